@@ -57,6 +57,10 @@ const char* b200_last_variant(void);
  * (bench.py's gpu_launches counter). */
 int64_t b200_launch_count(void);
 
+/* Waits inside kernels of the current device that ran out (each after about two seconds) since the library was
+ * loaded: a kernel whose wait runs out ends by itself and its output is not to be used.  Synchronises. */
+int b200_wait_timeouts(int64_t* total);
+
 /* Programmatic dependent launch (default on; env B200_PDL=0 turns it off): every kernel of the
  * library is launched with cudaLaunchAttributeProgrammaticStreamSerialization and orders its own
  * dependent accesses with griddepcontrol.wait, so consecutive kernels of a decode step overlap

@@ -22,6 +22,7 @@ _SIGNATURES = {
     "b200_last_error": (c_char_p, []),
     "b200_last_variant": (c_char_p, []),
     "b200_launch_count": (c_int64, []),
+    "b200_wait_timeouts": (c_int, [ctypes.POINTER(c_int64)]),
     "b200_set_pdl": (c_int, [c_int]),
     "b200_timing_enable": (c_int, [c_int]),
     "b200_timing_read": (c_int, [c_char_p, ctypes.POINTER(c_int64), ctypes.POINTER(ctypes.c_double)]),

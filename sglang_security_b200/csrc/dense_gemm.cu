@@ -2,26 +2,13 @@
 // (UnquantizedLinearMethod.apply = F.linear, python/sglang/srt/layers/linear.py:170-176; the
 // lm_head of the decode step, vocab_parallel_embedding.py / logits_processor.py:_get_logits):
 //   out[M, N] = x[M, K] . w[N, K]^T (+ bias[N]),  bf16 / f16 operands, fp32 accumulation in TMEM.
-// Same persistent TMA + tcgen05 kernel as the FP8 path (gemm_tc.cuh) with kind::f16; K-major
+// Same CTA-pair TMA + tcgen05 kernel as the FP8 path (gemm_pair.cuh) with kind::f16; K-major
 // operands, so the reference's [N, K] weight is used as stored.
-#include "gemm_tc.cuh"
+#include "gemm_pair.cuh"
 
 namespace b200 {
 
-template <int KIND, typename OutT, bool ACT = false>
-static int dense_gemm_launch(const void* x, int64_t ldx, const void* w, int64_t ldw,
-                             const GemmEpilogueParams& ep, cudaStream_t st) {
-  // 128 x 256 tiles once they fill the machine, else 128 x 128 (with cluster split-K when even
-  // those leave SMs idle) — the rule of the FP8 dispatch (fp8_gemm.cu)
-  const int64_t tiles256 = static_cast<int64_t>(ceil_div(ep.M, 128)) * ceil_div(ep.N, 256);
-  if (tiles256 >= device_sm_count())
-    return launch_gemm_tn<KIND, 256, 4, OutT, false, ACT>(x, ldx, w, ldw, ep, st, "dense_gemm");
-  return launch_gemm_tn<KIND, 128, 6, OutT, false, ACT>(x, ldx, w, ldw, ep, st, "dense_gemm", true);
-}
-
-}  // namespace b200
-
-namespace b200 {
+static WaitCounter wait_counter_registered(tc::wait_counter());
 
 static int gemm_16bit(const void* x, int64_t ldx, const void* w, int64_t ldw, const void* bias, void* out,
                       int64_t ldc, int M, int N, int K, bool act, float act_pos, float act_neg, int dtype,
@@ -48,10 +35,10 @@ static int gemm_16bit(const void* x, int64_t ldx, const void* w, int64_t ldw, co
   ep.act_neg = act_neg;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (act)
-    return dtype == B200_BF16 ? dense_gemm_launch<kKindBf16, __nv_bfloat16, true>(x, ldx, w, ldw, ep, st)
-                              : dense_gemm_launch<kKindF16, __half, true>(x, ldx, w, ldw, ep, st);
-  return dtype == B200_BF16 ? dense_gemm_launch<kKindBf16, __nv_bfloat16>(x, ldx, w, ldw, ep, st)
-                            : dense_gemm_launch<kKindF16, __half>(x, ldx, w, ldw, ep, st);
+    return dtype == B200_BF16 ? launch_gemm_pair<kKindBf16, __nv_bfloat16, true>(x, ldx, w, ldw, ep, st, "dense_gemm")
+                              : launch_gemm_pair<kKindF16, __half, true>(x, ldx, w, ldw, ep, st, "dense_gemm");
+  return dtype == B200_BF16 ? launch_gemm_pair<kKindBf16, __nv_bfloat16>(x, ldx, w, ldw, ep, st, "dense_gemm")
+                            : launch_gemm_pair<kKindF16, __half>(x, ldx, w, ldw, ep, st, "dense_gemm");
 }
 
 }  // namespace b200

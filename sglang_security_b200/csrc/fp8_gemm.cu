@@ -4,6 +4,7 @@
 //   out[M,N] = (A_e4m3[M,K] . B_e4m3[N,K]^T) * sa[m] * sb[n] (+ bias[n])  -> bf16 / f16
 // plus the TMA-descriptor helper shared by every tcgen05 kernel of the library.
 #include "fp8_gemm_smallm.cuh"
+#include "gemm_pair.cuh"
 
 #include <cstdlib>
 #include <mutex>
@@ -15,6 +16,8 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                                   const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+static WaitCounter wait_counter_registered(tc::wait_counter());
 
 static EncodeTiledFn get_encode_tiled() {
   static EncodeTiledFn fn = nullptr;
@@ -135,21 +138,6 @@ int smallm_pick_splits(int n_tiles, int num_kb) {
   return s;
 }
 
-// Mid-M regime (one or two 128-row token blocks): the output has far fewer 128x128 tiles than the
-// chip has SMs and a single CTA ingests only ~55 GB/s (measured: 48 CTAs -> 16 us for a 25 MB
-// weight, whatever M), so K is split until roughly every SM streams (B200_GEMM_SPLITK=0 disables,
-// =n forces n).  At least 4 K blocks per slice, at most 8 slices.
-int splitk_pick(int tiles, int num_kb, int sms) {
-  static int forced = env_int("B200_GEMM_SPLITK", -1);
-  if (forced == 0) return 1;
-  int s = forced > 0 ? forced : sms / (tiles > 0 ? tiles : 1);
-  if (s > 8) s = 8;
-  if (s > num_kb / 4) s = num_kb / 4;
-  if (s < 1) s = 1;
-  while (s > 1 && (s - 1) * ceil_div(num_kb, s) >= num_kb) --s;  // no empty slice
-  return s;
-}
-
 // Row-parallel fusion: the small-M kernel can reduce across the TP group in its epilogue when the
 // dense [M, N] partial fits one receive slot and the grid fits the flag table.
 // Policy measured on B200: at TP = 2 (profiles/r01_bench_allreduce_tp2.json) fusing wins while the
@@ -260,31 +248,9 @@ static int fp8_gemm_rowcol_impl(const void* a, int64_t lda, const void* b, int64
     if (rc || !comm || fuse_ar) return rc;
     return comm_all_reduce_rows(comm, out, ldc, M, N, out_dtype, stream);
   }
-  // Tile choice: 128x256 when there is enough work to fill the SMs with it, else 128x128.
-  const int sms = device_sm_count();
-  const int64_t tiles256 = static_cast<int64_t>(ceil_div(M, 128)) * ceil_div(N, 256);
-  bool big = tiles256 >= sms;
-  // Measured (profiles/r01_bench_gemm_tilewidth.json): in the weight-streaming regime below that
-  // the 256-wide tile does not pay even when it saves a wave (28672x4096, M <= 128: 34 vs 31.6 us;
-  // M = 192-256: 44-46 vs 46-47 us), so the rule stays.  B200_GEMM_BN = 128 / 256 forces the choice.
-  static const int force_bn = env_int("B200_GEMM_BN", 0);
-  if (force_bn == 128) big = false;
-  if (force_bn == 256) big = true;
-  int rc;
-  // pairs of M blocks share the weight tile by TMA multicast (B200_GEMM_MCAST=0 turns it off)
-  static const int mcast_on = env_int("B200_GEMM_MCAST", 1);
-  if (big && mcast_on && ceil_div(M, 128) % 2 == 0) {
-    rc = out_dtype == B200_BF16
-             ? launch_gemm_tn<kKindFp8, 256, 4, __nv_bfloat16, true>(a, lda, b, ldb, ep, st, "fp8_gemm")
-             : launch_gemm_tn<kKindFp8, 256, 4, __half, true>(a, lda, b, ldb, ep, st, "fp8_gemm");
-  } else
-  if (out_dtype == B200_BF16) {
-    rc = big ? launch_gemm_tn<kKindFp8, 256, 4, __nv_bfloat16>(a, lda, b, ldb, ep, st, "fp8_gemm")
-             : launch_gemm_tn<kKindFp8, 128, 6, __nv_bfloat16>(a, lda, b, ldb, ep, st, "fp8_gemm", true);
-  } else {
-    rc = big ? launch_gemm_tn<kKindFp8, 256, 4, __half>(a, lda, b, ldb, ep, st, "fp8_gemm")
-             : launch_gemm_tn<kKindFp8, 128, 6, __half>(a, lda, b, ldb, ep, st, "fp8_gemm", true);
-  }
+  const int rc = out_dtype == B200_BF16
+                     ? launch_gemm_pair<kKindFp8, __nv_bfloat16>(a, lda, b, ldb, ep, st, "fp8_gemm")
+                     : launch_gemm_pair<kKindFp8, __half>(a, lda, b, ldb, ep, st, "fp8_gemm");
   if (rc || !comm) return rc;
   return comm_all_reduce_rows(comm, out, ldc, M, N, out_dtype, stream);
 }

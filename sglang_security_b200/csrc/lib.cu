@@ -1,5 +1,5 @@
 // Library-level C-ABI entry points: version, error text, launch counter.
-#include "common.cuh"
+#include "tc_common.cuh"
 
 #include <cstdlib>
 #include <cstring>
@@ -36,6 +36,21 @@ void set_error(const char* fmt, ...) {
   va_start(ap, fmt);
   vsnprintf(g_error, sizeof(g_error), fmt, ap);
   va_end(ap);
+}
+
+static std::vector<const void*>& wait_counters() {
+  static std::vector<const void*> v;
+  return v;
+}
+WaitCounter::WaitCounter(const void* symbol) { wait_counters().push_back(symbol); }
+int wait_timeouts(int64_t* total) {
+  *total = 0;
+  for (const void* sym : wait_counters()) {
+    unsigned n = 0;
+    B200_CUDA_OK(cudaMemcpyFromSymbol(&n, sym, sizeof(n)));
+    *total += n;
+  }
+  return 0;
 }
 
 static thread_local char g_variant[256] = "";
@@ -140,5 +155,10 @@ const char* b200_last_error(void) { return b200::g_error; }
 const char* b200_last_variant(void) { return b200::last_variant(); }
 
 int64_t b200_launch_count(void) { return b200::g_launch_count.load(); }
+
+int b200_wait_timeouts(int64_t* total) {
+  B200_REQUIRE(total, "b200_wait_timeouts: null pointer");
+  return b200::wait_timeouts(total);
+}
 
 }  // extern "C"

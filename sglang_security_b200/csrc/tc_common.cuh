@@ -44,6 +44,21 @@ __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity) {
   while (!mbar_try_wait(bar, parity)) {
   }
 }
+// Bounded form: gives up after about two seconds, counts that in this translation unit's g_wait_timeouts
+// (b200_wait_timeouts() reads it) and lets the caller run to its end; once `dead`, a thread's later waits only
+// poll, so a lost signal costs one limit and not one per wait.
+static __device__ unsigned g_wait_timeouts;
+__device__ __forceinline__ void mbar_wait_bounded(uint32_t bar, uint32_t parity, bool& dead) {
+  if (mbar_try_wait(bar, parity)) return;
+  const long long t0 = clock64();
+  while (!dead) {
+    if (mbar_try_wait(bar, parity)) return;
+    if (clock64() - t0 > (1ll << 32)) {
+      dead = true;
+      atomicAdd(&g_wait_timeouts, 1u);
+    }
+  }
+}
 
 // ---- TMA ------------------------------------------------------------------------------------
 __device__ __forceinline__ void prefetch_tmap(const CUtensorMap* m) {
@@ -65,16 +80,6 @@ __device__ __forceinline__ void tma_load_2d_hint(uint32_t dst, const CUtensorMap
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint"
       " [%0], [%1, {%3, %4}], [%2], %5;\n" ::"r"(dst),
       "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(c0), "r"(c1), "l"(policy)
-      : "memory");
-}
-// Multicast variant: the box lands at the SAME shared offset in every CTA of `cta_mask` and credits
-// the mbarrier at the same offset in each of them.
-__device__ __forceinline__ void tma_load_2d_mcast(uint32_t dst, const CUtensorMap* m, uint32_t bar,
-                                                  int c0, int c1, uint16_t cta_mask) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes"
-      ".multicast::cluster [%0], [%1, {%3, %4}], [%2], %5;\n" ::"r"(dst),
-      "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(c0), "r"(c1), "h"(cta_mask)
       : "memory");
 }
 constexpr uint64_t kEvictFirst = 0x12F0000000000000ull;  // CacheHintSm90::EVICT_FIRST
@@ -123,14 +128,6 @@ __device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint64_t adesc, uint64_
 }
 // Arrive on `bar` once every tcgen05.mma issued so far by this thread has completed
 // (implies tcgen05.fence::before_thread_sync).
-// Same, arriving on the barrier at this offset in every CTA of `cta_mask`.
-__device__ __forceinline__ void mma_commit_mcast(uint32_t bar, uint16_t cta_mask) {
-  asm volatile(
-      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 "
-      "[%0], %1;\n" ::"r"(bar),
-      "h"(cta_mask)
-      : "memory");
-}
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
                    bar)
@@ -226,6 +223,14 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
+}  // namespace tc
+
+// Every translation unit with bounded waits registers its counter once: static WaitCounter name(tc::wait_counter()).
+struct WaitCounter {
+  explicit WaitCounter(const void* symbol);
+};
+namespace tc {
+static inline const void* wait_counter() { return static_cast<const void*>(&g_wait_timeouts); }
 }  // namespace tc
 
 // ---- host side: TMA descriptor creation without linking libcuda ----------------------------------
