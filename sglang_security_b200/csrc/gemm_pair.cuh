@@ -382,15 +382,17 @@ inline int pair_stages(int bn, int* smem) {
 // Tile width and K split for M tokens; clusters_of[s]: clusters of s pairs that are resident at once.
 // Estimated microseconds, from B200 measurements (e4m3, N 4096, K 4096 and 20480, 64 pairs): a 128-byte K block
 // takes 0.131 / 0.147 / 0.203 / 0.245 / 0.287 / 0.373 at 32 / 64 / 128 / 160 / 192 / 256 tokens (narrow tiles wait
-// for the ring, wide ones for the tensor cores), a launch 4 + bn / 250, a split 2.5 for the exchange of the
-// partials.  So one wave of narrow tiles beats two of wide ones, and a split pays where most pairs would idle; a
-// narrower tile or a split has to promise 5 %, since it reads more and the estimate is not better than that
-// (4096 x 4096, bf16, M 4096: 256 tokens 340 us at K 14336 where 192 "save" 3 % and took 355).
+// for the ring, wide ones for the tensor cores), a launch 4 + bn / 250, a split 2 + bn / 125 for the exchange of
+// the partials (e4m3, 512 x 4096 x 14336: 27.9 in two slices of 256 tokens, 26.3 in unsplit tiles of 128).  So one
+// wave of narrow tiles beats two of wide ones, and a split pays where most pairs would idle; a narrower tile or a
+// split has to promise 5 %, since it reads more and the estimate is not better than that.  From 2048 tokens on
+// the tile stays wide (bf16, 4096 x 4096 x 14336: 340 at 256 tokens, 355 at 192 although that saves part of a wave;
+// 2048 x 4096 x 4096 e4m3, the other way: 28.4 at 256, 27.4 at 160).
 inline PairPlan pair_pick(int M, int N, int num_kb, const int* clusters_of) {
   const int n_blocks = ceil_div(N, 256);
   PairPlan best;
   double best_us = 0;
-  for (int nb = ceil_div(M, 256); nb <= ceil_div(M, 32) && nb <= ceil_div(M, 256) + 12; ++nb) {
+  for (int nb = ceil_div(M, 256); nb <= ceil_div(M, 32) && nb <= ceil_div(M, 256) + (M < 2048 ? 12 : 0); ++nb) {
     const int bn = (ceil_div(M, nb) + 31) / 32 * 32;
     const int64_t tiles = static_cast<int64_t>(ceil_div(M, bn)) * n_blocks;
     const double wide = 0.040 + 0.0013 * bn, narrow = 0.115 + 0.0005 * bn;
@@ -400,7 +402,7 @@ inline PairPlan pair_pick(int M, int N, int num_kb, const int* clusters_of) {
       const int per = ceil_div(num_kb, S);
       if (S > 1 && (tiles > clusters_of[S] || per < 4 || (S - 1) * per >= num_kb)) continue;
       const int64_t waves = S > 1 ? 1 : (tiles + clusters_of[1] - 1) / clusters_of[1];
-      const double us = waves * (per * per_kb + 0.3) + 4.0 + bn / 250.0 + (S > 1 ? 2.5 : 0.0);
+      const double us = waves * (per * per_kb + 0.3) + 4.0 + bn / 250.0 + (S > 1 ? 2.0 + 0.008 * bn : 0.0);
       if (best.bn == 0 || us < 0.95 * best_us) {
         best.bn = bn;
         best.splits = S;
