@@ -250,50 +250,52 @@ attn_extend_kernel(const ExtendParams p) {
     tc::fence_proxy_async_smem();
     tc::mbar_arrive(bar_kv_full((n_kv - 1) & 1));
   } else if (warp == 4) {
-    // ===================== MMA issuer =====================
-    if (lane == 0) {
-      constexpr uint32_t fmt = sizeof(T) == 2 && std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
-      constexpr uint32_t idesc_qk = tc::make_idesc(fmt, fmt, 128, kKvTile, 0, 0);
-      constexpr uint32_t idesc_pv = tc::make_idesc(fmt, fmt, 128, D, 0, 1);  // V: MN-major B
-      const uint32_t tmem_s = tmem_base, tmem_o = tmem_base + C::O_COL;
-      auto issue_qk = [&](int j) {
-        const uint32_t sk = sbase + C::OFF_K + (j & 1) * C::KV_TILE_BYTES;
+    // ===================== MMA issuer (whole warp, one elected thread per batch of instructions) ==========
+    constexpr uint32_t fmt = sizeof(T) == 2 && std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
+    constexpr uint32_t idesc_qk = tc::make_idesc(fmt, fmt, 128, kKvTile, 0, 0);
+    constexpr uint32_t idesc_pv = tc::make_idesc(fmt, fmt, 128, D, 0, 1);  // V: MN-major B
+    const uint32_t tmem_s = tmem_base, tmem_o = tmem_base + C::O_COL;
+    const uint64_t qdesc = tc::make_smem_desc_sw128(sbase + C::OFF_Q, 1024, 16);
+    const uint64_t pdesc = tc::make_smem_desc_sw128(sbase + C::OFF_P, 1024, 16);
+    auto issue_qk = [&](int j) {
+      const uint64_t kdesc = tc::make_smem_desc_sw128(sbase + C::OFF_K + (j & 1) * C::KV_TILE_BYTES, 1024, 16);
+      if (tc::elect_one()) {
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk) {
           const uint32_t koff = (kk >> 2) * (128 * 128) + (kk & 3) * 32;   // Q panel / k-step
           const uint32_t boff = (kk >> 2) * (kKvTile * 128) + (kk & 3) * 32;
-          tc::mma_f16(tmem_s, tc::make_smem_desc_sw128(sbase + C::OFF_Q + koff, 1024, 16),
-                      tc::make_smem_desc_sw128(sk + boff, 1024, 16), idesc_qk, kk != 0 ? 1u : 0u);
+          tc::mma_f16(tmem_s, qdesc + (koff >> 4), kdesc + (boff >> 4), idesc_qk, kk != 0 ? 1u : 0u);
         }
         tc::mma_commit(bar_s_full);
-      };
-      tc::mbar_wait(bar_q, 0);
-      tc::mbar_wait(bar_kv_full(0), 0);
-      tc::tc_fence_after();
-      issue_qk(0);
-      for (int j = 0; j < n_kv; ++j) {
-        if (j + 1 < n_kv) {
-          tc::mbar_wait(bar_kv_full((j + 1) & 1), ((j + 1) >> 1) & 1u);
-          tc::mbar_wait(bar_s_free, j & 1u);  // softmax has pulled S(j) out of TMEM
-          tc::tc_fence_after();
-          issue_qk(j + 1);
-        }
-        tc::mbar_wait(bar_p_full, j & 1u);
+      }
+      __syncwarp();
+    };
+    tc::mbar_wait(bar_q, 0);
+    tc::mbar_wait(bar_kv_full(0), 0);
+    tc::tc_fence_after();
+    issue_qk(0);
+    for (int j = 0; j < n_kv; ++j) {
+      if (j + 1 < n_kv) {
+        tc::mbar_wait(bar_kv_full((j + 1) & 1), ((j + 1) >> 1) & 1u);
+        tc::mbar_wait(bar_s_free, j & 1u);  // softmax has pulled S(j) out of TMEM
         tc::tc_fence_after();
-        const uint32_t sv = sbase + C::OFF_V + (j & 1) * C::V_STAGE_BYTES;
+        issue_qk(j + 1);
+      }
+      tc::mbar_wait(bar_p_full, j & 1u);
+      tc::tc_fence_after();
+      // A = P [128 x 64 tokens], K-major; B = V rows kk*16.., MN-major: LBO = panel stride
+      const uint64_t vdesc = tc::make_smem_desc_sw128(sbase + C::OFF_V + (j & 1) * C::V_STAGE_BYTES, 1024, kKvTile * 128);
+      if (tc::elect_one()) {
 #pragma unroll
         for (int vh = 0; vh < NV; ++vh)
 #pragma unroll
-          for (int kk = 0; kk < kKvTile / 16; ++kk) {
-            // A = P [128 x 64 tokens], K-major; B = V rows kk*16.., MN-major: LBO = panel stride
-            tc::mma_f16(tmem_o + vh * D, tc::make_smem_desc_sw128(sbase + C::OFF_P + kk * 32, 1024, 16),
-                        tc::make_smem_desc_sw128(sv + vh * C::KV_TILE_BYTES + kk * 16 * 128, 1024,
-                                                 kKvTile * 128),
+          for (int kk = 0; kk < kKvTile / 16; ++kk)
+            tc::mma_f16(tmem_o + vh * D, pdesc + 2 * kk, vdesc + ((vh * C::KV_TILE_BYTES + kk * 16 * 128) >> 4),
                         idesc_pv, (j | kk) != 0 ? 1u : 0u);
-          }
         tc::mma_commit(bar_pv_full);
         tc::mma_commit(bar_kv_empty(j & 1));
       }
+      __syncwarp();
     }
   } else {
     // ===================== softmax / epilogue (warps 0-3, thread = query row) =====================

@@ -227,50 +227,54 @@ diff_attn_extend_kernel(const DiffExtendParams p) {
     cp_async_wait<0>();
     for (int j = max(0, n_kv - LAG); j < n_kv; ++j) publish(j);
   } else if (warp == 8) {
-    // ===================== MMA issuer =====================
-    if (lane == 0) {
-      constexpr uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
-      constexpr uint32_t idesc_qk = tc::make_idesc(fmt, fmt, 128, kDxTile, 0, 0);
-      constexpr uint32_t idesc_pv = tc::make_idesc(fmt, fmt, 128, DV, 0, 1);   // V: MN-major B
-      auto issue_qk = [&](int j, int m) {
-        const uint32_t sk = sbase + C::OFF_K + (j % ST) * C::K_BYTES;
+    // ===================== MMA issuer (whole warp, one elected thread per batch of instructions) ==========
+    constexpr uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
+    constexpr uint32_t idesc_qk = tc::make_idesc(fmt, fmt, 128, kDxTile, 0, 0);
+    constexpr uint32_t idesc_pv = tc::make_idesc(fmt, fmt, 128, DV, 0, 1);   // V: MN-major B
+    const uint64_t qdesc = tc::make_smem_desc_sw128(sbase + C::OFF_Q, 1024, 16);
+    auto issue_qk = [&](int j, int m) {
+      const uint64_t kdesc = tc::make_smem_desc_sw128(sbase + C::OFF_K + (j % ST) * C::K_BYTES, 1024, 16);
+      if (tc::elect_one()) {
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk) {
           const int k = m * (D / 16) + kk;             // 16-coordinate step of the whole [map 1 | map 2] row
           const uint32_t qoff = (k >> 2) * (128 * 128) + (k & 3) * 32;
           const uint32_t koff = (k >> 2) * (kDxTile * 128) + (k & 3) * 32;
-          tc::mma_f16(tmem_base + C::S_COL + m * kDxTile, tc::make_smem_desc_sw128(sbase + C::OFF_Q + qoff, 1024, 16),
-                      tc::make_smem_desc_sw128(sk + koff, 1024, 16), idesc_qk, kk != 0 ? 1u : 0u);
+          tc::mma_f16(tmem_base + C::S_COL + m * kDxTile, qdesc + (qoff >> 4), kdesc + (koff >> 4), idesc_qk,
+                      kk != 0 ? 1u : 0u);
         }
         tc::mma_commit(bar_s_full(m));
-      };
-      wait(bar_q, 0);
-      wait(bar_kv_full(0), 0);
-      tc::tc_fence_after();
-      issue_qk(0, 0);
-      issue_qk(0, 1);
-      for (int j = 0; j < n_kv; ++j) {
-        if (j + 1 < n_kv) {
-          wait(bar_kv_full((j + 1) % ST), ((j + 1) / ST) & 1);
-          for (int m = 0; m < 2; ++m) {
-            wait(bar_s_free(m), j & 1u);               // the softmax has pulled S_m(j) out of TMEM
-            tc::tc_fence_after();
-            issue_qk(j + 1, m);
-          }
-        }
-        const uint32_t sv = sbase + C::OFF_V + (j % ST) * C::V_BYTES;
+      }
+      __syncwarp();
+    };
+    wait(bar_q, 0);
+    wait(bar_kv_full(0), 0);
+    tc::tc_fence_after();
+    issue_qk(0, 0);
+    issue_qk(0, 1);
+    for (int j = 0; j < n_kv; ++j) {
+      if (j + 1 < n_kv) {
+        wait(bar_kv_full((j + 1) % ST), ((j + 1) / ST) & 1);
         for (int m = 0; m < 2; ++m) {
-          wait(bar_p_full(m), j & 1u);
+          wait(bar_s_free(m), j & 1u);                 // the softmax has pulled S_m(j) out of TMEM
           tc::tc_fence_after();
+          issue_qk(j + 1, m);
+        }
+      }
+      const uint64_t vdesc = tc::make_smem_desc_sw128(sbase + C::OFF_V + (j % ST) * C::V_BYTES, 1024, kDxTile * 128);
+      for (int m = 0; m < 2; ++m) {
+        wait(bar_p_full(m), j & 1u);
+        tc::tc_fence_after();
+        const uint64_t pdesc = tc::make_smem_desc_sw128(sbase + C::OFF_P + m * C::P_BYTES, 1024, 16);
+        if (tc::elect_one()) {
 #pragma unroll
           for (int kk = 0; kk < kDxTile / 16; ++kk)
-            tc::mma_f16(tmem_base + C::O_COL + m * DV,
-                        tc::make_smem_desc_sw128(sbase + C::OFF_P + m * C::P_BYTES + kk * 32, 1024, 16),
-                        tc::make_smem_desc_sw128(sv + kk * 16 * 128, 1024, kDxTile * 128), idesc_pv,
+            tc::mma_f16(tmem_base + C::O_COL + m * DV, pdesc + 2 * kk, vdesc + ((kk * 16 * 128) >> 4), idesc_pv,
                         (j | kk) != 0 ? 1u : 0u);
           tc::mma_commit(bar_pv_full(m));
+          if (m == 1) tc::mma_commit(bar_kv_empty(j % ST));
         }
-        tc::mma_commit(bar_kv_empty(j % ST));
+        __syncwarp();
       }
     }
   } else {

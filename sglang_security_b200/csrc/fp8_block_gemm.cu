@@ -89,53 +89,52 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
   griddep_wait();  // activations / scales come from the previous kernel
   griddep_launch_dependents();
 
+  // whole-warp loops, one elected thread per instruction (see gemm_pair.cuh)
   if (warp == 0) {
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
-        const int m_blk = tile % m_blocks, n_blk = tile / m_blocks;
-        for (int kb = 0; kb < num_kb; ++kb) {
-          tc::mbar_wait(empty_bar(stage), phase ^ 1u);
+    int stage = 0;
+    uint32_t phase = 0;
+    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
+      const int m_blk = tile % m_blocks, n_blk = tile / m_blocks;
+      for (int kb = 0; kb < num_kb; ++kb) {
+        tc::mbar_wait(empty_bar(stage), phase ^ 1u);
+        const uint32_t sa = smem_base + stage * STAGE_BYTES;
+        if (tc::elect_one()) {
           tc::mbar_arrive_expect_tx(full_bar(stage), STAGE_BYTES);
-          const uint32_t sa = smem_base + stage * STAGE_BYTES;
           tc::tma_load_2d(sa, &tmap_a, full_bar(stage), kb * BLOCK, m_blk * BLOCK);
           tc::tma_load_2d(sa + A_BYTES, &tmap_b, full_bar(stage), kb * BLOCK, n_blk * BN);
-          if (++stage == STAGES) {
-            stage = 0;
-            phase ^= 1u;
-          }
+        }
+        __syncwarp();
+        if (++stage == STAGES) {
+          stage = 0;
+          phase ^= 1u;
         }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = tc::make_idesc(0, 0, BLOCK, BN, 0, 0);
-      int stage = 0;
-      uint32_t phase = 0;
-      uint32_t it = 0;  // running K-block counter across tiles -> TMEM buffer ring
-      for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
-        for (int kb = 0; kb < num_kb; ++kb, ++it) {
-          const int buf = it % NBUF;
-          const uint32_t buf_phase = (it / NBUF) & 1u;
-          tc::mbar_wait(tempty_bar(buf), buf_phase ^ 1u);
-          tc::mbar_wait(full_bar(stage), phase);
-          tc::tc_fence_after();
-          const uint32_t sa = smem_base + stage * STAGE_BYTES;
-          const uint32_t sb = sa + A_BYTES;
-          const uint32_t tmem_d = tmem_base + buf * BN;
+    constexpr uint32_t idesc = tc::make_idesc(0, 0, BLOCK, BN, 0, 0);
+    int stage = 0;
+    uint32_t phase = 0;
+    uint32_t it = 0;  // running K-block counter across tiles -> TMEM buffer ring
+    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
+      for (int kb = 0; kb < num_kb; ++kb, ++it) {
+        const int buf = it % NBUF;
+        const uint32_t buf_phase = (it / NBUF) & 1u;
+        tc::mbar_wait(tempty_bar(buf), buf_phase ^ 1u);
+        tc::mbar_wait(full_bar(stage), phase);
+        tc::tc_fence_after();
+        const uint64_t adesc = tc::make_smem_desc_sw128(smem_base + stage * STAGE_BYTES, 1024, 16);
+        const uint64_t bdesc = tc::make_smem_desc_sw128(smem_base + stage * STAGE_BYTES + A_BYTES, 1024, 16);
+        const uint32_t tmem_d = tmem_base + buf * BN;
+        if (tc::elect_one()) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const uint64_t adesc = tc::make_smem_desc_sw128(sa + k * 32, 1024, 16);
-            const uint64_t bdesc = tc::make_smem_desc_sw128(sb + k * 32, 1024, 16);
-            tc::mma_f8f6f4(tmem_d, adesc, bdesc, idesc, k != 0 ? 1u : 0u);
-          }
+          for (int k = 0; k < 4; ++k) tc::mma_f8f6f4(tmem_d, adesc + 2 * k, bdesc + 2 * k, idesc, k != 0 ? 1u : 0u);
           tc::mma_commit(empty_bar(stage));
           tc::mma_commit(tfull_bar(buf));
-          if (++stage == STAGES) {
-            stage = 0;
-            phase ^= 1u;
-          }
+        }
+        __syncwarp();
+        if (++stage == STAGES) {
+          stage = 0;
+          phase ^= 1u;
         }
       }
     }

@@ -146,7 +146,7 @@ fp8_gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w,
   };
   auto wait_mma_done = [&](int i) { tc::mbar_wait(empty_bar(i % NW), (i / NW) & 1u); };
 
-  if (warp == 0 && lane == 0) {
+  if (warp == 0 && tc::elect_one()) {
     if ((smem_base & 1023u) != 0) __trap();
     tc::prefetch_tmap(&tmap_w);
     tc::prefetch_tmap(&tmap_x);
@@ -177,47 +177,51 @@ fp8_gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w,
   tc::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
 
+  // whole-warp loops, one elected thread per instruction (see gemm_pair.cuh)
   if (warp == 0) {
     // ===================== TMA producer: stream this rank's K slice of the weight tile ==========
-    if (lane == 0) {
-      for (int i = NW; i < nkb; ++i) {  // W runs NW blocks ahead of the MMA, X only NX blocks
-        wait_mma_done(i - NW);
+    for (int i = NW; i < nkb; ++i) {  // W runs NW blocks ahead of the MMA, X only NX blocks
+      wait_mma_done(i - NW);
+      if (tc::elect_one()) {
         issue_w(i);
         issue_x(i - NW + NX);
       }
-      for (int j = NX + (nkb > NW ? nkb - NW : 0); j < nkb; ++j) {
-        wait_mma_done(j - NX);
-        issue_x(j);
-      }
-      if (p.pdl_late) griddep_launch_dependents();  // every load of this CTA has been issued
+      __syncwarp();
     }
+    for (int j = NX + (nkb > NW ? nkb - NW : 0); j < nkb; ++j) {
+      wait_mma_done(j - NX);
+      if (tc::elect_one()) issue_x(j);
+      __syncwarp();
+    }
+    if (p.pdl_late) griddep_launch_dependents();  // every load of this CTA has been issued
   } else if (warp == 1) {
     // ===================== MMA issuer ==========================================================
-    if (lane == 0) {
-      constexpr uint32_t idesc = tc::make_idesc(0, 0, 128, MT, 0, 0);
-      for (int i = 0; i < nkb; ++i) {
-        const int buf = BLK ? i % NBUF : 0;
-        if (BLK) tc::mbar_wait(tempty_bar(buf), ((i / NBUF) & 1u) ^ 1u);
-        tc::mbar_wait(full_bar(i % NW), (i / NW) & 1u);
-        tc::tc_fence_after();
-        const uint32_t sw = smem_base + (i % NW) * C::W_BYTES;
-        const uint32_t sx = ring_x + (i % NX) * C::X_BYTES;
-        const uint32_t tmem_d = tmem_base + buf * MT;
+    constexpr uint32_t idesc = tc::make_idesc(0, 0, 128, MT, 0, 0);
+    for (int i = 0; i < nkb; ++i) {
+      const int buf = BLK ? i % NBUF : 0;
+      if (BLK) tc::mbar_wait(tempty_bar(buf), ((i / NBUF) & 1u) ^ 1u);
+      tc::mbar_wait(full_bar(i % NW), (i / NW) & 1u);
+      tc::tc_fence_after();
+      const uint64_t adesc = tc::make_smem_desc_sw128(smem_base + (i % NW) * C::W_BYTES, 1024, 16);
+      const uint64_t bdesc = tc::make_smem_desc_sw128(ring_x + (i % NX) * C::X_BYTES, 1024, 16);
+      const uint32_t tmem_d = tmem_base + buf * MT;
+      if (tc::elect_one()) {
 #pragma unroll
         for (int u = 0; u < C::KS; ++u) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const uint64_t adesc = tc::make_smem_desc_sw128(sw + u * C::W_SUB + k * 32, 1024, 16);
-            const uint64_t bdesc = tc::make_smem_desc_sw128(sx + u * C::X_SUB + k * 32, 1024, 16);
+          for (int k = 0; k < 4; ++k) {   // 32 bytes of K further on: 2 in the address field
             const uint32_t accum = BLK ? (k != 0) : ((i != 0) | (u != 0) | (k != 0));
-            tc::mma_f8f6f4(tmem_d, adesc, bdesc, idesc, accum ? 1u : 0u);
+            tc::mma_f8f6f4(tmem_d, adesc + (u * C::W_SUB >> 4) + 2 * k, bdesc + (u * C::X_SUB >> 4) + 2 * k, idesc,
+                           accum ? 1u : 0u);
           }
         }
         tc::mma_commit(empty_bar(i % NW));
         if (BLK) tc::mma_commit(tfull_bar(buf));
       }
-      if (!BLK && has_work) tc::mma_commit(tfull_bar(0));
+      __syncwarp();
     }
+    if (!BLK && has_work && tc::elect_one()) tc::mma_commit(tfull_bar(0));
+    __syncwarp();
   } else {
     // ===================== epilogue ===========================================================
     // S == 1: TMEM -> registers -> scales/bias -> global (a warp writes 32 consecutive channels).

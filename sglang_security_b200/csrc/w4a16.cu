@@ -272,13 +272,14 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
 
   if (warp == 0) {
     // ===================== TMA producer: activation tiles =====================
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      for (int tile = tile0; tile < num_tiles; tile += tile_step) {
-        const int m_blk = tile % m_blocks;
-        for (int kb = kb_begin; kb < kb_end; ++kb) {
-          tc::mbar_wait(empty_bar(stage), phase ^ 1u);
+    // (this and the two other issuing loops: whole warps, one elected thread per instruction; see gemm_pair.cuh)
+    int stage = 0;
+    uint32_t phase = 0;
+    for (int tile = tile0; tile < num_tiles; tile += tile_step) {
+      const int m_blk = tile % m_blocks;
+      for (int kb = kb_begin; kb < kb_end; ++kb) {
+        tc::mbar_wait(empty_bar(stage), phase ^ 1u);
+        if (tc::elect_one()) {
           tc::mbar_arrive_expect_tx(full_bar(stage), C::X_BYTES);
 #pragma unroll
           for (int j = 0; j < KS; ++j)
@@ -286,10 +287,11 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
             for (int h = 0; h < MH; ++h)
               tc::tma_load_2d(smem_base + stage * C::STAGE_BYTES + (j * MH + h) * (XBOX * 128),
                               &tmap_x, full_bar(stage), (kb * KS + j) * BK, m_blk * BM + h * XBOX);
-          if (++stage == ST) {
-            stage = 0;
-            phase ^= 1u;
-          }
+        }
+        __syncwarp();
+        if (++stage == ST) {
+          stage = 0;
+          phase ^= 1u;
         }
       }
     }
@@ -303,8 +305,8 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         const uint32_t dst = raw_base + rs * C::RAW_BYTES;
         const uint32_t zdst = dst + KS * kW4PackedBytes;
         if (p.raw_tma) {
-          if (lane == 0) {
-            tc::mbar_wait(rempty_bar(rs), rphase ^ 1u);
+          tc::mbar_wait(rempty_bar(rs), rphase ^ 1u);
+          if (tc::elect_one()) {
             tc::mbar_arrive_expect_tx(rfull_bar(rs),
                                       KS * (kW4PackedBytes + (zs_rows ? kW4ZsBytes : 0)));
             tc::tma_load_2d_hint(dst, &tmap_q, rfull_bar(rs), n_blk * (BN / 8), kb * KS * BK,
@@ -318,6 +320,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
               }
             }
           }
+          __syncwarp();
         } else {
           // rows whose pitch is not a multiple of 16 bytes: the 32 lanes copy the tile word by word
           tc::mbar_wait(rempty_bar(rs), rphase ^ 1u);
@@ -358,36 +361,35 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     }
   } else if (warp == 1) {
     // ===================== MMA issuer =====================
-    if (lane == 0) {
-      constexpr uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
-      // normal: A = x (K-major, 128 rows), B = weights (MN-major, N = 128)
-      // swap  : A = weights (MN-major, M = 128 output columns), B = x (K-major, N = MT tokens)
-      constexpr uint32_t idesc = SWAP ? tc::make_idesc(fmt, fmt, 128, BM, 1, 0)
-                                      : tc::make_idesc(fmt, fmt, 128, BN, 0, 1);
-      int stage = 0;
-      uint32_t phase = 0;
-      int local = 0;
-      for (int tile = tile0; tile < num_tiles; tile += tile_step, ++local) {
-        const int acc = local & 1;
-        tc::mbar_wait(tempty_bar(acc), ((local >> 1) & 1u) ^ 1u);
+    constexpr uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
+    // normal: A = x (K-major, 128 rows), B = weights (MN-major, N = 128)
+    // swap  : A = weights (MN-major, M = 128 output columns), B = x (K-major, N = MT tokens)
+    constexpr uint32_t idesc = SWAP ? tc::make_idesc(fmt, fmt, 128, BM, 1, 0)
+                                    : tc::make_idesc(fmt, fmt, 128, BN, 0, 1);
+    int stage = 0;
+    uint32_t phase = 0;
+    int local = 0;
+    for (int tile = tile0; tile < num_tiles; tile += tile_step, ++local) {
+      const int acc = local & 1;
+      tc::mbar_wait(tempty_bar(acc), ((local >> 1) & 1u) ^ 1u);
+      tc::tc_fence_after();
+      const uint32_t tmem_d = tmem_base + acc * C::ACC_COLS;
+      for (int kb = kb_begin; kb < kb_end; ++kb) {
+        tc::mbar_wait(full_bar(stage), phase);
         tc::tc_fence_after();
-        const uint32_t tmem_d = tmem_base + acc * C::ACC_COLS;
-        for (int kb = kb_begin; kb < kb_end; ++kb) {
-          tc::mbar_wait(full_bar(stage), phase);
-          tc::tc_fence_after();
-          const uint32_t sx = smem_base + stage * C::STAGE_BYTES;
-          const uint32_t sw = sx + C::X_BYTES;
+        const uint32_t sx = smem_base + stage * C::STAGE_BYTES;
+        // weight rows kk*16.. of a [64 k x 128 n] sub-tile; panels of 64 n are 64*128 B apart
+        const uint64_t wdesc0 = tc::make_smem_desc_sw128(sx + C::X_BYTES, 1024, BK * 128);
+        const uint64_t xdesc0 = tc::make_smem_desc_sw128(sx, 1024, 16);
+        if (tc::elect_one()) {
 #pragma unroll
           for (int j = 0; j < KS; ++j) {
 #pragma unroll
             for (int kk = 0; kk < BK / 16; ++kk) {
-              // weight rows kk*16.. of a [64 k x 128 n] sub-tile; panels of 64 n are 64*128 B apart
-              const uint64_t wdesc =
-                  tc::make_smem_desc_sw128(sw + j * C::BSUB + kk * 16 * 128, 1024, BK * 128);
+              const uint64_t wdesc = wdesc0 + ((j * C::BSUB + kk * 16 * 128) >> 4);
 #pragma unroll
               for (int h = 0; h < MH; ++h) {
-                const uint64_t xdesc = tc::make_smem_desc_sw128(
-                    sx + (j * MH + h) * (XBOX * 128) + kk * 32, 1024, 16);
+                const uint64_t xdesc = xdesc0 + (((j * MH + h) * (XBOX * 128) + kk * 32) >> 4);
                 const uint32_t accum = ((kb - kb_begin) | j | kk) != 0 ? 1u : 0u;
                 if (SWAP)
                   tc::mma_f16(tmem_d, wdesc, xdesc, idesc, accum);
@@ -397,13 +399,15 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
             }
           }
           tc::mma_commit(empty_bar(stage));
-          if (++stage == ST) {
-            stage = 0;
-            phase ^= 1u;
-          }
         }
-        tc::mma_commit(tfull_bar(acc));
+        __syncwarp();
+        if (++stage == ST) {
+          stage = 0;
+          phase ^= 1u;
+        }
       }
+      if (tc::elect_one()) tc::mma_commit(tfull_bar(acc));
+      __syncwarp();
     }
   } else if (warp < 6) {
     // ===================== epilogue (warps 2..5) =====================
