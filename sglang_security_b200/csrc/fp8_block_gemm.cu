@@ -24,7 +24,11 @@ struct BlockGemmParams {
   int64_t bs_row;
   const void* bias;
   int M, N, K;
+  // few tiles: a cluster of `splits` CTAs takes one tile, each a slice of K; see the epilogue
+  int splits, kb_per_split;
 };
+
+static WaitCounter wait_counter_registered(tc::wait_counter());
 
 // Tile 128 x 256: a 128 x 128 tile moves 64 KiB through shared memory (TMA in + UMMA out) per 256
 // tensor-core clocks, twice what an SM's shared memory delivers, and plateaued at 1.59 PFLOP/s
@@ -64,6 +68,12 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
   const int m_blocks = ceil_div(p.M, BLOCK), n_blocks = ceil_div(p.N, BN);
   const int num_tiles = m_blocks * n_blocks;
   const int num_kb = ceil_div(p.K, BLOCK);
+  const int S = p.splits;
+  const int rank = S > 1 ? static_cast<int>(cluster_ctarank()) : 0;
+  const int kb0 = S > 1 ? rank * p.kb_per_split : 0;
+  const int kb1 = S > 1 ? min(num_kb, kb0 + p.kb_per_split) : num_kb;
+  const int tile0 = static_cast<int>(blockIdx.x) / S, tile_step = static_cast<int>(gridDim.x) / S;
+  bool dead = false;                     // a wait of this thread ran out: the rest only poll
 
   if (warp == 0 && lane == 0) {
     tc::prefetch_tmap(&tmap_a);
@@ -93,10 +103,10 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
   if (warp == 0) {
     int stage = 0;
     uint32_t phase = 0;
-    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
+    for (int tile = tile0; tile < num_tiles; tile += tile_step) {
       const int m_blk = tile % m_blocks, n_blk = tile / m_blocks;
-      for (int kb = 0; kb < num_kb; ++kb) {
-        tc::mbar_wait(empty_bar(stage), phase ^ 1u);
+      for (int kb = kb0; kb < kb1; ++kb) {
+        tc::mbar_wait_bounded(empty_bar(stage), phase ^ 1u, dead);
         const uint32_t sa = smem_base + stage * STAGE_BYTES;
         if (tc::elect_one()) {
           tc::mbar_arrive_expect_tx(full_bar(stage), STAGE_BYTES);
@@ -115,12 +125,12 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
     int stage = 0;
     uint32_t phase = 0;
     uint32_t it = 0;  // running K-block counter across tiles -> TMEM buffer ring
-    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
-      for (int kb = 0; kb < num_kb; ++kb, ++it) {
+    for (int tile = tile0; tile < num_tiles; tile += tile_step) {
+      for (int kb = kb0; kb < kb1; ++kb, ++it) {
         const int buf = it % NBUF;
         const uint32_t buf_phase = (it / NBUF) & 1u;
-        tc::mbar_wait(tempty_bar(buf), buf_phase ^ 1u);
-        tc::mbar_wait(full_bar(stage), phase);
+        tc::mbar_wait_bounded(tempty_bar(buf), buf_phase ^ 1u, dead);
+        tc::mbar_wait_bounded(full_bar(stage), phase, dead);
         tc::tc_fence_after();
         const uint64_t adesc = tc::make_smem_desc_sw128(smem_base + stage * STAGE_BYTES, 1024, 16);
         const uint64_t bdesc = tc::make_smem_desc_sw128(smem_base + stage * STAGE_BYTES + A_BYTES, 1024, 16);
@@ -145,7 +155,7 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
     const OutT* bias = static_cast<const OutT*>(p.bias);
     const int nsb = ceil_div(p.N, BLOCK);  // weight scale blocks along N
     uint32_t it = 0;
-    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
+    for (int tile = tile0; tile < num_tiles; tile += tile_step) {
       const int m_blk = tile % m_blocks, n_blk = tile / m_blocks;
       const int row = m_blk * BLOCK + quarter * 32 + lane;
       const bool row_ok = row < p.M;
@@ -157,12 +167,12 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
       float2 acc[COLS / 2];
 #pragma unroll
       for (int j = 0; j < COLS / 2; ++j) acc[j] = make_float2(0.f, 0.f);
-      for (int kb = 0; kb < num_kb; ++kb, ++it) {
+      for (int kb = kb0; kb < kb1; ++kb, ++it) {
         const int buf = it % NBUF;
         const uint32_t buf_phase = (it / NBUF) & 1u;
         const float s = __ldg(as_row + kb * p.as_col) * __ldg(bs_row + kb);
         const float2 s2 = make_float2(s, s);
-        tc::mbar_wait(tfull_bar(buf), buf_phase);
+        tc::mbar_wait_bounded(tfull_bar(buf), buf_phase, dead);
         tc::tc_fence_after();
         const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * BN +
                                half * COLS;
@@ -183,7 +193,47 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
                 acc[c * 16 + j]);
         }
       }
-      if (row_ok && blk_ok) {
+      if (S > 1) {
+        // the slices' promoted fp32 sums meet over distributed shared memory: parked in the idle operand ring as
+        // [column][row], then rank r adds its share of the column groups in rank order (deterministic)
+        const uint32_t part = smem_base + (quarter * 32 + lane) * 4;
+#pragma unroll
+        for (int j = 0; j < COLS / 2; ++j) {
+          asm volatile("st.shared.f32 [%0], %1;\n" ::"r"(part + (half * COLS + 2 * j) * 512), "f"(acc[j].x) : "memory");
+          asm volatile("st.shared.f32 [%0], %1;\n" ::"r"(part + (half * COLS + 2 * j + 1) * 512), "f"(acc[j].y) : "memory");
+        }
+        __syncwarp();
+        cluster_sync_all();
+        for (int g = rank * 2 + half; g < BN / 8; g += 2 * S) {
+          float sum[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) sum[j] = 0.f;
+          for (int q = 0; q < S; ++q) {
+            const uint32_t src = map_to_rank(part + g * 8 * 512, q);
+            float t[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) t[j] = ld_cluster_f32(src + j * 512);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) sum[j] += t[j];
+          }
+          const int col0 = n_blk * BN + g * 8;
+          if (!row_ok || col0 >= p.N) continue;
+          OutT* o8 = out + static_cast<int64_t>(row) * p.ldc + col0;
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            if (bias && col0 + j < p.N) sum[j] += to_float<OutT>(bias[col0 + j]);
+          if (col0 + 8 <= p.N && (p.ldc & 7) == 0) {
+            *reinterpret_cast<uint4*>(o8) = make_uint4(pack_out2<OutT>(sum[0], sum[1]), pack_out2<OutT>(sum[2], sum[3]),
+                                                       pack_out2<OutT>(sum[4], sum[5]), pack_out2<OutT>(sum[6], sum[7]));
+          } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              if (col0 + j < p.N) o8[j] = from_float<OutT>(sum[j]);
+          }
+        }
+        __syncwarp();
+        cluster_sync_all();                // the peers have read this slice
+      } else if (row_ok && blk_ok) {
         OutT* orow = out + static_cast<int64_t>(row) * p.ldc;
         const int col0 = col_base;
         if (col0 + COLS <= p.N && (p.ldc & 7) == 0) {
@@ -215,32 +265,81 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
     }
   }
 
+  if (S > 1 && warp < 2) {               // the reduction's two barriers (one tile per cluster)
+    __syncwarp();
+    cluster_sync_all();
+    cluster_sync_all();
+  }
   tc::tc_fence_before();
   __syncthreads();
   if (warp == 1) tc::tmem_dealloc(tmem_base, NBUF * BN);
 }
 
+// Clusters of S CTAs of the 128-wide instance that are resident at once on the current device (0: none).
+template <typename OutT, int BN>
+static int block_clusters(int S) {
+  static std::atomic<int> cached[64][9];
+  auto kern = fp8_block_gemm_kernel<OutT, BN>;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  int n = cached[dev][S].load(std::memory_order_relaxed);
+  if (n == 0) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(S * 8);
+    cfg.blockDim = dim3(kBlkThreads);
+    cfg.dynamicSmemBytes = BlkCfg<BN>::SMEM;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = S;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, BlkCfg<BN>::SMEM) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) {
+      (void)cudaGetLastError();
+      n = -1;
+    }
+    cached[dev][S].store(n, std::memory_order_relaxed);
+  }
+  return n > 0 ? n : 0;
+}
+
 template <typename OutT, int BN>
 static int launch_block_gemm_bn(const void* a, int64_t lda, const void* b, int64_t ldb,
-                                const BlockGemmParams& p, cudaStream_t st) {
+                                const BlockGemmParams& p_in, cudaStream_t st) {
   constexpr int SMEM = BlkCfg<BN>::SMEM;
+  BlockGemmParams p = p_in;
   CUtensorMap ta, tb;
   int rc = make_tmap_2d(&ta, a, p.M, p.K, lda, 128, 128, 1, false);
   if (rc) return rc;
   rc = make_tmap_2d(&tb, b, p.N, p.K, ldb, BN, 128, 1, true);
   if (rc) return rc;
   auto kern = fp8_block_gemm_kernel<OutT, BN>;
-  static bool attr_done = false;
-  if (!attr_done) {
-    B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
-    attr_done = true;
-  }
+  const int resident = block_clusters<OutT, BN>(1);   // also raises the shared memory limit
+  B200_REQUIRE(resident > 0, "fp8_block_gemm_kernel does not fit this device");
   const int tiles = ceil_div(p.M, 128) * ceil_div(p.N, BN);
   const int sms = device_sm_count();
-  note_variant("fp8_block_gemm bn=%d tiles=%d", BN, tiles);
+  const int num_kb = ceil_div(p.K, 128);
+  p.splits = 1;
+  p.kb_per_split = num_kb;
+  if (BN == 128) {
+    // Largest split whose clusters are all resident, with 4 K blocks or more per slice.  Both sides on B200 (us,
+    // unsplit -> split, 128 tokens): 6144 x 4096 13.0 -> 12.3 in 2, 4096 x 14336 31.8 -> 16.3 in 4; with more
+    // tiles than half the SMs there is nothing to split for.
+    for (int S = sms / tiles < 8 ? sms / tiles : 8; S > 1; --S) {
+      const int per = ceil_div(num_kb, S);
+      if (per < 4 || (S - 1) * per >= num_kb || block_clusters<OutT, BN>(S) < tiles) continue;
+      p.splits = S;
+      p.kb_per_split = per;
+      break;
+    }
+  }
+  const int grid = p.splits > 1 ? tiles * p.splits : (tiles < sms ? tiles : sms);
+  note_variant("fp8_block_gemm bn=%d tiles=%d splits=%d", BN, tiles, p.splits);
   {
     ScopedKernelTimer timer("fp8_block_gemm", st);
-    B200_CUDA_OK(launch_kernel(kern, dim3(tiles < sms ? tiles : sms), dim3(kBlkThreads), SMEM, st, 1, pdl_family(p.M, kPdlGemmBig), ta, tb, p));
+    B200_CUDA_OK(launch_kernel(kern, dim3(grid), dim3(kBlkThreads), SMEM, st, p.splits, pdl_family(p.M, kPdlGemmBig), ta, tb, p));
   }
   B200_CHECK_LAUNCH("fp8_block_gemm_kernel");
   return 0;
@@ -273,9 +372,10 @@ static int fp8_gemm_block128_impl(const void* a, int64_t lda, const void* b, int
   B200_REQUIRE(out_dtype == B200_BF16 || out_dtype == B200_F16,
                "b200_fp8_gemm_block128: out dtype %d", out_dtype);
   cudaStream_t st0 = static_cast<cudaStream_t>(stream);
-  // (block-scaled: up to 64 tokens; the 128-token promotion loop is slower than the big tile)
+  // (block-scaled: up to 32 tokens; from there the promotion loops over 64 and 128 tokens per channel are slower
+  // than the big tile: 64 tokens, us, qkv / o / gate_up / down 21.2 / 15.1 / 54.4 / 32.7 against 11.8 / 9.5 / 26.5 / 15.9)
   const bool fuse_ar = M <= 64 && comm_can_fuse(comm, M, N);
-  if (fuse_ar || (M <= smallm_max_m() && (M <= 64 || smallm_forced()))) {  // decode regime: weight streaming, swap-AB + cluster split-K
+  if (fuse_ar || (M <= smallm_max_m() && (M <= 32 || smallm_forced()))) {  // decode regime: weight streaming, swap-AB + cluster split-K
     SmallMParams sp = {};
     if (fuse_ar) {
       sp.use_comm = 1;
