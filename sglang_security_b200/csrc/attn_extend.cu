@@ -104,6 +104,17 @@ __device__ __forceinline__ float fmax3(float a, float b, float c) {
   return d;
 }
 
+template <typename T>
+__device__ __forceinline__ uint32_t pack16(float a, float b) {
+  if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+    __nv_bfloat162 t = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<uint32_t*>(&t);
+  } else {
+    __half2 t = __floats2half2_rn(a, b);
+    return *reinterpret_cast<uint32_t*>(&t);
+  }
+}
+
 // FAST (round 2): the softmax warps are the limiter (ncu: issue 56 %, ALU 43 %, tensor 36 %), so the
 // per-element instruction count of the common tile is cut from ~7.5 to ~3: the causal / length mask
 // is applied only on tiles that cross the row's last visible key, the row max is taken on the RAW
@@ -542,6 +553,14 @@ attn_extend_kernel(const ExtendParams p) {
   if (warp == 4) tc::tmem_dealloc(tmem_base, C::TMEM_COLS);
 }
 
+}  // namespace b200
+
+#include "attn_extend_wide.cuh"
+
+namespace b200 {
+
+static WaitCounter wait_counter_registered(tc::wait_counter());
+
 // B200_EXTEND_FAST_SOFTMAX=0 selects the round-1 softmax for every call (read per launch: A/B tools flip it)
 static bool extend_fast_softmax_enabled() {
   const char* e = std::getenv("B200_EXTEND_FAST_SOFTMAX");
@@ -596,6 +615,9 @@ static int launch_extend(const ExtendParams& p, int n_values, int bs, int max_ex
   // a cap up to 40 keeps e^(-2 cap) a normal fp32 (and 16-bit) number: the one-pass capped form
   const float ref = p.score_bound > 0.f && p.score_bound < p.logit_cap ? p.score_bound : p.logit_cap;
   const bool fast = ref <= 40.f && p.qk_scale > 0.f && extend_fast_softmax_enabled();
+  // plain attention: two query tiles per CTA (all else, and every option, on the kernel above)
+  if (fast && p.logit_cap <= 0.f && p.window == 0 && !p.sink && !p.gate && !p.lse && n_values == 1 && p.v_head < 0)
+    return launch_extend_wide<T, D>(p, bs, max_extend_len, st);
   note_variant("attn_extend d=%d fast_softmax=%d values=%d", D, fast ? 1 : 0, n_values);
   if (n_values == 2)
     return fast ? launch_extend_inst<T, D, 1, 2>(p, bs, max_extend_len, st)

@@ -1,0 +1,353 @@
+// Extend attention without window, sink, gate or cap: two 128-row query tiles per CTA, P kept in tensor memory.
+//
+// attn_extend_kernel runs QK -> softmax -> PV as one serial chain per 64-key tile and CTA (1.3-1.6 us of latency
+// for 0.27 us of tensor work, two chains per SM).  Here one CTA per SM owns two query tiles that take turns: while
+// the softmax warps of one tile work, the tensor cores run PV and the next QK of the other.
+//
+//   warps 0-3, 4-7  softmax of tile 0 / 1: thread = query row; 128 scores in registers, bf16 / f16 P written back
+//                   over the scores in tensor memory (A operand of PV, so P never crosses shared memory); O is
+//                   rescaled only when a row's maximum grows by more than 2^8
+//   warp 8          MMA issuer: per key tile PV0 QK0' PV1 QK1' (whole warp, one elected thread)
+//   warps 9-11      gather of 128-key K and V tiles through req_to_token into a ring of tiles, in the
+//                   128-byte-swizzled layout; slots of the next tile are fetched a tile ahead
+//
+// Tensor memory: S0 | S1 (128 columns each, P in the first 64 of its S) | O0 | O1 (D columns each).
+// Shared memory per 128 keys: Q and K of two QK (128 KiB), V of two PV (64), the gather (64) = 2048 clocks at
+// 128 B/clk, as long as the tensor work and the 32768 exponentials take: the three bound it together.
+#pragma once
+
+namespace b200 {
+
+constexpr int kWideThreads = 384;
+constexpr int kWideTile = 128;                     // keys
+constexpr int kWideLoaders = 96;
+constexpr int kWideSoftmaxRegs = 200, kWideOtherRegs = 96;   // 256 x 200 + 128 x 96 <= 384 x 168 at launch
+
+template <int D>
+struct WideCfg {
+  static constexpr int TILE_BYTES = kWideTile * D * 2;        // a K, V or Q tile
+  static constexpr int SLOTS = D == 128 ? 5 : 10;             // K and V tiles in flight
+  static constexpr int OFF_RING = 2 * TILE_BYTES;             // after the two Q tiles
+  static constexpr int OFF_BAR = OFF_RING + SLOTS * TILE_BYTES;
+  static constexpr int N_BARS = 1 + 2 * SLOTS + 6;
+  static constexpr int SMEM_BYTES = OFF_BAR + N_BARS * 8 + 16;
+  static constexpr int O_COL = 256;
+  static_assert(SMEM_BYTES <= 227 * 1024, "tiles exceed shared memory");
+};
+
+namespace tc {
+// A operand from tensor memory (16-bit elements, two to a column), B from shared memory
+__device__ __forceinline__ void mma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(acc)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n" ::"r"(taddr),
+      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+}  // namespace tc
+
+template <typename T, int D>
+__global__ void __launch_bounds__(kWideThreads, 1)
+attn_extend_wide_kernel(const ExtendParams p) {
+  using C = WideCfg<D>;
+  constexpr int SL = C::SLOTS;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  const uint32_t sbase = smem_u32(smem);
+
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
+  const int lane = threadIdx.x & 31;
+
+  const int b = blockIdx.z;
+  const int ext = p.extend_lens[b];
+  const int prefix = p.prefix_lens[b];
+  const int tok_per_tile = 128 / p.pack;
+  // the latest query tiles see the most keys: they start first
+  const int tok0 = static_cast<int>(gridDim.x - 1 - blockIdx.x) * 2 * tok_per_tile;
+  if (tok0 >= ext) return;                         // uniform for the CTA
+  const int kvh = blockIdx.y / p.head_tiles;
+  const int head_base = kvh * p.group + (blockIdx.y - kvh * p.head_tiles) * p.pack;
+  const int kv_len = prefix + ext;
+  const int tiles = tok0 + tok_per_tile < ext ? 2 : 1;          // query tiles with any row
+  const int tok_last = min(tok0 + 2 * tok_per_tile, ext) - 1;
+  const int n_kv = ceil_div(p.causal ? prefix + tok_last + 1 : kv_len, kWideTile);
+  const int64_t q_row0 = p.extend_start[b];
+
+  const uint32_t bars = sbase + C::OFF_BAR;
+  const uint32_t bar_q = bars;
+  auto bar_full = [&](int s) { return bars + 8u * (1 + s); };
+  auto bar_empty = [&](int s) { return bars + 8u * (1 + SL + s); };
+  auto bar_s = [&](int t) { return bars + 8u * (1 + 2 * SL + t); };        // scores of tile t are complete
+  auto bar_p = [&](int t) { return bars + 8u * (3 + 2 * SL + t); };        // P of tile t is written
+  auto bar_o = [&](int t) { return bars + 8u * (5 + 2 * SL + t); };        // PV of tile t is complete
+  const uint32_t tmem_slot = bars + 8u * C::N_BARS;
+  bool dead = false;
+
+  if (threadIdx.x == 0) {
+    tc::mbar_init(bar_q, kWideLoaders);
+    for (int s = 0; s < SL; ++s) {
+      tc::mbar_init(bar_full(s), kWideLoaders);
+      tc::mbar_init(bar_empty(s), 1);
+    }
+    for (int t = 0; t < 2; ++t) {
+      tc::mbar_init(bar_s(t), 1);
+      tc::mbar_init(bar_p(t), 128);
+      tc::mbar_init(bar_o(t), 1);
+    }
+    tc::fence_barrier_init();
+  }
+  if (warp == 8) {
+    tc::tmem_alloc(tmem_slot, 512);
+    tc::tmem_relinquish();
+  }
+  tc::tc_fence_before();
+  __syncthreads();
+  tc::tc_fence_after();
+  const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(smem + C::OFF_BAR + 8 * C::N_BARS);
+
+  if (warp >= 8) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(kWideOtherRegs));
+    if (warp > 8) {
+      // ===================== gather =====================
+      const int lt = static_cast<int>(threadIdx.x) - 9 * 32;
+      constexpr int CPR = D / 8;                   // 16-byte chunks per row
+      constexpr int RPP = kWideLoaders / CPR;      // rows per pass
+      constexpr int PASSES = (kWideTile + RPP - 1) / RPP;
+      const int lrow = lt / CPR, lcol = lt - lrow * CPR;
+      const int32_t* rtt = p.req_to_token + p.req_pool_indices[b] * p.rtt_stride;
+      const int64_t row_bytes = p.kv_row_stride * 2;
+      const char* kbase = static_cast<const char*>(p.k_cache) + static_cast<int64_t>(kvh) * D * 2 + lcol * 16;
+      const char* vbase = static_cast<const char*>(p.v_cache) + static_cast<int64_t>(kvh) * D * 2 + lcol * 16;
+      int32_t slots[PASSES];
+      auto load_slots = [&](int j) {
+#pragma unroll
+        for (int i = 0; i < PASSES; ++i) {
+          const int r = lrow + RPP * i, pos = j * kWideTile + r;
+          slots[i] = (r < kWideTile && pos < kv_len) ? __ldg(rtt + pos) : 0;   // 0 = the pool's dummy row
+        }
+      };
+      load_slots(0);
+      for (int c = lt; c < tiles * 128 * CPR; c += kWideLoaders) {
+        const int r = c / CPR, col = c - r * CPR, t = r >> 7, rr = r & 127;
+        int tok = tok0 + r / p.pack;
+        if (tok >= ext) tok = ext - 1;             // padding rows repeat the last token (never stored)
+        const char* src = static_cast<const char*>(p.q) +
+                          ((q_row0 + tok) * p.q_stride + (head_base + r % p.pack) * D) * 2 + col * 16;
+        cp_async16(sbase + t * C::TILE_BYTES + swz_off<128>(rr, col), src);
+      }
+      // Unit u = 2 j + (0: K, 1: V) of key tile j goes to ring slot u % SL and is published LAG units later, when
+      // its copies have landed.  Waiting for unit u - SL to be consumed cannot stall: the issuer needs no unit
+      // past u - SL + 2 for that, and those up to u - 1 - LAG are published.
+      constexpr int LAG = SL - 3;
+      auto publish = [&](int u) {
+        tc::fence_proxy_async_smem();
+        if (u == 0) tc::mbar_arrive(bar_q);        // copied with unit 0
+        tc::mbar_arrive(bar_full(u % SL));
+      };
+      int slot = 0;
+      uint32_t phase = 0;
+      for (int j = 0; j < n_kv; ++j) {
+#pragma unroll
+        for (int kv = 0; kv < 2; ++kv) {
+          const int u = 2 * j + kv;
+          if (u >= SL) tc::mbar_wait_bounded(bar_empty(slot), phase ^ 1u, dead);
+          const uint32_t dst = sbase + C::OFF_RING + slot * C::TILE_BYTES;
+          const char* src = kv ? vbase : kbase;
+#pragma unroll
+          for (int i = 0; i < PASSES; ++i) {
+            const int r = lrow + RPP * i;
+            if (r < kWideTile) cp_async16(dst + swz_off<kWideTile>(r, lcol), src + static_cast<int64_t>(slots[i]) * row_bytes);
+          }
+          cp_async_commit();
+          if (kv == 1 && j + 1 < n_kv) load_slots(j + 1);
+          if (u >= LAG) {
+            cp_async_wait<LAG>();
+            publish(u - LAG);
+          }
+          if (++slot == SL) {
+            slot = 0;
+            phase ^= 1u;
+          }
+        }
+      }
+      cp_async_wait<0>();
+      for (int u = max(0, 2 * n_kv - LAG); u < 2 * n_kv; ++u) publish(u);
+    } else {
+      // ===================== MMA issuer =====================
+      constexpr uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
+      constexpr uint32_t idesc_qk = tc::make_idesc(fmt, fmt, 128, kWideTile, 0, 0);
+      constexpr uint32_t idesc_pv = tc::make_idesc(fmt, fmt, 128, D, 0, 1);    // V: MN-major B
+      const uint64_t qdesc = tc::make_smem_desc_sw128(sbase, 1024, 16);
+      auto wait_unit = [&](int u) {
+        tc::mbar_wait_bounded(bar_full(u % SL), (u / SL) & 1u, dead);
+        tc::tc_fence_after();
+      };
+      auto issue_qk = [&](int t, int j, bool last) {
+        const int s = (2 * j) % SL;
+        const uint64_t kdesc = tc::make_smem_desc_sw128(sbase + C::OFF_RING + s * C::TILE_BYTES, 1024, 16);
+        if (tc::elect_one()) {
+#pragma unroll
+          for (int kk = 0; kk < D / 16; ++kk) {
+            const uint32_t off = ((kk >> 2) * (128 * 128) + (kk & 3) * 32) >> 4;
+            tc::mma_f16(tmem_base + t * 128, qdesc + t * (C::TILE_BYTES >> 4) + off, kdesc + off, idesc_qk, kk != 0 ? 1u : 0u);
+          }
+          tc::mma_commit(bar_s(t));
+          if (last) tc::mma_commit(bar_empty(s));  // both tiles have used this K tile
+        }
+        __syncwarp();
+      };
+      tc::mbar_wait_bounded(bar_q, 0, dead);
+      wait_unit(0);
+      for (int t = 0; t < tiles; ++t) issue_qk(t, 0, t == tiles - 1);
+      for (int j = 0; j < n_kv; ++j) {
+        const int s = (2 * j + 1) % SL;
+        const uint64_t vdesc = tc::make_smem_desc_sw128(sbase + C::OFF_RING + s * C::TILE_BYTES, 1024, kWideTile * 128);
+        wait_unit(2 * j + 1);
+        for (int t = 0; t < tiles; ++t) {
+          tc::mbar_wait_bounded(bar_p(t), j & 1u, dead);
+          tc::tc_fence_after();
+          if (tc::elect_one()) {
+#pragma unroll
+            for (int kk = 0; kk < kWideTile / 16; ++kk)
+              tc::mma_f16_ts(tmem_base + C::O_COL + t * D, tmem_base + t * 128 + kk * 8, vdesc + ((kk * 16 * 128) >> 4),
+                             idesc_pv, (j | kk) != 0 ? 1u : 0u);
+            tc::mma_commit(bar_o(t));
+            if (t == tiles - 1) tc::mma_commit(bar_empty(s));
+          }
+          __syncwarp();
+          if (j + 1 < n_kv) {
+            if (t == 0) wait_unit(2 * j + 2);
+            issue_qk(t, j + 1, t == tiles - 1);    // overwrites P(j) of this tile: MMAs run in issue order
+          }
+        }
+      }
+    }
+  } else {
+    // ===================== softmax / epilogue =====================
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(kWideSoftmaxRegs));
+    const int t = warp >> 2;
+    if (t < tiles) {
+      const int r = (warp & 3) * 32 + lane;
+      const int tok = tok0 + t * tok_per_tile + r / p.pack;
+      const bool row_ok = tok < ext;
+      const int limit = p.causal ? prefix + min(tok, ext - 1) : kv_len - 1;    // last visible key
+      const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
+      const uint32_t tmem_s = tmem_base + lane_addr + t * 128;
+      const uint32_t tmem_o = tmem_base + lane_addr + C::O_COL + t * D;
+      const float2 sc2 = make_float2(p.qk_scale, p.qk_scale), one2 = make_float2(1.f, 1.f);
+      float m = -INFINITY, l = 0.f;
+      for (int j = 0; j < n_kv; ++j) {
+        tc::mbar_wait_bounded(bar_s(t), j & 1u, dead);
+        tc::tc_fence_after();
+        __syncwarp();
+        uint32_t v[4][32];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) tc::tmem_ld32(tmem_s + c * 32, v[c]);
+        tc::tmem_ld_wait();
+        const int k0 = j * kWideTile;
+        if (k0 + kWideTile - 1 > limit) {          // the tile crosses the row's last key
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int e = 0; e < 32; ++e)
+              if (k0 + c * 32 + e > limit) v[c][e] = 0xff800000u;              // -inf
+        }
+        float a[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+          for (int e = 0; e < 32; e += 2) a[c] = fmax3(a[c], __uint_as_float(v[c][e]), __uint_as_float(v[c][e + 1]));
+        const float mt = fmaxf(fmaxf(a[0], a[1]), fmaxf(a[2], a[3])) * p.qk_scale;   // scale > 0: -inf stays
+        const float m_new = fmaxf(m, mt);
+        if (__any_sync(0xffffffffu, m_new > m + kRescaleThreshold)) {          // also the first finite maximum
+          if (j > 0) {
+            tc::mbar_wait_bounded(bar_o(t), (j - 1) & 1u, dead);               // O holds tiles 0 .. j - 1
+            tc::tc_fence_after();
+            __syncwarp();
+            const float alpha = (m == -INFINITY) ? 0.f : fast_exp2(m - m_new);
+#pragma unroll 1
+            for (int cc = 0; cc < D / 16; ++cc) {
+              uint32_t o[16];
+              tc::tmem_ld16(tmem_o + cc * 16, o);
+              tc::tmem_ld_wait();
+#pragma unroll
+              for (int c = 0; c < 16; ++c) o[c] = __float_as_uint(__uint_as_float(o[c]) * alpha);
+              tc::tmem_st16(tmem_o + cc * 16, o);
+            }
+            l *= alpha;
+          }
+          m = m_new;
+        }
+        const float m_use = (m == -INFINITY) ? 0.f : m;
+        const float2 nm2 = make_float2(-m_use, -m_use);
+        float2 lsum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          uint32_t packed[16];
+#pragma unroll
+          for (int e = 0; e < 16; ++e) {
+            const float2 x = ffma2(make_float2(__uint_as_float(v[c][2 * e]), __uint_as_float(v[c][2 * e + 1])), sc2, nm2);
+            const float2 y = make_float2(fast_exp2(x.x), fast_exp2(x.y));
+            lsum[e & 1] = ffma2(y, one2, lsum[e & 1]);
+            packed[e] = pack16<T>(y.x, y.y);
+          }
+          tc::tmem_st16(tmem_s + c * 16, packed);  // over scores that are in registers by now
+        }
+        tc::tmem_st_wait();
+        l += (lsum[0].x + lsum[0].y) + (lsum[1].x + lsum[1].y);
+        tc::tc_fence_before();
+        tc::mbar_arrive(bar_p(t));
+      }
+      // ---- O / l -> out
+      tc::mbar_wait_bounded(bar_o(t), (n_kv - 1) & 1u, dead);
+      tc::tc_fence_after();
+      __syncwarp();
+      const float inv_l = l > 0.f ? p.out_scale / l : 0.f;
+      T* orow = static_cast<T*>(p.o) + (q_row0 + (row_ok ? tok : 0)) * p.o_stride +
+                static_cast<int64_t>(head_base + r % p.pack) * D;
+#pragma unroll 1
+      for (int cc = 0; cc < D / 32; ++cc) {
+        uint32_t o[32];
+        tc::tmem_ld32(tmem_o + cc * 32, o);
+        tc::tmem_ld_wait();
+        if (row_ok) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            uint32_t w[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              w[e] = pack16<T>(__uint_as_float(o[i * 8 + 2 * e]) * inv_l, __uint_as_float(o[i * 8 + 2 * e + 1]) * inv_l);
+            *reinterpret_cast<uint4*>(orow + cc * 32 + i * 8) = make_uint4(w[0], w[1], w[2], w[3]);
+          }
+        }
+      }
+    }
+  }
+
+  tc::tc_fence_before();
+  __syncthreads();
+  if (warp == 8) tc::tmem_dealloc(tmem_base, 512);
+}
+
+template <typename T, int D>
+static int launch_extend_wide(const ExtendParams& p, int bs, int max_extend_len, cudaStream_t st) {
+  using C = WideCfg<D>;
+  auto kern = attn_extend_wide_kernel<T, D>;
+  B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
+  const dim3 grid(ceil_div(max_extend_len, 256 / p.pack), p.Hkv * p.head_tiles, bs);
+  note_variant("attn_extend_wide d=%d", D);
+  {
+    ScopedKernelTimer timer("attn_extend", st);
+    kern<<<grid, kWideThreads, C::SMEM_BYTES, st>>>(p);
+  }
+  B200_CHECK_LAUNCH("attn_extend_wide_kernel");
+  return 0;
+}
+
+}  // namespace b200
