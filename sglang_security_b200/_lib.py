@@ -54,6 +54,7 @@ _SIGNATURES = {
                                 c_void_p, c_int, c_void_p]),
     "b200_attn_decode_workspace_bytes": (c_size_t, [c_int, c_int, c_int, c_int]),
     "b200_attn_decode_num_splits": (c_int, [c_int, c_int, c_int, c_int, c_int64, c_int]),
+    "b200_attn_decode_num_splits_ragged": (c_int, [c_int, c_int, c_int, c_int, c_int64, c_int64, c_int]),
     "b200_attn_decode_split_align": (c_int, [c_int, c_int]),
     "b200_attn_decode": (c_int, [c_void_p, c_int64, c_void_p, c_void_p, c_int64, c_void_p,
                                  c_int64, c_void_p, c_int64, c_void_p, c_void_p, c_int, c_int,

@@ -564,35 +564,80 @@ attn_decode_mma_kernel(const DecodeParams p) {
     decode_fused_tail<T, NW * 32>(tail_of(p), b, kvh * p.group + head0, heads_here, ceil_div(len, chunk), D);
 }
 
-// Merge of split partials: one CTA per (query head, request).
+// Merge of split partials: one warp per (query head, request), four columns per lane.  Latency-bound (a few hundred
+// KB): the split sums are read by all lanes at once and the first partial rows are requested before the sequence length
+// is known, so the chain is one round trip to L2, not one per split (1 request of 1500 tokens in 7 splits: 5.2 us, now
+// 3.8).  Sums run over the splits in order, as in attn_merge_quant_kernel: same bytes.
+constexpr int kMergeWarps = 4;
+constexpr int kMergeAhead = 8;
+
 template <typename T>
-__global__ void attn_merge_kernel(const float* __restrict__ part_o,
-                                  const float* __restrict__ part_lse, T* __restrict__ o,
-                                  int64_t o_stride, const int64_t* __restrict__ seq_lens, int Hq,
-                                  int Dv, int num_splits, int align,
-                                  const int32_t* __restrict__ row_list, const T* __restrict__ gate,
-                                  int64_t gate_stride) {
+__global__ void __launch_bounds__(kMergeWarps * 32)
+attn_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_lse, T* __restrict__ o,
+                  int64_t o_stride, const int64_t* __restrict__ seq_lens, int Hq, int Dv, int num_splits, int align,
+                  const int32_t* __restrict__ row_list, const T* __restrict__ gate, int64_t gate_stride) {
   griddep_wait();
   griddep_launch_dependents();
-  const int hq = blockIdx.x, b = blockIdx.y;
+  const int lane = threadIdx.x & 31;
+  const int hq = blockIdx.x * kMergeWarps + (threadIdx.x >> 5), b = blockIdx.y;
+  if (hq >= Hq) return;
+  const int64_t base = (static_cast<int64_t>(b) * Hq + hq) * num_splits;
+  const float* po = part_o + base * Dv;
+  // splits past the sequence are allocated but hold nothing: their values are not used
+  float4 x[kMergeAhead];
+  const int d0 = lane * 4;
+#pragma unroll
+  for (int i = 0; i < kMergeAhead; ++i)
+    x[i] = i < num_splits && d0 < Dv ? __ldcg(reinterpret_cast<const float4*>(po + static_cast<int64_t>(i) * Dv + d0))
+                                     : make_float4(0.f, 0.f, 0.f, 0.f);
+  const float lse0 = lane < num_splits ? __ldcg(part_lse + base + lane) : 0.f;
   const int len = static_cast<int>(seq_lens[b]);
   if (len <= 0) return;
-  const int chunk = split_chunk(len, num_splits, align);
-  const int nvalid = ceil_div(len, chunk);
-  const int64_t base = (static_cast<int64_t>(b) * Hq + hq) * num_splits;
-  float M = -INFINITY;
-  for (int s = 0; s < nvalid; ++s) M = fmaxf(M, __ldg(part_lse + base + s));
-  float den = 0.f;
-  for (int s = 0; s < nvalid; ++s) den += fast_exp2(__ldg(part_lse + base + s) - M);
-  const float inv = 1.f / den;
+  const int nvalid = ceil_div(len, split_chunk(len, num_splits, align));
+  float M = lane < nvalid ? lse0 : -INFINITY;
+  for (int s = 32 + lane; s < nvalid; s += 32) M = fmaxf(M, __ldcg(part_lse + base + s));
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, off));
   const int64_t row = row_list ? row_list[b] : b;
-  for (int d = threadIdx.x; d < Dv; d += blockDim.x) {
-    float num = 0.f;
-    for (int s = 0; s < nvalid; ++s)
-      num += fast_exp2(__ldg(part_lse + base + s) - M) * __ldg(part_o + (base + s) * Dv + d);
-    num *= inv;
-    if (gate) num *= sigmoid_f(to_float<T>(gate[row * gate_stride + hq * Dv + d]));
-    o[row * o_stride + hq * Dv + d] = from_float<T>(num);
+  for (int dd = 0; dd < Dv; dd += 128) {
+    const int d = dd + d0;
+    float den = 0.f;
+    float4 num = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int s0 = 0; s0 < nvalid; s0 += 32) {
+      const float lse = s0 == 0 ? lse0 : (s0 + lane < nvalid ? __ldcg(part_lse + base + s0 + lane) : 0.f);
+      const float w_lane = s0 + lane < nvalid ? fast_exp2(lse - M) : 0.f;
+      for (int s1 = s0; s1 < min(nvalid, s0 + 32); s1 += kMergeAhead) {
+        if (s1 > 0 || dd > 0) {
+#pragma unroll
+          for (int i = 0; i < kMergeAhead; ++i)
+            if (s1 + i < nvalid && d < Dv)
+              x[i] = __ldcg(reinterpret_cast<const float4*>(po + static_cast<int64_t>(s1 + i) * Dv + d));
+        }
+#pragma unroll
+        for (int i = 0; i < kMergeAhead; ++i) {
+          const float w = __shfl_sync(0xffffffffu, w_lane, (s1 + i) & 31);
+          if (s1 + i < nvalid) {
+            den += w;
+            num.x += w * x[i].x;
+            num.y += w * x[i].y;
+            num.z += w * x[i].z;
+            num.w += w * x[i].w;
+          }
+        }
+      }
+    }
+    if (d >= Dv) continue;
+    const float inv = 1.f / den;
+    float y[4] = {num.x * inv, num.y * inv, num.z * inv, num.w * inv};
+    if (gate) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (d + e < Dv) y[e] *= sigmoid_f(to_float<T>(gate[row * gate_stride + hq * Dv + d + e]));
+    }
+    T* dst = o + row * o_stride + hq * Dv + d;
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (d + e < Dv) dst[e] = from_float<T>(y[e]);
   }
 }
 
@@ -640,8 +685,10 @@ attn_merge_quant_kernel(const float* __restrict__ part_o, const float* __restric
       if (num_splits > 1) {
         const int64_t base = (static_cast<int64_t>(b) * Hq + h) * num_splits;
         float M = -INFINITY;
+#pragma unroll 8
         for (int s = 0; s < nvalid; ++s) M = fmaxf(M, __ldg(part_lse + base + s));
         float den = 0.f, num[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
         for (int s = 0; s < nvalid; ++s) {
           const float w = fast_exp2(__ldg(part_lse + base + s) - M);
           const float4 x = __ldg(reinterpret_cast<const float4*>(part_o + (base + s) * Dv + d));
@@ -917,7 +964,7 @@ size_t b200_attn_decode_workspace_bytes(int bs, int Hq, int Dv, int num_splits) 
   return rows * Dv * sizeof(float) + rows * sizeof(float);
 }
 
-int b200_attn_decode_num_splits(int bs, int Hkv, int group, int D, int64_t avg_len, int num_sms) {
+static int decode_num_splits(int bs, int Hkv, int group, int D, int64_t avg_len, int64_t max_len, int num_sms) {
   using namespace b200;
   if (bs <= 0 || Hkv <= 0 || group <= 0) return 1;
   if (num_sms <= 0) num_sms = 148;
@@ -927,36 +974,41 @@ int b200_attn_decode_num_splits(int bs, int Hkv, int group, int D, int64_t avg_l
   const int ctas_per_sm = decode_ctas_per_sm(D);
   const int64_t slots = static_cast<int64_t>(num_sms) * ctas_per_sm;
   const int align = decode_align();
-  // HBM-bound: what matters is that enough CTAs stay resident until the end, not whole waves —
-  // late CTAs run faster because they share the bandwidth with fewer neighbours.  Take the
-  // smallest split count that oversubscribes the resident slots by `kOver` (measured on cfg 2:
-  // s = 2 -> 1.7x beats s = 1 -> 0.86x by 20 % and s = 8 by 4 %), with at least 4 CTA tiles
-  // (192 tokens) per split.
-  constexpr double kOver = 1.5;
+  // Equal-length CTAs that all fit the resident slots at once finish together, while any overflow runs as a thin
+  // second wave: the largest count that fits one wave.  Per-rank shapes of Llama-3.1-8B at TP 2 / 4 / 8, batch
+  // 64 x 4k: 2 / 4 / 9 splits = 512 / 512 / 576 CTAs on 592 slots (90.8 / 50.7 / 29.9 us) against 93.9 / 56.4 /
+  // 35.3 us for the oversubscription rule below; 1 split (512 CTAs, no merge) 170.4 us against 174.4 + merge.
+  // Few requests are bound by the chain of tiles in a warp, so the splits go down to 64 tokens (us, splits of 192
+  // tokens -> this: 1 x 1500 tokens 10.9 -> 10.3, 5 x 2000 ragged 14.4 -> 12.3), but past 32 of them the merge takes
+  // back what the chain gives (1 x 8000, FP8 rows: 16.5 with 41, 14.4 with 12 to 32).
+  const int64_t by_slots = slots / base;
+  int64_t fit = by_slots < avg_len / 64 ? by_slots : avg_len / 64;
+  if (fit > 32) fit = 32;
+  // Few splits of unequal requests: the longest ones would run alone at the end, so twice the slots are filled
+  // (us, one wave or 1.5 -> 2.1 times the slots: 40 x up to 3000 tokens 61.3 -> 57.9, 64 x up to 4096 FP8 77.0 -> 69.3,
+  // 27 x up to 6000 FP8 50.4 -> 48.2).
+  const bool ragged = max_len * 8 > avg_len * 9 && by_slots < 4;
+  if (!ragged && fit >= 1 && (fit < by_slots || static_cast<double>(base * fit) >= 0.85 * static_cast<double>(slots)))
+    return static_cast<int>(fit);
+  // HBM-bound: what matters is that enough CTAs stay resident until the end, not whole waves — late CTAs run faster
+  // because they share the bandwidth with fewer neighbours.  The smallest split count that oversubscribes the
+  // resident slots (measured on cfg 2: s = 2 -> 1.7x beats s = 1 -> 0.86x by 20 % and s = 8 by 4 %), with at least 4
+  // CTA tiles (192 tokens) per split.
+  const double over = ragged ? 2.1 : 1.5;
   int64_t max_s = avg_len / (4 * align);
   if (max_s > 64) max_s = 64;
-  if (max_s < 1) max_s = 1;
-  // Few kv heads per rank (tensor parallel): equal-length CTAs that all fit the resident slots at
-  // once finish together, while any overflow runs as a thin second wave.  Measured on the per-rank
-  // shapes of Llama-3.1-8B at TP 2/4/8, batch 64 x 4k (profiles/r02_sweep_decode_tp_shapes.json):
-  // the best split count is the LARGEST one whose CTAs fit one wave — 2 / 4 / 9 splits = 512 / 512 /
-  // 576 CTAs on 592 slots (90.8 / 50.7 / 29.9 us) against 93.9 / 56.4 / 35.3 us for the
-  // oversubscription rule below.
-  {
-    const int64_t s1 = slots / base;
-    // (s1 == 1, the 512 CTAs of the whole-model bench shape: 170.4 us and no merge launch against
-    //  174.4 us + merge with two splits, profiles/r02_bench_n1.json)
-    if (s1 >= 1 && s1 <= max_s && static_cast<double>(base * s1) >= 0.85 * static_cast<double>(slots))
-      return static_cast<int>(s1);
-  }
-  int best = static_cast<int>(max_s);
-  for (int s = 1; s <= max_s; ++s) {
-    if (static_cast<double>(base * s) >= kOver * static_cast<double>(slots)) {
-      best = s;
-      break;
-    }
-  }
-  return best;
+  for (int s = 1; s <= max_s; ++s)
+    if (static_cast<double>(base * s) >= over * static_cast<double>(slots)) return s;
+  return static_cast<int>(max_s > fit ? max_s : (fit > 1 ? fit : 1));
+}
+
+int b200_attn_decode_num_splits(int bs, int Hkv, int group, int D, int64_t avg_len, int num_sms) {
+  return decode_num_splits(bs, Hkv, group, D, avg_len, avg_len, num_sms);
+}
+
+int b200_attn_decode_num_splits_ragged(int bs, int Hkv, int group, int D, int64_t avg_len, int64_t max_len,
+                                       int num_sms) {
+  return decode_num_splits(bs, Hkv, group, D, avg_len, max_len, num_sms);
 }
 
 static int attn_merge_impl(const float* part_o, const float* part_lse, void* o, int64_t o_stride,
@@ -970,8 +1022,9 @@ static int attn_merge_impl(const float* part_o, const float* part_lse, void* o, 
                num_splits, split_align);
   B200_REQUIRE(part_o && part_lse && o && seq_lens, "b200_attn_merge: null pointer");
   B200_REQUIRE(dtype == B200_BF16 || dtype == B200_F16, "b200_attn_merge: dtype %d", dtype);
-  dim3 grid(Hq, bs);
-  const int threads = Dv >= 128 ? 128 : 64;
+  B200_REQUIRE(Dv % 4 == 0, "b200_attn_merge: value dim %d", Dv);
+  dim3 grid(ceil_div(Hq, kMergeWarps), bs);
+  const int threads = kMergeWarps * 32;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   ScopedKernelTimer timer("attn_merge", st);
   if (dtype == B200_BF16)

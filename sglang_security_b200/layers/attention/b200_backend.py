@@ -97,12 +97,12 @@ class B200AttnBackend(AttentionBackend):
         return self._tickets
 
     # ------------------------------------------------------------------ metadata
-    def _num_splits(self, bs: int, head_dim: int, avg_len: int) -> int:
+    def _num_splits(self, bs: int, head_dim: int, avg_len: int, max_len: int = 0) -> int:
         if self.fixed_num_kv_splits > 0:
             return self.fixed_num_kv_splits
-        return self.lib.b200_attn_decode_num_splits(
+        return self.lib.b200_attn_decode_num_splits_ragged(
             bs, self.num_kv_head, self.num_head // self.num_kv_head, head_dim, int(avg_len),
-            self.num_sms)
+            max(int(avg_len), int(max_len)), self.num_sms)
 
     def _ensure_workspace(self, bs: int, num_splits: int) -> Optional[torch.Tensor]:
         need = self.lib.b200_attn_decode_workspace_bytes(bs, self.num_head, self.v_head_dim,
@@ -121,7 +121,9 @@ class B200AttnBackend(AttentionBackend):
                 return
             total = forward_batch.seq_lens_sum or bs * self.max_context_len
             head_dim = self.v_head_dim
-            s = self._num_splits(bs, head_dim, max(1, total // bs))
+            lens = getattr(forward_batch, "seq_lens_cpu", None)   # host copy, where the scheduler keeps one
+            longest = int(lens.max()) if lens is not None and lens.numel() else 0
+            s = self._num_splits(bs, head_dim, max(1, total // bs), longest)
             self.forward_metadata = ForwardMetadata(num_splits=s,
                                                     workspace=self._ensure_workspace(bs, s))
         else:
