@@ -226,6 +226,17 @@ int b200_attn_extend(const void* q, int64_t q_stride, const void* k_cache, const
 
 /* Same kernel with an output multiplier: extend over an FP8 KV pool runs on an exact 16-bit copy
  * of the requests' rows (b200_kv_dequant_gather) with scale * k_scale and out_scale = v_scale.    */
+/* b200_attn_extend_scaled for callers that know the longest request (max_kv_len = its prefix + new tokens, on the
+ * host): few query tiles over many keys are then spread over clusters.  0: not known. */
+int b200_attn_extend_known(const void* q, int64_t q_stride, const void* k_cache, const void* v_cache,
+                           int64_t kv_row_stride, void* o, int64_t o_stride, const int32_t* req_to_token,
+                           int64_t req_to_token_stride, const int64_t* req_pool_indices, const int64_t* seq_lens,
+                           const int32_t* extend_prefix_lens, const int32_t* extend_seq_lens,
+                           const int32_t* extend_start_loc, int bs, int max_extend_len, int max_kv_len, int Hq, int Hkv,
+                           int D, int Dv, float scale, float logit_cap, float out_scale, int causal, int dtype,
+                           void* stream);
+/* Start row of every request: exclusive sums of extend_seq_lens. */
+int b200_extend_starts(const int32_t* extend_seq_lens, int32_t* extend_start_loc, int bs, void* stream);
 int b200_attn_extend_scaled(const void* q, int64_t q_stride, const void* k_cache,
                             const void* v_cache, int64_t kv_row_stride, void* o, int64_t o_stride,
                             const int32_t* req_to_token, int64_t req_to_token_stride,

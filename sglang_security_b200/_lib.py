@@ -42,6 +42,10 @@ _SIGNATURES = {
                                         c_int64, c_void_p, c_int64, c_void_p, c_void_p, c_void_p,
                                         c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
                                         c_float, c_float, c_float, c_int, c_int, c_void_p]),
+    "b200_attn_extend_known": (c_int, [c_void_p, c_int64, c_void_p, c_void_p, c_int64, c_void_p, c_int64, c_void_p,
+                                       c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
+                                       c_int, c_int, c_int, c_int, c_float, c_float, c_float, c_int, c_int, c_void_p]),
+    "b200_extend_starts": (c_int, [c_void_p, c_void_p, c_int, c_void_p]),
     "b200_write_req_to_token": (c_int, [c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p,
                                         c_void_p, c_int, c_void_p]),
     "b200_get_last_loc": (c_int, [c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_int, c_void_p]),

@@ -24,7 +24,7 @@
 #include <cstdlib>
 #include <type_traits>
 
-#include "tc_common.cuh"
+#include "gemm_tc.cuh"
 
 namespace b200 {
 
@@ -62,6 +62,7 @@ struct ExtendParams {
   int64_t gate_stride;           // sigmoid(gate[row, head * D + d])
   float score_bound;             // > 0: no capped score exceeds it (unit-norm queries and keys), so it is the
                                  // reference of every exponent instead of the cap; 0: the cap itself
+  int kv_splits;                 // attn_extend_wide.cuh: CTAs of a cluster that share the keys of its query tiles
   float cap_poly[5];             // FAST == 2: cap * log2(e) * tanh(x) / x = sum_i cap_poly[i] x^(2i) on the
                                  // range the scores can take
 };
@@ -611,13 +612,18 @@ static void fit_cap_polynomial(double mult, double range, float* c) {
 }
 
 template <typename T, int D>
-static int launch_extend(const ExtendParams& p, int n_values, int bs, int max_extend_len, cudaStream_t st) {
+static int launch_extend(const ExtendParams& p, int n_values, int bs, int max_extend_len, int max_kv_len,
+                         cudaStream_t st) {
   // a cap up to 40 keeps e^(-2 cap) a normal fp32 (and 16-bit) number: the one-pass capped form
   const float ref = p.score_bound > 0.f && p.score_bound < p.logit_cap ? p.score_bound : p.logit_cap;
   const bool fast = ref <= 40.f && p.qk_scale > 0.f && extend_fast_softmax_enabled();
-  // plain attention: two query tiles per CTA (all else, and every option, on the kernel above)
-  if (fast && p.logit_cap <= 0.f && p.window == 0 && !p.sink && !p.gate && !p.lse && n_values == 1 && p.v_head < 0)
-    return launch_extend_wide<T, D>(p, bs, max_extend_len, st);
+  // Plain attention over 1024 keys or more: two query tiles per CTA.  All options, and shorter requests, on the kernel
+  // above, whose two CTAs per SM hide what a CTA of the other spends before its first and after its last tile
+  // (~8 us; us, this / that kernel: 8 x 512 fresh tokens 63.6 / 72.3, 8 x 1024 160 / 153, 8 x 1536 299 / 254, 24 new
+  // tokens behind 512 / 1024 / 1536 cached 21.9 / 20.1, 30.9 / 22.8, 39.2 / 21.3).
+  const int keys = max_kv_len > 0 ? max_kv_len : max_extend_len;
+  if (fast && keys >= 1024 && p.logit_cap <= 0.f && p.window == 0 && !p.sink && !p.gate && !p.lse && n_values == 1 && p.v_head < 0)
+    return launch_extend_wide<T, D>(p, bs, max_extend_len, max_kv_len, st);
   note_variant("attn_extend d=%d fast_softmax=%d values=%d", D, fast ? 1 : 0, n_values);
   if (n_values == 2)
     return fast ? launch_extend_inst<T, D, 1, 2>(p, bs, max_extend_len, st)
@@ -705,7 +711,8 @@ static int extend_heads_impl(const void* q, int64_t q_stride, const void* k_cach
                              int D, int Dv, float scale, float logit_cap, float out_scale, int causal,
                              int window, int keep_first, const float* sink, int v_head, int n_values,
                              int64_t o_plane, float* lse, int64_t lse_stride, int dtype, void* stream,
-                             const void* gate = nullptr, int64_t gate_stride = 0, float score_bound = 0.f) {
+                             const void* gate = nullptr, int64_t gate_stride = 0, float score_bound = 0.f,
+                             int max_kv_len = 0) {
   using namespace b200;
   B200_REQUIRE(!gate || (n_values == 1 && gate_stride % 8 == 0 && aligned16(gate)),
                "b200_attn_extend: the gate rows must be 16-byte aligned (stride %lld)",
@@ -770,10 +777,10 @@ static int extend_heads_impl(const void* q, int64_t q_stride, const void* k_cach
   B200_REQUIRE(bs <= 65535 && Hkv * p.head_tiles <= 65535, "b200_attn_extend: grid too large");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (dtype == B200_BF16)
-    return D == 128 ? launch_extend<__nv_bfloat16, 128>(p, n_values, bs, max_extend_len, st)
-                    : launch_extend<__nv_bfloat16, 64>(p, n_values, bs, max_extend_len, st);
-  return D == 128 ? launch_extend<__half, 128>(p, n_values, bs, max_extend_len, st)
-                  : launch_extend<__half, 64>(p, n_values, bs, max_extend_len, st);
+    return D == 128 ? launch_extend<__nv_bfloat16, 128>(p, n_values, bs, max_extend_len, max_kv_len, st)
+                    : launch_extend<__nv_bfloat16, 64>(p, n_values, bs, max_extend_len, max_kv_len, st);
+  return D == 128 ? launch_extend<__half, 128>(p, n_values, bs, max_extend_len, max_kv_len, st)
+                  : launch_extend<__half, 64>(p, n_values, bs, max_extend_len, max_kv_len, st);
 }
 
 int b200_attn_extend_heads(const void* q, int64_t q_stride, const void* k_cache, const void* v_cache,
@@ -819,6 +826,20 @@ int b200_attn_extend_lse(const void* q, int64_t q_stride, const void* k_cache, c
                            req_to_token_stride, req_pool_indices, seq_lens, extend_prefix_lens,
                            extend_seq_lens, extend_start_loc, bs, max_extend_len, Hq, Hkv, D, Dv, scale, 0.f,
                            1.f, 1, window, 0, nullptr, -1, 1, 0, lse, lse_stride, dtype, stream);
+}
+
+int b200_attn_extend_known(const void* q, int64_t q_stride, const void* k_cache, const void* v_cache,
+                           int64_t kv_row_stride, void* o, int64_t o_stride, const int32_t* req_to_token,
+                           int64_t req_to_token_stride, const int64_t* req_pool_indices, const int64_t* seq_lens,
+                           const int32_t* extend_prefix_lens, const int32_t* extend_seq_lens,
+                           const int32_t* extend_start_loc, int bs, int max_extend_len, int max_kv_len, int Hq, int Hkv,
+                           int D, int Dv, float scale, float logit_cap, float out_scale, int causal, int dtype,
+                           void* stream) {
+  return extend_heads_impl(q, q_stride, k_cache, v_cache, kv_row_stride, o, o_stride, req_to_token,
+                           req_to_token_stride, req_pool_indices, seq_lens, extend_prefix_lens,
+                           extend_seq_lens, extend_start_loc, bs, max_extend_len, Hq, Hkv, D, Dv, scale, logit_cap,
+                           out_scale, causal, 0, 0, nullptr, -1, 1, 0, nullptr, 0, dtype, stream, nullptr, 0, 0.f,
+                           max_kv_len);
 }
 
 }  // extern "C"

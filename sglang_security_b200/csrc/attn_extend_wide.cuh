@@ -11,6 +11,10 @@
 //   warps 9-11      gather of 128-key K and V tiles through req_to_token into a ring of tiles, in the
 //                   128-byte-swizzled layout; slots of the next tile are fetched a tile ahead
 //
+// Few query tiles (a short turn behind a long prefix): a cluster of S CTAs takes the query tiles of one CTA, each a
+// range of the keys; the unnormalised O, maximum and sum of every row meet in shared memory and are merged in rank
+// order over the cluster (deterministic).
+//
 // Tensor memory: S0 | S1 (128 columns each, P in the first 64 of its S) | O0 | O1 (D columns each).
 // Shared memory per 128 keys: Q and K of two QK (128 KiB), V of two PV (64), the gather (64) = 2048 clocks at
 // 128 B/clk, as long as the tensor work and the 32768 exponentials take: the three bound it together (D 128: 3450
@@ -35,6 +39,8 @@ struct WideCfg {
   static constexpr int N_BARS = 1 + 2 * SLOTS + 8;
   static constexpr int SMEM_BYTES = OFF_BAR + N_BARS * 8 + 16;
   static constexpr int O_COL = 256;
+  static constexpr int PART_ROW = D * 4 + 16;                 // a row's partial O, then m and l
+  static_assert(256 * PART_ROW <= OFF_BAR, "partial rows alias the operand tiles");
   static_assert(SMEM_BYTES <= 227 * 1024, "tiles exceed shared memory");
 };
 
@@ -56,7 +62,7 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
 }
 }  // namespace tc
 
-template <typename T, int D>
+template <typename T, int D, bool SPLIT>
 __global__ void __launch_bounds__(kWideThreads, 1)
 attn_extend_wide_kernel(const ExtendParams p) {
   using C = WideCfg<D>;
@@ -68,18 +74,23 @@ attn_extend_wide_kernel(const ExtendParams p) {
   const int lane = threadIdx.x & 31;
 
   const int b = blockIdx.z;
+  const int S = SPLIT ? p.kv_splits : 1;           // cluster size; every CTA of a cluster has the same query tiles
+  const int rank = S > 1 ? static_cast<int>(cluster_ctarank()) : 0;
   const int ext = p.extend_lens[b];
   const int prefix = p.prefix_lens[b];
   const int tok_per_tile = 128 / p.pack;
   // the latest query tiles see the most keys: they start first
-  const int tok0 = static_cast<int>(gridDim.x - 1 - blockIdx.x) * 2 * tok_per_tile;
-  if (tok0 >= ext) return;                         // uniform for the CTA
+  const int tok0 = static_cast<int>((gridDim.x - 1 - blockIdx.x) / S) * 2 * tok_per_tile;
+  if (tok0 >= ext) return;                         // uniform for the CTA and its cluster
   const int kvh = blockIdx.y / p.head_tiles;
   const int head_base = kvh * p.group + (blockIdx.y - kvh * p.head_tiles) * p.pack;
   const int kv_len = prefix + ext;
   const int tiles = tok0 + tok_per_tile < ext ? 2 : 1;          // query tiles with any row
   const int tok_last = min(tok0 + 2 * tok_per_tile, ext) - 1;
-  const int n_kv = ceil_div(p.causal ? prefix + tok_last + 1 : kv_len, kWideTile);
+  const int n_all = ceil_div(p.causal ? prefix + tok_last + 1 : kv_len, kWideTile);
+  const int per = ceil_div(n_all, S);
+  const int j0 = min(n_all, rank * per);           // this CTA's key tiles: loop index j stands for tile j0 + j
+  const int n_kv = min(n_all, j0 + per) - j0;      // 0: nothing left for this rank
   const int64_t q_row0 = p.extend_start[b];
 
   const uint32_t bars = sbase + C::OFF_BAR;
@@ -132,12 +143,12 @@ attn_extend_wide_kernel(const ExtendParams p) {
       auto load_slots = [&](int j) {
 #pragma unroll
         for (int i = 0; i < PASSES; ++i) {
-          const int r = lrow + RPP * i, pos = j * kWideTile + r;
+          const int r = lrow + RPP * i, pos = (j0 + j) * kWideTile + r;
           slots[i] = (r < kWideTile && pos < kv_len) ? __ldg(rtt + pos) : 0;   // 0 = the pool's dummy row
         }
       };
-      load_slots(0);
-      for (int c = lt; c < tiles * 128 * CPR; c += kWideLoaders) {
+      if (n_kv > 0) load_slots(0);
+      for (int c = lt; n_kv > 0 && c < tiles * 128 * CPR; c += kWideLoaders) {
         const int r = c / CPR, col = c - r * CPR, t = r >> 7, rr = r & 127;
         int tok = tok0 + r / p.pack;
         if (tok >= ext) tok = ext - 1;             // padding rows repeat the last token (never stored)
@@ -206,9 +217,11 @@ attn_extend_wide_kernel(const ExtendParams p) {
         }
         __syncwarp();
       };
-      tc::mbar_wait_bounded(bar_q, 0, dead);
-      wait_unit(0);
-      for (int t = 0; t < tiles; ++t) issue_qk(t, 0, t == tiles - 1);
+      if (n_kv > 0) {
+        tc::mbar_wait_bounded(bar_q, 0, dead);
+        wait_unit(0);
+        for (int t = 0; t < tiles; ++t) issue_qk(t, 0, t == tiles - 1);
+      }
       for (int j = 0; j < n_kv; ++j) {
         const int s = (2 * j + 1) % SL;
         const uint64_t vdesc = tc::make_smem_desc_sw128(sbase + C::OFF_RING + s * C::TILE_BYTES, 1024, kWideTile * 128);
@@ -261,7 +274,7 @@ attn_extend_wide_kernel(const ExtendParams p) {
         tc::tmem_ld_wait();
         tc::tmem_ld32(tmem_s + 64, v[2]);
         tc::tmem_ld32(tmem_s + 96, v[3]);
-        const int k0 = j * kWideTile;
+        const int k0 = (j0 + j) * kWideTile;
         float a[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
         const bool edge = k0 + kWideTile - 1 > limit;
         if (!edge) {
@@ -332,47 +345,163 @@ attn_extend_wide_kernel(const ExtendParams p) {
         }
         l += (lsum[0].x + lsum[0].y) + (lsum[1].x + lsum[1].y);
       }
-      // ---- O / l -> out
-      tc::mbar_wait_bounded(bar_o(t), (n_kv - 1) & 1u, dead);
+      if (n_kv > 0) {
+        tc::mbar_wait_bounded(bar_o(t), (n_kv - 1) & 1u, dead);
+        if (S > 1) tc::mbar_wait_bounded(bar_o(tiles - 1), (n_kv - 1) & 1u, dead);  // the last reader of shared memory
+      }
       tc::tc_fence_after();
       __syncwarp();
-      const float inv_l = l > 0.f ? p.out_scale / l : 0.f;
-      T* orow = static_cast<T*>(p.o) + (q_row0 + (row_ok ? tok : 0)) * p.o_stride +
-                static_cast<int64_t>(head_base + r % p.pack) * D;
+      if (S > 1) {
+        // this rank's O, m, l of the row; the operand tiles are idle (every MMA that read them is complete)
+        const uint32_t row_at = sbase + (t * 128 + r) * C::PART_ROW;
 #pragma unroll 1
-      for (int cc = 0; cc < D / 32; ++cc) {
-        uint32_t o[32];
-        tc::tmem_ld32(tmem_o + cc * 32, o);
-        tc::tmem_ld_wait();
-        if (row_ok) {
+        for (int cc = 0; cc < D / 32; ++cc) {
+          uint32_t o[32];
+          if (n_kv > 0) {
+            tc::tmem_ld32(tmem_o + cc * 32, o);
+            tc::tmem_ld_wait();
+          } else {
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            uint32_t w[4];
+            for (int i = 0; i < 32; ++i) o[i] = 0u;
+          }
 #pragma unroll
-            for (int e = 0; e < 4; ++e)
-              w[e] = pack16<T>(__uint_as_float(o[i * 8 + 2 * e]) * inv_l, __uint_as_float(o[i * 8 + 2 * e + 1]) * inv_l);
-            *reinterpret_cast<uint4*>(orow + cc * 32 + i * 8) = make_uint4(w[0], w[1], w[2], w[3]);
+          for (int i = 0; i < 8; ++i)
+            asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};\n" ::"r"(row_at + (cc * 32 + i * 4) * 4), "r"(o[4 * i]),
+                         "r"(o[4 * i + 1]), "r"(o[4 * i + 2]), "r"(o[4 * i + 3])
+                         : "memory");
+        }
+        asm volatile("st.shared.v2.f32 [%0], {%1,%2};\n" ::"r"(row_at + D * 4), "f"(m), "f"(l) : "memory");
+      } else {
+        // ---- O / l -> out
+        const float inv_l = l > 0.f ? p.out_scale / l : 0.f;
+        T* orow = static_cast<T*>(p.o) + (q_row0 + (row_ok ? tok : 0)) * p.o_stride +
+                  static_cast<int64_t>(head_base + r % p.pack) * D;
+#pragma unroll 1
+        for (int cc = 0; cc < D / 32; ++cc) {
+          uint32_t o[32];
+          tc::tmem_ld32(tmem_o + cc * 32, o);
+          tc::tmem_ld_wait();
+          if (row_ok) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              uint32_t w[4];
+#pragma unroll
+              for (int e = 0; e < 4; ++e)
+                w[e] = pack16<T>(__uint_as_float(o[i * 8 + 2 * e]) * inv_l, __uint_as_float(o[i * 8 + 2 * e + 1]) * inv_l);
+              *reinterpret_cast<uint4*>(orow + cc * 32 + i * 8) = make_uint4(w[0], w[1], w[2], w[3]);
+            }
           }
         }
       }
     }
   }
 
+  if (S > 1) {
+    __syncwarp();
+    cluster_sync_all();                            // every rank's rows are in its shared memory
+    // rank r writes rows r, r + S, ..: a warp per row, four columns per lane, all ranks' pieces requested together
+    // (4-byte reads with a row in every second lane took 60 us of remote accesses for 256 rows of 8 ranks)
+    const int rows = tiles * 128 / S;              // S divides 128
+    for (int i = warp; i < rows; i += kWideThreads / 32) {
+      const int rr = i * S + rank, t = rr >> 7, r = rr & 127;
+      const int tok = tok0 + t * tok_per_tile + r / p.pack;
+      if (tok >= ext) continue;                    // uniform for the warp
+      const uint32_t row_at = sbase + rr * C::PART_ROW;
+      float x[8][4];
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (q < S && lane * 4 < D)
+          asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];\n"
+                       : "=f"(x[q][0]), "=f"(x[q][1]), "=f"(x[q][2]), "=f"(x[q][3])
+                       : "r"(map_to_rank(row_at + lane * 16, q))
+                       : "memory");
+      float mq = -INFINITY, lq = 0.f;
+      if (lane < S)
+        asm volatile("ld.shared::cluster.v2.f32 {%0,%1}, [%2];\n"
+                     : "=f"(mq), "=f"(lq) : "r"(map_to_rank(row_at + D * 4, lane)) : "memory");
+      float M = mq;
+#pragma unroll
+      for (int off = 4; off > 0; off >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, off));
+      M = __shfl_sync(0xffffffffu, M, 0);
+      const float wq = mq == -INFINITY ? 0.f : fast_exp2(mq - M);
+      float den = 0.f, acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        if (q >= S) break;
+        const float w = __shfl_sync(0xffffffffu, wq, q);
+        den = fmaf(w, __shfl_sync(0xffffffffu, lq, q), den);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[e] = fmaf(w, x[q][e], acc[e]);
+      }
+      const float inv = den > 0.f ? p.out_scale / den : 0.f;
+      if (lane * 4 < D)
+        *reinterpret_cast<uint2*>(static_cast<T*>(p.o) + (q_row0 + tok) * p.o_stride +
+                                  static_cast<int64_t>(head_base + r % p.pack) * D + lane * 4) =
+            make_uint2(pack16<T>(acc[0] * inv, acc[1] * inv), pack16<T>(acc[2] * inv, acc[3] * inv));
+    }
+    __syncwarp();
+    cluster_sync_all();                            // the peers have read this rank's rows
+  }
   tc::tc_fence_before();
   __syncthreads();
   if (warp == 8) tc::tmem_dealloc(tmem_base, 512);
 }
 
+// Clusters of S CTAs that are resident at once on the current device (0: none).
 template <typename T, int D>
-static int launch_extend_wide(const ExtendParams& p, int bs, int max_extend_len, cudaStream_t st) {
+static int wide_clusters(int S) {
+  static std::atomic<int> cached[64][9];
+  auto kern = attn_extend_wide_kernel<T, D, true>;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  int n = cached[dev][S].load(std::memory_order_relaxed);
+  if (n == 0) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(S * 8);
+    cfg.blockDim = dim3(kWideThreads);
+    cfg.dynamicSmemBytes = WideCfg<D>::SMEM_BYTES;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = S;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, WideCfg<D>::SMEM_BYTES) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) {
+      (void)cudaGetLastError();
+      n = -1;
+    }
+    cached[dev][S].store(n, std::memory_order_relaxed);
+  }
+  return n > 0 ? n : 0;
+}
+
+template <typename T, int D>
+static int launch_extend_wide(const ExtendParams& p_in, int bs, int max_extend_len, int max_kv_len, cudaStream_t st) {
   using C = WideCfg<D>;
-  auto kern = attn_extend_wide_kernel<T, D>;
-  B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
-  const dim3 grid(ceil_div(max_extend_len, 256 / p.pack), p.Hkv * p.head_tiles, bs);
-  note_variant("attn_extend_wide d=%d", D);
+  ExtendParams p = p_in;
+  B200_CUDA_OK(cudaFuncSetAttribute(attn_extend_wide_kernel<T, D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    C::SMEM_BYTES));
+  const int resident = device_sm_count();
+  const int64_t ctas = static_cast<int64_t>(ceil_div(max_extend_len, 256 / p.pack)) * p.Hkv * p.head_tiles * bs;
+  // The longest request's keys are cut while whole clusters still fit the idle SMs and a CTA keeps three key tiles
+  // (~1.8 us each; launch and merge of a cluster cost ~3).  us, one CTA -> split:
+  // 64 tokens behind 8192, two kv heads 117 -> 36; 128 behind 4000, eight 68 -> 36; 30 behind 2000 47 -> 22.
+  p.kv_splits = 1;
+  for (int S = 8; S > 1 && ctas < resident; S /= 2)   // (the occupancy answer also raises the shared memory limit)
+    if (max_kv_len >= 3 * S * kWideTile && wide_clusters<T, D>(S) >= ctas) {
+      p.kv_splits = S;
+      break;
+    }
+  const dim3 grid(ceil_div(max_extend_len, 256 / p.pack) * p.kv_splits, p.Hkv * p.head_tiles, bs);
+  note_variant("attn_extend_wide d=%d splits=%d", D, p.kv_splits);
   {
     ScopedKernelTimer timer("attn_extend", st);
-    kern<<<grid, kWideThreads, C::SMEM_BYTES, st>>>(p);
+    if (p.kv_splits > 1)
+      B200_CUDA_OK(launch_kernel(attn_extend_wide_kernel<T, D, true>, grid, dim3(kWideThreads), C::SMEM_BYTES, st, p.kv_splits, 0, p));
+    else
+      B200_CUDA_OK(launch_kernel(attn_extend_wide_kernel<T, D, false>, grid, dim3(kWideThreads), C::SMEM_BYTES, st, 1, 0, p));
   }
   B200_CHECK_LAUNCH("attn_extend_wide_kernel");
   return 0;

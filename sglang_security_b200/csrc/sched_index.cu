@@ -133,9 +133,28 @@ compute_position_kernel(int64_t* __restrict__ positions, int32_t* __restrict__ e
   if (threadIdx.x == 0) extend_start_loc[b] = static_cast<int32_t>(start);
 }
 
+__global__ void __launch_bounds__(kIdxThreads)
+extend_starts_kernel(const int32_t* __restrict__ extend_seq_lens, int32_t* __restrict__ extend_start_loc) {
+  griddep_wait();
+  griddep_launch_dependents();
+  const int b = blockIdx.x;
+  const int64_t start = cta_prefix_sum(b, [&](int i) { return static_cast<int64_t>(extend_seq_lens[i]); });
+  if (threadIdx.x == 0) extend_start_loc[b] = static_cast<int32_t>(start);
+}
+
 }  // namespace b200
 
 extern "C" {
+
+int b200_extend_starts(const int32_t* extend_seq_lens, int32_t* extend_start_loc, int bs, void* stream) {
+  using namespace b200;
+  if (bs == 0) return 0;
+  B200_REQUIRE(extend_seq_lens && extend_start_loc && bs > 0, "b200_extend_starts: bad arguments");
+  B200_CUDA_OK(launch_kernel(extend_starts_kernel, dim3(bs), dim3(kIdxThreads), 0, static_cast<cudaStream_t>(stream), 1,
+                             pdl_family(bs, kPdlOther), extend_seq_lens, extend_start_loc));
+  B200_CHECK_LAUNCH("extend_starts_kernel");
+  return 0;
+}
 
 int b200_write_req_to_token(int32_t* req_to_token, int64_t req_to_token_stride,
                             const int64_t* req_pool_indices, const int64_t* pre_lens,

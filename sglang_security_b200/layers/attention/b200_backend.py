@@ -35,6 +35,7 @@ class ForwardMetadata:
     # extend only
     qo_indptr: Optional[torch.Tensor] = None
     max_extend_len: int = 0
+    max_kv_len: int = 0          # longest prefix + new tokens, 0 when the host does not know it
     total_extend: int = 0
     # dtype-converted copies of the ForwardBatch index tensors, kept alive for the whole forward
     # (one conversion per step, never a temporary whose block the allocator could hand out again
@@ -135,7 +136,11 @@ class B200AttnBackend(AttentionBackend):
         (forward_batch_info.py:348-369); the fallbacks mirror triton_backend.py:393-431."""
         ext = forward_batch.extend_seq_lens
         start = forward_batch.extend_start_loc
-        if start is None:
+        if start is None and ext.is_cuda and ext.dtype == torch.int32 and ext.is_contiguous():
+            start = torch.empty_like(ext)
+            _lib.check(self.lib.b200_extend_starts(ext.data_ptr(), start.data_ptr(), ext.numel(),
+                                                   _lib.current_stream()), "b200_extend_starts")
+        elif start is None:
             start = torch.zeros_like(ext)
             start[1:] = torch.cumsum(ext[:-1], dim=0)
         if forward_batch.extend_seq_lens_cpu is not None:
@@ -144,7 +149,11 @@ class B200AttnBackend(AttentionBackend):
         else:
             max_len = int(ext.max().item()) if ext.numel() else 0
             total = int(ext.sum().item()) if ext.numel() else 0
-        return ForwardMetadata(qo_indptr=start.to(torch.int32), max_extend_len=int(max_len),
+        max_kv = 0
+        if forward_batch.extend_seq_lens_cpu is not None and forward_batch.extend_prefix_lens_cpu is not None:
+            max_kv = max((p + e for p, e in zip(forward_batch.extend_prefix_lens_cpu,
+                                                forward_batch.extend_seq_lens_cpu)), default=0)
+        return ForwardMetadata(qo_indptr=start.to(torch.int32), max_extend_len=int(max_len), max_kv_len=int(max_kv),
                                total_extend=int(total))
 
     # ------------------------------------------------------------------ CUDA graph hooks
@@ -350,12 +359,12 @@ class B200AttnBackend(AttentionBackend):
             raise _lib.B200Error(
                 f"B200AttnBackend.forward_extend: KV cache dtype {k_cache.dtype} != q dtype "
                 f"{q.dtype} (supported pools: the activation dtype, float8_e4m3fn or float8_e5m2)")
-        rc = self.lib.b200_attn_extend_scaled(
+        rc = self.lib.b200_attn_extend_known(
             q.data_ptr(), q.stride(0), k_cache.data_ptr(), v_cache.data_ptr(), k_cache.stride(0),
             o.data_ptr(), o.stride(0), req_to_token.data_ptr(), req_to_token.stride(0),
             req_pool_indices.data_ptr(), seq_lens.data_ptr(),
             prefix_lens.data_ptr(), extend_lens.data_ptr(), md.qo_indptr.data_ptr(), bs,
-            md.max_extend_len, hq, hkv, d, dv, scaling, float(layer.logit_cap or 0.0), out_scale,
+            md.max_extend_len, md.max_kv_len, hq, hkv, d, dv, scaling, float(layer.logit_cap or 0.0), out_scale,
             1 if causal else 0, _lib.dtype_code(q.dtype), _lib.current_stream())
         _lib.check(rc, "b200_attn_extend")
         return o

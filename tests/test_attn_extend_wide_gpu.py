@@ -35,8 +35,24 @@ def test_tile_edges(hq, hkv, d, dtype):
     pack = next(p for p in (8, 4, 2, 1) if (hq // hkv) % p == 0)
     rows = 128 // pack                                   # tokens of a query tile
     ext = [1, rows - 1, rows, rows + 1, 2 * rows, 2 * rows + 1, 5, 1]
-    total = [1, 127, 128 + rows, 129 + rows, 2 * rows, 512 + 2 * rows, 1285, 641]
+    total = [1, 127, 128 + rows, 129 + rows, 2 * rows, 512 + 2 * rows, 1285, 641]   # 1285: the batch takes this kernel
     _run(scenarios.make_attention_case(seed=hq * 100 + d, hq=hq, hkv=hkv, d=d, seq_lens=total, extend_lens=ext, dtype=dtype))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("hq,hkv,d,seq,ext,splits", [
+    (4, 1, 128, [3300], [40], 8),                     # one query tile, eight ranks
+    (4, 1, 128, [3300, 200, 1], [64, 64, 1], 8),      # ranks without keys beside full ones
+    (8, 1, 128, [1700, 900], [32, 20], 4),
+    (7, 1, 64, [3073], [129], 8),                     # two query tiles, a rank with one key more
+    (4, 1, 128, [1290], [90], 2),
+])
+def test_keys_spread_over_clusters(hq, hkv, d, seq, ext, splits, dtype):
+    from sglang_security_b200 import _lib
+
+    case = scenarios.make_attention_case(seed=sum(seq) + d, hq=hq, hkv=hkv, d=d, seq_lens=seq, extend_lens=ext, dtype=dtype)
+    _run(case)
+    assert f"splits={splits}" in _lib.last_variant(), _lib.last_variant()
 
 
 @pytest.mark.parametrize("d", [64, 128])
