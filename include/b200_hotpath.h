@@ -379,6 +379,13 @@ int b200_w4a16_gemv(const void* x, int64_t ldx, const void* qweight, const void*
                     int K, int group_size, int dtype, void* stream);
 int b200_w4a16_gemv_config(int max_m, int splits);
 
+/* Prefill sizes with the stream copy (b200_w4a16_gemv_v2_repack): expands the weight into `workspace` (16-bit [N, K])
+ * and runs the CTA-pair GEMM.  N % 16 == 0, K % 64 == 0, group_size % 8 == 0. */
+size_t b200_w4a16_gemm_stream_workspace_bytes(int N, int K);
+int b200_w4a16_gemm_stream(const void* x, int64_t ldx, const void* qweight_stream, const void* zeros, const void* scales,
+                           const void* bias, void* out, int64_t ldc, int M, int N, int K, int group_size,
+                           void* workspace, size_t workspace_bytes, int dtype, void* stream);
+
 /* Decode-regime GEMV, second generation (csrc/w4a16_gemv2.cu): the same arithmetic as
  * b200_w4a16_gemv on a one-time STREAM repack of the packed weight — tiles of 16 output columns x
  * 64 k, 512 contiguous bytes, ordered [n / 16][k / 64], each lane's 16 bytes being its mma.sync A

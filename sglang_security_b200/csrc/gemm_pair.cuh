@@ -445,9 +445,10 @@ int pair_clusters(int S) {
   return n > 0 ? n : 0;
 }
 
+// old_weight: no kernel still in flight on the stream writes w (its first tiles are read before the dependency wait).
 template <int KIND, typename OutT, bool ACT = false>
 int launch_gemm_pair(const void* x, int64_t ldx, const void* w, int64_t ldw, const GemmEpilogueParams& ep,
-                     cudaStream_t st, const char* timer_name) {
+                     cudaStream_t st, const char* timer_name, bool old_weight = true) {
   constexpr int ELT = GemmKindTraits<KIND>::ELT;
   int clusters_of[kPairMaxSplits + 1] = {0};
   for (int s = 1; s <= kPairMaxSplits; ++s) clusters_of[s] = pair_clusters<KIND, OutT, ACT>(s);
@@ -485,7 +486,7 @@ int launch_gemm_pair(const void* x, int64_t ldx, const void* w, int64_t ldw, con
   {
     ScopedKernelTimer timer(timer_name, st);
     B200_CUDA_OK(launch_kernel(gemm_pair_kernel<KIND, OutT, ACT>, dim3(clusters * 2 * plan.splits), dim3(kPairThreads),
-                               plan.smem, st, 2 * plan.splits, kPdlGemmBig, tw, tx, p));
+                               plan.smem, st, 2 * plan.splits, old_weight ? kPdlGemmBig : 0, tw, tx, p));
   }
   B200_CHECK_LAUNCH("gemm_pair_kernel");
   return 0;

@@ -116,6 +116,29 @@ def w4a16_gemv_v2(x: torch.Tensor, qweight_stream: torch.Tensor, zeros: torch.Te
     return out
 
 
+def w4a16_gemm_stream(x: torch.Tensor, qweight_stream: torch.Tensor, zeros: torch.Tensor, scales: torch.Tensor,
+                      group_size: int, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """x [M, K] @ dequant(stream-layout weight) (+ bias) -> [M, N] in two passes: the weight is expanded to a 16-bit
+    [N, K] scratch tensor, then multiplied by the CTA-pair GEMM (csrc/w4a16_stream_gemm.cu)."""
+    _cuda(x, "w4a16_gemm_stream")
+    if x.dim() != 2 or x.stride(-1) != 1:
+        raise _lib.B200Error("w4a16_gemm_stream: x must be 2-D with contiguous rows")
+    m, k = x.shape
+    n = scales.shape[1]
+    if qweight_stream.numel() * 8 != k * n or scales.dtype != x.dtype or zeros.dtype != x.dtype:
+        raise _lib.B200Error("w4a16_gemm_stream: shape / dtype mismatch between x and the packed weight")
+    out = torch.empty((m, n), device=x.device, dtype=x.dtype)
+    if bias is not None and bias.dtype != x.dtype:
+        bias = bias.to(x.dtype)
+    ws = torch.empty(n * k, device=x.device, dtype=x.dtype)
+    rc = _lib.load().b200_w4a16_gemm_stream(x.data_ptr(), x.stride(0), qweight_stream.data_ptr(), zeros.data_ptr(),
+                                            scales.data_ptr(), _lib.ptr(bias), out.data_ptr(), out.stride(0), m, n, k,
+                                            group_size, ws.data_ptr(), ws.numel() * ws.element_size(),
+                                            _lib.dtype_code(x.dtype), _lib.current_stream())
+    _lib.check(rc, "b200_w4a16_gemm_stream")
+    return out
+
+
 def w4a16_gemv_v2_config(splits: int = 0) -> None:
     _lib.check(_lib.load().b200_w4a16_gemv_v2_config(int(splits)), "b200_w4a16_gemv_v2_config")
 
@@ -125,18 +148,30 @@ def w4a16_gemv_v2_config(splits: int = 0) -> None:
 GEMV_V2_MAX_M = int(os.environ.get("B200_W4A16_GEMV2_MAX_M", "16"))
 
 
+def stream_gemm_pays(m: int, n: int) -> bool:
+    """Expansion + GEMM against the fused kernel (us, Qwen2.5-32B at TP 2, fused / two passes): the expansion is spread
+    over enough tokens from 1500 on (gate_up 1500: 354 / 350, 2048: 466 / 425, 3001: 727 / 609; 1024: 235 / 248), and
+    narrow weights leave the fused kernel's tiles too few (777 tokens, qkv / o / down: 38.5 / 31.0, 41.8 / 27.1,
+    173 / 125)."""
+    return m >= 1500 or (m > 512 and n <= 8192)
+
+
 def stream_copy_enabled() -> bool:
     return os.environ.get("B200_W4A16_STREAM_COPY", "1") != "0"
 
 
 def w4a16_linear(x2: torch.Tensor, layer, bias: Optional[torch.Tensor]) -> torch.Tensor:
     """Dispatch of AWQ/GPTQ apply(): decode batches (M <= 16) stream the repacked weight through
-    the GEMV, everything else runs the fused dequant + tcgen05 GEMM on the [K, N/8] layout."""
+    the GEMV, large ones expand it once for the CTA-pair GEMM, everything else runs the fused dequant +
+    tcgen05 GEMM on the [K, N/8] layout."""
     stream = getattr(layer, "b200_qweight_stream", None)
     m = x2.shape[0]
     if stream is not None and 1 <= m <= GEMV_V2_MAX_M and gemv_v2_supported(
             m, layer.scales.shape[1], x2.shape[1], layer.w4a16_group_size):
         return w4a16_gemv_v2(x2, stream, layer.b200_zeros, layer.scales, layer.w4a16_group_size, bias)
+    if (stream is not None and stream_gemm_pays(m, layer.scales.shape[1]) and layer.w4a16_group_size % 8 == 0
+            and x2.stride(0) % 8 == 0 and x2.data_ptr() % 16 == 0):
+        return w4a16_gemm_stream(x2, stream, layer.b200_zeros, layer.scales, layer.w4a16_group_size, bias)
     packed = layer.b200_qweight if hasattr(layer, "b200_qweight") else layer.qweight  # GPTQ / AWQ
     return w4a16_gemm(x2, packed, layer.b200_zeros, layer.scales, layer.w4a16_group_size, bias)
 
