@@ -571,7 +571,21 @@ attn_decode_mma_kernel(const DecodeParams p) {
 constexpr int kMergeWarps = 4;
 constexpr int kMergeAhead = 8;
 
-template <typename T>
+// V columns per lane: 4, or 1 for rows that 16-byte loads do not fit
+template <int V>
+__device__ __forceinline__ void merge_load(float (&x)[V], const float* p) {
+  if constexpr (V == 4) {
+    const float4 f = __ldcg(reinterpret_cast<const float4*>(p));
+    x[0] = f.x;
+    x[1] = f.y;
+    x[2] = f.z;
+    x[3] = f.w;
+  } else {
+    x[0] = __ldcg(p);
+  }
+}
+
+template <typename T, int V>
 __global__ void __launch_bounds__(kMergeWarps * 32)
 attn_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_lse, T* __restrict__ o,
                   int64_t o_stride, const int64_t* __restrict__ seq_lens, int Hq, int Dv, int num_splits, int align,
@@ -584,12 +598,11 @@ attn_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ pa
   const int64_t base = (static_cast<int64_t>(b) * Hq + hq) * num_splits;
   const float* po = part_o + base * Dv;
   // splits past the sequence are allocated but hold nothing: their values are not used
-  float4 x[kMergeAhead];
-  const int d0 = lane * 4;
+  float x[kMergeAhead][V];
+  const int d0 = lane * V;
 #pragma unroll
   for (int i = 0; i < kMergeAhead; ++i)
-    x[i] = i < num_splits && d0 < Dv ? __ldcg(reinterpret_cast<const float4*>(po + static_cast<int64_t>(i) * Dv + d0))
-                                     : make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i < num_splits && d0 < Dv) merge_load<V>(x[i], po + static_cast<int64_t>(i) * Dv + d0);
   const float lse0 = lane < num_splits ? __ldcg(part_lse + base + lane) : 0.f;
   const int len = static_cast<int>(seq_lens[b]);
   if (len <= 0) return;
@@ -599,10 +612,11 @@ attn_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ pa
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, off));
   const int64_t row = row_list ? row_list[b] : b;
-  for (int dd = 0; dd < Dv; dd += 128) {
+  for (int dd = 0; dd < Dv; dd += 32 * V) {
     const int d = dd + d0;
-    float den = 0.f;
-    float4 num = make_float4(0.f, 0.f, 0.f, 0.f);
+    float den = 0.f, num[V];
+#pragma unroll
+    for (int e = 0; e < V; ++e) num[e] = 0.f;
     for (int s0 = 0; s0 < nvalid; s0 += 32) {
       const float lse = s0 == 0 ? lse0 : (s0 + lane < nvalid ? __ldcg(part_lse + base + s0 + lane) : 0.f);
       const float w_lane = s0 + lane < nvalid ? fast_exp2(lse - M) : 0.f;
@@ -610,34 +624,28 @@ attn_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ pa
         if (s1 > 0 || dd > 0) {
 #pragma unroll
           for (int i = 0; i < kMergeAhead; ++i)
-            if (s1 + i < nvalid && d < Dv)
-              x[i] = __ldcg(reinterpret_cast<const float4*>(po + static_cast<int64_t>(s1 + i) * Dv + d));
+            if (s1 + i < nvalid && d < Dv) merge_load<V>(x[i], po + static_cast<int64_t>(s1 + i) * Dv + d);
         }
 #pragma unroll
         for (int i = 0; i < kMergeAhead; ++i) {
           const float w = __shfl_sync(0xffffffffu, w_lane, (s1 + i) & 31);
           if (s1 + i < nvalid) {
             den += w;
-            num.x += w * x[i].x;
-            num.y += w * x[i].y;
-            num.z += w * x[i].z;
-            num.w += w * x[i].w;
+#pragma unroll
+            for (int e = 0; e < V; ++e) num[e] += w * x[i][e];
           }
         }
       }
     }
     if (d >= Dv) continue;
     const float inv = 1.f / den;
-    float y[4] = {num.x * inv, num.y * inv, num.z * inv, num.w * inv};
-    if (gate) {
-#pragma unroll
-      for (int e = 0; e < 4; ++e)
-        if (d + e < Dv) y[e] *= sigmoid_f(to_float<T>(gate[row * gate_stride + hq * Dv + d + e]));
-    }
     T* dst = o + row * o_stride + hq * Dv + d;
 #pragma unroll
-    for (int e = 0; e < 4; ++e)
-      if (d + e < Dv) dst[e] = from_float<T>(y[e]);
+    for (int e = 0; e < V; ++e) {
+      float y = num[e] * inv;
+      if (gate) y *= sigmoid_f(to_float<T>(gate[row * gate_stride + hq * Dv + d + e]));
+      dst[e] = from_float<T>(y);
+    }
   }
 }
 
@@ -1022,20 +1030,23 @@ static int attn_merge_impl(const float* part_o, const float* part_lse, void* o, 
                num_splits, split_align);
   B200_REQUIRE(part_o && part_lse && o && seq_lens, "b200_attn_merge: null pointer");
   B200_REQUIRE(dtype == B200_BF16 || dtype == B200_F16, "b200_attn_merge: dtype %d", dtype);
-  B200_REQUIRE(Dv % 4 == 0, "b200_attn_merge: value dim %d", Dv);
   dim3 grid(ceil_div(Hq, kMergeWarps), bs);
   const int threads = kMergeWarps * 32;
+  const bool wide = Dv % 4 == 0 && aligned16(part_o);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   ScopedKernelTimer timer("attn_merge", st);
-  if (dtype == B200_BF16)
-    B200_CUDA_OK(launch_kernel(attn_merge_kernel<__nv_bfloat16>, grid, dim3(threads), 0, st, 1, pdl_family(bs, kPdlMerge),
-                               part_o, part_lse, static_cast<__nv_bfloat16*>(o), o_stride, seq_lens,
-                               Hq, Dv, num_splits, align, row_list, static_cast<const __nv_bfloat16*>(gate),
-                               gate_stride));
-  else
-    B200_CUDA_OK(launch_kernel(attn_merge_kernel<__half>, grid, dim3(threads), 0, st, 1, pdl_family(bs, kPdlMerge), part_o,
-                               part_lse, static_cast<__half*>(o), o_stride, seq_lens, Hq, Dv,
-                               num_splits, align, row_list, static_cast<const __half*>(gate), gate_stride));
+#define LAUNCH_MERGE(T, V)                                                                                            \
+  B200_CUDA_OK(launch_kernel(attn_merge_kernel<T, V>, grid, dim3(threads), 0, st, 1, pdl_family(bs, kPdlMerge), part_o, \
+                             part_lse, static_cast<T*>(o), o_stride, seq_lens, Hq, Dv, num_splits, align, row_list,   \
+                             static_cast<const T*>(gate), gate_stride))
+  if (dtype == B200_BF16) {
+    if (wide) LAUNCH_MERGE(__nv_bfloat16, 4);
+    else LAUNCH_MERGE(__nv_bfloat16, 1);
+  } else {
+    if (wide) LAUNCH_MERGE(__half, 4);
+    else LAUNCH_MERGE(__half, 1);
+  }
+#undef LAUNCH_MERGE
   B200_CHECK_LAUNCH("attn_merge_kernel");
   return 0;
 }
