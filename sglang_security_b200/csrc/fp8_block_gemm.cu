@@ -10,7 +10,7 @@
 // "promote" it into fp32 registers with one packed FMA per element pair:
 //   acc[m, :] += (As[m,kb] * Bs[nb,kb]) * partial[m, :]
 // (a warpgroup owns 128 columns = one weight scale block, so the combined scale is a per-thread scalar) while
-// the MMA warp already works on the next K blocks.  Same TMA / mbarrier ring as gemm_tc.cuh.
+// the MMA warp already works on the next K blocks.  TMA / mbarrier ring and issue loops as in gemm_pair.cuh.
 #include "fp8_gemm_smallm.cuh"
 
 namespace b200 {

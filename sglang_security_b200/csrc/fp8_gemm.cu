@@ -219,14 +219,12 @@ static int fp8_gemm_rowcol_impl(const void* a, int64_t lda, const void* b, int64
   ep.N = N;
   ep.K = K;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // Decode regime: weight streaming, swap-AB + cluster split-K.  Measured crossover against the
-  // big-tile kernel with cluster split-K (profiles/r01_bench_gemm_midm_splitk.json): the swap-AB
-  // kernel wins up to M = 32; from M = 33 the 128x128 tile split over K is faster on every
-  // Llama-3.1-8B shape (10.8 vs 15.4-20.6 us at N = K = 4096, 17.2 vs 21.7-27 us at K = 14336).
+  // Decode regime: weight streaming, swap-AB + cluster split-K, two CTAs per SM.  Against the CTA-pair kernel (us, qkv /
+  // o / gate_up / down of Llama-3.1-8B): this one at 32 tokens 8.3 / 7.3 / 19.8 / 12.7, the pair kernel at 64 tokens 8.9 /
+  // 8.2 / - / 15.1, where this one's accumulators halve the CTAs per SM.
   const bool fuse_ar = comm_can_fuse(comm, M, N);
-  // Exception (profiles/r01_bench_gemm_midm_swap.json): a weight with more 128-row tiles than SMs
-  // (gate_up 28672x4096) cannot be split and runs the big tiles in two uneven waves; there the
-  // swap-AB kernel stays ahead up to M = 64 (27.4 vs 31.5 us at M = 48, 29.1 vs 31.7 at M = 64).
+  // A weight with more 128-row tiles than SMs (gate_up 28672x4096) streams best here up to 64 tokens: 21.8 us at 64,
+  // the pair kernel 23.5 at 128.
   const bool wide = ceil_div(N, 128) > device_sm_count();
   if (fuse_ar || (M <= smallm_max_m() && (M <= 32 || (wide && M <= 64) || smallm_forced()))) {
     SmallMParams sp = {};

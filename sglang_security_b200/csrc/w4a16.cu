@@ -21,7 +21,7 @@
 //   w4a16_gemm_kernel       : fused tcgen05 GEMM — x tiles by TMA (K-major A operand), weight tiles
 //                             dequantised in registers by 4 warps straight into 128-byte-swizzled
 //                             shared memory as an MN-major B operand; TMEM accumulators; same
-//                             mbarrier rings as gemm_tc.cuh.
+//                             mbarrier rings as gemm_pair.cuh.
 #include <cstdlib>
 #include <type_traits>
 
