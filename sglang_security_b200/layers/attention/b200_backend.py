@@ -123,7 +123,7 @@ class B200AttnBackend(AttentionBackend):
             total = forward_batch.seq_lens_sum or bs * self.max_context_len
             head_dim = self.v_head_dim
             lens = getattr(forward_batch, "seq_lens_cpu", None)   # host copy, where the scheduler keeps one
-            longest = int(lens.max()) if lens is not None and lens.numel() else 0
+            longest = int(lens.max()) if torch.is_tensor(lens) and not lens.is_cuda and lens.numel() else 0
             s = self._num_splits(bs, head_dim, max(1, total // bs), longest)
             self.forward_metadata = ForwardMetadata(num_splits=s,
                                                     workspace=self._ensure_workspace(bs, s))

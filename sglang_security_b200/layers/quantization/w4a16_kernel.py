@@ -171,7 +171,10 @@ def w4a16_linear(x2: torch.Tensor, layer, bias: Optional[torch.Tensor]) -> torch
         return w4a16_gemv_v2(x2, stream, layer.b200_zeros, layer.scales, layer.w4a16_group_size, bias)
     if (stream is not None and stream_gemm_pays(m, layer.scales.shape[1]) and layer.w4a16_group_size % 8 == 0
             and x2.stride(0) % 8 == 0 and x2.data_ptr() % 16 == 0):
-        return w4a16_gemm_stream(x2, stream, layer.b200_zeros, layer.scales, layer.w4a16_group_size, bias)
+        try:
+            return w4a16_gemm_stream(x2, stream, layer.b200_zeros, layer.scales, layer.w4a16_group_size, bias)
+        except torch.cuda.OutOfMemoryError:
+            pass    # no room for the expanded weight: the fused kernel needs none
     packed = layer.b200_qweight if hasattr(layer, "b200_qweight") else layer.qweight  # GPTQ / AWQ
     return w4a16_gemm(x2, packed, layer.b200_zeros, layer.scales, layer.w4a16_group_size, bias)
 

@@ -61,3 +61,25 @@ def test_layer_dispatch(m, two_pass):
     wide = torch.randn(m, k + 4, device="cuda", generator=g).to(dtype)[:, :k]     # rows the copies cannot start on
     out, _ = layer(wide.contiguous())
     _check(out, wide, OI.awq_dequantize_oracle(q, s, z, 128), None)
+
+
+def test_no_room_for_the_expanded_weight(monkeypatch):
+    """The layer still runs, on the fused kernel, where the scratch tensor cannot be had."""
+    from sglang_security_b200 import _lib
+    from sglang_security_b200.layers.quantization import w4a16_kernel as W
+
+    k, n, m, dtype = 512, 1024, 1500, torch.float16
+    q, z, s, g = _packed(k, n, 128, dtype, 5)
+    layer = torch.nn.Module()
+    layer.qweight, layer.scales, layer.w4a16_group_size = q, s, 128
+    layer.b200_zeros = W.unpack_zeros(z, dtype, awq_order=True, add_one=False)
+    layer.b200_qweight_stream = W.gemv_stream_repack(q)
+    x = torch.randn(m, k, device="cuda", generator=g).to(dtype)
+
+    def refuse(*a, **kw):
+        raise torch.cuda.OutOfMemoryError("no room")
+
+    monkeypatch.setattr(W, "w4a16_gemm_stream", refuse)
+    out = W.w4a16_linear(x, layer, None)
+    assert not _lib.last_variant().endswith("expanded")
+    _check(out, x, OI.awq_dequantize_oracle(q, s, z, 128), None)
