@@ -995,7 +995,8 @@ static int decode_num_splits(int bs, int Hkv, int group, int D, int64_t avg_len,
   // Few splits of unequal requests: the longest ones would run alone at the end, so twice the slots are filled
   // (us, one wave or 1.5 -> 2.1 times the slots: 40 x up to 3000 tokens 61.3 -> 57.9, 64 x up to 4096 FP8 77.0 -> 69.3,
   // 27 x up to 6000 FP8 50.4 -> 48.2).
-  const bool ragged = max_len * 8 > avg_len * 9 && by_slots < 4;
+  // Not for short requests, where the smaller splits' merge costs more than the even end gives.
+  const bool ragged = max_len * 8 > avg_len * 9 && by_slots < 4 && avg_len >= 1536;
   if (!ragged && fit >= 1 && (fit < by_slots || static_cast<double>(base * fit) >= 0.85 * static_cast<double>(slots)))
     return static_cast<int>(fit);
   // HBM-bound: what matters is that enough CTAs stay resident until the end, not whole waves — late CTAs run faster
