@@ -157,9 +157,12 @@ fp8_quant_row_kernel(const T* __restrict__ x, int64_t ldx, uint8_t* __restrict__
 // aligned (s_row = 1, s_col = padded M).
 // x / scale is a true division.  With r = 1 / scale rounded to nearest, q = x r and one remainder step
 // q + (x - q scale) r give the rounded quotient (Markstein 1990) up to halfway cases; that the e4m3 byte is the
-// division's for every significand of x and of the maximum is checked exhaustively by the tests.  The compiler's
-// division and one load in flight per lane bound the kernel: 3001 x 14336 bf16 took 46.5 us, now 32.5, of 20 us
+// division's for every significand of x and of the maximum is checked exhaustively by the tests.  That holds while
+// the remainder is exact: a quotient that is not rounded to zero is at least 2^-11, so its product with the scale is
+// a multiple of 2^-57 scale, which fp32 holds from a scale of 2^-92 on.  Smaller scales (a caller's eps; below 3e-39
+// their reciprocal is infinite) and infinite ones are divided by.  The compiler's division and one load in flight per lane bound the kernel: 3001 x 14336 bf16 took 46.5 us, now 32.5, of 20 us
 // of HBM time; 2048 x 4096 10.9, now 8.8.
+constexpr float kReciprocalMin = 0x1p-90f;
 template <typename T, int GPT>
 __global__ void __launch_bounds__(256)
 fp8_quant_group128_kernel(const T* __restrict__ x, int64_t ldx, uint8_t* __restrict__ q,
@@ -196,7 +199,7 @@ fp8_quant_group128_kernel(const T* __restrict__ x, int64_t ldx, uint8_t* __restr
     if (m[i] < 0) continue;
     const float s = amax / kFp8Max;
     if (lane == 0) scales[m[i] * s_row + g[i] * s_col] = s;
-    if (s < INFINITY) {
+    if (s >= kReciprocalMin && s < INFINITY) {
       const float r = 1.0f / s;
 #pragma unroll
       for (int e = 0; e < 4; ++e) {

@@ -17,11 +17,11 @@ def _group_ref(x, eps=1e-10):
     return y.to(FP8).view(x.shape), s.squeeze(-1)
 
 
-def _same(x):
+def _same(x, eps=1e-10):
     from sglang_security_b200.layers.quantization.fp8_kernel import per_token_group_quant_fp8
 
-    q, s = per_token_group_quant_fp8(x, 128)
-    rq, rs = _group_ref(x)
+    q, s = per_token_group_quant_fp8(x, 128, eps)
+    rq, rs = _group_ref(x, eps)
     assert torch.equal(s, rs)
     assert torch.equal(q.view(torch.uint8), rq.view(torch.uint8))
 
@@ -54,6 +54,31 @@ def test_group_special_values_and_sizes():
     x[1, 5], x[2, 200], x[3, 7] = float("inf"), float("-inf"), float("nan")
     x[4] *= 1e-6
     _same(x)
+
+
+@pytest.mark.parametrize("eps", [0.0, 1e-45, 1e-38, 1e-36, 2.0 ** -81, 1e-10])
+def test_group_small_scales(eps):
+    """Any eps is the caller's choice: scales down to the smallest subnormal (their reciprocal overflows), around the
+    line from which on they are divided by, and groups whose scale is eps itself."""
+    sig = 1.0 + torch.arange(128, device="cuda", dtype=torch.float32) / 128
+    for top in (-132, -128, -121, -118, -100, -84, -83, -82, -81, -40, 0, 30, 120):
+        peak = sig[torch.arange(0, 128, 5, device="cuda")] * 2.0 ** top
+        rows = torch.cat([sig * 2.0 ** (top - e) for e in range(10)])
+        rows = torch.minimum(rows.expand(len(peak), -1), peak[:, None])
+        rows = torch.nn.functional.pad(rows, (0, (-rows.shape[1]) % 127)).view(len(peak), -1, 127)
+        x = torch.cat([peak[:, None, None].expand(-1, rows.shape[1], 1), rows], -1).reshape(len(peak), -1).to(torch.bfloat16)
+        _same(x, eps)
+        _same(-x, eps)
+
+
+def test_group_scale_from_eps_exhaustively():
+    """Every bf16 value up to eps, of either sign, in groups whose maximum does not reach eps."""
+    for eps in (1e-10, 3e-7, 1.7e-20):
+        bits = torch.arange(0, 0x7f80, device="cuda", dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+        x = bits[bits.float() <= eps]
+        x = torch.cat([x, x.new_zeros((-x.numel()) % 128)]).view(-1, 128)
+        _same(x, eps)
+        _same(-x, eps)
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
