@@ -445,7 +445,8 @@ int pair_clusters(int S) {
   return n > 0 ? n : 0;
 }
 
-// old_weight: no kernel still in flight on the stream writes w (its first tiles are read before the dependency wait).
+// old_weight: the launch just before this one does not write w, whose first tiles are read before the dependency wait
+// where the launch is a dependent one (pdl_family: up to 512 tokens).
 template <int KIND, typename OutT, bool ACT = false>
 int launch_gemm_pair(const void* x, int64_t ldx, const void* w, int64_t ldw, const GemmEpilogueParams& ep,
                      cudaStream_t st, const char* timer_name, bool old_weight = true) {
@@ -486,7 +487,8 @@ int launch_gemm_pair(const void* x, int64_t ldx, const void* w, int64_t ldw, con
   {
     ScopedKernelTimer timer(timer_name, st);
     B200_CUDA_OK(launch_kernel(gemm_pair_kernel<KIND, OutT, ACT>, dim3(clusters * 2 * plan.splits), dim3(kPairThreads),
-                               plan.smem, st, 2 * plan.splits, old_weight ? kPdlGemmBig : 0, tw, tx, p));
+                               plan.smem, st, 2 * plan.splits, old_weight ? pdl_family(ep.M, kPdlGemmBig) : 0, tw, tx,
+                               p));
   }
   B200_CHECK_LAUNCH("gemm_pair_kernel");
   return 0;

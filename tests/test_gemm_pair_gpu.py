@@ -77,3 +77,21 @@ def test_repeatable_with_split_k():
     assert "splits=1" not in _lib.last_variant()
     for _ in range(5):
         assert torch.equal(first, gemm_16bit(x, w))
+
+
+@pytest.mark.parametrize("m", [513, 600, 2048])
+def test_weight_written_by_the_launch_before(m):
+    """Above 512 tokens a GEMM waits for the launch before it: a weight quantised right before it is read whole."""
+    from sglang_security_b200.layers.quantization.fp8_kernel import fp8_scaled_mm, sglang_per_token_quant_fp8
+
+    n, k = 6144, 4096
+    g = torch.Generator(device="cuda").manual_seed(m)
+    x, sa = sglang_per_token_quant_fp8(torch.randn(m, k, device="cuda", generator=g).to(torch.bfloat16))
+    for i in range(8):
+        weight = torch.randn(n, k, device="cuda", generator=g).to(torch.bfloat16)
+        torch.cuda.synchronize()
+        w, sb = sglang_per_token_quant_fp8(weight)          # the allocator hands out the last round's bytes again
+        out = fp8_scaled_mm(x, w.t(), sa, sb, torch.bfloat16)
+        torch.cuda.synchronize()
+        assert torch.equal(out, fp8_scaled_mm(x, w.t(), sa, sb, torch.bfloat16)), i
+        del w, sb, out, weight
