@@ -236,45 +236,3 @@ class B200AllReduce:
                 self._nvls_buf, self.nvls = None, False
             self.free_shared_buffer()
             self.disabled = True
-
-
-class LocalCommGroup:
-    """`world` communicators that live in ONE process on ONE device (every "rank" is driven from
-    its own CUDA stream).  Test/bench harness for the protocol on a single-GPU box: the kernels
-    are exactly the ones the multi-process path launches, only the buffers are not IPC-mapped."""
-
-    def __init__(self, world: int, max_size: int = _MAX_CAR_SIZE, device="cuda"):
-        lib = _lib.load()
-        self.world = world
-        self.device = torch.device(device)
-        nbytes = int(lib.b200_comm_buffer_bytes(world, max_size))
-        self._bufs = [torch.zeros(nbytes, dtype=torch.uint8, device=self.device)
-                      for _ in range(world)]
-        arr = (ctypes.c_void_p * world)(*[b.data_ptr() for b in self._bufs])
-        self.comms = []
-        for r in range(world):
-            h = ctypes.c_void_p()
-            _lib.check(lib.b200_comm_create(r, world, arr, nbytes, ctypes.byref(h)),
-                       "b200_comm_create")
-            self.comms.append(_LocalComm(h, r, world))
-        self.streams = [torch.cuda.Stream(device=self.device) for _ in range(world)]
-        torch.cuda.synchronize(self.device)
-
-    def close(self):
-        torch.cuda.synchronize(self.device)
-        for c in self.comms:
-            _lib.load().b200_comm_destroy(c.handle)
-        self.comms = []
-
-
-class _LocalComm:
-    def __init__(self, handle, rank, world):
-        self.handle, self.rank, self.world_size, self.disabled = handle, rank, world, False
-
-    def all_reduce(self, inp, *, out=None):
-        if out is None:
-            out = torch.empty_like(inp)
-        _lib.check(_lib.load().b200_comm_all_reduce(
-            self.handle, inp.data_ptr(), out.data_ptr(), inp.numel(), _lib.dtype_code(inp.dtype),
-            _lib.current_stream()), "b200_comm_all_reduce")
-        return out
