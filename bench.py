@@ -433,6 +433,7 @@ def run_b200(args):
         e2e_step(3 + i)
     ev1.record()
     barrier()
+    _lib.check_waits()
     e2e_ms = max_over_ranks(ev0.elapsed_time(ev1)) / args.steps
     e2e_value = bs / (e2e_ms * 1e-3)
     clocks = sampler.stop() if rank == 0 else None

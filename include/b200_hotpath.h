@@ -58,8 +58,13 @@ const char* b200_last_variant(void);
 int64_t b200_launch_count(void);
 
 /* Waits inside kernels of the current device that ran out (each after about two seconds) since the library was
- * loaded: a kernel whose wait runs out ends by itself and its output is not to be used.  Synchronises. */
+ * loaded: a kernel whose wait runs out ends by itself and its output is not to be used.  Synchronises the device. */
 int b200_wait_timeouts(int64_t* total);
+/* 1 if a wait has run out since the last report, 0 if not; reading clears it and does not synchronise (read it where
+ * the results' stream has been waited for).  The library's next launch of a kernel with bounded waits reports it too,
+ * by failing.  b200_wait_selftest lets one wait run out, after a millisecond, to show that the report arrives. */
+int b200_wait_error(void);
+int b200_wait_selftest(void* stream);
 
 /* Programmatic dependent launch (default on; env B200_PDL=0 turns it off): every kernel of the
  * library is launched with cudaLaunchAttributeProgrammaticStreamSerialization and orders its own

@@ -23,6 +23,8 @@ _SIGNATURES = {
     "b200_last_variant": (c_char_p, []),
     "b200_launch_count": (c_int64, []),
     "b200_wait_timeouts": (c_int, [ctypes.POINTER(c_int64)]),
+    "b200_wait_error": (c_int, []),
+    "b200_wait_selftest": (c_int, [c_void_p]),
     "b200_set_pdl": (c_int, [c_int]),
     "b200_timing_enable": (c_int, [c_int]),
     "b200_timing_read": (c_int, [c_char_p, ctypes.POINTER(c_int64), ctypes.POINTER(ctypes.c_double)]),
@@ -383,6 +385,13 @@ def check(status: int, what: str) -> None:
     if status != 0:
         msg = load().b200_last_error()
         raise B200Error(f"{what} failed (status {status}): {msg.decode() if msg else ''}")
+
+
+def check_waits() -> None:
+    """Raises where a wait inside a kernel ran out, so that what it left in its output is not taken for a result.  To be
+    called once the results' stream has been waited for (a host read of the tokens); reads one word of host memory."""
+    if load().b200_wait_error():
+        raise B200Error("a wait inside a kernel ran out: the results of this step are not to be used")
 
 
 def last_variant() -> str:

@@ -62,6 +62,7 @@ struct ExtendParams {
   int64_t gate_stride;           // sigmoid(gate[row, head * D + d])
   float score_bound;             // > 0: no capped score exceeds it (unit-norm queries and keys), so it is the
                                  // reference of every exponent instead of the cap; 0: the cap itself
+  int* wait_error;               // attn_extend_wide.cuh: tc::report_gave_up
   int kv_splits;                 // attn_extend_wide.cuh: CTAs of a cluster that share the keys of its query tiles
   float cap_poly[5];             // FAST == 2: cap * log2(e) * tanh(x) / x = sum_i cap_poly[i] x^(2i) on the
                                  // range the scores can take

@@ -100,7 +100,7 @@ attn_extend_wide_kernel(const ExtendParams p) {
   auto bar_s = [&](int t) { return bars + 8u * (1 + 2 * SL + t); };        // scores of tile t are complete
   auto bar_p = [&](int t, int h) { return bars + 8u * (3 + 2 * SL + 2 * t + h); };  // half h of P of tile t is written
   auto bar_o = [&](int t) { return bars + 8u * (7 + 2 * SL + t); };        // PV of tile t is complete
-  const uint32_t tmem_slot = bars + 8u * C::N_BARS;
+  const uint32_t tmem_slot = bars + 8u * C::N_BARS, gave_up = tmem_slot + 4;
   bool dead = false;
 
   if (threadIdx.x == 0) {
@@ -115,6 +115,7 @@ attn_extend_wide_kernel(const ExtendParams p) {
       tc::mbar_init(bar_p(t, 1), 128);
       tc::mbar_init(bar_o(t), 1);
     }
+    asm volatile("st.shared.u32 [%0], 0;\n" ::"r"(gave_up) : "memory");
     tc::fence_barrier_init();
   }
   if (warp == 8) {
@@ -171,7 +172,7 @@ attn_extend_wide_kernel(const ExtendParams p) {
 #pragma unroll
         for (int kv = 0; kv < 2; ++kv) {
           const int u = 2 * j + kv;
-          if (u >= SL) tc::mbar_wait_bounded(bar_empty(slot), phase ^ 1u, dead);
+          if (u >= SL) tc::mbar_wait_bounded(bar_empty(slot), phase ^ 1u, dead, gave_up);
           const uint32_t dst = sbase + C::OFF_RING + slot * C::TILE_BYTES;
           const char* src = kv ? vbase : kbase;
 #pragma unroll
@@ -200,7 +201,7 @@ attn_extend_wide_kernel(const ExtendParams p) {
       constexpr uint32_t idesc_pv = tc::make_idesc(fmt, fmt, 128, D, 0, 1);    // V: MN-major B
       const uint64_t qdesc = tc::make_smem_desc_sw128(sbase, 1024, 16);
       auto wait_unit = [&](int u) {
-        tc::mbar_wait_bounded(bar_full(u % SL), (u / SL) & 1u, dead);
+        tc::mbar_wait_bounded(bar_full(u % SL), (u / SL) & 1u, dead, gave_up);
         tc::tc_fence_after();
       };
       auto issue_qk = [&](int t, int j, bool last) {
@@ -218,7 +219,7 @@ attn_extend_wide_kernel(const ExtendParams p) {
         __syncwarp();
       };
       if (n_kv > 0) {
-        tc::mbar_wait_bounded(bar_q, 0, dead);
+        tc::mbar_wait_bounded(bar_q, 0, dead, gave_up);
         wait_unit(0);
         for (int t = 0; t < tiles; ++t) issue_qk(t, 0, t == tiles - 1);
       }
@@ -229,7 +230,7 @@ attn_extend_wide_kernel(const ExtendParams p) {
         for (int t = 0; t < tiles; ++t) {
 #pragma unroll
           for (int h = 0; h < 2; ++h) {            // the first 64 keys are multiplied while the others' P is made
-            tc::mbar_wait_bounded(bar_p(t, h), j & 1u, dead);
+            tc::mbar_wait_bounded(bar_p(t, h), j & 1u, dead, gave_up);
             tc::tc_fence_after();
             if (tc::elect_one()) {
 #pragma unroll
@@ -265,7 +266,7 @@ attn_extend_wide_kernel(const ExtendParams p) {
       const float2 sc2 = make_float2(p.qk_scale, p.qk_scale), one2 = make_float2(1.f, 1.f);
       float m = -INFINITY, l = 0.f;
       for (int j = 0; j < n_kv; ++j) {
-        tc::mbar_wait_bounded(bar_s(t), j & 1u, dead);
+        tc::mbar_wait_bounded(bar_s(t), j & 1u, dead, gave_up);
         tc::tc_fence_after();
         __syncwarp();
         uint32_t v[4][32];
@@ -306,7 +307,7 @@ attn_extend_wide_kernel(const ExtendParams p) {
         const float m_new = fmaxf(m, mt);
         if (__any_sync(0xffffffffu, m_new > m + kRescaleThreshold)) {          // also the first finite maximum
           if (j > 0) {
-            tc::mbar_wait_bounded(bar_o(t), (j - 1) & 1u, dead);               // O holds tiles 0 .. j - 1
+            tc::mbar_wait_bounded(bar_o(t), (j - 1) & 1u, dead, gave_up);      // O holds tiles 0 .. j - 1
             tc::tc_fence_after();
             __syncwarp();
             const float alpha = (m == -INFINITY) ? 0.f : fast_exp2(m - m_new);
@@ -346,8 +347,8 @@ attn_extend_wide_kernel(const ExtendParams p) {
         l += (lsum[0].x + lsum[0].y) + (lsum[1].x + lsum[1].y);
       }
       if (n_kv > 0) {
-        tc::mbar_wait_bounded(bar_o(t), (n_kv - 1) & 1u, dead);
-        if (S > 1) tc::mbar_wait_bounded(bar_o(tiles - 1), (n_kv - 1) & 1u, dead);  // the last reader of shared memory
+        tc::mbar_wait_bounded(bar_o(t), (n_kv - 1) & 1u, dead, gave_up);
+        if (S > 1) tc::mbar_wait_bounded(bar_o(tiles - 1), (n_kv - 1) & 1u, dead, gave_up);  // the last reader
       }
       tc::tc_fence_after();
       __syncwarp();
@@ -444,7 +445,10 @@ attn_extend_wide_kernel(const ExtendParams p) {
   }
   tc::tc_fence_before();
   __syncthreads();
-  if (warp == 8) tc::tmem_dealloc(tmem_base, 512);
+  if (warp == 8) {
+    tc::report_gave_up(gave_up, p.wait_error);
+    tc::tmem_dealloc(tmem_base, 512);
+  }
 }
 
 // Clusters of S CTAs that are resident at once on the current device (0: none).
@@ -481,6 +485,7 @@ template <typename T, int D>
 static int launch_extend_wide(const ExtendParams& p_in, int bs, int max_extend_len, int max_kv_len, cudaStream_t st) {
   using C = WideCfg<D>;
   ExtendParams p = p_in;
+  if (const int rc = wait_error_arm("attn_extend", &p.wait_error)) return rc;
   B200_CUDA_OK(cudaFuncSetAttribute(attn_extend_wide_kernel<T, D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     C::SMEM_BYTES));
   const int resident = device_sm_count();

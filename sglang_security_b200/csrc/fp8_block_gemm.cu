@@ -26,6 +26,7 @@ struct BlockGemmParams {
   int M, N, K;
   // few tiles: a cluster of `splits` CTAs takes one tile, each a slice of K; see the epilogue
   int splits, kb_per_split;
+  int* wait_error;  // tc::report_gave_up
 };
 
 static WaitCounter wait_counter_registered(tc::wait_counter());
@@ -59,7 +60,7 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
   auto empty_bar = [&](int s) { return bars + 8u * (STAGES + s); };
   auto tfull_bar = [&](int a) { return bars + 8u * (2 * STAGES + a); };
   auto tempty_bar = [&](int a) { return bars + 8u * (2 * STAGES + NBUF + a); };
-  const uint32_t tmem_slot = bars + 8u * (2 * STAGES + 2 * NBUF);
+  const uint32_t tmem_slot = bars + 8u * (2 * STAGES + 2 * NBUF), gave_up = tmem_slot + 4;
   volatile uint32_t* tmem_slot_ptr =
       reinterpret_cast<volatile uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
 
@@ -68,7 +69,7 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
   const int m_blocks = ceil_div(p.M, BLOCK), n_blocks = ceil_div(p.N, BN);
   const int num_tiles = m_blocks * n_blocks;
   const int num_kb = ceil_div(p.K, BLOCK);
-  const int S = p.splits;
+  const int S = BN == 128 ? p.splits : 1;   // wide tiles are never split
   const int rank = S > 1 ? static_cast<int>(cluster_ctarank()) : 0;
   const int kb0 = S > 1 ? rank * p.kb_per_split : 0;
   const int kb1 = S > 1 ? min(num_kb, kb0 + p.kb_per_split) : num_kb;
@@ -86,6 +87,7 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
       tc::mbar_init(tfull_bar(a), 1);
       tc::mbar_init(tempty_bar(a), 8);
     }
+    asm volatile("st.shared.u32 [%0], 0;\n" ::"r"(gave_up) : "memory");
     tc::fence_barrier_init();
   }
   if (warp == 1) {
@@ -106,7 +108,7 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
     for (int tile = tile0; tile < num_tiles; tile += tile_step) {
       const int m_blk = tile % m_blocks, n_blk = tile / m_blocks;
       for (int kb = kb0; kb < kb1; ++kb) {
-        tc::mbar_wait_bounded(empty_bar(stage), phase ^ 1u, dead);
+        tc::mbar_wait_bounded(empty_bar(stage), phase ^ 1u, dead, gave_up);
         const uint32_t sa = smem_base + stage * STAGE_BYTES;
         if (tc::elect_one()) {
           tc::mbar_arrive_expect_tx(full_bar(stage), STAGE_BYTES);
@@ -129,8 +131,8 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
       for (int kb = kb0; kb < kb1; ++kb, ++it) {
         const int buf = it % NBUF;
         const uint32_t buf_phase = (it / NBUF) & 1u;
-        tc::mbar_wait_bounded(tempty_bar(buf), buf_phase ^ 1u, dead);
-        tc::mbar_wait_bounded(full_bar(stage), phase, dead);
+        tc::mbar_wait_bounded(tempty_bar(buf), buf_phase ^ 1u, dead, gave_up);
+        tc::mbar_wait_bounded(full_bar(stage), phase, dead, gave_up);
         tc::tc_fence_after();
         const uint64_t adesc = tc::make_smem_desc_sw128(smem_base + stage * STAGE_BYTES, 1024, 16);
         const uint64_t bdesc = tc::make_smem_desc_sw128(smem_base + stage * STAGE_BYTES + A_BYTES, 1024, 16);
@@ -172,7 +174,7 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
         const uint32_t buf_phase = (it / NBUF) & 1u;
         const float s = __ldg(as_row + kb * p.as_col) * __ldg(bs_row + kb);
         const float2 s2 = make_float2(s, s);
-        tc::mbar_wait_bounded(tfull_bar(buf), buf_phase, dead);
+        tc::mbar_wait_bounded(tfull_bar(buf), buf_phase, dead, gave_up);
         tc::tc_fence_after();
         const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * BN +
                                half * COLS;
@@ -272,7 +274,10 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
   }
   tc::tc_fence_before();
   __syncthreads();
-  if (warp == 1) tc::tmem_dealloc(tmem_base, NBUF * BN);
+  if (warp == 1) {
+    tc::report_gave_up(gave_up, p.wait_error);
+    tc::tmem_dealloc(tmem_base, NBUF * BN);
+  }
 }
 
 // Clusters of S CTAs of the 128-wide instance that are resident at once on the current device (0: none).
@@ -311,7 +316,9 @@ static int launch_block_gemm_bn(const void* a, int64_t lda, const void* b, int64
   constexpr int SMEM = BlkCfg<BN>::SMEM;
   BlockGemmParams p = p_in;
   CUtensorMap ta, tb;
-  int rc = make_tmap_2d(&ta, a, p.M, p.K, lda, 128, 128, 1, false);
+  int rc = wait_error_arm("fp8_block_gemm", &p.wait_error);
+  if (rc) return rc;
+  rc = make_tmap_2d(&ta, a, p.M, p.K, lda, 128, 128, 1, false);
   if (rc) return rc;
   rc = make_tmap_2d(&tb, b, p.N, p.K, ldb, BN, 128, 1, true);
   if (rc) return rc;

@@ -38,6 +38,7 @@ struct PairParams {
   int splits, kb_per_split;
   int vec_ok;           // rows of `out` take 16-byte stores
   float act_pos, act_neg;
+  int* wait_error;      // tc::report_gave_up
 };
 
 constexpr int kPairMaxStages = 10, kPairMaxSplits = 4;
@@ -107,7 +108,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   auto empty_bar = [&](int s) { return bars + 8u * (kPairMaxStages + s); };
   auto tfull_bar = [&](int a) { return bars + 8u * (2 * kPairMaxStages + a); };
   auto tempty_bar = [&](int a) { return bars + 8u * (2 * kPairMaxStages + 2 + a); };
-  const uint32_t tmem_slot = bars + 8u * (2 * kPairMaxStages + 4);
+  const uint32_t tmem_slot = bars + 8u * (2 * kPairMaxStages + 4), gave_up = tmem_slot + 4;
 
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
@@ -136,6 +137,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
       tc::mbar_init(tfull_bar(a), 1);
       tc::mbar_init(tempty_bar(a), 16);            // the epilogue warps of both CTAs
     }
+    asm volatile("st.shared.u32 [%0], 0;\n" ::"r"(gave_up) : "memory");
     tc::fence_barrier_init();
   }
   if (warp == 1) tc::tmem_alloc_pair(tmem_slot, 512);
@@ -180,7 +182,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         if (ahead)
           --w_ahead;
         else
-          tc::mbar_wait_bounded(empty_bar(stage), phase ^ 1u, dead);
+          tc::mbar_wait_bounded(empty_bar(stage), phase ^ 1u, dead, gave_up);
         if (tc::elect_one()) {
           if (!ahead) {
             if (half == 0) tc::mbar_arrive_expect_tx(full_bar(stage), stage_tx);
@@ -196,7 +198,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
       }
     }
     for (int i = 0; i < p.stages; ++i) {           // every commit that targets this CTA has arrived
-      tc::mbar_wait_bounded(empty_bar(stage), phase ^ 1u, dead);
+      tc::mbar_wait_bounded(empty_bar(stage), phase ^ 1u, dead, gave_up);
       if (++stage == p.stages) {
         stage = 0;
         phase ^= 1u;
@@ -209,11 +211,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
       uint32_t phase = 0;
       for (int tile = cluster_id; tile < num_tiles; tile += clusters, ++local) {
         const int acc = local & 1;
-        tc::mbar_wait_bounded(tempty_bar(acc), ((local >> 1) & 1u) ^ 1u, dead);
+        tc::mbar_wait_bounded(tempty_bar(acc), ((local >> 1) & 1u) ^ 1u, dead, gave_up);
         tc::tc_fence_after();
         const uint32_t tmem_d = tmem_base + acc * 256;
         for (int kb = kb0; kb < kb1; ++kb) {
-          tc::mbar_wait_bounded(full_bar(stage), phase, dead);
+          tc::mbar_wait_bounded(full_bar(stage), phase, dead, gave_up);
           tc::tc_fence_after();
           const uint64_t adesc = tc::make_smem_desc_sw128(base + stage * stage_bytes, 1024, 16);
           const uint64_t bdesc = tc::make_smem_desc_sw128(base + stage * stage_bytes + W_BYTES, 1024, 16);
@@ -299,7 +301,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
       const float sb = p.sb && chan < p.N ? __ldg(p.sb + static_cast<int64_t>(chan) * p.sb_stride) : 1.0f;
       const float bias = p.bias && chan < p.N ? to_float<OutT>(static_cast<const OutT*>(p.bias)[chan]) : 0.0f;
       named_bar_sync_gemm(1, 256);                 // scales of this tile are in place
-      tc::mbar_wait_bounded(tfull_bar(acc), (local >> 1) & 1u, dead);
+      tc::mbar_wait_bounded(tfull_bar(acc), (local >> 1) & 1u, dead, gave_up);
       tc::tc_fence_after();
       __syncwarp();
       if (S > 1) {
@@ -363,7 +365,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   tc::tc_fence_before();
   __syncwarp();
   cluster_sync_all();                              // the peer may still signal this CTA's barriers
-  if (warp == 1) tc::tmem_dealloc_pair(tmem_base, 512);
+  if (warp == 1) {
+    tc::report_gave_up(gave_up, p.wait_error);
+    tc::tmem_dealloc_pair(tmem_base, 512);
+  }
 }
 
 struct PairPlan {
@@ -478,6 +483,8 @@ int launch_gemm_pair(const void* x, int64_t ldx, const void* w, int64_t ldw, con
   p.vec_ok = ep.ldc % 8 == 0 && aligned16(ep.out);
   p.act_pos = ep.act_pos;
   p.act_neg = ep.act_neg;
+  rc = wait_error_arm(timer_name, &p.wait_error);
+  if (rc) return rc;
   const int tiles = ceil_div(ep.M, plan.bn) * ceil_div(ep.N, 256);
   const int clusters = plan.splits > 1 || tiles < clusters_of[1] ? tiles : clusters_of[1];
   // mc: the 128-token blocks come in full pairs

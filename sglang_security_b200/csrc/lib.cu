@@ -45,12 +45,60 @@ static std::vector<const void*>& wait_counters() {
 WaitCounter::WaitCounter(const void* symbol) { wait_counters().push_back(symbol); }
 int wait_timeouts(int64_t* total) {
   *total = 0;
+  B200_CUDA_OK(cudaDeviceSynchronize());   // other streams' kernels too
   for (const void* sym : wait_counters()) {
     unsigned n = 0;
     B200_CUDA_OK(cudaMemcpyFromSymbol(&n, sym, sizeof(n)));
     *total += n;
   }
   return 0;
+}
+
+// Allocated by the first launch that needs it, which may be one that is being captured.
+static std::atomic<int*> g_wait_error{nullptr};
+int* wait_error_word() {
+  if (int* w = g_wait_error.load(std::memory_order_acquire)) return w;
+  static std::mutex mu;
+  std::lock_guard<std::mutex> lock(mu);
+  if (int* w = g_wait_error.load(std::memory_order_acquire)) return w;
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  (void)cudaThreadExchangeStreamCaptureMode(&mode);
+  int* w = nullptr;
+  if (cudaHostAlloc(reinterpret_cast<void**>(&w), sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+    (void)cudaGetLastError();
+    w = nullptr;
+  } else {
+    *w = 0;
+  }
+  (void)cudaThreadExchangeStreamCaptureMode(&mode);
+  g_wait_error.store(w, std::memory_order_release);
+  return w;
+}
+static int take_wait_error() {
+  volatile int* w = g_wait_error.load(std::memory_order_acquire);
+  if (!w || !*w) return 0;
+  *w = 0;
+  return 1;
+}
+int wait_error_arm(const char* who, int** word) {
+  *word = wait_error_word();
+  B200_REQUIRE(*word, "%s: no host-visible error word", who);
+  B200_REQUIRE(!take_wait_error(), "%s: a wait inside an earlier kernel ran out, its output is not to be used", who);
+  return 0;
+}
+
+static WaitCounter wait_counter_registered(tc::wait_counter());
+
+// One wait that nothing ends, with a limit of about a millisecond.
+__global__ void wait_selftest_kernel(int* error) {
+  __shared__ uint64_t bar;
+  __shared__ uint32_t gave_up;
+  tc::mbar_init(smem_u32(&bar), 1);
+  tc::fence_barrier_init();
+  gave_up = 0;
+  bool dead = false;
+  tc::mbar_wait_bounded(smem_u32(&bar), 0, dead, smem_u32(&gave_up), 1ll << 21);
+  tc::report_gave_up(smem_u32(&gave_up), error);
 }
 
 static thread_local char g_variant[256] = "";
@@ -159,6 +207,17 @@ int64_t b200_launch_count(void) { return b200::g_launch_count.load(); }
 int b200_wait_timeouts(int64_t* total) {
   B200_REQUIRE(total, "b200_wait_timeouts: null pointer");
   return b200::wait_timeouts(total);
+}
+
+int b200_wait_error(void) { return b200::take_wait_error(); }
+
+int b200_wait_selftest(void* stream) {
+  using namespace b200;
+  int* word = nullptr;
+  if (const int rc = wait_error_arm("b200_wait_selftest", &word)) return rc;
+  wait_selftest_kernel<<<1, 1, 0, static_cast<cudaStream_t>(stream)>>>(word);
+  B200_CHECK_LAUNCH("wait_selftest_kernel");
+  return 0;
 }
 
 }  // extern "C"

@@ -44,20 +44,36 @@ __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity) {
   while (!mbar_try_wait(bar, parity)) {
   }
 }
-// Bounded form: gives up after about two seconds, counts that in this translation unit's g_wait_timeouts
-// (b200_wait_timeouts() reads it) and lets the caller run to its end; once `dead`, a thread's later waits only
-// poll, so a lost signal costs one limit and not one per wait.
+// Bounded form: gives up after `limit` clocks (about two seconds), counts that in this translation unit's
+// g_wait_timeouts (b200_wait_timeouts() reads it), marks the block's word of shared memory at `gave_up` and lets the
+// caller run to its end; once `dead`, a thread's later waits only poll, so a lost signal costs one limit and not one
+// per wait.
 static __device__ unsigned g_wait_timeouts;
-__device__ __forceinline__ void mbar_wait_bounded(uint32_t bar, uint32_t parity, bool& dead) {
+__device__ __forceinline__ void mbar_wait_bounded(uint32_t bar, uint32_t parity, bool& dead, uint32_t gave_up,
+                                                  long long limit = 1ll << 32) {
   if (mbar_try_wait(bar, parity)) return;
   const long long t0 = clock64();
   while (!dead) {
     if (mbar_try_wait(bar, parity)) return;
-    if (clock64() - t0 > (1ll << 32)) {
+    if (clock64() - t0 > limit) {
       dead = true;
       atomicAdd(&g_wait_timeouts, 1u);
+      asm volatile("st.shared.u32 [%0], 1;\n" ::"r"(gave_up) : "memory");
     }
   }
+}
+// The end of a block with bounded waits, by one thread after the block has met: where a wait ran out, a millisecond
+// for the copies and MMAs that may still be in flight, and the host's error word (wait_error_word()) is marked, which
+// the library's next launch with bounded waits and b200_wait_error() report.
+__device__ __forceinline__ void report_gave_up(uint32_t gave_up, int* error) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1];\n" : "=r"(v) : "r"(gave_up) : "memory");
+  if (v == 0) return;
+  const long long t0 = clock64();
+  while (clock64() - t0 < (1ll << 21)) {
+  }
+  *static_cast<volatile int*>(error) = 1;
+  __threadfence_system();
 }
 
 // ---- TMA ------------------------------------------------------------------------------------
@@ -229,6 +245,10 @@ __device__ __forceinline__ bool elect_one() {
 struct WaitCounter {
   explicit WaitCounter(const void* symbol);
 };
+// The word of host memory that a kernel marks when a wait runs out; null where none can be had.
+int* wait_error_word();
+// Every launch with bounded waits begins here: fails where an earlier one gave up (and clears that), else -> *word.
+int wait_error_arm(const char* who, int** word);
 namespace tc {
 static inline const void* wait_counter() { return static_cast<const void*>(&g_wait_timeouts); }
 }  // namespace tc

@@ -33,6 +33,7 @@ def main(argv=None) -> int:
 
     import torch
 
+    from .. import _lib
     from ..managers.schedule_batch import Req, StepItem
     from ..managers.scheduler import Scheduler
     from ..model_executor.model_runner import ModelRunner
@@ -63,6 +64,7 @@ def main(argv=None) -> int:
         logits = sched.run_step(items, layer_hook=hook) if items else None
         if logits is not None:
             data = logits.float().cpu().contiguous().numpy().astype("<f4")
+            _lib.check_waits()
             tmp = os.path.join(a.out, f".{step['step']}.f32.part")
             with open(tmp, "wb") as f:
                 f.write(data.tobytes())

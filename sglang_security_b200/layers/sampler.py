@@ -7,6 +7,7 @@ from typing import List
 
 import torch
 
+from .. import _lib
 from .dense_kernel import argmax_rows
 
 
@@ -27,6 +28,11 @@ class Sampler:
 
     def __call__(self, logits: torch.Tensor, reqs: List) -> List[int]:
         """logits [n, vocab] (one row per request) -> n token ids."""
+        tokens = self._pick(logits, reqs)
+        _lib.check_waits()      # the tokens have been read: every kernel behind them has ended
+        return tokens
+
+    def _pick(self, logits: torch.Tensor, reqs: List) -> List[int]:
         if all(r.sampling_params.temperature <= 0 for r in reqs):
             rows = logits
             if rows.dtype in (torch.bfloat16, torch.float16):
