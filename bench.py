@@ -1,18 +1,18 @@
 #!/usr/bin/env python
 """bench.py — headline benchmark of the B200 hot path.
 
-Metric (BASELINE.json): decode tokens/s of Llama-3.1-8B FP8 (W8A8: per-channel e4m3 weights, dynamic
+Metric: decode tokens/s of Llama-3.1-8B FP8 (W8A8: per-channel e4m3 weights, dynamic
 per-token e4m3 activations) at 1/2/4/8 B200, plus the decode-attention kernel's HBM GB/s vs peak.
 
-Workload: batch 64 decode at 4k context (the geometry BASELINE configs[1] fixes for the attention
-roofline, run here with the whole model of configs[2]).  One "step" = ONE WHOLE-MODEL DECODE STEP,
+Workload: batch 64 decode at 4k context (the geometry of the attention roofline, run here with the
+whole model).  One "step" = ONE WHOLE-MODEL DECODE STEP,
 what the reference's `bench_one_batch.py:234-263` times: vocab-parallel embedding -> 32 x
 (RMSNorm->FP8 quant, qkv GEMM, RoPE + KV-pool write, paged split-KV decode attention, o_proj GEMM
 [+ TP all-reduce], RMSNorm->quant, gate_up GEMM, SiLU*mul->quant, down GEMM [+ TP all-reduce]) ->
 final RMSNorm -> lm_head (+ all-gather of the vocab slices) -> greedy argmax.  Random-init weights
 of the real geometry, synthetic token ids, random page table (page_size 1, worst-case gather).
 
-N > 1 (torchrun, one rank per GPU): tensor parallel by heads / columns (SURVEY §8e) with the
+N > 1 (torchrun, one rank per GPU): tensor parallel by heads / columns with the
 all-reduce after every row-parallel GEMM in the timed path (NVLink peer-memory kernel or NCCL, as
 `RowParallelLinear` decides) — total work is fixed => "strong" scaling.
 
@@ -53,8 +53,7 @@ UNIT = "tokens/s"
 
 # --------------------------------------------------------------------------------------------
 def split_kernel_bytes(bs, ctx, hq, hkv, d, kv_elt=2, elt=2):
-    """Algorithmic bytes of ONE attn_decode split-kernel launch: K+V rows, q, o, slot indices
-    (SURVEY §8d cfg 2)."""
+    """Algorithmic bytes of ONE attn_decode split-kernel launch: K+V rows, q, o, slot indices."""
     return bs * ctx * hkv * 2 * d * kv_elt + bs * hq * d * elt * 2 + bs * ctx * 4
 
 

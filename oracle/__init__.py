@@ -1,11 +1,11 @@
 """oracle/ — TEST INFRASTRUCTURE ONLY.
 
-CPU restatements of the reference's algorithms for the hot path (SURVEY.md §8c).  Only
+CPU restatements of the reference's algorithms for the hot path.  Only
 `tests/`, `__graft_entry__.smoke()` and `bench.py`'s cpu_baseline / `--impl reference` legs may
 import this package, and only as the checker or the timed CPU baseline — never as (part of) the
 product path.  Nothing under `sglang_security_b200/` imports it.
 
-Pinning status (details in DESIGN.md §3):
+Pinning status:
   attention decode/extend : pinned — checked against outputs of the reference's own
       torch_native_backend.py run in the authoring container (tests/golden/attn_*.pt, generated
       by oracle/gen_golden.py), against the reference sgl-kernel CPU kernels (oracle/_ref) and
@@ -20,6 +20,6 @@ Pinning status (details in DESIGN.md §3):
       alloc_extend / alloc_decode by the reference's own Triton kernels run in Triton's CPU
       interpreter (tests/golden/sched_index.pt, sched_alloc.pt).
   GPTQ                    : arithmetic lives in vllm 0.8.4 (absent, CUDA only): packing order pinned
-      by vllm's gptq_pack (tests/golden/gptq_pack_vllm.pt); dequant arithmetic checked on the GPU box
+      by vllm's gptq_pack (tests/golden/gptq_pack_vllm.pt); dequant arithmetic checked on a GPU
       against the image's vllm wheel (tests/test_gptq_vs_vllm_gpu.py) - unpinned in the CPU suite.
 """

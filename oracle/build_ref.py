@@ -1,9 +1,9 @@
 """Compile the reference's own CPU attention kernels into oracle/_ref/ (authoring container only).
 
-TEST INFRASTRUCTURE ONLY.  Sources are compiled WHERE THEY LIE under /root/reference
+TEST INFRASTRUCTURE ONLY.  Sources are compiled WHERE THEY LIE in the reference tree
 (sgl-kernel/csrc/cpu/decode.cpp, extend.cpp, gemm.cpp, gemm_fp8.cpp + headers); nothing is copied into this repo.  Only
 the outputs (two .so files and build_info.json) land in oracle/_ref/, which is git-ignored but
-travels to the GPU box.  Two ISA variants are built because the GPU box's host CPU may differ:
+travels with the working tree.  Two ISA variants are built because another machine's CPU may differ:
   native  : -march=native of the authoring container (AVX512-BF16 + AMX kernels, the reference's
             own CMake flag, sgl-kernel/csrc/cpu/CMakeLists.txt:46)
   generic : -march=x86-64-v3 (the reference's scalar/at::vec fallbacks)
@@ -66,7 +66,7 @@ def _compile(variant: str, march: str) -> str:
 
 def build(force: bool = False):
     if not os.path.isdir(REF_CPU):
-        return None  # GPU box: only the prebuilt files are used
+        return None  # no reference here: only the prebuilt files are used
     os.makedirs(OUT, exist_ok=True)
     info_path = os.path.join(OUT, "build_info.json")
     srcs = [os.path.join(HERE, "ref_shim.cpp"), *[os.path.join(REF_CPU, f) for f in REF_SOURCES],

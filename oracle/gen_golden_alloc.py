@@ -3,8 +3,8 @@
 They are Triton kernels; their source text is extracted UNMODIFIED (ast line ranges, decorators
 included) into a scratch module and executed on CPU tensors with Triton's interpreter
 (TRITON_INTERPRET=1), launched exactly as PagedTokenToKVPoolAllocator.alloc_extend / alloc_decode
-launch them (paged_allocator.py:217-262).  Run here (needs /root/reference and triton); the fixture
-travels to the GPU box.  TEST INFRASTRUCTURE ONLY."""
+launch them (paged_allocator.py:217-262).  Run here (needs the reference tree and triton); the fixture
+is committed.  TEST INFRASTRUCTURE ONLY."""
 import ast
 import importlib.util
 import os

@@ -6,7 +6,7 @@ the constructor would set (memory_pool.py:119-123,264-300); the one import insid
 (cuda_graph_runner.get_is_capture_mode) is answered by a stub module returning False, which is its
 value outside graph capture.  Covers float8_e4m3fn and float8_e5m2 pools, bf16 / f16 activations,
 with and without k_scale / v_scale, out-of-range values (e4m3: NaN byte; e5m2: Inf byte), subnormals.
-Run here (needs /root/reference); the fixture travels to the GPU box.  TEST INFRASTRUCTURE ONLY."""
+Needs the reference tree; the fixture is committed.  TEST INFRASTRUCTURE ONLY."""
 import ast
 import os
 import sys

@@ -11,8 +11,8 @@ OWN torch-native implementations of the quantised-linear ops, whose source is ex
 
 These are the functions the reference's own tests compare its CUDA kernels with (the kernels
 themselves cannot be built offline).  Inputs follow the reference tests' distributions
-(test_fp8_gemm.py:16-25, test_block_fp8.py:369-384, test_awq_dequant.py:81-103).  Run here (needs
-/root/reference); the fixtures travel to the GPU box.  TEST INFRASTRUCTURE ONLY.
+(test_fp8_gemm.py:16-25, test_block_fp8.py:369-384, test_awq_dequant.py:81-103).  Needs the
+reference tree; the fixtures are committed.  TEST INFRASTRUCTURE ONLY.
 """
 import ast
 import os

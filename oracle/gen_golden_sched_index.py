@@ -2,7 +2,7 @@
 whose source is extracted unmodified (ast) from the read-only reference tree:
   get_last_loc_torch      python/sglang/srt/managers/schedule_batch.py
   compute_position_torch  python/sglang/srt/model_executor/forward_batch_info.py
-Run here (needs /root/reference); the fixture travels to the GPU box.  TEST INFRASTRUCTURE ONLY."""
+Needs the reference tree; the fixture is committed.  TEST INFRASTRUCTURE ONLY."""
 import ast
 import os
 import sys

@@ -1,11 +1,11 @@
 """Load pieces of the UNMODIFIED reference by file path (authoring container only).
 
-TEST INFRASTRUCTURE ONLY.  `/root/reference` does not exist on the GPU box, so nothing that runs
-there may call this module; it is used by oracle/gen_golden.py to produce tests/golden/*.pt and by
+TEST INFRASTRUCTURE ONLY.  The reference tree is not there where the GPU tests run, so nothing of them
+may call this module; it is used by oracle/gen_golden.py to produce tests/golden/*.pt and by
 the `not gpu` tests that re-check the restatement against the live reference when it is present.
 
 `import sglang` itself fails in this image (pins torch 2.6 / triton 3.2 / transformers 4.52), so
-single files are executed with the minimum of stub modules (SURVEY.md appendix A.1).
+single files are executed with the minimum of stub modules.
 """
 from __future__ import annotations
 

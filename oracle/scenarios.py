@@ -97,8 +97,8 @@ def digest(case) -> str:
     return h.hexdigest()
 
 
-# The parity cases: name -> kwargs of make_attention_case.  Shapes cover the geometries of the
-# BASELINE configs (Llama-3.1-8B group 4 / D 128, Qwen2.5-0.5B group 7 / D 64, 70B@TP8 group 8,
+# The parity cases: name -> kwargs of make_attention_case.  Shapes cover the measured
+# geometries (Llama-3.1-8B group 4 / D 128, Qwen2.5-0.5B group 7 / D 64, 70B@TP8 group 8,
 # MHA) with ragged lengths around the kernel's tile sizes (16/32/64) and a shared radix prefix.
 DECODE_CASES = {
     "decode_llama_g4_d128": dict(seed=11, hq=8, hkv=2, d=128, seq_lens=[1, 17, 64, 130, 257]),

@@ -2,8 +2,8 @@
 
 `python -m sglang_security_b200.build` compiles every `csrc/*.cu` into
 `sglang_security_b200/lib/libb200hotpath.so`.  nvcc cross-compiles without a GPU, so the
-same command is the "does it build" check on the CPU box; the resulting .so is git-ignored but
-travels to the GPU box with the working tree.
+same command is the "does it build" check on a machine without a GPU; the resulting .so is git-ignored but
+travels with the working tree.
 """
 from __future__ import annotations
 

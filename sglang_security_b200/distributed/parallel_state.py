@@ -1,5 +1,5 @@
 """Tensor-parallel group plumbing: one process per GPU, torch.distributed (NCCL over
-NVLink 5 / NVSwitch on the B200 box, gloo in the CPU tests).  Mirrors the call surface the linear
+NVLink 5 / NVSwitch on B200, gloo in the CPU tests).  Mirrors the call surface the linear
 layers use in the reference (python/sglang/srt/distributed/communication_op.py:11-20,
 parallel_state.py:398-461, 1047-1200): the all-reduce sits only at the row-parallel boundaries."""
 from __future__ import annotations

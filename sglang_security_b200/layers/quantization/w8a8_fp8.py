@@ -1,5 +1,5 @@
 """W8A8Fp8Config / W8A8Fp8LinearMethod: static per-channel weight scales x dynamic per-token
-activation scales (python/sglang/srt/layers/quantization/w8a8_fp8.py:28-183) — BASELINE's
+activation scales (python/sglang/srt/layers/quantization/w8a8_fp8.py:28-183) — the
 "per-channel" FP8 configuration."""
 from __future__ import annotations
 

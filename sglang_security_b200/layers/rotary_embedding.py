@@ -92,7 +92,7 @@ class RotaryEmbedding(nn.Module):
     def forward_with_kv_write(self, positions, query, key, value, layer, forward_batch):
         """Rotate q/k in place and write (k, v) of every token to the KV pool rows
         forward_batch.out_cache_loc — the buffers are fetched through get_key_buffer /
-        get_value_buffer per call so pool-side hooks keep firing (SURVEY §8b)."""
+        get_value_buffer per call so pool-side hooks keep firing."""
         pool = forward_batch.token_to_kv_pool
         k_cache = pool.get_key_buffer(layer.layer_id)
         v_cache = pool.get_value_buffer(layer.layer_id)
@@ -155,7 +155,7 @@ def get_rope(head_size: int, rotary_dim: int, max_position: int, base: float,
              is_neox_style: bool = True, rope_scaling: Optional[dict] = None,
              dtype: torch.dtype = torch.bfloat16) -> RotaryEmbedding:
     """Subset of the reference factory (rotary_embedding.py:1083-1300 get_rope): unscaled RoPE and
-    the `llama3` scaling the BASELINE models (Llama-3.1-8B / 70B) use.  Every other rope_scaling
+    the `llama3` scaling that Llama-3.1-8B / 70B use.  Every other rope_scaling
     type raises instead of silently building unscaled tables."""
     if rope_scaling is None:
         return RotaryEmbedding(head_size, rotary_dim, max_position, base, is_neox_style, dtype)

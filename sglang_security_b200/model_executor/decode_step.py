@@ -12,7 +12,7 @@ What `bench_one_batch.py` times in the reference (python/sglang/bench_one_batch.
     next_token_ids = argmax(logits)
 
 This is NOT a model zoo or a model runner: it only strings `B200DecoderLayer`s together on
-random-init weights of a named geometry so that BASELINE.json's headline metric (decode tokens/s of
+random-init weights of a named geometry so that the headline metric (decode tokens/s of
 the whole model, TP all-reduce included) can be measured through the hot path.  The scheduler's
 per-step work (slot allocation, req_to_token writes) is done by the caller.
 """
@@ -56,7 +56,7 @@ class ModelGeometry:
     rms_eps: float = 1e-5
 
 
-# public HF configs of the models BASELINE.json names
+# public HF configs of the measured models
 GEOMETRIES = {
     "llama3.1-8b": ModelGeometry("llama3.1-8b", 4096, 32, 8, 128, 14336, 32, 128256, 500000.0, False),
     "llama3.1-70b": ModelGeometry("llama3.1-70b", 8192, 64, 8, 128, 28672, 80, 128256, 500000.0, False),

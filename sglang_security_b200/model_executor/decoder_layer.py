@@ -10,8 +10,8 @@ qkv bias):
     hidden, residual = post_attention_layernorm(hidden, residual)
     hidden = down_proj(SiluAndMul(gate_up_proj(hidden)))
 
-With `fuse=True` (default) the steps either side of the GEMMs / attention use the fused kernels
-(SURVEY §8f rows 1-2): RMSNorm->FP8 quant, RoPE->KV-pool write, SiLU*mul->FP8 quant — 11 launches
+With `fuse=True` (default) the steps either side of the GEMMs / attention use the fused kernels:
+RMSNorm->FP8 quant, RoPE->KV-pool write, SiLU*mul->FP8 quant — 11 launches
 per layer in decode instead of 16.  With `fuse=False` every op is launched separately exactly in
 the reference's order (used by the tests to prove both give the same result).
 The scheduler / model runner stay the reference's: this class only needs `forward_batch`.

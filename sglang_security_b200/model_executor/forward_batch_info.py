@@ -1,6 +1,6 @@
 """Field-compatible stand-in for the reference's ForwardBatch / ForwardMode.
 
-Only the fields the attention backend consumes are kept (SURVEY.md §8a3; reference
+Only the fields the attention backend consumes are kept (reference
 python/sglang/srt/model_executor/forward_batch_info.py:54-118 for the mode predicates and
 :139-259 for the batch fields).  In a real deployment the reference's own classes are passed in;
 these exist so that tests, bench.py and smoke() can drive the backend without importing sglang.

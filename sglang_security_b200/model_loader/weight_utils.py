@@ -1,5 +1,5 @@
 """FP8 KV-cache scaling factors: the JSON file of `--quantization-param-path` and the checkpoint
-parameter names — host side of SURVEY §8(f) rank 1.  Same function names, arguments, return values
+parameter names.  Same function names, arguments, return values
 and failure behaviour as the reference (python/sglang/srt/model_loader/weight_utils.py:670-857); the
 reference validates the document with pydantic models, this is a plain-Python check of the same rules.
 Pinned to the reference's own functions run on its own fixtures (tests/golden/kv_cache_scales.pt)."""

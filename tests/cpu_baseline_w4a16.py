@@ -1,8 +1,8 @@
 #!/usr/bin/env python
-"""CPU baseline of the AWQ INT4 (W4A16, group 128) linear path — SURVEY §8(d) "CPU baseline" item 3:
+"""CPU baseline of the AWQ INT4 (W4A16, group 128) linear path:
 the reference's torch-native route `awq_dequantize_torch + matmul` (sgl-kernel/tests/
 test_awq_dequant.py:9-57 restated in oracle/int4.py, pinned by tests/golden/awq_dequant.pt), on all
-host cores, at the per-rank shapes of Qwen2.5-32B TP 2 (BASELINE cfg 4) for decode-size batches.
+host cores, at the per-rank shapes of Qwen2.5-32B TP 2 for decode-size batches.
 A reported baseline next to the GPU numbers of profiles/r02_bench_w4a16_gemv2.json — not a target.
 Needs no GPU.  Lives under tests/ because it executes oracle/ code (only tests/, smoke() and bench.py's
 cpu_baseline leg may); not collected by pytest.  Run: python tests/cpu_baseline_w4a16.py"""

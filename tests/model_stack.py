@@ -43,7 +43,7 @@ def init_weights(cfg: StackConfig, seed: int = 0, std: float = 0.02, decisive_em
     tie_word_embeddings) and the embedding gets that std, so the residual stream carries a token
     signal as large as the 24 layers' contributions: the greedy token then wins by a margin far
     above the bf16 / fp8 numeric noise instead of being a near-tie among 32000 random logits
-    (SURVEY §8d cfg 1: random-init logits are nearly tied, report the margin)."""
+    (random-init logits are nearly tied, so the margin is reported)."""
     g = torch.Generator().manual_seed(seed)
     r = lambda *s: (torch.randn(*s, generator=g) * std).to(torch.bfloat16)
     qkv_out = (cfg.heads + 2 * cfg.kv_heads) * cfg.head_dim
@@ -240,7 +240,7 @@ class Stack:
 
 def run_shared_prefix_session(stack: Stack, prefix_ids, suffix_ids: List[torch.Tensor],
                               decode_steps: int, forced_tokens=None):
-    """cfg 1: (A) extend one request with the shared prefix, (B) extend bs requests
+    """(A) extend one request with the shared prefix, (B) extend bs requests
     that reuse the SAME prefix slots plus their own suffix, (C) greedy decode.  If forced_tokens
     is given the decode inputs are taken from it (teacher forcing) instead of this run's argmax.
     Returns (tokens [steps+1, bs], logits list)."""

@@ -11,7 +11,7 @@ import harness
 pytestmark = pytest.mark.gpu
 GOLDEN = os.path.join(os.path.dirname(__file__), "golden")
 
-# bf16/f16 attention tolerance (SURVEY §8c note iii): max-abs <= 3e-2, relative L2 <= 1e-2
+# bf16/f16 attention tolerance: max-abs <= 3e-2, relative L2 <= 1e-2
 MAX_ABS, REL_L2 = 3e-2, 1e-2
 
 
@@ -160,7 +160,7 @@ def test_decode_cuda_graph_capture_and_replay(index_dtype):
 
 
 def test_decode_full_size_properties():
-    """BASELINE config 2 geometry at full size (bs 64 x 4k, Hq 32 / Hkv 8 / D 128): checked through
+    """The Llama-3.1-8B decode batch at full size (bs 64 x 4k, Hq 32 / Hkv 8 / D 128): checked through
     size-independent properties — (1) a request whose cached V rows are all the same vector must
     return exactly that vector (softmax weights sum to 1); (2) permuting the slot assignment of a
     request (same K/V content at different slots) leaves the output unchanged; (3) a sampled

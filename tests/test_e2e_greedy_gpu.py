@@ -1,4 +1,4 @@
-"""BASELINE config 1 end to end: Qwen2.5-0.5B geometry, random-init bf16 weights, a 512-token shared
+"""End to end: Qwen2.5-0.5B geometry, random-init bf16 weights, a 512-token shared
 radix prefix, 8 requests x 16 own tokens, 32 greedy decode steps — the B200 path (attention backend
 + linear layers through the C-ABI) against the CPU oracle stack on the same weights."""
 import pytest
@@ -134,7 +134,7 @@ def _free_running(cfg, embed_std, decode_steps, bs, prefix, own, noise_budget):
 
 
 def test_greedy_free_running_identical_bf16_cfg1():
-    """BASELINE cfg 1 at full geometry (Qwen2.5-0.5B: 24 layers, hidden 896, 14/2 heads, D 64, qkv
+    """Full geometry (Qwen2.5-0.5B: 24 layers, hidden 896, 14/2 heads, D 64, qkv
     bias, tied head), 512-token shared radix prefix, 8 requests x 16 own tokens, 32 greedy decode
     steps: 264 greedy tokens, zero mismatches."""
     cfg = MS.StackConfig()

@@ -1,8 +1,8 @@
-"""GPU parity of the FP8 (e4m3) KV-cache path — SURVEY §8(f) rank 1: quantising set_kv_buffer
+"""GPU parity of the FP8 (e4m3) KV-cache path: quantising set_kv_buffer
 (bit-exact with the reference's div_ -> .to(float8_e4m3fn) -> index_put, memory_pool.py:390-412,
 restated in oracle/pools.py) and paged decode attention over the e4m3 pool
 (oracle/attention.py: unmodified torch_native math on the de-quantised cache with the FlashInfer
-backend's k_scale / v_scale semantics).  Tolerances: max-abs <= 3e-2, rel-l2 <= 1e-2 (SURVEY §8c)."""
+backend's k_scale / v_scale semantics).  Tolerances: max-abs <= 3e-2, rel-l2 <= 1e-2."""
 from types import SimpleNamespace
 
 import pytest

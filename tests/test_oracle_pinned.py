@@ -24,7 +24,7 @@ def test_awq_dequant_oracle_equals_reference_function():
         out = OI.awq_dequantize_oracle(c["qweight"], c["scales"], c["qzeros"], c["group"])
         assert out.dtype == c["out"].dtype
         assert torch.equal(out.view(torch.int16), c["out"].view(torch.int16))
-        # the integer unpack itself (bit-exact target of north_star)
+        # the integer unpack itself (bit-exact)
         w = OI.unpack_awq_int4(c["qweight"])
         assert w.min() >= 0 and w.max() <= 15
 

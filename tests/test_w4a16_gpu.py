@@ -57,7 +57,7 @@ def test_gptq_repack_and_zero_unpack_bit_exact():
 def _awq_layer(k, n, group, dtype, seed, realistic=False):
     g = torch.Generator().manual_seed(seed)
     if realistic:
-        # asymmetric group quantisation of N(0, 0.02) weights (SURVEY §8d cfg 4 "realistic variant")
+        # asymmetric group quantisation of N(0, 0.02) weights
         w = torch.randn((k, n), generator=g) * 0.02
         wg = w.view(k // group, group, n)
         lo, hi = wg.amin(1), wg.amax(1)
@@ -98,7 +98,7 @@ def test_awq_linear_method(m, k, n, group, dtype):
             qweight.cuda(), scales.cuda(), qzeros.cuda(), group), bias.cuda()).cpu()
     else:
         ref = O.w4a16_linear_oracle(x, O.awq_dequantize_oracle(qweight, scales, qzeros, group), bias)
-    # reference tolerance for x @ dequant in 16 bit: rtol 1e-2 (SURVEY §8d cfg 4)
+    # reference tolerance for x @ dequant in 16 bit: rtol 1e-2
     err = (out.cpu().float() - ref.float()).abs()
     tol = 1e-2 * ref.float().abs() + 1e-2 * ref.float().abs().max()
     assert (err <= tol).all(), (err.max().item(), ref.float().abs().max().item())

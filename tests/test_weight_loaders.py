@@ -3,7 +3,7 @@
 `loaded_shard_id`, per-rank windows, kv-head replication, int4 packing, block-scale grids and
 per-shard scalar scales.  Every case loads the SAME full checkpoint on every simulated rank and
 compares the rank's parameter with a hand-computed slice; GPTQ row-parallel g_idx handling
- and the Llama-3.1 rope_scaling table (pinned to the reference's get_rope output)."""
+and the Llama-3.1 rope_scaling table (pinned to the reference's get_rope output)."""
 import os
 
 import pytest
@@ -136,7 +136,7 @@ def test_fp8_block_scale_grid_windows():
 
 def test_gptq_row_parallel_ignores_global_g_idx_without_desc_act():
     """AutoGPTQ stores g_idx = arange(K) // group with GLOBAL group ids even when desc_act=False;
-    a K shard of rank > 0 must still be treated as the trivial mapping (ADVICE r1)."""
+    a K shard of rank > 0 must still be treated as the trivial mapping."""
     k, n, group, tp = 256, 16, 64, 2
     cfg = GPTQConfig(4, group, False)
     for rank in range(tp):

@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Whole-model decode step through the B200 hot path: BASELINE.json's headline metric
+"""Whole-model decode step through the B200 hot path: the headline metric
 "decode tokens/s (Llama-3-8B FP8) at 1/2/4/8 B200" measured on random-init weights.
 
 One step = embedding lookup -> L x B200DecoderLayer (fused RMSNorm->quant, FP8/INT4/bf16 linear,

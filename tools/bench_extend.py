@@ -1,6 +1,6 @@
 #!/usr/bin/env python
 """Extend (prefill with a cached radix prefix) attention throughput on the tcgen05 kernel:
-TFLOP/s = 4 * Hq * D * sum_b ext_b * (prefix_b + (ext_b + 1) / 2) / time  (SURVEY section 8d cfg 5),
+TFLOP/s = 4 * Hq * D * sum_b ext_b * (prefix_b + (ext_b + 1) / 2) / time,
 against the measured dense bf16 peak.  Shapes: Llama-3.1-8B heads (Hq 32, Hkv 8, D 128) on one GPU
 and the per-rank heads of Llama-3.1-70B at TP=8 (Hq 8, Hkv 1), radix hit-rate sweep
 h = prefix / ctx in {0, 0.5, 0.9}.  Times the kernel with CUDA events through the library timing
@@ -19,10 +19,10 @@ import torch
 
 def main():
     ap = argparse.ArgumentParser()
-    ap.add_argument("--out", default=os.path.join(ROOT, "gpurun_out", "bench_extend.json"))
+    ap.add_argument("--out", default=os.path.join(ROOT, "build", "bench_extend.json"))
     ap.add_argument("--iters", type=int, default=5)
     ap.add_argument("--quick", action="store_true")
-    ap.add_argument("--ab", action="store_true", help="also time the round-1 softmax instance")
+    ap.add_argument("--ab", action="store_true", help="also time the plain softmax instance")
     ap.add_argument("--headline", action="store_true", help="Llama-3.1-8B heads only (6 points)")
     args = ap.parse_args()
     from sglang_security_b200 import _lib
@@ -79,7 +79,7 @@ def main():
                 backend.init_forward_metadata(fb)
 
                 def timed(fast):
-                    # the library reads B200_EXTEND_FAST_SOFTMAX per launch (0 = round-1 softmax)
+                    # the library reads B200_EXTEND_FAST_SOFTMAX per launch (0 = the plain softmax)
                     os.environ["B200_EXTEND_FAST_SOFTMAX"] = "1" if fast else "0"
                     for _ in range(2):
                         layer(q, k, v, fb)

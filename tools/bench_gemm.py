@@ -39,7 +39,7 @@ def main():
     ap.add_argument("--ms", default="1,16,64,256,1024,4096,8192,16384")
     ap.add_argument("--smallm-sweep", action="store_true",
                     help="for M <= 128 also time the big-tile kernel and forced cluster split-K factors")
-    ap.add_argument("--out", default=os.path.join(ROOT, "gpurun_out", "bench_gemm.json"))
+    ap.add_argument("--out", default=os.path.join(ROOT, "build", "bench_gemm.json"))
     args = ap.parse_args()
     dev = "cuda"
     flush = torch.empty(256 << 20, dtype=torch.uint8, device=dev)

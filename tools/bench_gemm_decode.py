@@ -63,7 +63,7 @@ def main():
     ap.add_argument("--shapes", default="", help="optional NxK,NxK filter overriding --model")
     ap.add_argument("--variants", default="auto", help="comma list: auto,big,s1,s2,s3,s4,s6,s8")
     ap.add_argument("--kinds", default="rowcol,block128,torch_rowwise")
-    ap.add_argument("--out", default=os.path.join(ROOT, "gpurun_out", "bench_gemm_decode.json"))
+    ap.add_argument("--out", default=os.path.join(ROOT, "build", "bench_gemm_decode.json"))
     args = ap.parse_args()
     dev = "cuda"
     rows = []

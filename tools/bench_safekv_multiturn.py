@@ -1,8 +1,8 @@
 #!/usr/bin/env python
-"""BASELINE cfg 5: multi-turn shared-prefix load with the SafeKV private / shared prefix split,
+"""Multi-turn shared-prefix load with the SafeKV private / shared prefix split,
 radix hit-rate sweep — prefill (extend) and decode tokens/s of the whole model against hit rate.
 
-The SafeKV policy itself stays on the host, untouched (north_star): this tool only MODELS its
+The SafeKV policy itself stays on the host, untouched: this tool only MODELS its
 reuse rule to produce the (extend_prefix_lens, extend_seq_lens) the scheduler would hand the model
 runner, and then runs the real B200 hot path on them.  Rule restated from the fork's
 RadixCache._match_prefix_helper (python/sglang/srt/mem_cache/radix_cache.py:333-349): a cached node

@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""BASELINE cfg 4: Qwen2.5-32B AWQ INT4 W4A16 g128 per-rank GEMMs at TP=2 / TP=4, GEMV -> GEMM
+"""Qwen2.5-32B AWQ INT4 W4A16 g128 per-rank GEMMs at TP=2 / TP=4, GEMV -> GEMM
 crossover sweep.  Every launch streams distinct weights (copies rotate over > 2x L2) from a CUDA
 graph.  Columns: the HBM-bound GEMV (M <= 16), the tcgen05 dequant-GEMM, and the reference's own
 approach on the same GPU (awq_dequantize to a 16-bit [K, N] tensor + library matmul, awq.py:203-215).
@@ -33,7 +33,7 @@ def main():
     ap.add_argument("--splits2", default="", help="extra forced split-K factors for the stream GEMV")
     ap.add_argument("--skip-ref", action="store_true")
     ap.add_argument("--dtype", default="float16")
-    ap.add_argument("--out", default=os.path.join(ROOT, "gpurun_out", "bench_w4a16.json"))
+    ap.add_argument("--out", default=os.path.join(ROOT, "build", "bench_w4a16.json"))
     args = ap.parse_args()
     dev, dt, group = "cuda", getattr(torch, args.dtype), 128
     rows = []

@@ -14,7 +14,7 @@ import subprocess
 import sys
 from collections import OrderedDict
 
-OURS = ("attn_", "kv_write", "kv_indices", "gemm_tn", "fp8_", "w4a16", "awq_", "b200", "quant",
+OURS = ("attn_", "kv_write", "kv_indices", "gemm_", "fp8_", "w4a16", "awq_", "b200", "quant",
         "rmsnorm", "rope", "silu", "allreduce", "gptq")
 
 FULL_KEYS = [

@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Tuning sweep of the decode-attention kernel on the cfg-2 geometry (run on the GPU box).
+"""Tuning sweep of the decode-attention kernel at Llama-3.1-8B's decode batch.
 
 Times attn_decode_split (+ merge) per launch with the library's per-kernel CUDA events while
 rotating over several layers' pools (each ~1 GB, so L2 never helps) and prints achieved GB/s of
@@ -82,7 +82,7 @@ def main():
     ap.add_argument("--tp-shapes", action="store_true",
                     help="per-rank head geometry of Llama-3.1-8B at TP 2/4/8 over a range of split counts")
     ap.add_argument("--kv-dtype", default="bf16", choices=["bf16", "fp8"])
-    ap.add_argument("--out", default=os.path.join(ROOT, "gpurun_out", "sweep_decode.json"))
+    ap.add_argument("--out", default=os.path.join(ROOT, "build", "sweep_decode.json"))
     args = ap.parse_args()
     peak = 6541.5
     try:
