@@ -567,9 +567,10 @@ attn_decode_mma_kernel(const DecodeParams p) {
 // Merge of split partials: one warp per (query head, request), four columns per lane.  Latency-bound (a few hundred
 // KB): the split sums are read by all lanes at once and the first partial rows are requested before the sequence length
 // is known, so the chain is one round trip to L2, not one per split (1 request of 1500 tokens in 7 splits: 5.2 us, now
-// 3.8).  Sums run over the splits in order, as in attn_merge_quant_kernel: same bytes.
+// 3.8).  BYCOLS, for more splits than the rows requested ahead: the four warps of a CTA share the columns of a head, one
+// column per lane, so that 32 rows are requested together (64 splits are two round trips, not eight).
+// Sums run over the splits in order, as in attn_merge_quant_kernel: same bytes.
 constexpr int kMergeWarps = 4;
-constexpr int kMergeAhead = 8;
 
 // V columns per lane: 4, or 1 for rows that 16-byte loads do not fit
 template <int V>
@@ -585,23 +586,25 @@ __device__ __forceinline__ void merge_load(float (&x)[V], const float* p) {
   }
 }
 
-template <typename T, int V>
+template <typename T, int V, bool BYCOLS>
 __global__ void __launch_bounds__(kMergeWarps * 32)
 attn_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_lse, T* __restrict__ o,
                   int64_t o_stride, const int64_t* __restrict__ seq_lens, int Hq, int Dv, int num_splits, int align,
                   const int32_t* __restrict__ row_list, const T* __restrict__ gate, int64_t gate_stride) {
   griddep_wait();
   griddep_launch_dependents();
-  const int lane = threadIdx.x & 31;
-  const int hq = blockIdx.x * kMergeWarps + (threadIdx.x >> 5), b = blockIdx.y;
+  constexpr int AHEAD = BYCOLS ? 32 : 8;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int hq = BYCOLS ? blockIdx.x : blockIdx.x * kMergeWarps + warp, b = blockIdx.y;
   if (hq >= Hq) return;
   const int64_t base = (static_cast<int64_t>(b) * Hq + hq) * num_splits;
   const float* po = part_o + base * Dv;
   // splits past the sequence are allocated but hold nothing: their values are not used
-  float x[kMergeAhead][V];
-  const int d0 = lane * V;
+  float x[AHEAD][V];
+  const int dd0 = BYCOLS ? warp * 32 * V : 0, step = BYCOLS ? kMergeWarps * 32 * V : 32 * V;
+  const int d0 = dd0 + lane * V;
 #pragma unroll
-  for (int i = 0; i < kMergeAhead; ++i)
+  for (int i = 0; i < AHEAD; ++i)
     if (i < num_splits && d0 < Dv) merge_load<V>(x[i], po + static_cast<int64_t>(i) * Dv + d0);
   const float lse0 = lane < num_splits ? __ldcg(part_lse + base + lane) : 0.f;
   const int len = static_cast<int>(seq_lens[b]);
@@ -612,22 +615,22 @@ attn_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ pa
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, off));
   const int64_t row = row_list ? row_list[b] : b;
-  for (int dd = 0; dd < Dv; dd += 32 * V) {
-    const int d = dd + d0;
+  for (int dd = dd0; dd < Dv; dd += step) {
+    const int d = dd + lane * V;
     float den = 0.f, num[V];
 #pragma unroll
     for (int e = 0; e < V; ++e) num[e] = 0.f;
     for (int s0 = 0; s0 < nvalid; s0 += 32) {
       const float lse = s0 == 0 ? lse0 : (s0 + lane < nvalid ? __ldcg(part_lse + base + s0 + lane) : 0.f);
       const float w_lane = s0 + lane < nvalid ? fast_exp2(lse - M) : 0.f;
-      for (int s1 = s0; s1 < min(nvalid, s0 + 32); s1 += kMergeAhead) {
-        if (s1 > 0 || dd > 0) {
+      for (int s1 = s0; s1 < min(nvalid, s0 + 32); s1 += AHEAD) {
+        if (s1 > 0 || dd > dd0) {
 #pragma unroll
-          for (int i = 0; i < kMergeAhead; ++i)
+          for (int i = 0; i < AHEAD; ++i)
             if (s1 + i < nvalid && d < Dv) merge_load<V>(x[i], po + static_cast<int64_t>(s1 + i) * Dv + d);
         }
 #pragma unroll
-        for (int i = 0; i < kMergeAhead; ++i) {
+        for (int i = 0; i < AHEAD; ++i) {
           const float w = __shfl_sync(0xffffffffu, w_lane, (s1 + i) & 31);
           if (s1 + i < nvalid) {
             den += w;
@@ -1031,21 +1034,24 @@ static int attn_merge_impl(const float* part_o, const float* part_lse, void* o, 
                num_splits, split_align);
   B200_REQUIRE(part_o && part_lse && o && seq_lens, "b200_attn_merge: null pointer");
   B200_REQUIRE(dtype == B200_BF16 || dtype == B200_F16, "b200_attn_merge: dtype %d", dtype);
-  dim3 grid(ceil_div(Hq, kMergeWarps), bs);
+  const bool bycols = num_splits > 8;
+  dim3 grid(bycols ? Hq : ceil_div(Hq, kMergeWarps), bs);
   const int threads = kMergeWarps * 32;
   const bool wide = Dv % 4 == 0 && aligned16(part_o);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   ScopedKernelTimer timer("attn_merge", st);
-#define LAUNCH_MERGE(T, V)                                                                                            \
-  B200_CUDA_OK(launch_kernel(attn_merge_kernel<T, V>, grid, dim3(threads), 0, st, 1, pdl_family(bs, kPdlMerge), part_o, \
-                             part_lse, static_cast<T*>(o), o_stride, seq_lens, Hq, Dv, num_splits, align, row_list,   \
-                             static_cast<const T*>(gate), gate_stride))
+#define LAUNCH_MERGE(T, V, C)                                                                                         \
+  B200_CUDA_OK(launch_kernel(attn_merge_kernel<T, V, C>, grid, dim3(threads), 0, st, 1, pdl_family(bs, kPdlMerge),    \
+                             part_o, part_lse, static_cast<T*>(o), o_stride, seq_lens, Hq, Dv, num_splits, align,     \
+                             row_list, static_cast<const T*>(gate), gate_stride))
   if (dtype == B200_BF16) {
-    if (wide) LAUNCH_MERGE(__nv_bfloat16, 4);
-    else LAUNCH_MERGE(__nv_bfloat16, 1);
+    if (bycols) LAUNCH_MERGE(__nv_bfloat16, 1, true);
+    else if (wide) LAUNCH_MERGE(__nv_bfloat16, 4, false);
+    else LAUNCH_MERGE(__nv_bfloat16, 1, false);
   } else {
-    if (wide) LAUNCH_MERGE(__half, 4);
-    else LAUNCH_MERGE(__half, 1);
+    if (bycols) LAUNCH_MERGE(__half, 1, true);
+    else if (wide) LAUNCH_MERGE(__half, 4, false);
+    else LAUNCH_MERGE(__half, 1, false);
   }
 #undef LAUNCH_MERGE
   B200_CHECK_LAUNCH("attn_merge_kernel");
