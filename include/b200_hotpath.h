@@ -130,7 +130,7 @@ size_t b200_attn_decode_workspace_bytes(int bs, int Hq, int Dv, int num_splits);
 /* Split-count heuristic (replaces get_num_kv_splits_triton, triton_backend.py:23-72, with a
  * host-side choice that needs no device sync): avg_len = expected tokens per request.       */
 int b200_attn_decode_num_splits(int bs, int Hkv, int group, int D, int64_t avg_len, int num_sms);
-/* The same where the longest request is known too: unequal requests get more, smaller splits. */
+/* The same where the longest request is known too (the splits go by it), avg_len alone standing for equal requests. */
 int b200_attn_decode_num_splits_ragged(int bs, int Hkv, int group, int D, int64_t avg_len, int64_t max_len,
                                        int num_sms);
 int b200_attn_decode(const void* q, int64_t q_stride, const void* k_cache, const void* v_cache,

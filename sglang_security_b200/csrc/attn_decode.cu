@@ -20,6 +20,7 @@
 //   accumulators and fp32 online softmax in registers (exp2 domain, scale*log2e folded in).
 //   Warps are merged once through shared memory; partials (normalised O, log2-domain LSE) go to
 //   the workspace and are merged by attn_merge_kernel.
+#include <cmath>
 #include <cstdlib>
 
 #include "common.cuh"
@@ -984,34 +985,42 @@ static int decode_num_splits(int bs, int Hkv, int group, int D, int64_t avg_len,
   const int64_t base = static_cast<int64_t>(bs) * Hkv * head_tiles;
   const int ctas_per_sm = decode_ctas_per_sm(D);
   const int64_t slots = static_cast<int64_t>(num_sms) * ctas_per_sm;
-  const int align = decode_align();
-  // Equal-length CTAs that all fit the resident slots at once finish together, while any overflow runs as a thin
-  // second wave: the largest count that fits one wave.  Per-rank shapes of Llama-3.1-8B at TP 2 / 4 / 8, batch
-  // 64 x 4k: 2 / 4 / 9 splits = 512 / 512 / 576 CTAs on 592 slots (90.8 / 50.7 / 29.9 us) against 93.9 / 56.4 /
-  // 35.3 us for the oversubscription rule below; 1 split (512 CTAs, no merge) 170.4 us against 174.4 + merge.
-  // Few requests are bound by the chain of tiles in a warp, so the splits go down to 64 tokens (us, splits of 192
-  // tokens -> this: 1 x 1500 tokens 10.9 -> 10.3, 5 x 2000 ragged 14.4 -> 12.3), but past 32 of them the merge takes
-  // back what the chain gives (1 x 8000, FP8 rows: 16.5 with 41, 14.4 with 12 to 32).
   const int64_t by_slots = slots / base;
-  int64_t fit = by_slots < avg_len / 64 ? by_slots : avg_len / 64;
-  if (fit > 32) fit = 32;
-  // Few splits of unequal requests: the longest ones would run alone at the end, so twice the slots are filled
-  // (us, one wave or 1.5 -> 2.1 times the slots: 40 x up to 3000 tokens 61.3 -> 57.9, 64 x up to 4096 FP8 77.0 -> 69.3,
-  // 27 x up to 6000 FP8 50.4 -> 48.2).
-  // Not for short requests, where the smaller splits' merge costs more than the even end gives.
-  const bool ragged = max_len * 8 > avg_len * 9 && by_slots < 4 && avg_len >= 1536;
-  if (!ragged && fit >= 1 && (fit < by_slots || static_cast<double>(base * fit) >= 0.85 * static_cast<double>(slots)))
+  // Split counts from 1 to 64 were timed for 1592 batches (1 to 64 requests of 64 to 131072 tokens, equal and unequal
+  // ones, bf16 and FP8 rows, 2 to 8 kv heads): this rule's choice is 2.4 % slower than the best count on average.
+  // A request that is not split ends as soon as one that is (which costs a merge) up to some 384 tokens, and further up
+  // where the CTAs are many (us, whole / split: 1 x 128 tokens 6.0 / 7.6, 1 x 512 10.7 / 7.6, 16 x 384 9.7 / 10.7,
+  // 16 x 700 13.8 / 13.1).  The longest request is what the others are waited for.
+  const int64_t longest = avg_len > max_len ? avg_len : max_len;
+  if (longest < (base <= 40 ? 384 : 576)) return 1;
+  // Up to one wave of CTAs, the chain of 48-token tiles in a CTA (0.4 to 0.6 us a tile) stands against what a split adds
+  // to the merge and the launch (about 0.07 us): L / 48 / s * 0.6 + 0.07 s is least near s = sqrt(L / 6) (us, 1 request:
+  // 1500 tokens 9.3 in 8, 7.7 in 16, 9.1 in 64; 131072 tokens 116 in 32, 92 in 64).
+  int64_t fit = static_cast<int64_t>(std::sqrt(static_cast<double>(longest) / 6.0) + 0.5);
+  if (fit > 64) fit = 64;
+  if (fit < by_slots) return static_cast<int>(fit);
+  fit = by_slots;
+  // Equal-length CTAs that all fit the resident slots at once finish together, while any overflow runs as a thin
+  // second wave: the largest count that fits one wave, where that fills three quarters of it.  Per-rank shapes of
+  // Llama-3.1-8B at TP 2 / 4 / 8, batch 64 x 4k: 2 / 4 / 9 splits = 512 / 512 / 576 CTAs on 592 slots (90.8 / 50.7 /
+  // 29.9 us) against 93.9 / 56.4 / 35.3 us for the oversubscription rule below; 1 split (512 CTAs, no merge) 170.4 us
+  // against 174.4 + merge.
+  // Not for few splits of unequal requests, where the longest ones would run alone at the end (us, one wave or 1.5 ->
+  // 2.1 times the slots: 40 x up to 3000 tokens 61.3 -> 57.9, 64 x up to 4096 FP8 77.0 -> 69.3, 27 x up to 6000 FP8
+  // 50.4 -> 48.2); short ones lose more to the merge than the even end gives.
+  const bool unequal = max_len * 8 > avg_len * 9;
+  if (fit >= 1 && static_cast<double>(base * fit) >= 0.75 * static_cast<double>(slots) &&
+      !(unequal && by_slots < 4 && avg_len >= 1536))
     return static_cast<int>(fit);
-  // HBM-bound: what matters is that enough CTAs stay resident until the end, not whole waves — late CTAs run faster
-  // because they share the bandwidth with fewer neighbours.  The smallest split count that oversubscribes the
-  // resident slots (measured on cfg 2: s = 2 -> 1.7x beats s = 1 -> 0.86x by 20 % and s = 8 by 4 %), with at least 4
-  // CTA tiles (192 tokens) per split.
-  const double over = ragged ? 2.1 : 1.5;
-  int64_t max_s = avg_len / (4 * align);
-  if (max_s > 64) max_s = 64;
-  for (int s = 1; s <= max_s; ++s)
-    if (static_cast<double>(base * s) >= over * static_cast<double>(slots)) return s;
-  return static_cast<int>(max_s > fit ? max_s : (fit > 1 ? fit : 1));
+  // HBM-bound: what matters is that enough CTAs stay resident until the end, not whole waves: late CTAs run faster
+  // because they share the bandwidth with fewer neighbours.  The smallest split count that oversubscribes the resident
+  // slots, where the requests are long enough for it (40 equal requests, 1 / 3 splits: 1024 tokens 37.6 / 39.9 us, 3000
+  // tokens 94.4 / 88.6).
+  const double over = unequal ? 2.1 : 1.5;
+  const int64_t least = unequal ? 192 : 640;
+  for (int64_t s = 1; s < 64 && avg_len >= least * s; ++s)
+    if (static_cast<double>(base * s) >= over * static_cast<double>(slots)) return static_cast<int>(s);
+  return static_cast<int>(fit > 1 ? fit : 1);
 }
 
 int b200_attn_decode_num_splits(int bs, int Hkv, int group, int D, int64_t avg_len, int num_sms) {

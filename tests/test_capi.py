@@ -56,6 +56,41 @@ def test_host_side_helpers_need_no_gpu(lib_path):
     assert lib.b200_attn_decode_split_align(128, 4) == 48  # 3 warps x 16-token tiles
 
 
+@pytest.mark.parametrize("bs,hkv,group,d,avg,longest,splits", [
+    # short requests are not split, few ones from 384 tokens on, many from 576 on
+    (1, 8, 4, 128, 128, 0, 1), (1, 8, 4, 128, 383, 0, 1), (1, 8, 4, 128, 384, 0, 8), (16, 8, 4, 128, 512, 0, 1),
+    (16, 8, 4, 128, 700, 0, 4), (5, 8, 4, 128, 300, 400, 8),
+    # few requests: splits grow with the root of the longest, up to 64
+    (1, 8, 4, 128, 1500, 0, 16), (1, 8, 4, 128, 4096, 0, 26), (1, 2, 4, 128, 16384, 0, 52), (1, 8, 4, 128, 131072, 0, 64),
+    (1, 8, 4, 128, 1000000, 0, 64), (2, 2, 7, 64, 1000, 4096, 26),
+    # one full wave of CTAs
+    (5, 8, 4, 128, 8192, 0, 14), (40, 4, 5, 128, 2048, 0, 3), (64, 8, 4, 128, 4096, 0, 1), (64, 8, 4, 128, 131072, 0, 1),
+    # a wave that would be half empty: oversubscribed where the requests are long enough
+    (40, 8, 4, 128, 1024, 0, 1), (40, 8, 4, 128, 3000, 0, 3),
+    # unequal requests with few splits: twice the slots
+    (64, 8, 4, 128, 2500, 4096, 3), (27, 8, 4, 128, 3600, 6000, 6), (64, 8, 4, 128, 1000, 1100, 1),
+])
+def test_split_rule(lib_path, bs, hkv, group, d, avg, longest, splits):
+    from sglang_security_b200 import _lib
+
+    lib = _lib.load()
+    if longest == 0:
+        assert lib.b200_attn_decode_num_splits(bs, hkv, group, d, avg, 148) == splits
+        longest = avg
+    assert lib.b200_attn_decode_num_splits_ragged(bs, hkv, group, d, avg, longest, 148) == splits
+
+
+def test_split_rule_stays_within_the_workspace_of_graphs(lib_path):
+    from sglang_security_b200 import _lib
+
+    lib = _lib.load()
+    for bs in (1, 3, 17, 64, 300, 5000):
+        for hkv in (1, 2, 8, 32):
+            for avg in (1, 47, 500, 3000, 70000, 1 << 22):
+                for longest in (avg, 3 * avg, 1 << 23):
+                    assert 1 <= lib.b200_attn_decode_num_splits_ragged(bs, hkv, 4, 128, avg, longest, 148) <= 64
+
+
 def test_noalloc_decode_rejects_oversize_requests_before_touching_the_gpu(lib_path):
     """b200_attn_decode_noalloc: the size check against the built-in 8 MiB scratch comes before any
     CUDA call, so it can be exercised here (pointers are never dereferenced)."""
