@@ -331,12 +331,13 @@ static int launch_block_gemm_bn(const void* a, int64_t lda, const void* b, int64
   p.splits = 1;
   p.kb_per_split = num_kb;
   if (BN == 128) {
-    // Largest split whose clusters are all resident, with 4 K blocks or more per slice.  Both sides on B200 (us,
-    // unsplit -> split, 128 tokens): 6144 x 4096 13.0 -> 12.3 in 2, 4096 x 14336 31.8 -> 16.3 in 4; with more
-    // tiles than half the SMs there is nothing to split for.
+    // Largest split whose clusters are all resident, with 4 K blocks or more per slice, where it takes 12 blocks or
+    // more off the chain: the exchange of the partials costs as much as that (split - whole, us, median of 25 to 34
+    // problems of 33 to 777 tokens: 3 blocks saved +1.7, 8 +1.0, 10 0, 12 -0.4, 16 -1.2, 24 -2.9; 4096 x 14336, 128
+    // tokens 31.8 -> 16.3 in 4).  With more tiles than half the SMs there is nothing to split for.
     for (int S = sms / tiles < 8 ? sms / tiles : 8; S > 1; --S) {
       const int per = ceil_div(num_kb, S);
-      if (per < 4 || (S - 1) * per >= num_kb || block_clusters<OutT, BN>(S) < tiles) continue;
+      if (per < 4 || num_kb - per < 12 || (S - 1) * per >= num_kb || block_clusters<OutT, BN>(S) < tiles) continue;
       p.splits = S;
       p.kb_per_split = per;
       break;
