@@ -27,6 +27,7 @@ struct BlockGemmParams {
   // few tiles: a cluster of `splits` CTAs takes one tile, each a slice of K; see the epilogue
   int splits, kb_per_split;
   int* wait_error;  // tc::report_gave_up
+  int vec_ok;       // rows of `out` take 16-byte stores
 };
 
 static WaitCounter wait_counter_registered(tc::wait_counter());
@@ -224,7 +225,7 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
 #pragma unroll
           for (int j = 0; j < 8; ++j)
             if (bias && col0 + j < p.N) sum[j] += to_float<OutT>(bias[col0 + j]);
-          if (col0 + 8 <= p.N && (p.ldc & 7) == 0) {
+          if (col0 + 8 <= p.N && p.vec_ok) {
             *reinterpret_cast<uint4*>(o8) = make_uint4(pack_out2<OutT>(sum[0], sum[1]), pack_out2<OutT>(sum[2], sum[3]),
                                                        pack_out2<OutT>(sum[4], sum[5]), pack_out2<OutT>(sum[6], sum[7]));
           } else {
@@ -238,7 +239,7 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
       } else if (row_ok && blk_ok) {
         OutT* orow = out + static_cast<int64_t>(row) * p.ldc;
         const int col0 = col_base;
-        if (col0 + COLS <= p.N && (p.ldc & 7) == 0) {
+        if (col0 + COLS <= p.N && p.vec_ok) {
 #pragma unroll
           for (int v = 0; v < COLS / 8; ++v) {
             uint32_t packed[4];
@@ -328,6 +329,7 @@ static int launch_block_gemm_bn(const void* a, int64_t lda, const void* b, int64
   const int tiles = ceil_div(p.M, 128) * ceil_div(p.N, BN);
   const int sms = device_sm_count();
   const int num_kb = ceil_div(p.K, 128);
+  p.vec_ok = p.ldc % 8 == 0 && aligned16(p.out);
   p.splits = 1;
   p.kb_per_split = num_kb;
   if (BN == 128) {

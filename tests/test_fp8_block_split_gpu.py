@@ -1,5 +1,6 @@
 """Block-scaled FP8 GEMM with K split over a cluster, against float64: ragged last slices, a ragged last K block, channel
-counts that 128 does not divide, a bias.
+counts that 128 does not divide, a bias, and rows of the output that 16-byte stores do not fit (a row stride that 8 does
+not divide, a first row that does not start on 16 bytes).
 
 Bound per element: one rounding to the output type (2^-8 of the result for bf16, 2^-11 for f16) and fp32 sums of K scaled
 products in any order, K * 2^-24 of the sum of their magnitudes."""
@@ -55,3 +56,21 @@ def test_split(m, n, k, split, dtype):
         assert (_splits() > 1) == split
         _check(out, ref if c is None else ref + c.double(), mags if c is None else mags + c.double().abs(), k)
         assert torch.equal(out, fp8_blockwise_scaled_mm(a, b, sa, sb, dtype, c))
+
+
+@pytest.mark.parametrize("m,n,k", [(40, 200, 2176), (40, 256, 512), (64, 136, 4096), (200, 4096, 256)])
+@pytest.mark.parametrize("pad,shift", [(4, 0), (8, 1), (8, 4), (7, 3)])
+def test_rows_that_wide_stores_do_not_fit(m, n, k, pad, shift):
+    """The output as a window of a larger tensor: its neighbours keep their values."""
+    from sglang_security_b200 import _lib
+
+    a, b, sa, sb, bias, ref, mags = _problem(m, n, k, torch.bfloat16)
+    ld = (n + 7) // 8 * 8 + pad
+    whole = torch.full((m * ld + 16,), 7.0, device="cuda", dtype=torch.bfloat16)
+    out = whole[shift:shift + m * ld].view(m, ld)
+    rc = _lib.load().b200_fp8_gemm_block128(
+        a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0), sa.data_ptr(), sa.stride(0), sa.stride(1), sb.data_ptr(),
+        sb.stride(0), bias.data_ptr(), out.data_ptr(), ld, m, n, k, _lib.dtype_code(torch.bfloat16), _lib.current_stream())
+    _lib.check(rc, "b200_fp8_gemm_block128")
+    _check(out[:, :n], ref + bias.double(), mags + bias.double().abs(), k)
+    assert bool((out[:, n:] == 7.0).all()) and bool((whole[:shift] == 7.0).all()) and bool((whole[shift + m * ld:] == 7.0).all())
