@@ -612,19 +612,50 @@ static void fit_cap_polynomial(double mult, double range, float* c) {
   for (int i = 0; i < N; ++i) c[i] = static_cast<float>(a[i]);
 }
 
+// Expected microseconds of a plain call on either kernel, from 594 calls timed on both (1 to 8 requests of 1 to 8192 new
+// tokens, 1024 to 8192 keys, groups of 4, 5 and 7 heads): a fixed part per CTA and a time per key tile, times the waves
+// of CTAs (a wave that is not full costs most of a whole one; with more than one wave the causal half of the new tokens
+// is not seen).  Half of the estimates are within 5 %, nine in ten within 22 %; the kernel that they pick is 0.9 % slower
+// than the better one on average (the two-tile kernel for all of them 2.2 %, and up to 38 % where its CTAs need a second
+// wave: 8 turns of 64 tokens behind 1000, groups of 5, 34 us here, 45 there; up to 26 % at head size 64: 256 tokens
+// behind 768 21 / 26).
+static double extend_waves(double ctas, int resident, double tail) {
+  const double x = ctas / resident;
+  return x <= 1.0 ? 1.0 : x + tail * (std::ceil(x) - x);
+}
+static double extend_keys(const ExtendParams& p, int max_extend_len, int keys, double waves) {
+  return p.causal && waves > 1.0 ? keys - 0.5 * max_extend_len : keys;
+}
+static double narrow_us(int D, const ExtendParams& p, int bs, int max_extend_len, int keys) {
+  const int sms = device_sm_count();
+  const double ctas = static_cast<double>(ceil_div(max_extend_len, 128 / p.pack)) * p.Hkv * p.head_tiles * bs;
+  const double waves = extend_waves(ctas, 2 * sms, 0.75);
+  const double tile = ctas <= sms ? (D == 128 ? 1.07 : 0.76) : (D == 128 ? 1.46 : 1.04);   // alone on its SM, or two
+  return waves * (9.0 + extend_keys(p, max_extend_len, keys, waves) / kKvTile * tile);
+}
+static double wide_us(int D, const ExtendParams& p, int max_extend_len, int keys, int64_t ctas, int splits) {
+  const double waves = extend_waves(static_cast<double>(ctas), device_sm_count(), D == 128 ? 0.9 : 0.75);
+  const double tile = max_extend_len <= 128 / p.pack ? (D == 128 ? 1.4 : 1.04) : (D == 128 ? 1.96 : 1.93);   // one query tile, or two
+  const double tiles = std::ceil(extend_keys(p, max_extend_len, keys, waves) / kWideTile / splits);
+  return 3.0 + waves * ((D == 128 ? 11.0 : 8.0) + tiles * tile) + (splits > 1 ? 3.2 : 0.0);
+}
+
 template <typename T, int D>
 static int launch_extend(const ExtendParams& p, int n_values, int bs, int max_extend_len, int max_kv_len,
                          cudaStream_t st) {
   // a cap up to 40 keeps e^(-2 cap) a normal fp32 (and 16-bit) number: the one-pass capped form
   const float ref = p.score_bound > 0.f && p.score_bound < p.logit_cap ? p.score_bound : p.logit_cap;
   const bool fast = ref <= 40.f && p.qk_scale > 0.f && extend_fast_softmax_enabled();
-  // Plain attention over 1024 keys or more: two query tiles per CTA.  All options, and shorter requests, on the kernel
-  // above, whose two CTAs per SM hide what a CTA of the other spends before its first and after its last tile
-  // (~8 us; us, this / that kernel: 8 x 512 fresh tokens 63.6 / 72.3, 8 x 1024 160 / 153, 8 x 1536 299 / 254, 24 new
-  // tokens behind 512 / 1024 / 1536 cached 21.9 / 20.1, 30.9 / 22.8, 39.2 / 21.3).
+  // Plain attention over 1024 keys or more: two query tiles per CTA where that is expected to end sooner.  All options,
+  // and shorter requests, on the kernel above, whose two CTAs per SM hide what a CTA of the other spends before its first
+  // and after its last tile (~8 us; us, this / that kernel: 8 x 512 fresh tokens 63.6 / 72.3).
   const int keys = max_kv_len > 0 ? max_kv_len : max_extend_len;
-  if (fast && keys >= 1024 && p.logit_cap <= 0.f && p.window == 0 && !p.sink && !p.gate && !p.lse && n_values == 1 && p.v_head < 0)
-    return launch_extend_wide<T, D>(p, bs, max_extend_len, max_kv_len, st);
+  if (fast && keys >= 1024 && p.logit_cap <= 0.f && p.window == 0 && !p.sink && !p.gate && !p.lse && n_values == 1 && p.v_head < 0) {
+    int splits = 1;
+    const int64_t ctas = wide_ctas<T, D>(p, bs, max_extend_len, max_kv_len, &splits);
+    if (wide_us(D, p, max_extend_len, keys, ctas, splits) <= narrow_us(D, p, bs, max_extend_len, keys))
+      return launch_extend_wide<T, D>(p, bs, max_extend_len, splits, st);
+  }
   note_variant("attn_extend d=%d fast_softmax=%d values=%d", D, fast ? 1 : 0, n_values);
   if (n_values == 2)
     return fast ? launch_extend_inst<T, D, 1, 2>(p, bs, max_extend_len, st)

@@ -481,24 +481,29 @@ static int wide_clusters(int S) {
   return n > 0 ? n : 0;
 }
 
+// CTAs of a call before its keys are split, and the split: the longest request's keys are cut while whole clusters still
+// fit the idle SMs and a CTA keeps three key tiles (~1.8 us each; launch and merge of a cluster cost ~3).  us, one CTA ->
+// split: 64 tokens behind 8192, two kv heads 117 -> 36; 128 behind 4000, eight 68 -> 36; 30 behind 2000 47 -> 22.
 template <typename T, int D>
-static int launch_extend_wide(const ExtendParams& p_in, int bs, int max_extend_len, int max_kv_len, cudaStream_t st) {
+static int64_t wide_ctas(const ExtendParams& p, int bs, int max_extend_len, int max_kv_len, int* splits) {
+  const int64_t ctas = static_cast<int64_t>(ceil_div(max_extend_len, 256 / p.pack)) * p.Hkv * p.head_tiles * bs;
+  *splits = 1;
+  for (int S = 8; S > 1 && ctas < device_sm_count(); S /= 2)   // (the occupancy answer also raises the shared memory limit)
+    if (max_kv_len >= 3 * S * kWideTile && wide_clusters<T, D>(S) >= ctas) {
+      *splits = S;
+      break;
+    }
+  return ctas;
+}
+
+template <typename T, int D>
+static int launch_extend_wide(const ExtendParams& p_in, int bs, int max_extend_len, int splits, cudaStream_t st) {
   using C = WideCfg<D>;
   ExtendParams p = p_in;
   if (const int rc = wait_error_arm("attn_extend", &p.wait_error)) return rc;
   B200_CUDA_OK(cudaFuncSetAttribute(attn_extend_wide_kernel<T, D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     C::SMEM_BYTES));
-  const int resident = device_sm_count();
-  const int64_t ctas = static_cast<int64_t>(ceil_div(max_extend_len, 256 / p.pack)) * p.Hkv * p.head_tiles * bs;
-  // The longest request's keys are cut while whole clusters still fit the idle SMs and a CTA keeps three key tiles
-  // (~1.8 us each; launch and merge of a cluster cost ~3).  us, one CTA -> split:
-  // 64 tokens behind 8192, two kv heads 117 -> 36; 128 behind 4000, eight 68 -> 36; 30 behind 2000 47 -> 22.
-  p.kv_splits = 1;
-  for (int S = 8; S > 1 && ctas < resident; S /= 2)   // (the occupancy answer also raises the shared memory limit)
-    if (max_kv_len >= 3 * S * kWideTile && wide_clusters<T, D>(S) >= ctas) {
-      p.kv_splits = S;
-      break;
-    }
+  p.kv_splits = splits;
   const dim3 grid(ceil_div(max_extend_len, 256 / p.pack) * p.kv_splits, p.Hkv * p.head_tiles, bs);
   note_variant("attn_extend_wide d=%d splits=%d", D, p.kv_splits);
   {
