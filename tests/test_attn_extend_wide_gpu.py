@@ -65,3 +65,58 @@ def test_growing_scores_rescale(d):
     case.k_cache[slots] *= ramp[:, None, None].to(case.k_cache.dtype)
     case.k_new *= ramp[1200:, None, None].to(case.k_new.dtype)
     _run(case)
+
+
+@pytest.mark.parametrize("hq,hkv,d,prefix,ext,splits", [
+    (4, 1, 128, [1300, 40, 0], [70, 33, 1], 2),
+    (4, 1, 128, [3400, 100], [30, 65], 8),
+    (8, 1, 64, [2940, 500], [40, 17], 4),
+    (8, 8, 128, [900, 1000, 1100, 20, 300], [400, 270, 129, 400, 1], 1),
+])
+def test_every_key_visible(hq, hkv, d, prefix, ext, splits):
+    """No causal mask (encoder layers): every new token sees all keys of its request, also on keys spread over ranks."""
+    from sglang_security_b200 import _lib
+
+    g = torch.Generator(device="cuda").manual_seed(sum(prefix) + d)
+    total = [p + e for p, e in zip(prefix, ext)]
+    slots = torch.randperm(sum(total), device="cuda", generator=g) + 1
+    r2t = torch.zeros(len(ext), max(total), device="cuda", dtype=torch.int32)
+    rows, at = [], 0
+    for b, n in enumerate(total):
+        r2t[b, :n] = slots[at:at + n].to(torch.int32)
+        at += n
+    kc, vc = (torch.randn(sum(total) + 1, hkv, d, device="cuda", generator=g).to(torch.bfloat16) for _ in range(2))
+    q = torch.randn(sum(ext), hq * d, device="cuda", generator=g).to(torch.bfloat16)
+    o = torch.empty_like(q)
+    i32 = lambda x: torch.tensor(x, device="cuda", dtype=torch.int32)
+    lens, pre = i32(ext), i32(prefix)
+    starts = torch.empty_like(lens)
+    lib, st = _lib.load(), _lib.current_stream()
+    _lib.check(lib.b200_extend_starts(lens.data_ptr(), starts.data_ptr(), len(ext), st), "b200_extend_starts")
+    idx, seq = torch.arange(len(ext), device="cuda"), torch.tensor(total, device="cuda")
+    _lib.check(lib.b200_attn_extend_known(
+        q.data_ptr(), q.stride(0), kc.data_ptr(), vc.data_ptr(), hkv * d, o.data_ptr(), o.stride(0), r2t.data_ptr(),
+        r2t.stride(0), idx.data_ptr(), seq.data_ptr(), pre.data_ptr(), lens.data_ptr(), starts.data_ptr(), len(ext),
+        max(ext), max(total), hq, hkv, d, d, d ** -0.5, 0.0, 1.0, 0, _lib.dtype_code(q.dtype), st), "b200_attn_extend_known")
+    assert _lib.last_variant() == f"attn_extend_wide d={d} splits={splits}"
+    row = 0
+    for b, n in enumerate(total):
+        at = r2t[b, :n].long()
+        for h in range(hq):
+            kb, vb = kc[at, h // (hq // hkv)].double(), vc[at, h // (hq // hkv)].double()
+            qb = q[row:row + ext[b], h * d:(h + 1) * d].double()
+            ref = (qb @ kb.t() * d ** -0.5).softmax(-1) @ vb
+            got = o[row:row + ext[b], h * d:(h + 1) * d].double()
+            assert (got - ref).abs().max() <= 0.047 and (got - ref).norm() <= 6e-3 * ref.norm()
+        row += ext[b]
+
+
+@pytest.mark.parametrize("bs", [1, 2, 255, 256, 257, 1000])
+def test_start_rows(bs):
+    from sglang_security_b200 import _lib
+
+    lens = torch.randint(0, 9000, (bs,), device="cuda", dtype=torch.int32)
+    starts = torch.full_like(lens, -1)
+    _lib.check(_lib.load().b200_extend_starts(lens.data_ptr(), starts.data_ptr(), bs, _lib.current_stream()),
+               "b200_extend_starts")
+    assert torch.equal(starts.long(), lens.long().cumsum(0) - lens.long())
