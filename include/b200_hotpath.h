@@ -389,6 +389,8 @@ int b200_w4a16_gemv_config(int max_m, int splits);
 /* Prefill sizes with the stream copy (b200_w4a16_gemv_v2_repack): expands the weight into `workspace` (16-bit [N, K])
  * and runs the CTA-pair GEMM.  N % 16 == 0, K % 64 == 0, group_size % 8 == 0. */
 size_t b200_w4a16_gemm_stream_workspace_bytes(int N, int K);
+/* 1 where this is expected to be faster than b200_w4a16_gemm. */
+int b200_w4a16_gemm_stream_pays(int M, int N, int K);
 int b200_w4a16_gemm_stream(const void* x, int64_t ldx, const void* qweight_stream, const void* zeros, const void* scales,
                            const void* bias, void* out, int64_t ldc, int M, int N, int K, int group_size,
                            void* workspace, size_t workspace_bytes, int dtype, void* stream);

@@ -835,6 +835,21 @@ int b200_w4a16_repack_gptq(const void* qweight, const int32_t* perm, void* out, 
   return 0;
 }
 
+// Expansion + CTA-pair GEMM (w4a16_stream_gemm.cu) against the fused kernel, from 200 problems of 520 to 3072 tokens timed
+// on both (the rule's choice is 0.5 % slower than the better one on average).  The expansion is spread over enough
+// tokens from about 1200 on (us, fused / two passes: 27648 x 5120, 1300 tokens 347 / 315; 4096 x 4096, 1300: 62 / 44).
+// Below, it costs more than it gives where the fused kernel's tiles fill one wave (4096 x 4096, 1024 tokens 32.5 / 35.3;
+// 4096 x 1024, 1024 tokens 13.9 / 16.3), and of wide weights it has the most to write (13824 x 5120, 900 tokens 109 /
+// 120).  Small weights never pay the second launch (1024 x 1024, 2048 tokens 10.6 / 14.0).
+int b200_w4a16_gemm_stream_pays(int M, int N, int K) {
+  using namespace b200;
+  if (M <= 512 || static_cast<int64_t>(N) * K < (1 << 21)) return 0;
+  if (M >= 1200) return 1;
+  const int sms = device_sm_count(), bm = w4_pick_bm(M, N, K, sms);
+  if (static_cast<int64_t>(ceil_div(M, bm)) * ceil_div(N, 128) > sms) return N <= 8192;
+  return static_cast<double>(M) * N < (bm == 256 ? 0.6 : 0.7) * sms * bm * 128.0;
+}
+
 int b200_w4a16_gemm(const void* x, int64_t ldx, const void* qweight, const void* zeros,
                     const void* scales, const void* bias, void* out, int64_t ldc, int M, int N,
                     int K, int group_size, int dtype, void* stream) {

@@ -148,12 +148,8 @@ def w4a16_gemv_v2_config(splits: int = 0) -> None:
 GEMV_V2_MAX_M = int(os.environ.get("B200_W4A16_GEMV2_MAX_M", "16"))
 
 
-def stream_gemm_pays(m: int, n: int) -> bool:
-    """Expansion + GEMM against the fused kernel (us, Qwen2.5-32B at TP 2, fused / two passes): the expansion is spread
-    over enough tokens from 1500 on (gate_up 1500: 354 / 350, 2048: 466 / 425, 3001: 727 / 609; 1024: 235 / 248), and
-    narrow weights leave the fused kernel's tiles too few (777 tokens, qkv / o / down: 38.5 / 31.0, 41.8 / 27.1,
-    173 / 125)."""
-    return m >= 1500 or (m > 512 and n <= 8192)
+def stream_gemm_pays(m: int, n: int, k: int) -> bool:
+    return bool(_lib.load().b200_w4a16_gemm_stream_pays(int(m), int(n), int(k)))
 
 
 def stream_copy_enabled() -> bool:
@@ -169,7 +165,7 @@ def w4a16_linear(x2: torch.Tensor, layer, bias: Optional[torch.Tensor]) -> torch
     if stream is not None and 1 <= m <= GEMV_V2_MAX_M and gemv_v2_supported(
             m, layer.scales.shape[1], x2.shape[1], layer.w4a16_group_size):
         return w4a16_gemv_v2(x2, stream, layer.b200_zeros, layer.scales, layer.w4a16_group_size, bias)
-    if (stream is not None and stream_gemm_pays(m, layer.scales.shape[1]) and layer.w4a16_group_size % 8 == 0
+    if (stream is not None and stream_gemm_pays(m, layer.scales.shape[1], x2.shape[1]) and layer.w4a16_group_size % 8 == 0
             and x2.stride(0) % 8 == 0 and x2.data_ptr() % 16 == 0):
         try:
             return w4a16_gemm_stream(x2, stream, layer.b200_zeros, layer.scales, layer.w4a16_group_size, bias)

@@ -46,7 +46,7 @@ def test_layer_dispatch(m, two_pass):
     from sglang_security_b200.layers.linear import ColumnParallelLinear
     from sglang_security_b200.layers.quantization.awq import AWQConfig
 
-    k, n, dtype = 512, 1024, torch.float16
+    k, n, dtype = 2048, 1024, torch.float16               # 2^21 weights: the smallest that are expanded
     q, z, s, g = _packed(k, n, 128, dtype, m)
     layer = ColumnParallelLinear(k, n, bias=False, params_dtype=dtype, quant_config=AWQConfig(4, 128, True), tp_rank=0,
                                  tp_size=1).cuda()
@@ -68,7 +68,7 @@ def test_no_room_for_the_expanded_weight(monkeypatch):
     from sglang_security_b200 import _lib
     from sglang_security_b200.layers.quantization import w4a16_kernel as W
 
-    k, n, m, dtype = 512, 1024, 1500, torch.float16
+    k, n, m, dtype = 2048, 1024, 1500, torch.float16
     q, z, s, g = _packed(k, n, 128, dtype, 5)
     layer = torch.nn.Module()
     layer.qweight, layer.scales, layer.w4a16_group_size = q, s, 128
