@@ -10,7 +10,8 @@ import torch
 from torch.nn import Parameter
 
 from .base_config import LinearMethodBase, QuantizationConfig, set_weight_attrs
-from .w4a16_kernel import gemv_stream_repack, stream_copy_enabled, unpack_zeros, w4a16_linear
+from .w4a16_kernel import (gemv_stream_repack, reserve_expand_scratch, stream_copy_enabled, unpack_zeros,
+                           w4a16_linear)
 
 
 def is_layer_skipped_awq(prefix: str, modules_to_not_convert: List[str]) -> bool:
@@ -106,6 +107,8 @@ class AWQLinearMethod(LinearMethodBase):
         # (+0.5 byte per weight; B200_W4A16_STREAM_COPY=0 keeps only the [K, N/8] layout)
         layer.b200_qweight_stream = (gemv_stream_repack(layer.qweight.data)
                                      if stream_copy_enabled() else None)
+        layer.b200_expand_scratch = reserve_expand_scratch(layer.b200_qweight_stream, layer.scales.shape[1],
+                                                           layer.qweight.data.shape[0])
 
     def apply(self, layer: torch.nn.Module, x: torch.Tensor,
               bias: Optional[torch.Tensor] = None) -> torch.Tensor:

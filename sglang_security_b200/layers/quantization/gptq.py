@@ -13,7 +13,7 @@ import torch
 from torch.nn import Parameter
 
 from .base_config import LinearMethodBase, QuantizationConfig, set_weight_attrs
-from .w4a16_kernel import (gemv_stream_repack, repack_gptq, stream_copy_enabled, unpack_zeros,
+from .w4a16_kernel import (gemv_stream_repack, repack_gptq, reserve_expand_scratch, stream_copy_enabled, unpack_zeros,
                            w4a16_linear)
 
 
@@ -123,6 +123,8 @@ class GPTQLinearMethod(LinearMethodBase):
         # (+0.5 byte per weight; B200_W4A16_STREAM_COPY=0 keeps only the [K, N/8] layout)
         layer.b200_qweight_stream = (gemv_stream_repack(layer.b200_qweight)
                                      if stream_copy_enabled() else None)
+        layer.b200_expand_scratch = reserve_expand_scratch(layer.b200_qweight_stream, layer.scales.shape[1],
+                                                           layer.b200_qweight.shape[0])
 
     def apply(self, layer: torch.nn.Module, x: torch.Tensor,
               bias: Optional[torch.Tensor] = None) -> torch.Tensor:

@@ -1,7 +1,10 @@
 """INT4 weight-only kernels bound through the C-ABI (AWQ dequant, one-time repacks, fused GEMM)."""
 from __future__ import annotations
 
+import contextlib
 import os
+import threading
+import weakref
 from typing import Optional
 
 import torch
@@ -116,10 +119,75 @@ def w4a16_gemv_v2(x: torch.Tensor, qweight_stream: torch.Tensor, zeros: torch.Te
     return out
 
 
+class ExpandScratch:
+    """Device memory for the 16-bit form of one int4 weight at a time (w4a16_gemm_stream: 283 MB for 27648 x 5120).
+
+    One per device, shared by the layers that were loaded there and as large as the largest of their weights.  It is
+    taken when weights are loaded, before a KV pool is sized to what is left of the card, and given back with the last
+    layer that holds it.  Threads take turns at launching; a launch on another stream than the last one's waits for that
+    one on the device."""
+    _of_device = weakref.WeakValueDictionary()
+    _guard = threading.Lock()
+
+    def __init__(self, device: torch.device):
+        self.device, self.buf, self.lock = device, None, threading.Lock()
+        self.home = self.last = self.done = None      # streams of the allocation and of the last use, its end
+
+    @classmethod
+    def reserve(cls, device: torch.device, nbytes: int) -> "ExpandScratch":
+        """The device's scratch, of nbytes or more (or of what it had before, where there is no room for that)."""
+        with cls._guard:
+            scratch = cls._of_device.get(device.index)
+            if scratch is None:
+                scratch = cls._of_device[device.index] = cls(device)
+        with scratch.lock:
+            if scratch.size() < nbytes:
+                try:
+                    scratch.buf = torch.empty(nbytes, dtype=torch.uint8, device=device)
+                except torch.cuda.OutOfMemoryError:
+                    return scratch
+                scratch.home = scratch.last = torch.cuda.current_stream(device)
+                scratch.done = scratch.home.record_event()
+        return scratch
+
+    def size(self) -> int:
+        return 0 if self.buf is None else self.buf.numel()
+
+    @contextlib.contextmanager
+    def borrow(self):
+        """The memory, for launches on the current stream inside the block."""
+        with self.lock:
+            stream = torch.cuda.current_stream(self.device)
+            if stream != self.last:
+                stream.wait_event(self.done)
+            if stream != self.home:
+                self.buf.record_stream(stream)
+            try:
+                yield self.buf
+            finally:
+                self.last = stream
+                self.done.record(stream)
+
+    def __deepcopy__(self, memo):
+        return self
+
+    def __reduce__(self):
+        return ExpandScratch.reserve, (self.device, self.size())
+
+
+def reserve_expand_scratch(qweight_stream: Optional[torch.Tensor], n: int, k: int) -> Optional[ExpandScratch]:
+    """Of a layer whose weights have been loaded; None for one that w4a16_gemm_stream never takes."""
+    if qweight_stream is None or not stream_gemm_pays(1 << 20, n, k):
+        return None
+    return ExpandScratch.reserve(qweight_stream.device, _lib.load().b200_w4a16_gemm_stream_workspace_bytes(n, k))
+
+
 def w4a16_gemm_stream(x: torch.Tensor, qweight_stream: torch.Tensor, zeros: torch.Tensor, scales: torch.Tensor,
-                      group_size: int, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
+                      group_size: int, bias: Optional[torch.Tensor] = None,
+                      scratch: Optional[ExpandScratch] = None) -> torch.Tensor:
     """x [M, K] @ dequant(stream-layout weight) (+ bias) -> [M, N] in two passes: the weight is expanded to a 16-bit
-    [N, K] scratch tensor, then multiplied by the CTA-pair GEMM (csrc/w4a16_stream_gemm.cu)."""
+    [N, K] scratch tensor, then multiplied by the CTA-pair GEMM (csrc/w4a16_stream_gemm.cu).  Without `scratch`, and in
+    a graph that is being captured (whose launches run whenever it is replayed), the scratch tensor is the call's own."""
     _cuda(x, "w4a16_gemm_stream")
     if x.dim() != 2 or x.stride(-1) != 1:
         raise _lib.B200Error("w4a16_gemm_stream: x must be 2-D with contiguous rows")
@@ -130,11 +198,15 @@ def w4a16_gemm_stream(x: torch.Tensor, qweight_stream: torch.Tensor, zeros: torc
     out = torch.empty((m, n), device=x.device, dtype=x.dtype)
     if bias is not None and bias.dtype != x.dtype:
         bias = bias.to(x.dtype)
-    ws = torch.empty(n * k, device=x.device, dtype=x.dtype)
-    rc = _lib.load().b200_w4a16_gemm_stream(x.data_ptr(), x.stride(0), qweight_stream.data_ptr(), zeros.data_ptr(),
-                                            scales.data_ptr(), _lib.ptr(bias), out.data_ptr(), out.stride(0), m, n, k,
-                                            group_size, ws.data_ptr(), ws.numel() * ws.element_size(),
-                                            _lib.dtype_code(x.dtype), _lib.current_stream())
+    if scratch is None or torch.cuda.is_current_stream_capturing():
+        memory = contextlib.nullcontext(torch.empty(2 * n * k, device=x.device, dtype=torch.uint8))
+    else:
+        memory = scratch.borrow()
+    with memory as ws:
+        rc = _lib.load().b200_w4a16_gemm_stream(x.data_ptr(), x.stride(0), qweight_stream.data_ptr(), zeros.data_ptr(),
+                                                scales.data_ptr(), _lib.ptr(bias), out.data_ptr(), out.stride(0), m, n, k,
+                                                group_size, ws.data_ptr(), ws.numel(), _lib.dtype_code(x.dtype),
+                                                _lib.current_stream())
     _lib.check(rc, "b200_w4a16_gemm_stream")
     return out
 
@@ -165,12 +237,17 @@ def w4a16_linear(x2: torch.Tensor, layer, bias: Optional[torch.Tensor]) -> torch
     if stream is not None and 1 <= m <= GEMV_V2_MAX_M and gemv_v2_supported(
             m, layer.scales.shape[1], x2.shape[1], layer.w4a16_group_size):
         return w4a16_gemv_v2(x2, stream, layer.b200_zeros, layer.scales, layer.w4a16_group_size, bias)
-    if (stream is not None and stream_gemm_pays(m, layer.scales.shape[1], x2.shape[1]) and layer.w4a16_group_size % 8 == 0
+    n = layer.scales.shape[1]
+    if (stream is not None and stream_gemm_pays(m, n, x2.shape[1]) and layer.w4a16_group_size % 8 == 0
             and x2.stride(0) % 8 == 0 and x2.data_ptr() % 16 == 0):
-        try:
-            return w4a16_gemm_stream(x2, stream, layer.b200_zeros, layer.scales, layer.w4a16_group_size, bias)
-        except torch.cuda.OutOfMemoryError:
-            pass    # no room for the expanded weight: the fused kernel needs none
+        # the fused kernel needs no memory: it takes over where the expanded weight found none when it was loaded, and
+        # where a capture finds none
+        scratch = getattr(layer, "b200_expand_scratch", None)
+        if scratch is None or (scratch.size() >= 2 * n * x2.shape[1] and scratch.device == x2.device):
+            try:
+                return w4a16_gemm_stream(x2, stream, layer.b200_zeros, layer.scales, layer.w4a16_group_size, bias, scratch)
+            except torch.cuda.OutOfMemoryError:
+                pass
     packed = layer.b200_qweight if hasattr(layer, "b200_qweight") else layer.qweight  # GPTQ / AWQ
     return w4a16_gemm(x2, packed, layer.b200_zeros, layer.scales, layer.w4a16_group_size, bias)
 

@@ -83,3 +83,108 @@ def test_no_room_for_the_expanded_weight(monkeypatch):
     out = W.w4a16_linear(x, layer, None)
     assert not _lib.last_variant().endswith("expanded")
     _check(out, x, OI.awq_dequantize_oracle(q, s, z, 128), None)
+
+
+def _awq_layer(k, n, dtype, seed):
+    from sglang_security_b200.layers.linear import ColumnParallelLinear
+    from sglang_security_b200.layers.quantization.awq import AWQConfig
+
+    q, z, s, g = _packed(k, n, 128, dtype, seed)
+    layer = ColumnParallelLinear(k, n, bias=False, params_dtype=dtype, quant_config=AWQConfig(4, 128, True), tp_rank=0,
+                                 tp_size=1).cuda()
+    for p, v in ((layer.qweight, q), (layer.qzeros, z), (layer.scales, s)):
+        p.data.copy_(v)
+    layer.quant_method.process_weights_after_loading(layer)
+    return layer, OI.awq_dequantize_oracle(q, s, z, 128), g
+
+
+def test_scratch_is_taken_with_the_weights_and_given_back():
+    """A call allocates its output and no more; all layers of the device hold the same memory, also a copied and an
+    unpickled one; it grows with a larger weight and goes with the last layer."""
+    import copy
+    import gc
+    import pickle
+
+    from sglang_security_b200 import _lib
+    from sglang_security_b200.layers.quantization.w4a16_kernel import ExpandScratch
+
+    gc.collect()
+    dtype, m = torch.float16, 1500
+    a, wa, g = _awq_layer(2048, 1024, dtype, 1)
+    scratch = a.b200_expand_scratch
+    assert scratch.size() >= 2048 * 1024 * 2
+    b, wb, _ = _awq_layer(2048, 4096, dtype, 2)
+    assert b.b200_expand_scratch is scratch and scratch.size() >= 2048 * 4096 * 2
+    assert copy.deepcopy(scratch) is scratch and pickle.loads(pickle.dumps(scratch)) is scratch
+    x = torch.randn(m, 2048, device="cuda", generator=g).to(dtype)
+    for layer, w, n in ((a, wa, 1024), (b, wb, 4096)):
+        out, _ = layer(x)
+        torch.cuda.synchronize()
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        again, _ = layer(x)
+        assert torch.cuda.max_memory_allocated() - before <= m * n * 2 + 4096
+        assert _lib.last_variant().endswith("expanded")
+        assert torch.equal(out, again)
+        _check(out, x, w, None)
+    small, _, _ = _awq_layer(512, 1024, dtype, 3)
+    assert small.b200_expand_scratch is None                              # never expanded
+    held = torch.cuda.memory_allocated()
+    size = scratch.size()
+    del a, b, layer, scratch
+    gc.collect()
+    assert torch.device("cuda", 0).index not in ExpandScratch._of_device and torch.cuda.memory_allocated() <= held - size
+
+
+def test_no_room_when_the_weights_were_loaded(monkeypatch):
+    """The fused kernel runs, and the allocator is not asked for the expanded weight again."""
+    from sglang_security_b200 import _lib
+    from sglang_security_b200.layers.quantization import w4a16_kernel as W
+
+    real = torch.empty
+    asked = []
+
+    def empty(*a, **kw):
+        if kw.get("dtype") == torch.uint8:
+            asked.append(a)
+            raise torch.cuda.OutOfMemoryError("no room")
+        return real(*a, **kw)
+
+    monkeypatch.setattr(W.torch, "empty", empty)
+    layer, w, g = _awq_layer(2048, 1024, torch.float16, 4)
+    assert len(asked) == 1 and layer.b200_expand_scratch.size() == 0
+    x = torch.randn(1500, 2048, device="cuda", generator=g).to(torch.float16)
+    for _ in range(3):
+        out, _ = layer(x)
+        assert not _lib.last_variant().endswith("expanded")
+    assert len(asked) == 1
+    _check(out, x, w, None)
+
+
+def test_layers_on_two_streams_and_in_a_graph():
+    """Layers that share the scratch, launched in turns on two streams without a synchronisation, beside replays of a
+    captured one."""
+    dtype, m = torch.float16, 1500
+    a, wa, g = _awq_layer(4096, 2048, dtype, 5)
+    b, wb, _ = _awq_layer(4096, 2048, dtype, 6)
+    x = torch.randn(m, 4096, device="cuda", generator=g).to(dtype)
+    ra, rb = a(x)[0].clone(), b(x)[0].clone()
+    _check(ra, x, wa, None)
+    _check(rb, x, wb, None)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        captured, _ = a(x)
+    s1, s2, s3 = (torch.cuda.Stream() for _ in range(3))
+    torch.cuda.synchronize()
+    outs = []
+    for _ in range(6):
+        with torch.cuda.stream(s1):
+            outs.append((a(x)[0], ra))
+        with torch.cuda.stream(s2):
+            outs.append((b(x)[0], rb))
+        with torch.cuda.stream(s3):
+            graph.replay()
+    torch.cuda.synchronize()
+    for o, r in outs:
+        assert torch.equal(o, r)
+    assert torch.equal(captured, ra)
