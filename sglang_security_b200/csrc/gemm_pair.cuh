@@ -487,10 +487,8 @@ int launch_gemm_pair(const void* x, int64_t ldx, const void* w, int64_t ldw, con
   if (rc) return rc;
   const int tiles = ceil_div(ep.M, plan.bn) * ceil_div(ep.N, 256);
   const int clusters = plan.splits > 1 || tiles < clusters_of[1] ? tiles : clusters_of[1];
-  // mc: the 128-token blocks come in full pairs
-  note_variant("gemm_tn kind=%d bn=%d stages=%d mc=%d splits=%d out=%s grid=%d", KIND, plan.bn, plan.stages,
-               ceil_div(ep.M, 128) % 2 == 0 ? 1 : 0, plan.splits, std::is_same<OutT, __half>::value ? "f16" : "bf16",
-               clusters * 2 * plan.splits);
+  note_variant("gemm_tn kind=%d bn=%d stages=%d splits=%d out=%s grid=%d", KIND, plan.bn, plan.stages, plan.splits,
+               std::is_same<OutT, __half>::value ? "f16" : "bf16", clusters * 2 * plan.splits);
   {
     ScopedKernelTimer timer(timer_name, st);
     B200_CUDA_OK(launch_kernel(gemm_pair_kernel<KIND, OutT, ACT>, dim3(clusters * 2 * plan.splits), dim3(kPairThreads),

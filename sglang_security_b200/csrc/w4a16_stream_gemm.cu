@@ -112,7 +112,11 @@ int b200_w4a16_gemm_stream(const void* x, int64_t ldx, const void* qweight_strea
   const int rc = dtype == B200_F16
                      ? launch_gemm_pair<kKindF16, __half>(x, ldx, workspace, K, ep, st, "w4a16_gemm", false)
                      : launch_gemm_pair<kKindBf16, __nv_bfloat16>(x, ldx, workspace, K, ep, st, "w4a16_gemm", false);
-  note_variant("w4a16_gemm bm=256 swap=0 splits=1 expanded");
+  if (rc == 0) {
+    char pair[128];
+    std::snprintf(pair, sizeof(pair), "%s", b200_last_variant());
+    note_variant("w4a16_expand + %s expanded", pair);
+  }
   return rc;
 }
 

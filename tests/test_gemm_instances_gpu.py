@@ -3,13 +3,15 @@ against the oracle functions run on the GPU in fp32 (TF32 off; the checker may u
 the product may not).  Every case asserts WHICH kernel instance the dispatcher picked
 (b200_last_variant) so a shape cannot silently fall back to a smaller tile.
 
-  FP8 per-token x per-channel: 128x256 tiles, CTA pairs with TMA-multicast weights (even number of
-      M blocks, bf16 and f16), the non-multicast 128x256 path (odd), 128x128 tiles with cluster
-      split-K; all four Llama-3.1-8B shapes of BASELINE cfg 3 at M in {512, 2048, 8192}
+  FP8 per-token x per-channel: CTA pairs on 256-token tiles and narrower ones, even and odd numbers of 128-token
+      blocks, bf16 and f16, a channel count that 256 does not divide; all four Llama-3.1-8B shapes at M in
+      {512, 2048, 8192}
   FP8 block-scaled: the 128x256-tile kernel (needs >= 1.5 tiles per SM)
   W4A16: the 256-row (two-accumulator) instance and the 128-row persistent instance on the
-      Qwen2.5-32B TP=2 shapes of cfg 4
+      Qwen2.5-32B TP=2 shapes, and the layer on whichever of fused kernel and two passes it picks
 """
+import re
+
 import pytest
 import torch
 
@@ -63,16 +65,13 @@ def test_fp8_rowcol_cfg3_shapes(m, n, k):
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     assert v.startswith("gemm_tn kind=0"), v
     assert ("bn=256" in v) == (tiles256 >= sms), (v, tiles256)
-    if tiles256 >= sms:
-        assert "mc=1" in v, v          # even number of M blocks -> multicast pairs
 
 
-@pytest.mark.parametrize("m,out_dtype,mc", [(2048, torch.bfloat16, 1), (2048, torch.float16, 1),
-                                            (2176, torch.bfloat16, 0), (2176, torch.float16, 0),
-                                            (4096 + 128, torch.bfloat16, 0)])
-def test_fp8_rowcol_bn256_multicast_and_plain(m, out_dtype, mc):
-    """fp8_gemm.cu tile dispatch: even ceil(M/128) -> CTA pairs sharing the weight tile by TMA
-    multicast; odd -> the plain 128x256 persistent kernel.  Ragged N (not a multiple of 256)."""
+@pytest.mark.parametrize("m,out_dtype", [(2048, torch.bfloat16), (2048, torch.float16), (2176, torch.bfloat16),
+                                         (2176, torch.float16), (4096 + 128, torch.bfloat16)])
+def test_fp8_rowcol_several_tiles_per_pair(m, out_dtype):
+    """More tiles than CTA pairs: accumulators, ring and staged scales go on from tile to tile.  Ragged N (not a multiple
+    of 256), even and odd numbers of 128-token blocks."""
     from sglang_security_b200.layers.quantization.fp8_kernel import fp8_scaled_mm
 
     n, k = 6144 + 80, 1152
@@ -82,7 +81,9 @@ def test_fp8_rowcol_bn256_multicast_and_plain(m, out_dtype, mc):
     sb = torch.rand((n,), generator=g, device="cuda") * 1e-3
     out = fp8_scaled_mm(a, b.t(), sa, sb, out_dtype)
     v = _variant()
-    assert "bn=256" in v and f"mc={mc}" in v and ("f16" if out_dtype == torch.float16 else "bf16") in v, v
+    assert v.startswith("gemm_tn kind=0") and "splits=1" in v and ("out=f16" if out_dtype == torch.float16 else "out=bf16") in v, v
+    bn, grid = (int(re.search(rf"{name}=(\d+)", v).group(1)) for name in ("bn", "grid"))
+    assert -(-m // bn) * -(-n // 256) > grid // 2, v
     ref = OF.scaled_mm_oracle(a, b.t(), sa, sb, out_dtype, None)
     torch.testing.assert_close(out, ref, rtol=0.02, atol=1)
     scale = max(1.0, ref.float().abs().max().item())
@@ -141,7 +142,7 @@ def test_block_oracle_gpu_form_equals_cpu_oracle():
 
 
 def _awq_realistic(k, n, group, dtype, g):
-    """Asymmetric group quantisation of N(0, 0.02) weights (SURVEY §8d cfg 4 realistic variant)."""
+    """Asymmetric group quantisation of N(0, 0.02) weights."""
     w = torch.randn((k, n), generator=g, device="cuda") * 0.02
     wg = w.view(k // group, group, n)
     lo, hi = wg.amin(1), wg.amax(1)
@@ -158,10 +159,12 @@ def _awq_realistic(k, n, group, dtype, g):
                                       (512, 3584, 5120, 128), (2048, 5120, 13824, 256)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_w4a16_large_m_instances(m, n, k, bm, dtype):
-    """Qwen2.5-32B TP=2 shapes (cfg 4) at prefill-chunk M: the 256-row two-accumulator instance
-    (w4a16.cu w4_pick_bm) and the 128-row persistent one, through AWQLinearMethod.apply."""
+    """Qwen2.5-32B TP=2 shapes at prefill-chunk M: the 256-row two-accumulator instance
+    (w4a16.cu w4_pick_bm) and the 128-row persistent one, called directly (the layer expands the weight at most of these
+    sizes, and takes this kernel where there is no room for that), and AWQLinearMethod.apply."""
     from sglang_security_b200.layers.linear import ColumnParallelLinear
     from sglang_security_b200.layers.quantization.awq import AWQConfig
+    from sglang_security_b200.layers.quantization.w4a16_kernel import stream_gemm_pays, w4a16_gemm
 
     group = 128
     g = torch.Generator(device="cuda").manual_seed(m + n + k)
@@ -175,15 +178,18 @@ def test_w4a16_large_m_instances(m, n, k, bm, dtype):
     layer.scales.data.copy_(scales)
     layer.bias.data.copy_(bias)
     layer.quant_method.process_weights_after_loading(layer)
-    out, _ = layer(x)
+    fused = lambda: w4a16_gemm(x, layer.qweight, layer.b200_zeros, layer.scales, group, layer.bias)
+    out = fused()
     v = _variant()
     assert v.startswith(f"w4a16_gemm bm={bm} swap=0"), v
     w = OI.awq_dequantize_oracle(qweight, scales, qzeros, group)
     ref = OI.w4a16_linear_oracle(x, w, bias)
-    err = (out.float() - ref.float()).abs()
     tol = 1e-2 * ref.float().abs() + 1e-2 * ref.float().abs().max()
-    assert (err <= tol).all(), (err.max().item(), ref.float().abs().max().item())
-    # regression: the packed ring used to be released to its TMA refill without a cross-proxy fence
-    # (stale weights whenever the MMA pipe was the bottleneck, different on every run)
-    out2, _ = layer(x)
-    assert torch.equal(out, out2), "w4a16 GEMM is not deterministic run to run"
+    for call in (fused, lambda: layer(x)[0]):
+        out = call()
+        err = (out.float() - ref.float()).abs()
+        assert (err <= tol).all(), (err.max().item(), ref.float().abs().max().item())
+        # regression: the packed ring used to be released to its TMA refill without a cross-proxy fence
+        # (stale weights whenever the MMA pipe was the bottleneck, different on every run)
+        assert torch.equal(out, call()), "w4a16 GEMM is not deterministic run to run"
+    assert _variant().startswith("w4a16_expand + gemm_tn") == stream_gemm_pays(m, n, k), _variant()
