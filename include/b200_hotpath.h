@@ -231,8 +231,6 @@ int b200_attn_extend(const void* q, int64_t q_stride, const void* k_cache, const
                      int D, int Dv, float scale, float logit_cap, int causal, int dtype,
                      void* stream);
 
-/* Same kernel with an output multiplier: extend over an FP8 KV pool runs on an exact 16-bit copy
- * of the requests' rows (b200_kv_dequant_gather) with scale * k_scale and out_scale = v_scale.    */
 /* b200_attn_extend_scaled for callers that know the longest request (max_kv_len = its prefix + new tokens, on the
  * host): few query tiles over many keys are then spread over clusters.  0: not known. */
 int b200_attn_extend_known(const void* q, int64_t q_stride, const void* k_cache, const void* v_cache,
@@ -244,6 +242,8 @@ int b200_attn_extend_known(const void* q, int64_t q_stride, const void* k_cache,
                            void* stream);
 /* Start row of every request: exclusive sums of extend_seq_lens. */
 int b200_extend_starts(const int32_t* extend_seq_lens, int32_t* extend_start_loc, int bs, void* stream);
+/* Same kernel with an output multiplier: extend over an FP8 KV pool runs on an exact 16-bit copy
+ * of the requests' rows (b200_kv_dequant_gather) with scale * k_scale and out_scale = v_scale.    */
 int b200_attn_extend_scaled(const void* q, int64_t q_stride, const void* k_cache,
                             const void* v_cache, int64_t kv_row_stride, void* o, int64_t o_stride,
                             const int32_t* req_to_token, int64_t req_to_token_stride,
@@ -412,7 +412,7 @@ int b200_w4a16_gemv_v2(const void* x, int64_t ldx, const void* qweight_stream, c
 int b200_w4a16_gemv_v2_supported(int M, int N, int K, int group_size);
 int b200_w4a16_gemv_v2_config(int splits);
 
-/* ---- steps either side of the GEMMs / attention (SURVEY section 8f rows 1-2) ------------------ */
+/* ---- steps either side of the GEMMs / attention ------------------ */
 /* (residual +) RMSNorm, optionally fused with the FP8 activation quantiser of the linear layer that
  * consumes it.  Replaces RMSNorm.forward (python/sglang/srt/layers/layernorm.py:61-108; oracle =
  * forward_native :88-108; GPU = sgl_kernel rmsnorm / fused_add_rmsnorm) followed by
@@ -502,7 +502,7 @@ int b200_fp8_gemm_rowcol_ar(void* comm, const void* a, int64_t lda, const void* 
 int b200_comm_fuse_config(int max_m);
 
 /* NVLS: all-reduce with the additions done inside the NVSwitch (multimem.ld_reduce over a multicast
- * mapping; csrc/comm_nvls.cu).  SURVEY section 8f row 3; reference analogue = the one-shot kernel of
+ * mapping; csrc/comm_nvls.cu).  Reference analogue = the one-shot kernel of
  * custom_all_reduce.cuh:203-225 (adds on the SM) and NCCL's NVLS algorithms.  Life cycle (host side:
  * distributed/device_communicators/b200_all_reduce.py):
  *   b200_nvls_supported()                      1 when device + driver offer multicast objects

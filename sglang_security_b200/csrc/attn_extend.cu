@@ -117,13 +117,13 @@ __device__ __forceinline__ uint32_t pack16(float a, float b) {
   }
 }
 
-// FAST (round 2): the softmax warps are the limiter (ncu: issue 56 %, ALU 43 %, tensor 36 %), so the
+// FAST: the softmax warps are the limiter (ncu: issue 56 %, ALU 43 %, tensor 36 %), so the
 // per-element instruction count of the common tile is cut from ~7.5 to ~3: the causal / length mask
 // is applied only on tiles that cross the row's last visible key, the row max is taken on the RAW
 // scores with three-input max (scale > 0 commutes with max), scale and max-subtraction are ONE
 // packed FFMA2 per two elements (exp2(s * scale - m)), and the row sum accumulates with FFMA2.
 // Same values up to fp32 rounding of the fused multiply-add.  Not used with logit capping or a
-// non-positive scale (dispatch falls back to the FAST = false instance, unchanged from round 1).
+// non-positive scale (dispatch falls back to the FAST = false instance).
 // FAST == 2: capped scores whose bound keeps |x| = |raw * scale / cap| below kCapPolyMax: tanh is a polynomial
 // there (fitted by the host to the range), so a score costs one exponential, as without a cap, and packed
 // multiply-adds instead of an exponential and a division; the bound is the reference of every exponent.
@@ -563,7 +563,7 @@ namespace b200 {
 
 static WaitCounter wait_counter_registered(tc::wait_counter());
 
-// B200_EXTEND_FAST_SOFTMAX=0 selects the round-1 softmax for every call (read per launch: A/B tools flip it)
+// B200_EXTEND_FAST_SOFTMAX=0 selects the FAST = 0 softmax for every call (read per launch: A/B tools flip it)
 static bool extend_fast_softmax_enabled() {
   const char* e = std::getenv("B200_EXTEND_FAST_SOFTMAX");
   return !(e && e[0] == '0');
@@ -635,7 +635,8 @@ static double narrow_us(int D, const ExtendParams& p, int bs, int max_extend_len
 }
 static double wide_us(int D, const ExtendParams& p, int max_extend_len, int keys, int64_t ctas, int splits) {
   const double waves = extend_waves(static_cast<double>(ctas), device_sm_count(), D == 128 ? 0.9 : 0.75);
-  const double tile = max_extend_len <= 128 / p.pack ? (D == 128 ? 1.4 : 1.04) : (D == 128 ? 1.96 : 1.93);   // one query tile, or two
+  const bool one = max_extend_len <= 128 / p.pack;             // query tile a CTA, or two
+  const double tile = D == 128 ? (one ? 1.4 : 1.96) : (one ? 1.04 : 1.93);
   const double tiles = std::ceil(extend_keys(p, max_extend_len, keys, waves) / kWideTile / splits);
   return 3.0 + waves * ((D == 128 ? 11.0 : 8.0) + tiles * tile) + (splits > 1 ? 3.2 : 0.0);
 }

@@ -1,5 +1,5 @@
 // NVLS: all-reduce whose additions happen INSIDE the NVSwitch (multimem.ld_reduce over a multicast
-// mapping) — SURVEY §8f row 3.  Reference analogue: the one-shot kernel of the custom all-reduce
+// mapping).  Reference analogue: the one-shot kernel of the custom all-reduce
 // (sgl-kernel/csrc/allreduce/custom_all_reduce.cuh:203-225, policy custom_all_reduce.py:414-437),
 // which pulls every peer's buffer over NVLink and adds on the SM; NCCL's NVLS algorithms are the
 // library form of what is done here.

@@ -1,4 +1,4 @@
-// The steps either side of every GEMM / attention call of a decoder layer (SURVEY §8f rows 1-2),
+// The steps either side of every GEMM / attention call of a decoder layer,
 // fused so that a decode step launches one kernel where the reference launches two or three:
 //
 //   b200_rmsnorm        (residual +) RMSNorm [-> FP8 per-token / per-128-group quant]

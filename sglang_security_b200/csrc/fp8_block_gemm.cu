@@ -383,7 +383,7 @@ static int fp8_gemm_block128_impl(const void* a, int64_t lda, const void* b, int
                "b200_fp8_gemm_block128: out dtype %d", out_dtype);
   cudaStream_t st0 = static_cast<cudaStream_t>(stream);
   // (block-scaled: up to 32 tokens; from there the promotion loops over 64 and 128 tokens per channel are slower
-  // than the big tile: 64 tokens, us, qkv / o / gate_up / down 21.2 / 15.1 / 54.4 / 32.7 against 11.8 / 9.5 / 26.5 / 15.9)
+  // than the big tile: 64 tokens, us, qkv / o / gate_up / down 21.3 / 15.1 / 56.0 / 33.7 against 11.8 / 9.7 / 28.0 / 17.3)
   const bool fuse_ar = M <= 64 && comm_can_fuse(comm, M, N);
   if (fuse_ar || (M <= smallm_max_m() && (M <= 32 || smallm_forced()))) {  // decode regime: weight streaming, swap-AB + cluster split-K
     SmallMParams sp = {};

@@ -2,7 +2,7 @@
 //
 // Replaces the same reference ops as fp8_gemm.cu / fp8_block_gemm.cu (sgl_kernel.fp8_scaled_mm,
 // fp8_gemm_kernel.cu:1071-1146; fp8_blockwise_scaled_mm / w8a8_block_fp8_matmul,
-// fp8_kernel.py:774-891) for the decode batch sizes of BASELINE cfg 3 (M = 1..128).
+// fp8_kernel.py:774-891) for the decode batch sizes (M = 1..128).
 //
 // Why a second kernel: with M <= 128 there is exactly one 128-row token tile, so the big-tile
 // kernel launches only N/128 CTAs (32..48 for the attention projections) and most SMs never touch

@@ -8,9 +8,9 @@
 // waves (pair_pick).  What bounds it: wide tiles the tensor cores (0.37 us per K block of 256 x 256, the library's
 // rate too), narrow ones the ring's round trip of ~1.3 us, small problems the ~4 us of launch, fill and epilogue.
 // Measured against one CTA per 128x256 / 128x128 tile with a one-lane producer and issuer (N x K of Llama-3.1-8B's
-// qkv / o / gate_up / down, us before -> now): e4m3 M 300: 14.2 / 13.7 / 47.8 / 36.6 -> 11.1 / 11.2 / 38.3 / 20.1;
-// e4m3 M 2048: 45.3 / 31.0 / 191 / 96.1 -> 40.6 / 28.4 / 175 / 89.6; bf16 M 777: 53.3 / 41.9 / 165 / 128 -> 34.3 /
-// 24.9 / 145 / 77.8.
+// qkv / o / gate_up / down, weights from HBM, us before -> now): e4m3 M 300: 14.9 / 13.3 / 46.8 / 37.8 -> 11.3 / 9.7 /
+// 35.9 / 21.5; e4m3 M 2048: 44.8 / 30.7 / 194 / 93.3 -> 39.3 / 27.8 / 174 / 85.0; bf16 M 777: 54.5 / 42.4 / 163 / 129 ->
+// 34.2 / 25.3 / 142 / 73.2.
 //
 //   warp 0    TMA producer, in both CTAs; the bytes of both are credited to the leader's full barrier
 //   warp 1    MMA issuer (leader only); commits multicast to both CTAs' empty / accumulator barriers

@@ -23,9 +23,9 @@ std::atomic<int> g_pdl_on{pdl_default()};
 int pdl_max_tokens() {
   static int v = [] {
     const char* e = std::getenv("B200_PDL_MAX_M");
-    // 512: re-measured in round 2 on the whole-model decode step (profiles/r02_bench_pdl.json): batch
+    // 512: measured on the whole-model decode step (profiles/r02_bench_pdl.json): batch
     // 64 x 4k 8.11 ms with PDL against 8.25 ms without; batch 128 / 256 @ 1k 5.99 / 9.62 ms against
-    // 6.20 / 9.84 ms with a limit of 64 tokens (round 1 had measured a loss from 64 tokens on)
+    // 6.20 / 9.84 ms with a limit of 64 tokens
     return (e && *e) ? std::atoi(e) : 512;
   }();
   return v;

@@ -1,4 +1,4 @@
-// Scheduler-side index kernels around the attention hot path (SURVEY §8f rank 4): pure int64 /
+// Scheduler-side index kernels around the attention hot path: pure int64 /
 // int32 index arithmetic, bit-exact with the reference's Triton kernels.
 //   b200_write_req_to_token  write_req_to_token_pool_triton   managers/schedule_batch.py:1789-1823
 //   b200_get_last_loc        get_last_loc_kernel / _torch     managers/schedule_batch.py:1838-1893

@@ -207,7 +207,7 @@ class B200AttnBackend(AttentionBackend):
         k_cache = pool.get_key_buffer(layer.layer_id)
         v_cache = pool.get_value_buffer(layer.layer_id)
         if k.dtype != k_cache.dtype:
-            # quantised KV cache (FP8): scaling/cast order is owned by the pool (SURVEY §8f rank 1)
+            # quantised KV cache (FP8): scaling/cast order is owned by the pool
             ks, vs = self._kv_scales(layer)
             pool.set_kv_buffer(layer, forward_batch.out_cache_loc, k, v, ks, vs)
         else:
@@ -237,8 +237,7 @@ class B200AttnBackend(AttentionBackend):
         window = getattr(layer, "sliding_window_size", None)
         if window is not None and window > 0:
             raise NotImplementedError(
-                f"B200AttnBackend: sliding_window_size={window} is not implemented "
-                "(no BASELINE config uses a window)")
+                f"B200AttnBackend: sliding_window_size={window} is not implemented")
         if getattr(layer, "is_cross_attention", False):
             raise NotImplementedError("B200AttnBackend: cross-attention layers are not implemented")
 
