@@ -70,9 +70,10 @@ int b200_wait_selftest(void* stream);
  * library is launched with cudaLaunchAttributeProgrammaticStreamSerialization and orders its own
  * dependent accesses with griddepcontrol.wait, so consecutive kernels of a decode step overlap
  * launch latency, prologue and weight prefetch with the tail of their predecessor (also inside a
- * captured CUDA graph).  Only up to 512 tokens (env B200_PDL_MAX_M), and there one access is not ordered:
- * a GEMM may read its weight operand before the launch just before it has ended, so that launch must not
- * be a kernel of this library that writes the weight.  Returns the previous setting. */
+ * captured CUDA graph).  Up to 512 tokens (env B200_PDL_MAX_M; 16-bit and per-channel FP8 GEMMs at
+ * every count unless it is set).  Up to 512 tokens one access is not ordered: a GEMM may read its weight
+ * operand before the launch just before it has ended, so that launch must not be a kernel of this library
+ * that writes the weight.  Returns the previous setting. */
 int b200_set_pdl(int on);
 
 /* Per-kernel device timing for bench.py's roofline leg: while enabled, the dominant kernels are

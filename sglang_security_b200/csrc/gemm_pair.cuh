@@ -37,6 +37,7 @@ struct PairParams {
   int stages;           // operand ring
   int splits, kb_per_split;
   int vec_ok;           // rows of `out` take 16-byte stores
+  int early_w;          // the first weight tiles may be read before the dependency wait
   float act_pos, act_neg;
   int* wait_error;      // tc::report_gave_up
 };
@@ -147,10 +148,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   tc::tc_fence_after();
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
 
-  // the weight never depends on the previous kernel: its first stages are requested before the dependency wait
+  // where the weight does not depend on the previous kernel, its first stages are requested before the dependency wait
   int w_ahead = 0;
   const uint32_t stage_tx = 2u * (W_BYTES + x_bytes);
-  if (warp == 0 && cluster_id < num_tiles) {
+  if (warp == 0 && cluster_id < num_tiles && p.early_w) {
     const int n_row = (cluster_id / tok_blocks) * 256 + static_cast<int>(half) * 128;
     w_ahead = min(p.stages, kb1 - kb0);
     if (tc::elect_one()) {
@@ -451,8 +452,8 @@ int pair_clusters(int S) {
   return n > 0 ? n : 0;
 }
 
-// old_weight: the launch just before this one does not write w, whose first tiles are read before the dependency wait
-// where the launch is a dependent one (pdl_family: up to 512 tokens).
+// old_weight: the launch just before this one does not write w, whose first tiles are read before the dependency wait up
+// to pdl_max_tokens() tokens; above, w is read after it.
 template <int KIND, typename OutT, bool ACT = false>
 int launch_gemm_pair(const void* x, int64_t ldx, const void* w, int64_t ldw, const GemmEpilogueParams& ep,
                      cudaStream_t st, const char* timer_name, bool old_weight = true) {
@@ -482,6 +483,8 @@ int launch_gemm_pair(const void* x, int64_t ldx, const void* w, int64_t ldw, con
   p.splits = plan.splits;
   p.kb_per_split = plan.kb_per_split;
   p.vec_ok = ep.ldc % 8 == 0 && aligned16(ep.out);
+  const int family = old_weight ? pdl_gemm_family(ep.M, kPdlGemmBig) : 0;
+  p.early_w = family == 0 || ep.M <= pdl_max_tokens();
   p.act_pos = ep.act_pos;
   p.act_neg = ep.act_neg;
   rc = wait_error_arm(timer_name, &p.wait_error);
@@ -493,8 +496,7 @@ int launch_gemm_pair(const void* x, int64_t ldx, const void* w, int64_t ldw, con
   {
     ScopedKernelTimer timer(timer_name, st);
     B200_CUDA_OK(launch_kernel(gemm_pair_kernel<KIND, OutT, ACT>, dim3(clusters * 2 * plan.splits), dim3(kPairThreads),
-                               plan.smem, st, 2 * plan.splits, old_weight ? pdl_family(ep.M, kPdlGemmBig) : 0, tw, tx,
-                               p));
+                               plan.smem, st, 2 * plan.splits, family, tw, tx, p));
   }
   B200_CHECK_LAUNCH("gemm_pair_kernel");
   return 0;

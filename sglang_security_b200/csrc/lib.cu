@@ -20,15 +20,25 @@ static int pdl_default() {
 }
 std::atomic<int> g_pdl_on{pdl_default()};
 
+static const char* pdl_limit() {
+  const char* e = std::getenv("B200_PDL_MAX_M");
+  return e && *e ? e : nullptr;
+}
+
 int pdl_max_tokens() {
   static int v = [] {
-    const char* e = std::getenv("B200_PDL_MAX_M");
+    const char* e = pdl_limit();
     // 512: measured on the whole-model decode step (profiles/r02_bench_pdl.json): batch
     // 64 x 4k 8.11 ms with PDL against 8.25 ms without; batch 128 / 256 @ 1k 5.99 / 9.62 ms against
     // 6.20 / 9.84 ms with a limit of 64 tokens
-    return (e && *e) ? std::atoi(e) : 512;
+    return e ? std::atoi(e) : 512;
   }();
   return v;
+}
+
+int pdl_gemm_family(int tokens, int family) {
+  static const bool limited = pdl_limit() != nullptr;
+  return limited ? pdl_family(tokens, family) : family;
 }
 
 void set_error(const char* fmt, ...) {
