@@ -20,7 +20,6 @@
 //   accumulators and fp32 online softmax in registers (exp2 domain, scale*log2e folded in).
 //   Warps are merged once through shared memory; partials (normalised O, log2-domain LSE) go to
 //   the workspace and are merged by attn_merge_kernel.
-#include <cmath>
 #include <cstdlib>
 
 #include "common.cuh"
@@ -568,8 +567,8 @@ attn_decode_mma_kernel(const DecodeParams p) {
 // Merge of split partials: one warp per (query head, request), four columns per lane.  Latency-bound (a few hundred
 // KB): the split sums are read by all lanes at once and the first partial rows are requested before the sequence length
 // is known, so the chain is one round trip to L2, not one per split (1 request of 1500 tokens in 7 splits: 5.2 us, now
-// 3.8).  BYCOLS, for more splits than the rows requested ahead: the four warps of a CTA share the columns of a head, one
-// column per lane, so that 32 rows are requested together (64 splits are two round trips, not eight).
+// 3.8).  BYCOLS, for more splits than the rows requested ahead: the four warps of a CTA share the columns
+// of a head, one column per lane, so that 32 rows are requested together (64 splits are two round trips, not eight).
 // Sums run over the splits in order, as in attn_merge_quant_kernel: same bytes.
 constexpr int kMergeWarps = 4;
 
@@ -986,22 +985,32 @@ static int decode_num_splits(int bs, int Hkv, int group, int D, int64_t avg_len,
   const int ctas_per_sm = decode_ctas_per_sm(D);
   const int64_t slots = static_cast<int64_t>(num_sms) * ctas_per_sm;
   const int64_t by_slots = slots / base;
-  // Split counts from 1 to 64 were timed for 1592 batches (1 to 64 requests of 64 to 131072 tokens, equal and unequal
-  // ones, bf16 and FP8 rows, 2 to 8 kv heads): this rule's choice is 2.4 % slower than the best count on average.
-  // A request that is not split ends as soon as one that is (which costs a merge) up to some 384 tokens, and further up
-  // where the CTAs are many (us, whole / split: 1 x 128 tokens 6.0 / 7.6, 1 x 512 10.7 / 7.6, 16 x 384 9.7 / 10.7,
-  // 16 x 700 13.8 / 13.1).  The longest request is what the others are waited for.
+  // Up to one wave of CTAs: the chain of 48-token tiles in a CTA, which is slower with more CTAs on its SM, against the
+  // merge launch and what each split adds to it.  Microseconds fitted to 1592 batches (1 to 64 requests of 64 to 131072
+  // tokens, equal and unequal ones, bf16 and FP8 rows, 2 to 8 kv heads), each timed at up to 20 split counts; the
+  // choice is 2.0 % slower than the best of them on average.  The longest request is what the others are waited for.
+  // (us, 1 request: 128 tokens 5.8 whole, 7.4 in 2; 512 tokens 10.6 whole, 7.6 in 8, 7.1 in 12; 1500 tokens 9.3 in 8,
+  // 7.7 in 16, 9.1 in 64; 131072 tokens 116 in 32, 92 in 64; 16 requests: 384 tokens 9.6 whole, 10.5 in 2; 700 tokens
+  // 13.9 whole, 12.9 in 4, 15.4 in 8.)  From 900 tokens on, with fewer than 4 splits in the wave, the bandwidth
+  // decides.
   const int64_t longest = avg_len > max_len ? avg_len : max_len;
-  if (longest < (base <= 40 ? 384 : 576)) return 1;
-  // Up to one wave of CTAs, the chain of 48-token tiles in a CTA (0.4 to 0.6 us a tile) stands against what a split adds
-  // to the merge and the launch (about 0.07 us): L / 48 / s * 0.6 + 0.07 s is least near s = sqrt(L / 6) (us, 1 request:
-  // 1500 tokens 9.3 in 8, 7.7 in 16, 9.1 in 64; 131072 tokens 116 in 32, 92 in 64).
-  int64_t fit = static_cast<int64_t>(std::sqrt(static_cast<double>(longest) / 6.0) + 0.5);
-  if (fit > 64) fit = 64;
-  if (fit < by_slots) return static_cast<int>(fit);
-  fit = by_slots;
+  const int64_t align = decode_align();
+  constexpr double kTile[4] = {0.46, 0.62, 0.90, 0.82};        // 1 to 4 CTAs an SM
+  int64_t fit = 1;
+  double fit_us = 0.0;
+  for (int64_t s = 1; s <= 64 && (s == 1 || (s <= by_slots && s * align <= longest)); ++s) {
+    const int64_t tiles = ((longest + s - 1) / s + align - 1) / align;
+    const int64_t on_sm = (base * s + num_sms - 1) / num_sms;
+    const double us = 0.04 * s * (1.0 + 0.001 * base) + (s > 1 ? 2.0 + 0.009 * base : 0.0) +
+                      tiles * (on_sm <= 4 ? kTile[on_sm - 1] : 0.25 * kTile[3] * on_sm);
+    if (s == 1 || us < fit_us) {
+      fit = s;
+      fit_us = us;
+    }
+  }
+  if (by_slots >= 4 || longest < 900) return static_cast<int>(fit);
   // Equal-length CTAs that all fit the resident slots at once finish together, while any overflow runs as a thin
-  // second wave: the largest count that fits one wave, where that fills three quarters of it.  Per-rank shapes of
+  // second wave: the estimate's count, where one wave fills three quarters of the slots.  Per-rank shapes of
   // Llama-3.1-8B at TP 2 / 4 / 8, batch 64 x 4k: 2 / 4 / 9 splits = 512 / 512 / 576 CTAs on 592 slots (90.8 / 50.7 /
   // 29.9 us) against 93.9 / 56.4 / 35.3 us for the oversubscription rule below; 1 split (512 CTAs, no merge) 170.4 us
   // against 174.4 + merge.
@@ -1009,18 +1018,18 @@ static int decode_num_splits(int bs, int Hkv, int group, int D, int64_t avg_len,
   // 2.1 times the slots: 40 x up to 3000 tokens 61.3 -> 57.9, 64 x up to 4096 FP8 77.0 -> 69.3, 27 x up to 6000 FP8
   // 50.4 -> 48.2); short ones lose more to the merge than the even end gives.
   const bool unequal = max_len * 8 > avg_len * 9;
-  if (fit >= 1 && static_cast<double>(base * fit) >= 0.75 * static_cast<double>(slots) &&
-      !(unequal && by_slots < 4 && avg_len >= 1536))
+  if (by_slots >= 1 && static_cast<double>(base * by_slots) >= 0.75 * static_cast<double>(slots) &&
+      !(unequal && avg_len >= 1536))
     return static_cast<int>(fit);
   // HBM-bound: what matters is that enough CTAs stay resident until the end, not whole waves: late CTAs run faster
   // because they share the bandwidth with fewer neighbours.  The smallest split count that oversubscribes the resident
-  // slots, where the requests are long enough for it (40 equal requests, 1 / 3 splits: 1024 tokens 37.6 / 39.9 us, 3000
+  // slots, where the requests are long enough for it (40 equal requests, 1 / 3 splits: 1024 tokens 37.2 / 40.0 us, 3000
   // tokens 94.4 / 88.6).
   const double over = unequal ? 2.1 : 1.5;
   const int64_t least = unequal ? 192 : 640;
   for (int64_t s = 1; s < 64 && avg_len >= least * s; ++s)
     if (static_cast<double>(base * s) >= over * static_cast<double>(slots)) return static_cast<int>(s);
-  return static_cast<int>(fit > 1 ? fit : 1);
+  return static_cast<int>(fit);
 }
 
 int b200_attn_decode_num_splits(int bs, int Hkv, int group, int D, int64_t avg_len, int num_sms) {

@@ -185,8 +185,10 @@ class B200AttnBackend(AttentionBackend):
             raise ValueError(f"B200AttnBackend: cuda graph capture of {forward_mode!r} unsupported")
         if spec_info is not None:
             raise NotImplementedError("speculative decoding is outside the B200 hot-path scope")
-        # The split count is frozen into the captured launch: choose it for a nominal context.
-        s = min(64, self._num_splits(bs, self.v_head_dim, min(self.max_context_len, 4096)))
+        # The split count is frozen into the captured launch: choose it for a nominal context.  One request, 8 kv
+        # heads, 1500 / 4096 / 16384 / 65536 tokens, us: 18 splits (best for 4096) 7.8 / 10.1 / 18.8 / 92.9, the 32 of
+        # 6144 tokens 8.4 / 9.9 / 16.3 / 63.3; with many requests both lengths give the same count.
+        s = min(64, self._num_splits(bs, self.v_head_dim, min(self.max_context_len, 6144)))
         self.forward_metadata = ForwardMetadata(num_splits=s, workspace=self._graph_workspace)
         self._stage_graph_indices(self.forward_metadata, bs, req_pool_indices, seq_lens)
 

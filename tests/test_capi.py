@@ -57,12 +57,12 @@ def test_host_side_helpers_need_no_gpu(lib_path):
 
 
 @pytest.mark.parametrize("bs,hkv,group,d,avg,longest,splits", [
-    # short requests are not split, few ones from 384 tokens on, many from 576 on
-    (1, 8, 4, 128, 128, 0, 1), (1, 8, 4, 128, 383, 0, 1), (1, 8, 4, 128, 384, 0, 8), (16, 8, 4, 128, 512, 0, 1),
-    (16, 8, 4, 128, 700, 0, 4), (5, 8, 4, 128, 300, 400, 8),
-    # few requests: splits grow with the root of the longest, up to 64
-    (1, 8, 4, 128, 1500, 0, 16), (1, 8, 4, 128, 4096, 0, 26), (1, 2, 4, 128, 16384, 0, 52), (1, 8, 4, 128, 131072, 0, 64),
-    (1, 8, 4, 128, 1000000, 0, 64), (2, 2, 7, 64, 1000, 4096, 26),
+    # short requests are not split, few ones from some 300 tokens on, many from some 600 on
+    (1, 8, 4, 128, 128, 0, 1), (1, 8, 4, 128, 300, 0, 4), (1, 8, 4, 128, 384, 0, 8), (16, 8, 4, 128, 384, 0, 1),
+    (16, 8, 4, 128, 512, 0, 1), (16, 8, 4, 128, 700, 0, 4), (5, 8, 4, 128, 300, 400, 5),
+    # few requests: splits grow with the longest, up to 64
+    (1, 8, 4, 128, 1500, 0, 16), (1, 8, 4, 128, 4096, 0, 18), (1, 2, 4, 128, 16384, 0, 57), (1, 8, 4, 128, 131072, 0, 64),
+    (1, 8, 4, 128, 1000000, 0, 64), (2, 2, 7, 64, 1000, 4096, 29),
     # one full wave of CTAs
     (5, 8, 4, 128, 8192, 0, 14), (40, 4, 5, 128, 2048, 0, 3), (64, 8, 4, 128, 4096, 0, 1), (64, 8, 4, 128, 131072, 0, 1),
     # a wave that would be half empty: oversubscribed where the requests are long enough
