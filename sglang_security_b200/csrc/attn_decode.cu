@@ -567,7 +567,7 @@ attn_decode_mma_kernel(const DecodeParams p) {
 // Merge of split partials: one warp per (query head, request), four columns per lane.  Latency-bound (a few hundred
 // KB): the split sums are read by all lanes at once and the first partial rows are requested before the sequence length
 // is known, so the chain is one round trip to L2, not one per split (1 request of 1500 tokens in 7 splits: 5.2 us, now
-// 3.8).  BYCOLS, for more splits than the rows requested ahead: the four warps of a CTA share the columns
+// 3.8).  BYCOLS, for more splits than the rows requested ahead and few heads: the four warps of a CTA share the columns
 // of a head, one column per lane, so that 32 rows are requested together (64 splits are two round trips, not eight).
 // Sums run over the splits in order, as in attn_merge_quant_kernel: same bytes.
 constexpr int kMergeWarps = 4;
@@ -1052,7 +1052,10 @@ static int attn_merge_impl(const float* part_o, const float* part_lse, void* o, 
                num_splits, split_align);
   B200_REQUIRE(part_o && part_lse && o && seq_lens, "b200_attn_merge: null pointer");
   B200_REQUIRE(dtype == B200_BF16 || dtype == B200_F16, "b200_attn_merge: dtype %d", dtype);
-  const bool bycols = num_splits > 8;
+  // By columns while their CTAs, one per head, are at most two an SM: more CTAs cost what the round trips save (us, with
+  // the split kernel, a warp per head / by columns: 32 heads in 9 splits 8.1 / 7.4, 128 in 14 11.0 / 10.7, 256 in 10
+  // 13.4 / 12.9, 320 in 16 16.4 / 17.1, 512 in 10 18.8 / 19.4, 1024 in 12 44.2 / 44.8).
+  const bool bycols = num_splits > 8 && static_cast<int64_t>(bs) * Hq <= 2 * device_sm_count();
   dim3 grid(bycols ? Hq : ceil_div(Hq, kMergeWarps), bs);
   const int threads = kMergeWarps * 32;
   const bool wide = Dv % 4 == 0 && aligned16(part_o);

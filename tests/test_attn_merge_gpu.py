@@ -1,5 +1,6 @@
 """b200_attn_merge on its own: fewer and more splits than a warp's lanes and than the rows requested ahead, splits past
-a short request (whose partials hold garbage), value sizes with and without 16-byte rows, against float64.
+a short request (whose partials hold garbage), value sizes with and without 16-byte rows, few heads and
+more than two an SM, against float64.
 Bound: one rounding of the result plus fp32 sums over the splits."""
 import pytest
 import torch
@@ -8,11 +9,12 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("splits,dv", [(2, 128), (8, 64), (9, 128), (33, 128), (70, 192), (5, 6), (11, 37)])
-def test_merge(splits, dv, dtype):
+@pytest.mark.parametrize("splits,dv,hq", [(2, 128, 5), (8, 64, 5), (9, 128, 5), (33, 128, 5), (70, 192, 5), (5, 6, 5), (11, 37, 5),
+                                          (9, 128, 110), (33, 64, 110), (11, 37, 110)])
+def test_merge(splits, dv, hq, dtype):
     from sglang_security_b200 import _lib
 
-    align, bs, hq = 48, 3, 5
+    align, bs = 48, 3
     lens = torch.tensor([splits * align, 1, max(1, splits // 2) * align - 7], device="cuda", dtype=torch.int64)
     g = torch.Generator(device="cuda").manual_seed(splits + dv)
     po = torch.randn(bs, hq, splits, dv, device="cuda", generator=g)
