@@ -243,6 +243,35 @@ int b200_attn_extend_known(const void* q, int64_t q_stride, const void* k_cache,
                            void* stream);
 /* Start row of every request: exclusive sums of extend_seq_lens. */
 int b200_extend_starts(const int32_t* extend_seq_lens, int32_t* extend_start_loc, int bs, void* stream);
+/* One extend of one attention layer in one call: the new tokens' rows go to the pool (k == NULL: they are there),
+ * an FP8 pool's rows of the requests are copied to 16 bits (b200_kv_dequant_dense) into `scratch`, attention as
+ * b200_attn_extend_known.  Fields of 8 bytes, in this order.  */
+typedef struct {
+  const void* q;
+  int64_t q_stride;
+  void *k_cache, *v_cache;
+  int64_t kv_row_stride;              /* elements; Hkv * D where rows are written or the pool is FP8 */
+  void* o;
+  int64_t o_stride;
+  const int32_t* req_to_token;
+  int64_t req_to_token_stride;
+  const int64_t *req_pool_indices, *seq_lens;
+  const int32_t *prefix_lens, *extend_lens, *extend_start;
+  const void *k, *v;                  /* new rows, [num_new, Hkv * D] with these strides in elements */
+  int64_t k_stride, v_stride;
+  const int64_t* loc;
+  int64_t num_new;
+  void* scratch;                      /* FP8 pool only: b200_extend_layer_scratch_bytes */
+  int64_t scratch_bytes, total_kv;    /* total_kv: sum of seq_lens */
+  int64_t bs, max_extend_len, max_kv_len, Hq, Hkv, D, Dv;
+  int64_t causal, dtype, pool_fp8;            /* B200_BF16 / B200_F16; 0 pool of that type, 1 e4m3, 2 e5m2 */
+  double scale, logit_cap, k_scale, v_scale;
+  int64_t has_scale;                  /* the new rows are divided by k_scale / v_scale before the cast */
+  void* stream;
+} b200_extend_layer_args;
+int b200_extend_layer(const b200_extend_layer_args* args);
+size_t b200_extend_layer_scratch_bytes(int64_t total_kv, int64_t row_elems, int64_t bs, int64_t max_kv_len);
+
 /* Same kernel with an output multiplier: extend over an FP8 KV pool runs on an exact 16-bit copy
  * of the requests' rows (b200_kv_dequant_gather) with scale * k_scale and out_scale = v_scale.    */
 int b200_attn_extend_scaled(const void* q, int64_t q_stride, const void* k_cache,
@@ -285,6 +314,12 @@ int b200_kv_dequant_gather(const void* k_cache, const void* v_cache, int row_ele
                            const int32_t* kv_indptr, void* k_out, void* v_out, int32_t* dense_rtt,
                            int64_t dense_rtt_stride, int bs, int64_t max_len, int dtype,
                            void* stream);
+/* Same; kv_indptr may be NULL (the prefix sum is taken on the device) and dense_indices, int64 [bs], receives the
+ * row of dense_rtt of every request (0 .. bs - 1; NULL: not wanted).                                            */
+int b200_kv_dequant_dense(const void* k_cache, const void* v_cache, int row_elems, const int32_t* req_to_token,
+                          int64_t req_to_token_stride, const int64_t* req_pool_indices, const int64_t* seq_lens,
+                          const int32_t* kv_indptr, void* k_out, void* v_out, int32_t* dense_rtt, int64_t dense_rtt_stride,
+                          int64_t* dense_indices, int bs, int64_t max_len, int dtype, void* stream);
 
 /* ---- FP8 activation quantisation ----------------------------------------- */
 /* Per-token dynamic (static_scale == NULL): scales[m] = absmax(x[m,:]) / 448, q = sat(x * (1/scale))

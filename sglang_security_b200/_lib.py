@@ -7,6 +7,7 @@ PyTorch-eager substitute.
 from __future__ import annotations
 
 import ctypes
+import struct
 from ctypes import c_char_p, c_float, c_int, c_int64, c_size_t, c_void_p
 from pathlib import Path
 
@@ -16,6 +17,9 @@ _lib = None
 # dtype codes (enum b200_dtype)
 BF16, F16, F32, FP8_E4M3 = 0, 1, 2, 3
 KV_FP8_E5M2 = 0x100  # B200_KV_FP8_E5M2: flag on the dtype argument of the FP8-KV-pool entry points
+
+# b200_extend_layer_args: 8-byte fields in the order of the header
+EXTEND_LAYER_ARGS = struct.Struct("=Pq2PqPqPq2P3P2P2qPqP2q7q3q4dqP".replace("P", "Q"))
 
 _SIGNATURES = {
     "b200_version": (c_int, []),
@@ -47,6 +51,11 @@ _SIGNATURES = {
     "b200_attn_extend_known": (c_int, [c_void_p, c_int64, c_void_p, c_void_p, c_int64, c_void_p, c_int64, c_void_p,
                                        c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                                        c_int, c_int, c_int, c_int, c_float, c_float, c_float, c_int, c_int, c_void_p]),
+    "b200_extend_layer": (c_int, [c_char_p]),
+    "b200_extend_layer_scratch_bytes": (c_size_t, [c_int64, c_int64, c_int64, c_int64]),
+    "b200_kv_dequant_dense": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_int64, c_void_p, c_void_p, c_void_p,
+                                      c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_int, c_int64, c_int,
+                                      c_void_p]),
     "b200_extend_starts": (c_int, [c_void_p, c_void_p, c_int, c_void_p]),
     "b200_w4a16_gemm_stream_workspace_bytes": (c_size_t, [c_int, c_int]),
     "b200_w4a16_gemm_stream_pays": (c_int, [c_int, c_int, c_int]),
@@ -423,14 +432,18 @@ def ptr(t):
     return None if t is None else t.data_ptr()
 
 
-def dtype_code(torch_dtype) -> int:
-    import torch
+_dtype_codes = {}
 
-    table = {torch.bfloat16: BF16, torch.float16: F16, torch.float32: F32,
-             torch.float8_e4m3fn: FP8_E4M3}
-    if torch_dtype not in table:
+
+def dtype_code(torch_dtype) -> int:
+    if not _dtype_codes:
+        import torch
+
+        _dtype_codes.update({torch.bfloat16: BF16, torch.float16: F16, torch.float32: F32,
+                             torch.float8_e4m3fn: FP8_E4M3})
+    if torch_dtype not in _dtype_codes:
         raise B200Error(f"dtype {torch_dtype} is not supported by the B200 hot path")
-    return table[torch_dtype]
+    return _dtype_codes[torch_dtype]
 
 
 def is_fp8_kv(torch_dtype) -> bool:
@@ -446,7 +459,16 @@ def kv_dtype_code(act_dtype, pool_dtype) -> int:
     return dtype_code(act_dtype) | (KV_FP8_E5M2 if pool_dtype == torch.float8_e5m2 else 0)
 
 
-def current_stream() -> int:
-    import torch
+_raw_stream = None
 
-    return torch.cuda.current_stream().cuda_stream
+
+def current_stream() -> int:
+    """Handle of the current stream of the current device (what torch.cuda.current_stream().cuda_stream gives, without
+    the Stream object that it builds on every call)."""
+    global _raw_stream
+    if _raw_stream is None:
+        import torch
+
+        torch.cuda.current_stream()   # initialises CUDA
+        _raw_stream = (torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice)
+    return _raw_stream[0](_raw_stream[1]())

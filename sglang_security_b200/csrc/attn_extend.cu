@@ -875,4 +875,63 @@ int b200_attn_extend_known(const void* q, int64_t q_stride, const void* k_cache,
                            max_kv_len);
 }
 
+static size_t align256(size_t n) { return (n + 255) & ~static_cast<size_t>(255); }
+
+size_t b200_extend_layer_scratch_bytes(int64_t total_kv, int64_t row_elems, int64_t bs, int64_t max_kv_len) {
+  return 2 * align256(static_cast<size_t>(total_kv) * row_elems * 2) + align256(static_cast<size_t>(bs) * 8) +
+         align256(static_cast<size_t>(bs) * ((max_kv_len + 3) / 4 * 4) * 4);
+}
+
+int b200_extend_layer(const b200_extend_layer_args* a) {
+  B200_REQUIRE(a, "b200_extend_layer: null pointer");
+  const int64_t row = a->Hkv * a->D;
+  const int dtype = static_cast<int>(a->dtype), bs = static_cast<int>(a->bs);
+  const int pool_dtype = dtype | (a->pool_fp8 == 2 ? B200_KV_FP8_E5M2 : 0);
+  B200_REQUIRE(a->kv_row_stride == row || (!a->k && !a->pool_fp8), "b200_extend_layer: pool rows of %lld elements for %lld heads",
+               static_cast<long long>(a->kv_row_stride), static_cast<long long>(a->Hkv));
+  if (a->k) {
+    const int n = static_cast<int>(a->num_new);
+    const int rc = a->pool_fp8
+                       ? b200_kv_write_fp8(a->k, a->v, a->k_stride, a->v_stride, a->k_cache, a->v_cache, a->loc, n,
+                                           static_cast<int>(row), static_cast<float>(a->k_scale),
+                                           static_cast<float>(a->v_scale), static_cast<int>(a->has_scale), pool_dtype, a->stream)
+                       : b200_kv_write(a->k, a->v, a->k_stride * 2, a->v_stride * 2, a->k_cache, a->v_cache, a->loc, n,
+                                       static_cast<int>(row * 2), static_cast<int>(row * 2), a->stream);
+    if (rc) return rc;
+  }
+  if (bs == 0 || a->max_extend_len == 0) return 0;
+  const void *kc = a->k_cache, *vc = a->v_cache;
+  const int32_t* rtt = a->req_to_token;
+  const int64_t* idx = a->req_pool_indices;
+  int64_t rtt_stride = a->req_to_token_stride;
+  double scale = a->scale, out_scale = 1.0;
+  if (a->pool_fp8) {
+    // the tcgen05 kernels want 16-bit operands: an exact dense copy; the scales ride on the softmax scale and the output
+    B200_REQUIRE(a->scratch && static_cast<size_t>(a->scratch_bytes) >=
+                                   b200_extend_layer_scratch_bytes(a->total_kv, row, a->bs, a->max_kv_len),
+                 "b200_extend_layer: scratch of %lld bytes is too small", static_cast<long long>(a->scratch_bytes));
+    char* at = static_cast<char*>(a->scratch);
+    const size_t rows = align256(static_cast<size_t>(a->total_kv) * row * 2);
+    void *k16 = at, *v16 = at + rows;
+    int64_t* dense_idx = reinterpret_cast<int64_t*>(at + 2 * rows);
+    int32_t* dense = reinterpret_cast<int32_t*>(at + 2 * rows + align256(static_cast<size_t>(bs) * 8));
+    rtt_stride = (a->max_kv_len + 3) / 4 * 4;
+    const int rc = b200_kv_dequant_dense(kc, vc, static_cast<int>(row), rtt, a->req_to_token_stride, idx, a->seq_lens, nullptr,
+                                         k16, v16, dense, rtt_stride, dense_idx, bs, a->max_kv_len, pool_dtype, a->stream);
+    if (rc) return rc;
+    kc = k16;
+    vc = v16;
+    rtt = dense;
+    idx = dense_idx;
+    scale *= a->k_scale;
+    out_scale = a->v_scale;
+  }
+  const int Hq = static_cast<int>(a->Hq), Hkv = static_cast<int>(a->Hkv), D = static_cast<int>(a->D);
+  return extend_heads_impl(a->q, a->q_stride, kc, vc, a->kv_row_stride, a->o, a->o_stride, rtt, rtt_stride, idx, a->seq_lens, a->prefix_lens,
+                           a->extend_lens, a->extend_start, bs, static_cast<int>(a->max_extend_len), Hq, Hkv, D, static_cast<int>(a->Dv),
+                           static_cast<float>(scale), static_cast<float>(a->logit_cap), static_cast<float>(out_scale),
+                           static_cast<int>(a->causal), 0, 0, nullptr, -1, 1, 0, nullptr, 0, dtype, a->stream, nullptr, 0, 0.f,
+                           static_cast<int>(a->max_kv_len));
+}
+
 }  // extern "C"

@@ -79,12 +79,25 @@ __global__ void kv_dequant_gather_kernel(const uint8_t* __restrict__ k8, const u
                                          const int64_t* __restrict__ seq_lens,
                                          const int32_t* __restrict__ kv_indptr, T* __restrict__ k_out,
                                          T* __restrict__ v_out, int32_t* __restrict__ dense_rtt,
-                                         int64_t dense_rtt_stride, int e5m2) {
+                                         int64_t dense_rtt_stride, int64_t* __restrict__ dense_idx, int e5m2) {
   griddep_wait();
   griddep_launch_dependents();
   const int b = blockIdx.y;
   const int len = static_cast<int>(seq_lens[b]);
-  const int base = kv_indptr[b];
+  int base;
+  if (kv_indptr) {
+    base = kv_indptr[b];
+  } else {                                         // first dense row: the tokens of the requests before this one
+    __shared__ int warp_sum[8];
+    int sum = 0;
+    for (int i = threadIdx.x; i < b; i += blockDim.x) sum += static_cast<int>(seq_lens[i]);
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    if ((threadIdx.x & 31) == 0) warp_sum[threadIdx.x >> 5] = sum;
+    __syncthreads();
+    base = 0;
+    for (int w = 0; w < 8; ++w) base += warp_sum[w];
+  }
+  if (dense_idx && blockIdx.x == 0 && threadIdx.x == 0) dense_idx[b] = b;
   const int32_t* rtt = req_to_token + req_pool_indices[b] * rtt_stride;
   const int chunks = row_elems / 8;
   const int64_t total = static_cast<int64_t>(len) * chunks;
@@ -236,10 +249,18 @@ int b200_kv_dequant_gather(const void* k_cache, const void* v_cache, int row_ele
                            const int32_t* kv_indptr, void* k_out, void* v_out, int32_t* dense_rtt,
                            int64_t dense_rtt_stride, int bs, int64_t max_len, int dtype,
                            void* stream) {
+  B200_REQUIRE(bs == 0 || max_len == 0 || kv_indptr, "b200_kv_dequant_gather: null pointer");
+  return b200_kv_dequant_dense(k_cache, v_cache, row_elems, req_to_token, req_to_token_stride, req_pool_indices, seq_lens,
+                               kv_indptr, k_out, v_out, dense_rtt, dense_rtt_stride, nullptr, bs, max_len, dtype, stream);
+}
+
+int b200_kv_dequant_dense(const void* k_cache, const void* v_cache, int row_elems, const int32_t* req_to_token,
+                          int64_t req_to_token_stride, const int64_t* req_pool_indices, const int64_t* seq_lens,
+                          const int32_t* kv_indptr, void* k_out, void* v_out, int32_t* dense_rtt, int64_t dense_rtt_stride,
+                          int64_t* dense_indices, int bs, int64_t max_len, int dtype, void* stream) {
   using namespace b200;
   if (bs == 0 || max_len == 0) return 0;
-  B200_REQUIRE(k_cache && v_cache && req_to_token && req_pool_indices && seq_lens && kv_indptr &&
-                   k_out && v_out && dense_rtt,
+  B200_REQUIRE(k_cache && v_cache && req_to_token && req_pool_indices && seq_lens && k_out && v_out && dense_rtt,
                "b200_kv_dequant_gather: null pointer");
   B200_REQUIRE(row_elems > 0 && row_elems % 8 == 0 && bs > 0 && bs <= 65535,
                "b200_kv_dequant_gather: bad sizes (row_elems=%d bs=%d)", row_elems, bs);
@@ -265,13 +286,13 @@ int b200_kv_dequant_gather(const void* k_cache, const void* v_cache, int row_ele
                          static_cast<const uint8_t*>(v_cache), row_elems, req_to_token,
                          req_to_token_stride, req_pool_indices, seq_lens, kv_indptr,
                          static_cast<__nv_bfloat16*>(k_out), static_cast<__nv_bfloat16*>(v_out),
-                         dense_rtt, dense_rtt_stride, e5m2);
+                         dense_rtt, dense_rtt_stride, dense_indices, e5m2);
   else
     lerr = launch_kernel(kv_dequant_gather_kernel<__half>, grid, dim3(256), 0, st, 1, kPdlOther & 0,
                          static_cast<const uint8_t*>(k_cache), static_cast<const uint8_t*>(v_cache),
                          row_elems, req_to_token, req_to_token_stride, req_pool_indices, seq_lens,
                          kv_indptr, static_cast<__half*>(k_out), static_cast<__half*>(v_out),
-                         dense_rtt, dense_rtt_stride, e5m2);
+                         dense_rtt, dense_rtt_stride, dense_indices, e5m2);
   B200_CUDA_OK(lerr);
   B200_CHECK_LAUNCH("b200_kv_dequant_gather");
   return 0;

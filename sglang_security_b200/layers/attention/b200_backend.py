@@ -9,7 +9,10 @@ and calls the sm_100a kernels through the C-ABI (include/b200_hotpath.h):
   forward_decode : b200_kv_write -> b200_attn_decode_fused (split-KV gather kernel whose last CTA per
                    request merges the splits and, on request, quantises the row for o_proj);
                    B200_ATTN_FUSED_TAIL=0 restores split kernel + merge kernel
-  forward_extend : b200_kv_write -> b200_attn_extend (tcgen05 prefix rectangle + causal triangle)
+  forward_extend : b200_extend_layer: pool write, 16-bit copy of an FP8 pool's rows, attention (tcgen05 prefix
+                   rectangle + causal triangle) in one native call.  Short extends are bound by the host: 64 fresh
+                   tokens took 62 us a call in three native calls with torch's Stream objects, 37 in one; behind an
+                   FP8 pool, whose prefix sum and row table were torch operations, 146, now 46.
 
 All per-step metadata is computed without a device->host sync; buffers are persistent so the
 decode step can be captured in a CUDA graph.
@@ -24,7 +27,7 @@ import os
 import torch
 
 from ... import _lib
-from ...mem_cache.memory_pool import kv_write
+from ...mem_cache.memory_pool import MHATokenToKVPool, kv_write
 from .base_attn_backend import AttentionBackend
 
 
@@ -41,6 +44,15 @@ class ForwardMetadata:
     # (one conversion per step, never a temporary whose block the allocator could hand out again
     # before the launch has read it); keyed by (data_ptr, dtype, numel) of the source
     converted: Dict[tuple, torch.Tensor] = field(default_factory=dict)
+    extent: Optional[tuple] = None
+
+    def kv_extent(self, forward_batch, seq_lens) -> tuple:
+        """(sum, maximum) of the sequence lengths, from the host's copy where there is one; once per forward."""
+        if self.extent is None:
+            cpu = getattr(forward_batch, "seq_lens_cpu", None)
+            lens = (seq_lens if cpu is None else cpu).tolist()
+            self.extent = sum(lens), max(lens)
+        return self.extent
 
     def as_dtype(self, t: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
         if t.dtype == dtype:
@@ -326,72 +338,85 @@ class B200AttnBackend(AttentionBackend):
             q = q.contiguous()
         o = q.new_empty((q.shape[0], hq * dv))
         pool = forward_batch.token_to_kv_pool
-        if save_kv_cache:
-            # new tokens' K/V go to the pool first; the kernel then gathers prefix AND new keys
-            # from the pool, exactly like the oracle (torch_native_backend.py:196-199)
-            k_cache, v_cache = self._save_kv(layer, forward_batch, k, v)
-        else:
-            k_cache = pool.get_key_buffer(layer.layer_id)
-            v_cache = pool.get_value_buffer(layer.layer_id)
+        k_cache = pool.get_key_buffer(layer.layer_id)
+        v_cache = pool.get_value_buffer(layer.layer_id)
         md = self.forward_metadata
         bs = forward_batch.batch_size
-        if q.shape[0] == 0 or bs == 0 or md.max_extend_len == 0:
+        empty = q.shape[0] == 0 or bs == 0 or md.max_extend_len == 0
+        if not empty:
+            self._check_layer(layer)
+        # new tokens' K/V go to the pool first; the kernel then gathers prefix AND new keys from the pool, exactly
+        # like the oracle (torch_native_backend.py:196-199)
+        rows = None
+        if save_kv_cache:
+            rows = None if empty else self._new_rows(k, v, k_cache, v_cache, pool, forward_batch.out_cache_loc, hkv, d)
+            if rows is None:
+                self._save_kv(layer, forward_batch, k, v)
+        if empty:
             return o
+        fp8 = _lib.is_fp8_kv(k_cache.dtype)
+        if not fp8 and k_cache.dtype != q.dtype:
+            raise _lib.B200Error(
+                f"B200AttnBackend.forward_extend: KV cache dtype {k_cache.dtype} != q dtype "
+                f"{q.dtype} (supported pools: the activation dtype, float8_e4m3fn or float8_e5m2)")
         attn_type = getattr(layer, "attn_type", None)
         causal = not (layer.is_cross_attention or
                       getattr(attn_type, "value", attn_type) == "encoder_only")
         req_to_token = forward_batch.req_to_token_pool.req_to_token
-        self._check_layer(layer)
         req_pool_indices = md.as_dtype(forward_batch.req_pool_indices, torch.int64)
         seq_lens = md.as_dtype(forward_batch.seq_lens, torch.int64)
         prefix_lens = md.as_dtype(forward_batch.extend_prefix_lens, torch.int32)
         extend_lens = md.as_dtype(forward_batch.extend_seq_lens, torch.int32)
-        scaling, out_scale = float(layer.scaling), 1.0
-        if _lib.is_fp8_kv(k_cache.dtype):
-            # FP8 pool: the tcgen05 kernel wants 16-bit operands, so the requests' rows are first
-            # copied (exactly) into a dense 16-bit scratch; scales ride on the softmax scale / output
-            k_cache, v_cache, req_to_token, req_pool_indices = self._dequant_for_extend(
-                forward_batch, k_cache, v_cache, req_to_token, req_pool_indices, seq_lens, hkv * d,
-                q.dtype)
+        ks = vs = scratch = None
+        total_kv = scratch_bytes = 0
+        max_kv = md.max_kv_len
+        if fp8:
+            # the kernel works on an exact dense 16-bit copy of the requests' rows
             ks, vs = self._kv_scales(layer)
-            scaling *= 1.0 if ks is None else ks
-            out_scale = 1.0 if vs is None else vs
-        elif k_cache.dtype != q.dtype:
-            raise _lib.B200Error(
-                f"B200AttnBackend.forward_extend: KV cache dtype {k_cache.dtype} != q dtype "
-                f"{q.dtype} (supported pools: the activation dtype, float8_e4m3fn or float8_e5m2)")
-        rc = self.lib.b200_attn_extend_known(
-            q.data_ptr(), q.stride(0), k_cache.data_ptr(), v_cache.data_ptr(), k_cache.stride(0),
-            o.data_ptr(), o.stride(0), req_to_token.data_ptr(), req_to_token.stride(0),
-            req_pool_indices.data_ptr(), seq_lens.data_ptr(),
-            prefix_lens.data_ptr(), extend_lens.data_ptr(), md.qo_indptr.data_ptr(), bs,
-            md.max_extend_len, md.max_kv_len, hq, hkv, d, dv, scaling, float(layer.logit_cap or 0.0), out_scale,
-            1 if causal else 0, _lib.dtype_code(q.dtype), _lib.current_stream())
-        _lib.check(rc, "b200_attn_extend")
+            if rows is not None and (ks is None) != (vs is None):
+                raise _lib.B200Error("forward_extend: k_scale and v_scale must be given together")
+            total_kv, max_kv = md.kv_extent(forward_batch, seq_lens)
+            scratch_bytes = self.lib.b200_extend_layer_scratch_bytes(total_kv, hkv * d, bs, max_kv)
+            scratch = torch.empty(scratch_bytes, dtype=torch.uint8, device=q.device)
+        kp = vp = kst = vst = locp = n_new = 0
+        if rows is not None:
+            k, v, loc = rows
+            kp, vp, kst, vst, locp, n_new = k.data_ptr(), v.data_ptr(), k.stride(0), v.stride(0), loc.data_ptr(), loc.numel()
+        args = _lib.EXTEND_LAYER_ARGS.pack(
+            q.data_ptr(), q.stride(0), k_cache.data_ptr(), v_cache.data_ptr(), k_cache.stride(0), o.data_ptr(), o.stride(0),
+            req_to_token.data_ptr(), req_to_token.stride(0), req_pool_indices.data_ptr(), seq_lens.data_ptr(),
+            prefix_lens.data_ptr(), extend_lens.data_ptr(), md.qo_indptr.data_ptr(), kp, vp, kst, vst, locp, n_new,
+            0 if scratch is None else scratch.data_ptr(), scratch_bytes, total_kv, bs, md.max_extend_len, max_kv, hq, hkv, d, dv,
+            1 if causal else 0, _lib.dtype_code(q.dtype),
+            0 if not fp8 else 2 if k_cache.dtype == torch.float8_e5m2 else 1, float(layer.scaling),
+            float(layer.logit_cap or 0.0), 1.0 if ks is None else ks, 1.0 if vs is None else vs, 0 if ks is None else 1,
+            _lib.current_stream())
+        _lib.check(self.lib.b200_extend_layer(args), "b200_attn_extend")
         return o
 
-    def _dequant_for_extend(self, forward_batch, k_cache, v_cache, req_to_token, req_pool_indices,
-                            seq_lens, row_elems, dtype):
-        """-> (k16, v16, dense_req_to_token, dense_req_pool_indices) for an e4m3 / e5m2 pool."""
-        bs = seq_lens.numel()
-        cpu = getattr(forward_batch, "seq_lens_cpu", None)
-        if cpu is not None:
-            total, max_len = int(cpu.sum()), int(cpu.max())
-        else:
-            total, max_len = int(seq_lens.sum().item()), int(seq_lens.max().item())
-        indptr = torch.zeros(bs + 1, dtype=torch.int32, device=seq_lens.device)
-        indptr[1:] = torch.cumsum(seq_lens, dim=0)
-        k16 = torch.empty((total, row_elems), dtype=dtype, device=seq_lens.device)
-        v16 = torch.empty_like(k16)
-        stride = (max_len + 3) // 4 * 4
-        dense_rtt = torch.empty((bs, stride), dtype=torch.int32, device=seq_lens.device)
-        rc = self.lib.b200_kv_dequant_gather(
-            k_cache.data_ptr(), v_cache.data_ptr(), row_elems, req_to_token.data_ptr(),
-            req_to_token.stride(0), req_pool_indices.data_ptr(), seq_lens.data_ptr(),
-            indptr.data_ptr(), k16.data_ptr(), v16.data_ptr(), dense_rtt.data_ptr(), stride, bs,
-            max_len, _lib.kv_dtype_code(dtype, k_cache.dtype), _lib.current_stream())
-        _lib.check(rc, "b200_kv_dequant_gather")
-        return k16, v16, dense_rtt, torch.arange(bs, dtype=torch.int64, device=seq_lens.device)
+    @staticmethod
+    def _new_rows(k, v, k_cache, v_cache, pool, loc, hkv, d):
+        """-> (k, v, loc) as b200_extend_layer stores them, or None where the pool stores them itself."""
+        if not (k.is_cuda and loc.dtype == torch.int64 and loc.is_contiguous() and k.dtype == v.dtype):
+            return None
+        if k.dtype != k_cache.dtype and not (type(pool) is MHATokenToKVPool and _lib.is_fp8_kv(k_cache.dtype)
+                                             and k.dtype in (torch.bfloat16, torch.float16)):
+            return None
+        n = loc.numel()
+        if n == 0 or not (k_cache.is_contiguous() and v_cache.is_contiguous()):
+            return None
+        out = []
+        for t, cache in ((k, k_cache), (v, v_cache)):
+            if t.numel() != n * hkv * d or cache.numel() != cache.shape[0] * hkv * d:
+                return None
+            st = t.stride()
+            if t.dim() == 3 and t.shape[1] == hkv and st[2] == 1 and (st[1] == d or hkv == 1) and t.shape[0] == n:
+                out.append(t)                       # rows of hkv * d elements with a stride
+            elif t.dim() == 2 and st[1] == 1 and t.shape[0] == n:
+                out.append(t)
+            else:
+                return None
+        return out[0], out[1], loc
 
     def support_triton(self):
         return False
