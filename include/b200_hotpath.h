@@ -422,6 +422,14 @@ int b200_w4a16_gemv(const void* x, int64_t ldx, const void* qweight, const void*
                     int K, int group_size, int dtype, void* stream);
 int b200_w4a16_gemv_config(int max_m, int splits);
 
+/* 17 to 512 tokens with the stream copy (b200_w4a16_gemv_v2_repack): the dequantised weights go from registers to
+ * tensor memory (csrc/w4a16_ts.cu); W as b200_w4a16_gemm.  N % 16 == 0, K % 64 == 0, group 32 or a multiple of 64.
+ * _takes: 1 for the problems that it accepts, those that it is expected to be faster for.                         */
+int b200_w4a16_gemm_ts_takes(int M, int N, int K, int group_size);
+int b200_w4a16_gemm_ts(const void* x, int64_t ldx, const void* qweight_stream, const void* zeros, const void* scales,
+                       const void* bias, void* out, int64_t ldc, int M, int N, int K, int group_size, int dtype,
+                       void* stream);
+
 /* Prefill sizes with the stream copy (b200_w4a16_gemv_v2_repack): expands the weight into `workspace` (16-bit [N, K])
  * and runs the CTA-pair GEMM.  N % 16 == 0, K % 64 == 0, group_size % 8 == 0. */
 size_t b200_w4a16_gemm_stream_workspace_bytes(int N, int K);

@@ -57,6 +57,9 @@ _SIGNATURES = {
                                       c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_int, c_int64, c_int,
                                       c_void_p]),
     "b200_extend_starts": (c_int, [c_void_p, c_void_p, c_int, c_void_p]),
+    "b200_w4a16_gemm_ts": (c_int, [c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int,
+                                   c_int, c_int, c_int, c_int, c_void_p]),
+    "b200_w4a16_gemm_ts_takes": (c_int, [c_int, c_int, c_int, c_int]),
     "b200_w4a16_gemm_stream_workspace_bytes": (c_size_t, [c_int, c_int]),
     "b200_w4a16_gemm_stream_pays": (c_int, [c_int, c_int, c_int]),
     "b200_w4a16_gemm_stream": (c_int, [c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64,

@@ -119,6 +119,30 @@ def w4a16_gemv_v2(x: torch.Tensor, qweight_stream: torch.Tensor, zeros: torch.Te
     return out
 
 
+def w4a16_gemm_ts(x: torch.Tensor, qweight_stream: torch.Tensor, zeros: torch.Tensor, scales: torch.Tensor,
+                  group_size: int, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """x [M, K] @ dequant(stream-layout weight) (+ bias) -> [M, N] for the problems of ts_takes() (csrc/w4a16_ts.cu)."""
+    _cuda(x, "w4a16_gemm_ts")
+    if x.dim() != 2 or x.stride(-1) != 1:
+        raise _lib.B200Error("w4a16_gemm_ts: x must be 2-D with contiguous rows")
+    m, k = x.shape
+    n = scales.shape[1]
+    if qweight_stream.numel() * 8 != k * n or scales.dtype != x.dtype or zeros.dtype != x.dtype:
+        raise _lib.B200Error("w4a16_gemm_ts: shape / dtype mismatch between x and the packed weight")
+    out = torch.empty((m, n), device=x.device, dtype=x.dtype)
+    if bias is not None and bias.dtype != x.dtype:
+        bias = bias.to(x.dtype)
+    rc = _lib.load().b200_w4a16_gemm_ts(x.data_ptr(), x.stride(0), qweight_stream.data_ptr(), zeros.data_ptr(),
+                                        scales.data_ptr(), _lib.ptr(bias), out.data_ptr(), out.stride(0), m, n, k,
+                                        group_size, _lib.dtype_code(x.dtype), _lib.current_stream())
+    _lib.check(rc, "b200_w4a16_gemm_ts")
+    return out
+
+
+def ts_takes(m: int, n: int, k: int, group_size: int) -> bool:
+    return bool(_lib.load().b200_w4a16_gemm_ts_takes(int(m), int(n), int(k), int(group_size)))
+
+
 class ExpandScratch:
     """Device memory for the 16-bit form of one int4 weight at a time (w4a16_gemm_stream: 283 MB for 27648 x 5120).
 
@@ -230,14 +254,18 @@ def stream_copy_enabled() -> bool:
 
 def w4a16_linear(x2: torch.Tensor, layer, bias: Optional[torch.Tensor]) -> torch.Tensor:
     """Dispatch of AWQ/GPTQ apply(): decode batches (M <= 16) stream the repacked weight through
-    the GEMV, large ones expand it once for the CTA-pair GEMM, everything else runs the fused dequant +
-    tcgen05 GEMM on the [K, N/8] layout."""
+    the GEMV, those up to 512 tokens whose tiles fit one wave dequantise it into tensor memory, large ones
+    expand it once for the CTA-pair GEMM, everything else runs the fused dequant + tcgen05 GEMM on the
+    [K, N/8] layout."""
     stream = getattr(layer, "b200_qweight_stream", None)
     m = x2.shape[0]
     if stream is not None and 1 <= m <= GEMV_V2_MAX_M and gemv_v2_supported(
             m, layer.scales.shape[1], x2.shape[1], layer.w4a16_group_size):
         return w4a16_gemv_v2(x2, stream, layer.b200_zeros, layer.scales, layer.w4a16_group_size, bias)
     n = layer.scales.shape[1]
+    if (stream is not None and x2.stride(0) % 8 == 0 and x2.data_ptr() % 16 == 0
+            and ts_takes(m, n, x2.shape[1], layer.w4a16_group_size)):
+        return w4a16_gemm_ts(x2, stream, layer.b200_zeros, layer.scales, layer.w4a16_group_size, bias)
     if (stream is not None and stream_gemm_pays(m, n, x2.shape[1]) and layer.w4a16_group_size % 8 == 0
             and x2.stride(0) % 8 == 0 and x2.data_ptr() % 16 == 0):
         # the fused kernel needs no memory: it takes over where the expanded weight found none when it was loaded, and
