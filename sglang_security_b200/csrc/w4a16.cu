@@ -559,6 +559,11 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         tile += tile_step;
       }
       if (tile >= num_tiles) break;
+      // Where RAWS is no multiple of DG, a slot passes from one group to another with each lap, and the copies of a stage
+      // may land after those of the next one: a group that is ahead would take the phase before last of `full` for its own,
+      // dequantise the words of an older stage and release the slot for the other group (wrong sums, or a ring that stands
+      // still).  So the slot's last owner has to have released it, which is after its copies had landed.
+      if (RAWS % DG != 0) tc::mbar_wait(rempty_bar(rs), rphase ^ 1u);
       tc::mbar_wait(rfull_bar(rs), rphase);
       const uint32_t rsrc = raw_base + rs * C::RAW_BYTES;
       uint32_t q[KS][RPT];
