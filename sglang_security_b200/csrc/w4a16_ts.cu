@@ -433,8 +433,8 @@ static void ts_rings(TsPlan* pl, int raw) {
 
 // Tile width, K split and form for M tokens; false where the kernels of w4a16.cu / w4a16_stream_gemm.cu are faster.
 // Measured (f16, us): a 64-k stage takes 0.22 + 0.0004 bn of a CTA alone on its SM, 0.19 + 0.0007 bn times their number where
-// several share one; a split 2 + 0.02 bn for the exchange of the partials.  More than 1.6 CTAs an SM were slower than fewer
-// (clusters do not pack).  Three CTAs an SM, each half of K, only where that fills them and two would leave every second SM
+// several share one; a split 2 + 0.02 bn for the exchange of the partials.  More than 1.63 CTAs an SM (240 of 148) were slower
+// than fewer (clusters do not pack).  Three CTAs an SM, each half of K, only where that fills them and two would leave every second SM
 // half idle (27648 x 5120, 16 / 64 tokens: 34.6 / 38.6 with two, 29.9 / 34.9 with three).
 // Above 128 tokens a weight is dequantised again for every block of tokens: worth it while the tiles fit one wave, which the
 // 128-token tiles of w4a16.cu take as long for without a split of K (us, there / here: 3584 x 5120, 200 tokens 27.4 / 20.2;
@@ -461,7 +461,7 @@ static bool ts_plan(int M, int N, int K, int raw, TsPlan* pl) {
     double best = 0;
     for (int S = 1; S <= 8; ++S) {
       const int per = ceil_div(KB, S), load = ceil_div(tiles * S, sms);
-      if (S > 1 && (per < 4 || (S - 1) * per >= KB || tiles * S > sms * 1.62)) continue;
+      if (S > 1 && (per < 4 || (S - 1) * per >= KB || tiles * S > sms * 1.63)) continue;
       const double us = per * (load == 1 ? 0.22 + 0.0004 * pl->bn : load * (0.19 + 0.0007 * pl->bn)) +
                         (S > 1 ? 2.0 + 0.02 * pl->bn : 0.0);
       if (S == 1 || us < best) {
