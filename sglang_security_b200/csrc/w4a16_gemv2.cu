@@ -37,7 +37,6 @@
 namespace b200 {
 
 constexpr int kG2Threads = 256;
-constexpr int kG2Depth = 6;  // LDG.128 in flight per lane (3 KiB per warp)
 
 struct Gemv2Params {
   const void* x;
@@ -137,13 +136,19 @@ __device__ __forceinline__ uint32_t g2_hmul2(uint32_t a, uint32_t b) {
   return r;
 }
 
-// MT = number of 8-token tiles (1: M <= 8, 2: M <= 16).  SPG = 32-k steps per quantisation group
+// MT = number of 8-token tiles (1: M <= 8, 2: M <= 16).  CTAS = CTAs per SM.  With two tiles, two CTAs keep six loads a
+// lane in flight (512 bytes each a warp); three keep four, and the partial tile takes the place of x, so that a K slice as
+// long as before fits: for grids that end a wave earlier with them (us, two / three a SM, f16, 9 and 16 tokens, Qwen2.5-32B
+// at TP 2, all four linears: 86.3 / 70.1 and 89.5 / 73.3; Llama-3.1-8B bf16 65.1 / 59.7 and 76.9 / 67.9; where both take
+// one wave, at TP 4, 35.0 / 36.6).
+//  SPG = 32-k steps per quantisation group
 // known at compile time (1, 2, 4 = groups of 32, 64, 128: the fold sits at fixed places of the
 // unrolled round, no counters) or 0 = any other group size (run-time step counter).
-template <typename T, int MT, int SPG>
-__global__ void __launch_bounds__(kG2Threads, MT == 1 ? 3 : 2)
+template <typename T, int MT, int SPG, int CTAS>
+__global__ void __launch_bounds__(kG2Threads, CTAS)
 w4a16_gemv2_kernel(const Gemv2Params p) {
   using MG = G2Magic<T>;
+  constexpr int DEPTH = MT == 2 && CTAS == 3 ? 4 : 6;
   extern __shared__ __align__(128) uint8_t smem[];
   const uint32_t sbase = smem_u32(smem);
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
@@ -160,9 +165,9 @@ w4a16_gemv2_kernel(const Gemv2Params p) {
 
   // ---- 1. weights do not depend on the previous kernel: put the first loads in flight now ------
   const uint4* wp = p.qw + (static_cast<int64_t>(nt) * KB + kb0) * 32 + lane;
-  uint4 buf[kG2Depth];
+  uint4 buf[DEPTH];
 #pragma unroll
-  for (int i = 0; i < kG2Depth; ++i)
+  for (int i = 0; i < DEPTH; ++i)
     buf[i] = (warp_ok && i < nkb) ? g2_ldg_stream(wp + i * 32) : make_uint4(0, 0, 0, 0);
 
   // ---- 2. scales and zero points of this slice's groups as fp32: [group][0 = s, 1 = z][128 columns]
@@ -203,7 +208,7 @@ w4a16_gemv2_kernel(const Gemv2Params p) {
   {
     const T* xg = static_cast<const T*>(p.x);
     const int cpr = nkb * 8;  // 16-byte chunks per row
-    for (int r = warp; r <= rows; r += 8) {
+    for (int r = warp; r < rows + (rows < MT * 8); r += 8) {
       const bool real = r < rows;
       const uint4* src = reinterpret_cast<const uint4*>(xg + static_cast<int64_t>(real ? r : 0) * p.ldx +
                                                         kb0 * 64);
@@ -321,23 +326,23 @@ w4a16_gemv2_kernel(const Gemv2Params p) {
       fold();
     }
   };
-  // tile j of a round (64 k = two steps); with a compile-time SPG a round of 6 tiles = 12 steps starts
-  // on a group boundary (12 % SPG == 0), so the fold positions are compile-time too
+  // tile j of a round (64 k = two steps); with a compile-time SPG a round of DEPTH tiles starts on a
+  // group boundary (2 DEPTH % SPG == 0), so the fold positions are compile-time too
   auto tile = [&](const uint4& w, int j, uint32_t xround) {
     step(w.x, w.y, xround + j * 128, SPG && ((2 * j + 1) % SPG == 0));
     step(w.z, w.w, xround + j * 128 + 64, SPG && ((2 * j + 2) % SPG == 0));
   };
-  static_assert(SPG == 0 || (2 * kG2Depth) % SPG == 0, "a round must hold whole groups");
+  static_assert(SPG == 0 || (2 * DEPTH) % SPG == 0, "a round must hold whole groups");
 
   if (warp_ok) {
     int base = 0;
-    const uint4* wq = wp + kG2Depth * 32;  // the tile kG2Depth ahead of the round's first
+    const uint4* wq = wp + DEPTH * 32;  // the tile DEPTH ahead of the round's first
     uint32_t xround = 0;
-    // steady state: every tile of this round has a successor kG2Depth tiles ahead
+    // steady state: every tile of this round has a successor DEPTH tiles ahead
 #pragma unroll 1
-    for (; base + 2 * kG2Depth <= nkb; base += kG2Depth, wq += kG2Depth * 32, xround += kG2Depth * 128) {
+    for (; base + 2 * DEPTH <= nkb; base += DEPTH, wq += DEPTH * 32, xround += DEPTH * 128) {
 #pragma unroll
-      for (int j = 0; j < kG2Depth; ++j) {
+      for (int j = 0; j < DEPTH; ++j) {
         const uint4 w = buf[j];
         buf[j] = g2_ldg_stream(wq + j * 32);
         tile(w, j, xround);
@@ -345,12 +350,12 @@ w4a16_gemv2_kernel(const Gemv2Params p) {
     }
     // tail: at most two rounds, loads predicated
 #pragma unroll 1
-    for (; base < nkb; base += kG2Depth, wq += kG2Depth * 32, xround += kG2Depth * 128) {
+    for (; base < nkb; base += DEPTH, wq += DEPTH * 32, xround += DEPTH * 128) {
 #pragma unroll
-      for (int j = 0; j < kG2Depth; ++j) {
+      for (int j = 0; j < DEPTH; ++j) {
         if (base + j < nkb) {
           const uint4 w = buf[j];
-          if (base + j + kG2Depth < nkb) buf[j] = g2_ldg_stream(wq + j * 32);
+          if (base + j + DEPTH < nkb) buf[j] = g2_ldg_stream(wq + j * 32);
           tile(w, j, xround);
         }
       }
@@ -359,7 +364,9 @@ w4a16_gemv2_kernel(const Gemv2Params p) {
   griddep_launch_dependents();
 
   // ---- split-K reduction in fixed rank order through distributed shared memory ------------------
-  float* part = reinterpret_cast<float*>(smem + p.part_off);  // [MT * 8][128]
+  if (MT == 2 && CTAS == 3) __syncthreads();  // the partial tile takes the place of x
+  const int part_off = MT == 2 && CTAS == 3 ? 0 : p.part_off;
+  float* part = reinterpret_cast<float*>(smem + part_off);  // [MT * 8][128]
 #pragma unroll
   for (int m = 0; m < MT; ++m)
 #pragma unroll
@@ -379,7 +386,7 @@ w4a16_gemv2_kernel(const Gemv2Params p) {
     const float bias_n = (bias && n < p.N) ? to_float<T>(bias[n]) : 0.f;
     for (int item = threadIdx.x; item < p.M * cpr; item += kG2Threads) {
       const int m = item >> cshift;
-      const uint32_t local = sbase + p.part_off + (m * 128 + c) * 4;
+      const uint32_t local = sbase + part_off + (m * 128 + c) * 4;
       float sum = 0.f;
       if (S == 1) {
         sum = part[m * 128 + c];
@@ -434,7 +441,7 @@ static bool gemv2_shape_ok(int M, int N, int K, int group) {
 }
 
 struct Gemv2Plan {
-  int S, kb_per_rank, xs_stride, sz_off, sum_off, part_off, smem;
+  int ctas, S, kb_per_rank, xs_stride, sz_off, sum_off, part_off, smem;
 };
 
 static bool gemv2_plan(int M, int N, int K, int group, Gemv2Plan* pl) {
@@ -467,11 +474,20 @@ static bool gemv2_plan(int M, int N, int K, int group, Gemv2Plan* pl) {
     pl->S = S;
     pl->kb_per_rank = kb_per_rank;
     pl->xs_stride = xs_stride;
-    pl->sz_off = (M + 1) * xs_stride;  // M token rows + the shared zero row
+    pl->sz_off = (M + (M < MT * 8)) * xs_stride;  // M token rows + the shared zero row
     pl->sum_off = pl->sz_off + ng * 1024;
     pl->part_off = pl->sum_off + ng * 2 * MT * 8 * 4;
     pl->smem = pl->part_off + MT * 8 * 128 * 4;
     if (pl->smem <= 72 * 1024 || S >= 8) break;  // keep >= 3 CTAs per SM when K allows
+  }
+  pl->ctas = MT == 1 ? 3 : 2;
+  if (MT == 2 && pl->part_off <= 75 * 1024) {
+    const int sms = device_sm_count(), grid = n_groups * pl->S;
+    if (ceil_div(grid, 3 * sms) < ceil_div(grid, 2 * sms)) {
+      pl->ctas = 3;
+      pl->smem = pl->part_off > MT * 8 * 128 * 4 ? pl->part_off : MT * 8 * 128 * 4;
+      pl->part_off = 0;
+    }
   }
   return pl->smem <= 200 * 1024;
 }
@@ -545,23 +561,25 @@ int b200_w4a16_gemv_v2(const void* x, int64_t ldx, const void* qweight_stream, c
   void (*kern)(const Gemv2Params) = nullptr;
   const int spg = group_size == 128 ? 4 : group_size == 64 ? 2 : group_size == 32 ? 1 : 0;
   const int mt = M <= 8 ? 1 : 2;
-#define B200_G2_PICK(T_, MT_)                                                             \
-  (spg == 4   ? w4a16_gemv2_kernel<T_, MT_, 4>                                            \
-   : spg == 2 ? w4a16_gemv2_kernel<T_, MT_, 2>                                            \
-   : spg == 1 ? w4a16_gemv2_kernel<T_, MT_, 1>                                            \
-              : w4a16_gemv2_kernel<T_, MT_, 0>)
+#define B200_G2_PICK(T_, MT_, CTAS_)                                                      \
+  (spg == 4   ? w4a16_gemv2_kernel<T_, MT_, 4, CTAS_>                                     \
+   : spg == 2 ? w4a16_gemv2_kernel<T_, MT_, 2, CTAS_>                                     \
+   : spg == 1 ? w4a16_gemv2_kernel<T_, MT_, 1, CTAS_>                                     \
+              : w4a16_gemv2_kernel<T_, MT_, 0, CTAS_>)
+#define B200_G2_FORM(T_) (mt == 1 ? B200_G2_PICK(T_, 1, 3) : pl.ctas == 2 ? B200_G2_PICK(T_, 2, 2) : B200_G2_PICK(T_, 2, 3))
   if (dtype == B200_F16)
-    kern = mt == 1 ? B200_G2_PICK(__half, 1) : B200_G2_PICK(__half, 2);
+    kern = B200_G2_FORM(__half);
   else
-    kern = mt == 1 ? B200_G2_PICK(__nv_bfloat16, 1) : B200_G2_PICK(__nv_bfloat16, 2);
+    kern = B200_G2_FORM(__nv_bfloat16);
+#undef B200_G2_FORM
 #undef B200_G2_PICK
-  const int ai = (dtype == B200_F16 ? 0 : 8) + (mt - 1) * 4 + (spg == 4 ? 3 : spg);
-  static int attr_smem[16] = {};
+  const int ai = (dtype == B200_F16 ? 0 : 12) + (mt - 1 + (mt == 2 && pl.ctas == 3)) * 4 + (spg == 4 ? 3 : spg);
+  static int attr_smem[24] = {};
   if (pl.smem > attr_smem[ai]) {
     B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, pl.smem));
     attr_smem[ai] = pl.smem;
   }
-  note_variant("w4a16_gemv2 mt=%d spg=%d splits=%d tiles=%d", mt, spg, pl.S, n_groups);
+  note_variant("w4a16_gemv2 mt=%d spg=%d splits=%d tiles=%d%s", mt, spg, pl.S, n_groups, mt == 2 && pl.ctas == 3 ? " ctas=3" : "");
   {
     ScopedKernelTimer timer("w4a16_gemv2", st);
     B200_CUDA_OK(launch_kernel(kern, dim3(n_groups * pl.S), dim3(kG2Threads), pl.smem, st, pl.S,
