@@ -261,8 +261,11 @@ typedef struct {
   int64_t k_stride, v_stride;
   const int64_t* loc;
   int64_t num_new;
-  void* scratch;                      /* FP8 pool only: b200_extend_layer_scratch_bytes */
-  int64_t scratch_bytes, total_kv;    /* total_kv: sum of seq_lens */
+  void* scratch;                      /* b200_extend_layer_scratch_bytes; less (an FP8 pool's copy only, or NULL): the
+                                       * keys of long requests are not spread evenly over the SMs */
+  int64_t scratch_bytes;
+  int64_t total_kv;                   /* sum of seq_lens (FP8 pool) */
+  const int32_t* host_lens;           /* HOST memory, read during the call: new tokens, prefix of every request; or NULL */
   int64_t bs, max_extend_len, max_kv_len, Hq, Hkv, D, Dv;
   int64_t causal, dtype, pool_fp8;            /* B200_BF16 / B200_F16; 0 pool of that type, 1 e4m3, 2 e5m2 */
   double scale, logit_cap, k_scale, v_scale;
@@ -270,7 +273,8 @@ typedef struct {
   void* stream;
 } b200_extend_layer_args;
 int b200_extend_layer(const b200_extend_layer_args* args);
-size_t b200_extend_layer_scratch_bytes(int64_t total_kv, int64_t row_elems, int64_t bs, int64_t max_kv_len);
+size_t b200_extend_layer_scratch_bytes(int64_t pool_fp8, int64_t total_kv, int64_t bs, int64_t max_kv_len, int64_t Hkv,
+                                       int64_t D);
 
 /* Same kernel with an output multiplier: extend over an FP8 KV pool runs on an exact 16-bit copy
  * of the requests' rows (b200_kv_dequant_gather) with scale * k_scale and out_scale = v_scale.    */

@@ -19,7 +19,7 @@ BF16, F16, F32, FP8_E4M3 = 0, 1, 2, 3
 KV_FP8_E5M2 = 0x100  # B200_KV_FP8_E5M2: flag on the dtype argument of the FP8-KV-pool entry points
 
 # b200_extend_layer_args: 8-byte fields in the order of the header
-EXTEND_LAYER_ARGS = struct.Struct("=Pq2PqPqPq2P3P2P2qPqP2q7q3q4dqP".replace("P", "Q"))
+EXTEND_LAYER_ARGS = struct.Struct("=Pq2PqPqPq2P3P2P2qPqP2qP7q3q4dqP".replace("P", "Q"))
 
 _SIGNATURES = {
     "b200_version": (c_int, []),
@@ -52,7 +52,7 @@ _SIGNATURES = {
                                        c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                                        c_int, c_int, c_int, c_int, c_float, c_float, c_float, c_int, c_int, c_void_p]),
     "b200_extend_layer": (c_int, [c_char_p]),
-    "b200_extend_layer_scratch_bytes": (c_size_t, [c_int64, c_int64, c_int64, c_int64]),
+    "b200_extend_layer_scratch_bytes": (c_size_t, [c_int64, c_int64, c_int64, c_int64, c_int64, c_int64]),
     "b200_kv_dequant_dense": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_int64, c_void_p, c_void_p, c_void_p,
                                       c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_int, c_int64, c_int,
                                       c_void_p]),

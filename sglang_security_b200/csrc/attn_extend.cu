@@ -20,8 +20,10 @@
 //               (M128 N=D K16 x 4, V consumed as an MN-major B operand); owns the TMEM allocation.
 //   warps 5-7 : gather loaders (cp.async double buffer, slot ids from req_to_token).
 // Two CTAs are co-resident per SM so one CTA's softmax overlaps the other's MMAs.
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
+#include <functional>
 #include <type_traits>
 
 #include "gemm_tc.cuh"
@@ -558,6 +560,7 @@ attn_extend_kernel(const ExtendParams p) {
 }  // namespace b200
 
 #include "attn_extend_wide.cuh"
+#include "attn_extend_flat.cuh"
 
 namespace b200 {
 
@@ -641,9 +644,62 @@ static double wide_us(int D, const ExtendParams& p, int max_extend_len, int keys
   return 3.0 + waves * ((D == 128 ? 11.0 : 8.0) + tiles * tile) + (splits > 1 ? 3.2 : 0.0);
 }
 
+// What the host may know beside the longest request
+struct ExtendHost {
+  void* workspace = nullptr;        // attn_extend_flat.cuh
+  size_t workspace_bytes = 0;
+  const int32_t* lens = nullptr;    // new tokens and prefix of every request, or null
+};
+// When the two-tile kernel's last CTA ends: its CTAs in the order of the grid, each to the SM that is free first.  From 68
+// calls timed (within 6 %, head size 64 2 %; without the requests' lengths, and so the order, 20 %).
+constexpr int kFlatMaxSms = 256;
+static double wide_last_us(int D, const ExtendParams& p, int bs, int max_extend_len, const int32_t* lens) {
+  const int sms = device_sm_count(), tok_cta = 256 / p.pack, heads = p.Hkv * p.head_tiles, blocks = ceil_div(max_extend_len, tok_cta);
+  const float once = D == 128 ? 12.f : 10.f, tile = D == 128 ? 1.9f : 1.7f, half = D == 128 ? 0.75f : 0.6f;
+  float free_at[kFlatMaxSms] = {}, last = 0.f;           // a heap, the earliest first
+  for (int b = 0; b < bs; ++b)
+    for (int h = 0; h < heads; ++h)
+      for (int q = blocks - 1; q >= 0; --q) {                // the longest of a head first, as in the grid
+        const int left = lens[2 * b] - q * tok_cta;
+        float& at = free_at[sms - 1];
+        std::pop_heap(free_at, free_at + sms, std::greater<float>());
+        at += left <= 0 ? 0.5f : once + flat_tiles(lens[2 * b + 1], lens[2 * b], q, tok_cta, 1) * tile * (left <= tok_cta / 2 ? half : 1.f);
+        if (at > last) last = at;
+        std::push_heap(free_at, free_at + sms, std::greater<float>());
+      }
+  return 3.0 + last;
+}
+// Whether the persistent kernel takes a causal call, from 151 calls timed on all kernels (groups of 4, 5 and 7 heads, head
+// sizes 64 and 128, 1 to 30 equal and ragged requests of 64 to 8192 new tokens behind 0 to 8000).  Its time is a fixed part
+// (the plan, the first loads, the last store, the merge) and every SM's equal share of items and key tiles (within 6 %); it
+// has to be a twentieth less than the others'.  Not above four waves of the two-tile kernel's CTAs, whose last one is a
+// small part there (2 x 8192 fresh tokens 944 us there, 1052 here), which also bounds the work of this estimate (~8 us).
+// 48 of the calls come here, 12 % faster on average, 4 % slower at worst (us, there / here: groups of 4, 8 x 512 behind 1536
+// 115 / 109, behind 4000 211 / 189, 3 x 100 behind 7000 146 / 61; head size 64, 2 x 1000 behind 7000 113 / 76).
+static bool flat_pays(int D, const ExtendParams& p, int bs, int max_extend_len, int64_t ctas, int splits, double wide, double narrow,
+                      const ExtendHost& host) {
+  const int sms = device_sm_count(), tok_cta = 256 / p.pack;
+  if (!p.causal || !host.lens || ctas > 4 * sms || sms > kFlatMaxSms) return false;
+  double items = 0, tiles = 0;
+  for (int b = 0; b < bs; ++b)
+    for (int q = 0; q * tok_cta < host.lens[2 * b]; ++q) {
+      items += 1;
+      tiles += flat_tiles(host.lens[2 * b + 1], host.lens[2 * b], q, tok_cta, 1);
+    }
+  const double share = static_cast<double>(p.Hkv) * p.head_tiles / sms;
+  const double flat = D == 128 ? 28.7 + (2.03 * tiles + 8.2 * items) * share : 18.8 + (1.9 * tiles + 5.6 * items) * share;
+  if (flat >= 0.95 * narrow) return false;
+  return flat < 0.95 * (splits > 1 ? wide : wide_last_us(D, p, bs, max_extend_len, host.lens));
+}
+// B200_EXTEND_FLAT: 0 never, 1 wherever it can (read per launch, for tests and A/B); else -1: by the estimates
+static int extend_flat_choice() {
+  const char* e = std::getenv("B200_EXTEND_FLAT");
+  return e && (e[0] == '0' || e[0] == '1') ? e[0] - '0' : -1;
+}
+
 template <typename T, int D>
 static int launch_extend(const ExtendParams& p, int n_values, int bs, int max_extend_len, int max_kv_len,
-                         cudaStream_t st) {
+                         const ExtendHost& host, cudaStream_t st) {
   // a cap up to 40 keeps e^(-2 cap) a normal fp32 (and 16-bit) number: the one-pass capped form
   const float ref = p.score_bound > 0.f && p.score_bound < p.logit_cap ? p.score_bound : p.logit_cap;
   const bool fast = ref <= 40.f && p.qk_scale > 0.f && extend_fast_softmax_enabled();
@@ -651,10 +707,15 @@ static int launch_extend(const ExtendParams& p, int n_values, int bs, int max_ex
   // and shorter requests, on the kernel above, whose two CTAs per SM hide what a CTA of the other spends before its first
   // and after its last tile (~8 us; us, this / that kernel: 8 x 512 fresh tokens 63.6 / 72.3).
   const int keys = max_kv_len > 0 ? max_kv_len : max_extend_len;
-  if (fast && keys >= 1024 && p.logit_cap <= 0.f && p.window == 0 && !p.sink && !p.gate && !p.lse && n_values == 1 && p.v_head < 0) {
+  if (fast && keys >= kWideMinKeys && p.logit_cap <= 0.f && p.window == 0 && !p.sink && !p.gate && !p.lse && n_values == 1 && p.v_head < 0) {
     int splits = 1;
     const int64_t ctas = wide_ctas<T, D>(p, bs, max_extend_len, max_kv_len, &splits);
-    if (wide_us(D, p, max_extend_len, keys, ctas, splits) <= narrow_us(D, p, bs, max_extend_len, keys))
+    const double wide = wide_us(D, p, max_extend_len, keys, ctas, splits), narrow = narrow_us(D, p, bs, max_extend_len, keys);
+    const int choice = extend_flat_choice();
+    if (choice != 0 && host.workspace && bs <= kFlatMaxBs && host.workspace_bytes >= flat_workspace_bytes<D>(device_sm_count()) &&
+        (choice == 1 || flat_pays(D, p, bs, max_extend_len, ctas, splits, wide, narrow, host)))
+      return launch_extend_flat<T, D>(p, bs, static_cast<float*>(host.workspace), host.workspace_bytes, st);
+    if (wide <= narrow)
       return launch_extend_wide<T, D>(p, bs, max_extend_len, splits, st);
   }
   note_variant("attn_extend d=%d fast_softmax=%d values=%d", D, fast ? 1 : 0, n_values);
@@ -745,7 +806,7 @@ static int extend_heads_impl(const void* q, int64_t q_stride, const void* k_cach
                              int window, int keep_first, const float* sink, int v_head, int n_values,
                              int64_t o_plane, float* lse, int64_t lse_stride, int dtype, void* stream,
                              const void* gate = nullptr, int64_t gate_stride = 0, float score_bound = 0.f,
-                             int max_kv_len = 0) {
+                             int max_kv_len = 0, const b200::ExtendHost& host = b200::ExtendHost()) {
   using namespace b200;
   B200_REQUIRE(!gate || (n_values == 1 && gate_stride % 8 == 0 && aligned16(gate)),
                "b200_attn_extend: the gate rows must be 16-byte aligned (stride %lld)",
@@ -810,10 +871,10 @@ static int extend_heads_impl(const void* q, int64_t q_stride, const void* k_cach
   B200_REQUIRE(bs <= 65535 && Hkv * p.head_tiles <= 65535, "b200_attn_extend: grid too large");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (dtype == B200_BF16)
-    return D == 128 ? launch_extend<__nv_bfloat16, 128>(p, n_values, bs, max_extend_len, max_kv_len, st)
-                    : launch_extend<__nv_bfloat16, 64>(p, n_values, bs, max_extend_len, max_kv_len, st);
-  return D == 128 ? launch_extend<__half, 128>(p, n_values, bs, max_extend_len, max_kv_len, st)
-                  : launch_extend<__half, 64>(p, n_values, bs, max_extend_len, max_kv_len, st);
+    return D == 128 ? launch_extend<__nv_bfloat16, 128>(p, n_values, bs, max_extend_len, max_kv_len, host, st)
+                    : launch_extend<__nv_bfloat16, 64>(p, n_values, bs, max_extend_len, max_kv_len, host, st);
+  return D == 128 ? launch_extend<__half, 128>(p, n_values, bs, max_extend_len, max_kv_len, host, st)
+                  : launch_extend<__half, 64>(p, n_values, bs, max_extend_len, max_kv_len, host, st);
 }
 
 int b200_attn_extend_heads(const void* q, int64_t q_stride, const void* k_cache, const void* v_cache,
@@ -876,10 +937,18 @@ int b200_attn_extend_known(const void* q, int64_t q_stride, const void* k_cache,
 }
 
 static size_t align256(size_t n) { return (n + 255) & ~static_cast<size_t>(255); }
-
-size_t b200_extend_layer_scratch_bytes(int64_t total_kv, int64_t row_elems, int64_t bs, int64_t max_kv_len) {
+static size_t extend_dense_bytes(int64_t total_kv, int64_t row_elems, int64_t bs, int64_t max_kv_len) {
   return 2 * align256(static_cast<size_t>(total_kv) * row_elems * 2) + align256(static_cast<size_t>(bs) * 8) +
          align256(static_cast<size_t>(bs) * ((max_kv_len + 3) / 4 * 4) * 4);
+}
+
+size_t b200_extend_layer_scratch_bytes(int64_t pool_fp8, int64_t total_kv, int64_t bs, int64_t max_kv_len, int64_t Hkv,
+                                       int64_t D) {
+  using namespace b200;
+  size_t n = pool_fp8 ? extend_dense_bytes(total_kv, Hkv * D, bs, max_kv_len) : 0;
+  if (max_kv_len >= kWideMinKeys && bs <= kFlatMaxBs)
+    n += D == 128 ? flat_workspace_bytes<128>(device_sm_count()) : D == 64 ? flat_workspace_bytes<64>(device_sm_count()) : 0;
+  return n;
 }
 
 int b200_extend_layer(const b200_extend_layer_args* a) {
@@ -905,10 +974,14 @@ int b200_extend_layer(const b200_extend_layer_args* a) {
   const int64_t* idx = a->req_pool_indices;
   int64_t rtt_stride = a->req_to_token_stride;
   double scale = a->scale, out_scale = 1.0;
+  b200::ExtendHost host;
+  host.workspace = a->scratch;
+  host.workspace_bytes = static_cast<size_t>(a->scratch_bytes);
+  host.lens = a->host_lens;
   if (a->pool_fp8) {
     // the tcgen05 kernels want 16-bit operands: an exact dense copy; the scales ride on the softmax scale and the output
-    B200_REQUIRE(a->scratch && static_cast<size_t>(a->scratch_bytes) >=
-                                   b200_extend_layer_scratch_bytes(a->total_kv, row, a->bs, a->max_kv_len),
+    const size_t dense_bytes = extend_dense_bytes(a->total_kv, row, a->bs, a->max_kv_len);
+    B200_REQUIRE(a->scratch && static_cast<size_t>(a->scratch_bytes) >= dense_bytes,
                  "b200_extend_layer: scratch of %lld bytes is too small", static_cast<long long>(a->scratch_bytes));
     char* at = static_cast<char*>(a->scratch);
     const size_t rows = align256(static_cast<size_t>(a->total_kv) * row * 2);
@@ -919,6 +992,8 @@ int b200_extend_layer(const b200_extend_layer_args* a) {
     const int rc = b200_kv_dequant_dense(kc, vc, static_cast<int>(row), rtt, a->req_to_token_stride, idx, a->seq_lens, nullptr,
                                          k16, v16, dense, rtt_stride, dense_idx, bs, a->max_kv_len, pool_dtype, a->stream);
     if (rc) return rc;
+    host.workspace = at + dense_bytes;
+    host.workspace_bytes = static_cast<size_t>(a->scratch_bytes) - dense_bytes;
     kc = k16;
     vc = v16;
     rtt = dense;
@@ -931,7 +1006,7 @@ int b200_extend_layer(const b200_extend_layer_args* a) {
                            a->extend_lens, a->extend_start, bs, static_cast<int>(a->max_extend_len), Hq, Hkv, D, static_cast<int>(a->Dv),
                            static_cast<float>(scale), static_cast<float>(a->logit_cap), static_cast<float>(out_scale),
                            static_cast<int>(a->causal), 0, 0, nullptr, -1, 1, 0, nullptr, 0, dtype, a->stream, nullptr, 0, 0.f,
-                           static_cast<int>(a->max_kv_len));
+                           static_cast<int>(a->max_kv_len), host);
 }
 
 }  // extern "C"

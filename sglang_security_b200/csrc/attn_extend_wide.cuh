@@ -27,8 +27,9 @@ namespace b200 {
 
 constexpr int kWideThreads = 384;
 constexpr int kWideTile = 128;                     // keys
+constexpr int kWideMinKeys = 1024;                 // shorter requests: attn_extend_kernel
 constexpr int kWideLoaders = 96;
-constexpr int kWideSoftmaxRegs = 200, kWideOtherRegs = 96;   // 256 x 200 + 128 x 96 <= 384 x 168 at launch
+constexpr int kWideSoftmaxRegs = 192, kWideOtherRegs = 120;   // 256 x 192 + 128 x 120 <= 384 x 168 at launch; no spills
 
 template <int D>
 struct WideCfg {

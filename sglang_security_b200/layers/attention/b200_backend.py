@@ -19,6 +19,7 @@ decode step can be captured in a CUDA graph.
 """
 from __future__ import annotations
 
+from array import array
 from dataclasses import dataclass, field
 from typing import Dict, Optional
 
@@ -40,6 +41,7 @@ class ForwardMetadata:
     max_extend_len: int = 0
     max_kv_len: int = 0          # longest prefix + new tokens, 0 when the host does not know it
     total_extend: int = 0
+    host_lens: Optional[array] = None   # new tokens, prefix of every request, where long requests may share the SMs
     # dtype-converted copies of the ForwardBatch index tensors, kept alive for the whole forward
     # (one conversion per step, never a temporary whose block the allocator could hand out again
     # before the launch has read it); keyed by (data_ptr, dtype, numel) of the source
@@ -161,12 +163,14 @@ class B200AttnBackend(AttentionBackend):
         else:
             max_len = int(ext.max().item()) if ext.numel() else 0
             total = int(ext.sum().item()) if ext.numel() else 0
-        max_kv = 0
+        max_kv, host_lens = 0, None
         if forward_batch.extend_seq_lens_cpu is not None and forward_batch.extend_prefix_lens_cpu is not None:
-            max_kv = max((p + e for p, e in zip(forward_batch.extend_prefix_lens_cpu,
-                                                forward_batch.extend_seq_lens_cpu)), default=0)
+            pairs = list(zip(forward_batch.extend_seq_lens_cpu, forward_batch.extend_prefix_lens_cpu))
+            max_kv = max((p + e for e, p in pairs), default=0)
+            if max_kv >= 1024:
+                host_lens = array("i", [n for pair in pairs for n in pair])
         return ForwardMetadata(qo_indptr=start.to(torch.int32), max_extend_len=int(max_len), max_kv_len=int(max_kv),
-                               total_extend=int(total))
+                               total_extend=int(total), host_lens=host_lens)
 
     # ------------------------------------------------------------------ CUDA graph hooks
     def init_cuda_graph_state(self, max_bs: int):
@@ -376,17 +380,24 @@ class B200AttnBackend(AttentionBackend):
             if rows is not None and (ks is None) != (vs is None):
                 raise _lib.B200Error("forward_extend: k_scale and v_scale must be given together")
             total_kv, max_kv = md.kv_extent(forward_batch, seq_lens)
-            scratch_bytes = self.lib.b200_extend_layer_scratch_bytes(total_kv, hkv * d, bs, max_kv)
-            scratch = torch.empty(scratch_bytes, dtype=torch.uint8, device=q.device)
+        if fp8 or max_kv >= 1024:       # where the keys may be spread over the SMs
+            scratch_bytes = self.lib.b200_extend_layer_scratch_bytes(1 if fp8 else 0, total_kv, bs, max_kv, hkv, d)
+            try:
+                scratch = torch.empty(scratch_bytes, dtype=torch.uint8, device=q.device)
+            except torch.cuda.OutOfMemoryError:          # an FP8 pool's dense copy at least, or nothing
+                scratch_bytes = self.lib.b200_extend_layer_scratch_bytes(1, total_kv, bs, max_kv, hkv * d, 1) if fp8 else 0
+                scratch = torch.empty(scratch_bytes, dtype=torch.uint8, device=q.device) if fp8 else None
         kp = vp = kst = vst = locp = n_new = 0
         if rows is not None:
             k, v, loc = rows
             kp, vp, kst, vst, locp, n_new = k.data_ptr(), v.data_ptr(), k.stride(0), v.stride(0), loc.data_ptr(), loc.numel()
+        lens = md.host_lens.buffer_info()[0] if md.host_lens is not None and len(md.host_lens) == 2 * bs else 0
         args = _lib.EXTEND_LAYER_ARGS.pack(
             q.data_ptr(), q.stride(0), k_cache.data_ptr(), v_cache.data_ptr(), k_cache.stride(0), o.data_ptr(), o.stride(0),
             req_to_token.data_ptr(), req_to_token.stride(0), req_pool_indices.data_ptr(), seq_lens.data_ptr(),
             prefix_lens.data_ptr(), extend_lens.data_ptr(), md.qo_indptr.data_ptr(), kp, vp, kst, vst, locp, n_new,
-            0 if scratch is None else scratch.data_ptr(), scratch_bytes, total_kv, bs, md.max_extend_len, max_kv, hq, hkv, d, dv,
+            0 if scratch is None else scratch.data_ptr(), scratch_bytes, total_kv, lens, bs,
+            md.max_extend_len, max_kv, hq, hkv, d, dv,
             1 if causal else 0, _lib.dtype_code(q.dtype),
             0 if not fp8 else 2 if k_cache.dtype == torch.float8_e5m2 else 1, float(layer.scaling),
             float(layer.logit_cap or 0.0), 1.0 if ks is None else ks, 1.0 if vs is None else vs, 0 if ks is None else 1,
