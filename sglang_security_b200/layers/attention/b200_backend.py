@@ -353,7 +353,8 @@ class B200AttnBackend(AttentionBackend):
         # like the oracle (torch_native_backend.py:196-199)
         rows = None
         if save_kv_cache:
-            rows = None if empty else self._new_rows(k, v, k_cache, v_cache, pool, forward_batch.out_cache_loc, hkv, d)
+            rows = None if empty else self._new_rows(q.dtype, k, v, k_cache, v_cache, pool, forward_batch.out_cache_loc,
+                                                     hkv, d)
             if rows is None:
                 self._save_kv(layer, forward_batch, k, v)
         if empty:
@@ -406,12 +407,17 @@ class B200AttnBackend(AttentionBackend):
         return o
 
     @staticmethod
-    def _new_rows(k, v, k_cache, v_cache, pool, loc, hkv, d):
-        """-> (k, v, loc) as b200_extend_layer stores them, or None where the pool stores them itself."""
-        if not (k.is_cuda and loc.dtype == torch.int64 and loc.is_contiguous() and k.dtype == v.dtype):
+    def _new_rows(q_dtype, k, v, k_cache, v_cache, pool, loc, hkv, d):
+        """-> (k, v, loc) as b200_extend_layer stores them, or None where _save_kv stores them.
+
+        The native call has one type, that of q, for q and the new rows: rows of another one (the other 16-bit type,
+        bytes that are in the pool's FP8 type already, 32 bits) are not for it."""
+        if not (k.is_cuda and loc.dtype == torch.int64 and loc.is_contiguous()):
             return None
-        if k.dtype != k_cache.dtype and not (type(pool) is MHATokenToKVPool and _lib.is_fp8_kv(k_cache.dtype)
-                                             and k.dtype in (torch.bfloat16, torch.float16)):
+        if q_dtype not in (torch.bfloat16, torch.float16) or k.dtype != q_dtype or v.dtype != q_dtype:
+            return None
+        if v_cache.dtype != k_cache.dtype or (k_cache.dtype != q_dtype and not (
+                type(pool) is MHATokenToKVPool and _lib.is_fp8_kv(k_cache.dtype))):
             return None
         n = loc.numel()
         if n == 0 or not (k_cache.is_contiguous() and v_cache.is_contiguous()):
