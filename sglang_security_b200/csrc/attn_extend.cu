@@ -959,6 +959,8 @@ int b200_extend_layer(const b200_extend_layer_args* a) {
   B200_REQUIRE(a->kv_row_stride == row || (!a->k && !a->pool_fp8), "b200_extend_layer: pool rows of %lld elements for %lld heads",
                static_cast<long long>(a->kv_row_stride), static_cast<long long>(a->Hkv));
   if (a->k) {
+    // rows of other types would be stored with half or twice their width before the attention refuses the type
+    B200_REQUIRE(dtype == B200_BF16 || dtype == B200_F16, "b200_extend_layer: new rows of dtype %d", dtype);
     const int n = static_cast<int>(a->num_new);
     const int rc = a->pool_fp8
                        ? b200_kv_write_fp8(a->k, a->v, a->k_stride, a->v_stride, a->k_cache, a->v_cache, a->loc, n,

@@ -97,3 +97,20 @@ def test_a_32_bit_pool_is_written_whole_before_its_type_is_refused():
     assert isinstance(r.out, _lib.B200Error)
     kv_write(r.k, r.v, *r.before, r.loc)
     assert torch.equal(r.pool.k_buffer[0], r.before[0]) and torch.equal(r.pool.v_buffer[0], r.before[1])
+
+
+@pytest.mark.parametrize("pool_fp8", [0, 1, 2])
+def test_the_native_call_refuses_new_rows_of_other_types_before_it_writes(pool_fp8):
+    """No rows and no requests: nothing would be launched, and the type is refused all the same."""
+    lib, at = _lib.load(), torch.zeros(64, dtype=torch.uint8).data_ptr()
+
+    def call(dtype):
+        return lib.b200_extend_layer(_lib.EXTEND_LAYER_ARGS.pack(
+            at, 128, at, at, 128, at, 128, at, 8, at, at, at, at, at, at, at, 128, 128, at, 0, 0, 0, 0, 0,
+            0, 0, 0, 2, 2, 64, 64, 1, dtype, pool_fp8, 1.0, 0.0, 1.0, 1.0, 0, 0))
+
+    assert call(_lib.BF16) == 0 and call(_lib.F16) == 0
+    for dtype in (_lib.F32, _lib.FP8_E4M3, 7):
+        assert call(dtype) != 0
+        with pytest.raises(_lib.B200Error, match="new rows of dtype"):
+            _lib.check(call(dtype), "b200_extend_layer")
