@@ -273,8 +273,16 @@ typedef struct {
   void* stream;
 } b200_extend_layer_args;
 int b200_extend_layer(const b200_extend_layer_args* args);
+/* The most scratch that such a call uses: an FP8 pool's copy and the persistent kernel's workspace. */
 size_t b200_extend_layer_scratch_bytes(int64_t pool_fp8, int64_t total_kv, int64_t bs, int64_t max_kv_len, int64_t Hkv,
                                        int64_t D);
+/* For callers with many layers of one batch, who choose once: an FP8 pool's copy alone; the persistent kernel's workspace
+ * where the estimates choose that kernel for the call (scale: with k_scale on it), else 0; the call itself, whose scratch
+ * is the sum of both and which takes that kernel (flat != 0) or another (flat == 0) without estimating again. */
+size_t b200_extend_layer_dense_bytes(int64_t total_kv, int64_t bs, int64_t max_kv_len, int64_t Hkv, int64_t D);
+size_t b200_extend_layer_flat_bytes(int64_t bs, int64_t max_extend_len, int64_t max_kv_len, int64_t Hq, int64_t Hkv,
+                                    int64_t D, int64_t causal, double scale, double logit_cap, const int32_t* host_lens);
+int b200_extend_layer_planned(const b200_extend_layer_args* args, int flat);
 
 /* Same kernel with an output multiplier: extend over an FP8 KV pool runs on an exact 16-bit copy
  * of the requests' rows (b200_kv_dequant_gather) with scale * k_scale and out_scale = v_scale.    */

@@ -8,7 +8,7 @@ from __future__ import annotations
 
 import ctypes
 import struct
-from ctypes import c_char_p, c_float, c_int, c_int64, c_size_t, c_void_p
+from ctypes import c_char_p, c_double, c_float, c_int, c_int64, c_size_t, c_void_p
 from pathlib import Path
 
 _LIB_PATH = Path(__file__).resolve().parent / "lib" / "libb200hotpath.so"
@@ -52,6 +52,10 @@ _SIGNATURES = {
                                        c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                                        c_int, c_int, c_int, c_int, c_float, c_float, c_float, c_int, c_int, c_void_p]),
     "b200_extend_layer": (c_int, [c_char_p]),
+    "b200_extend_layer_planned": (c_int, [c_char_p, c_int]),
+    "b200_extend_layer_dense_bytes": (c_size_t, [c_int64, c_int64, c_int64, c_int64, c_int64]),
+    "b200_extend_layer_flat_bytes": (c_size_t, [c_int64, c_int64, c_int64, c_int64, c_int64, c_int64, c_int64, c_double,
+                                                c_double, c_void_p]),
     "b200_extend_layer_scratch_bytes": (c_size_t, [c_int64, c_int64, c_int64, c_int64, c_int64, c_int64]),
     "b200_kv_dequant_dense": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_int64, c_void_p, c_void_p, c_void_p,
                                       c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_int, c_int64, c_int,

@@ -649,6 +649,7 @@ struct ExtendHost {
   void* workspace = nullptr;        // attn_extend_flat.cuh
   size_t workspace_bytes = 0;
   const int32_t* lens = nullptr;    // new tokens and prefix of every request, or null
+  int flat = -1;                    // the persistent kernel: chosen before the call (1), not (0), to be chosen in the call (-1)
 };
 // When the two-tile kernel's last CTA ends: its CTAs in the order of the grid, each to the SM that is free first.  From 68
 // calls timed (within 6 %, head size 64 2 %; without the requests' lengths, and so the order, 20 %).
@@ -673,23 +674,24 @@ static double wide_last_us(int D, const ExtendParams& p, int bs, int max_extend_
 // sizes 64 and 128, 1 to 30 equal and ragged requests of 64 to 8192 new tokens behind 0 to 8000).  Its time is a fixed part
 // (the plan, the first loads, the last store, the merge) and every SM's equal share of items and key tiles (within 6 %); it
 // has to be a twentieth less than the others'.  Not above four waves of the two-tile kernel's CTAs, whose last one is a
-// small part there (2 x 8192 fresh tokens 944 us there, 1052 here), which also bounds the work of this estimate (~8 us).
+// small part there (2 x 8192 fresh tokens 944 us there, 1052 here), which also bounds the work of this estimate (~8 us:
+// callers with many layers of one batch ask b200_extend_layer_flat_bytes once).
 // 48 of the calls come here, 12 % faster on average, 4 % slower at worst (us, there / here: groups of 4, 8 x 512 behind 1536
 // 115 / 109, behind 4000 211 / 189, 3 x 100 behind 7000 146 / 61; head size 64, 2 x 1000 behind 7000 113 / 76).
 static bool flat_pays(int D, const ExtendParams& p, int bs, int max_extend_len, int64_t ctas, int splits, double wide, double narrow,
-                      const ExtendHost& host) {
+                      const int32_t* lens) {
   const int sms = device_sm_count(), tok_cta = 256 / p.pack;
-  if (!p.causal || !host.lens || ctas > 4 * sms || sms > kFlatMaxSms) return false;
+  if (!p.causal || !lens || ctas > 4 * sms || sms > kFlatMaxSms) return false;
   double items = 0, tiles = 0;
   for (int b = 0; b < bs; ++b)
-    for (int q = 0; q * tok_cta < host.lens[2 * b]; ++q) {
+    for (int q = 0; q * tok_cta < lens[2 * b]; ++q) {
       items += 1;
-      tiles += flat_tiles(host.lens[2 * b + 1], host.lens[2 * b], q, tok_cta, 1);
+      tiles += flat_tiles(lens[2 * b + 1], lens[2 * b], q, tok_cta, 1);
     }
   const double share = static_cast<double>(p.Hkv) * p.head_tiles / sms;
   const double flat = D == 128 ? 28.7 + (2.03 * tiles + 8.2 * items) * share : 18.8 + (1.9 * tiles + 5.6 * items) * share;
   if (flat >= 0.95 * narrow) return false;
-  return flat < 0.95 * (splits > 1 ? wide : wide_last_us(D, p, bs, max_extend_len, host.lens));
+  return flat < 0.95 * (splits > 1 ? wide : wide_last_us(D, p, bs, max_extend_len, lens));
 }
 // B200_EXTEND_FLAT: 0 never, 1 wherever it can (read per launch, for tests and A/B); else -1: by the estimates
 static int extend_flat_choice() {
@@ -697,23 +699,35 @@ static int extend_flat_choice() {
   return e && (e[0] == '0' || e[0] == '1') ? e[0] - '0' : -1;
 }
 
+// a cap up to 40 keeps e^(-2 cap) a normal fp32 (and 16-bit) number: the one-pass capped form
+static bool extend_fast(const ExtendParams& p) {
+  const float ref = p.score_bound > 0.f && p.score_bound < p.logit_cap ? p.score_bound : p.logit_cap;
+  return ref <= 40.f && p.qk_scale > 0.f && extend_fast_softmax_enabled();
+}
+// What the kernels with two query tiles a CTA take
+static bool extend_plain(const ExtendParams& p, int n_values, int keys) {
+  return extend_fast(p) && keys >= kWideMinKeys && p.logit_cap <= 0.f && p.window == 0 && !p.sink && !p.gate && !p.lse &&
+         n_values == 1 && p.v_head < 0;
+}
+static size_t flat_bytes(int D) {
+  return D == 128 ? flat_workspace_bytes<128>(device_sm_count()) : flat_workspace_bytes<64>(device_sm_count());
+}
+
 template <typename T, int D>
 static int launch_extend(const ExtendParams& p, int n_values, int bs, int max_extend_len, int max_kv_len,
                          const ExtendHost& host, cudaStream_t st) {
-  // a cap up to 40 keeps e^(-2 cap) a normal fp32 (and 16-bit) number: the one-pass capped form
-  const float ref = p.score_bound > 0.f && p.score_bound < p.logit_cap ? p.score_bound : p.logit_cap;
-  const bool fast = ref <= 40.f && p.qk_scale > 0.f && extend_fast_softmax_enabled();
+  const bool fast = extend_fast(p);
   // Plain attention over 1024 keys or more: two query tiles per CTA where that is expected to end sooner.  All options,
   // and shorter requests, on the kernel above, whose two CTAs per SM hide what a CTA of the other spends before its first
   // and after its last tile (~8 us; us, this / that kernel: 8 x 512 fresh tokens 63.6 / 72.3).
   const int keys = max_kv_len > 0 ? max_kv_len : max_extend_len;
-  if (fast && keys >= kWideMinKeys && p.logit_cap <= 0.f && p.window == 0 && !p.sink && !p.gate && !p.lse && n_values == 1 && p.v_head < 0) {
+  if (extend_plain(p, n_values, keys)) {
     int splits = 1;
     const int64_t ctas = wide_ctas<T, D>(p, bs, max_extend_len, max_kv_len, &splits);
     const double wide = wide_us(D, p, max_extend_len, keys, ctas, splits), narrow = narrow_us(D, p, bs, max_extend_len, keys);
     const int choice = extend_flat_choice();
-    if (choice != 0 && host.workspace && bs <= kFlatMaxBs && host.workspace_bytes >= flat_workspace_bytes<D>(device_sm_count()) &&
-        (choice == 1 || flat_pays(D, p, bs, max_extend_len, ctas, splits, wide, narrow, host)))
+    if (choice != 0 && host.flat != 0 && host.workspace && bs <= kFlatMaxBs && host.workspace_bytes >= flat_bytes(D) &&
+        (choice == 1 || host.flat == 1 || flat_pays(D, p, bs, max_extend_len, ctas, splits, wide, narrow, host.lens)))
       return launch_extend_flat<T, D>(p, bs, static_cast<float*>(host.workspace), host.workspace_bytes, st);
     if (wide <= narrow)
       return launch_extend_wide<T, D>(p, bs, max_extend_len, splits, st);
@@ -731,6 +745,31 @@ static int launch_extend(const ExtendParams& p, int n_values, int bs, int max_ex
   }
   return fast ? launch_extend_inst<T, D, 1>(p, bs, max_extend_len, st)
               : launch_extend_inst<T, D, 0>(p, bs, max_extend_len, st);
+}
+
+// heads of one GQA group packed into the 128-row tile: largest power of two dividing the group
+static void extend_pack(ExtendParams* p, int Hq, int Hkv) {
+  p->Hq = Hq;
+  p->Hkv = Hkv;
+  p->group = Hq / Hkv;
+  int pack = 1;
+  while (pack < 8 && p->group % (pack * 2) == 0) pack *= 2;
+  p->pack = pack;
+  p->head_tiles = p->group / pack;
+}
+static float extend_qk_scale(float scale, float logit_cap) { return logit_cap > 0.f ? scale : scale * 1.4426950408889634f; }
+
+// Whether a plain call goes to the persistent kernel (launch_extend), without making it
+template <int D>
+static bool flat_chosen(const ExtendParams& p, int bs, int max_extend_len, int max_kv_len, const int32_t* lens) {
+  const int keys = max_kv_len > 0 ? max_kv_len : max_extend_len, choice = extend_flat_choice();
+  if (choice == 0 || bs > kFlatMaxBs || !extend_plain(p, 1, keys)) return false;
+  if (choice == 1) return true;
+  if (!p.causal || !lens) return false;            // (flat_pays; before the occupancy is asked for)
+  int splits = 1;
+  const int64_t ctas = wide_ctas<__nv_bfloat16, D>(p, bs, max_extend_len, max_kv_len, &splits);   // the same for f16
+  return flat_pays(D, p, bs, max_extend_len, ctas, splits, wide_us(D, p, max_extend_len, keys, ctas, splits),
+                   narrow_us(D, p, bs, max_extend_len, keys), lens);
 }
 
 }  // namespace b200
@@ -846,17 +885,10 @@ static int extend_heads_impl(const void* q, int64_t q_stride, const void* k_cach
   p.prefix_lens = extend_prefix_lens;
   p.extend_lens = extend_seq_lens;
   p.extend_start = extend_start_loc;
-  p.Hq = Hq;
-  p.Hkv = Hkv;
-  p.group = Hq / Hkv;
-  // heads of one GQA group packed into the 128-row tile: largest power of two dividing the group
-  int pack = 1;
-  while (pack < 8 && p.group % (pack * 2) == 0) pack *= 2;
-  p.pack = pack;
-  p.head_tiles = p.group / pack;
+  extend_pack(&p, Hq, Hkv);
   p.logit_cap = logit_cap;
   p.out_scale = out_scale;
-  p.qk_scale = logit_cap > 0.f ? scale : scale * 1.4426950408889634f;
+  p.qk_scale = extend_qk_scale(scale, logit_cap);
   p.causal = causal;
   p.window = window;
   p.keep_first = window > 0 ? keep_first : 0;
@@ -947,11 +979,33 @@ size_t b200_extend_layer_scratch_bytes(int64_t pool_fp8, int64_t total_kv, int64
   using namespace b200;
   size_t n = pool_fp8 ? extend_dense_bytes(total_kv, Hkv * D, bs, max_kv_len) : 0;
   if (max_kv_len >= kWideMinKeys && bs <= kFlatMaxBs)
-    n += D == 128 ? flat_workspace_bytes<128>(device_sm_count()) : D == 64 ? flat_workspace_bytes<64>(device_sm_count()) : 0;
+    n += D == 128 || D == 64 ? flat_bytes(static_cast<int>(D)) : 0;
   return n;
 }
+size_t b200_extend_layer_dense_bytes(int64_t total_kv, int64_t bs, int64_t max_kv_len, int64_t Hkv, int64_t D) {
+  return extend_dense_bytes(total_kv, Hkv * D, bs, max_kv_len);
+}
 
-int b200_extend_layer(const b200_extend_layer_args* a) {
+size_t b200_extend_layer_flat_bytes(int64_t bs, int64_t max_extend_len, int64_t max_kv_len, int64_t Hq, int64_t Hkv, int64_t D,
+                                    int64_t causal, double scale, double logit_cap, const int32_t* host_lens) {
+  using namespace b200;
+  if (bs <= 0 || max_extend_len <= 0 || Hkv <= 0 || Hq <= 0 || Hq % Hkv != 0 || (D != 64 && D != 128)) return 0;
+  ExtendParams p = {};
+  extend_pack(&p, static_cast<int>(Hq), static_cast<int>(Hkv));
+  p.causal = causal ? 1 : 0;
+  p.logit_cap = static_cast<float>(logit_cap);
+  p.qk_scale = extend_qk_scale(static_cast<float>(scale), p.logit_cap);
+  p.v_head = -1;
+  const int n = static_cast<int>(bs), ext = static_cast<int>(max_extend_len), kv = static_cast<int>(max_kv_len);
+  const bool flat = D == 128 ? flat_chosen<128>(p, n, ext, kv, host_lens) : flat_chosen<64>(p, n, ext, kv, host_lens);
+  return flat ? flat_bytes(static_cast<int>(D)) : 0;
+}
+
+static int extend_layer_impl(const b200_extend_layer_args* a, int flat);
+int b200_extend_layer(const b200_extend_layer_args* a) { return extend_layer_impl(a, -1); }
+int b200_extend_layer_planned(const b200_extend_layer_args* a, int flat) { return extend_layer_impl(a, flat ? 1 : 0); }
+
+static int extend_layer_impl(const b200_extend_layer_args* a, int flat) {
   B200_REQUIRE(a, "b200_extend_layer: null pointer");
   const int64_t row = a->Hkv * a->D;
   const int dtype = static_cast<int>(a->dtype), bs = static_cast<int>(a->bs);
@@ -980,6 +1034,7 @@ int b200_extend_layer(const b200_extend_layer_args* a) {
   host.workspace = a->scratch;
   host.workspace_bytes = static_cast<size_t>(a->scratch_bytes);
   host.lens = a->host_lens;
+  host.flat = flat;
   if (a->pool_fp8) {
     // the tcgen05 kernels want 16-bit operands: an exact dense copy; the scales ride on the softmax scale and the output
     const size_t dense_bytes = extend_dense_bytes(a->total_kv, row, a->bs, a->max_kv_len);

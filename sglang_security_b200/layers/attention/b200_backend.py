@@ -47,6 +47,7 @@ class ForwardMetadata:
     # before the launch has read it); keyed by (data_ptr, dtype, numel) of the source
     converted: Dict[tuple, torch.Tensor] = field(default_factory=dict)
     extent: Optional[tuple] = None
+    flat_bytes: Dict[tuple, int] = field(default_factory=dict)   # of forward_extend's choice, by a layer's form
 
     def kv_extent(self, forward_batch, seq_lens) -> tuple:
         """(sum, maximum) of the sequence lengths, from the host's copy where there is one; once per forward."""
@@ -381,18 +382,29 @@ class B200AttnBackend(AttentionBackend):
             if rows is not None and (ks is None) != (vs is None):
                 raise _lib.B200Error("forward_extend: k_scale and v_scale must be given together")
             total_kv, max_kv = md.kv_extent(forward_batch, seq_lens)
-        if fp8 or max_kv >= 1024:       # where the keys may be spread over the SMs
-            scratch_bytes = self.lib.b200_extend_layer_scratch_bytes(1 if fp8 else 0, total_kv, bs, max_kv, hkv, d)
+            scratch_bytes = self.lib.b200_extend_layer_dense_bytes(total_kv, bs, max_kv, hkv, d)
+        lens = md.host_lens.buffer_info()[0] if md.host_lens is not None and len(md.host_lens) == 2 * bs else 0
+        flat = 0
+        if max_kv >= 1024:
+            # whether the persistent kernel takes it, and its workspace: once per forward, not in every layer
+            scale = float(layer.scaling) * (1.0 if ks is None else ks)
+            form = (bs, max_kv, hq, hkv, d, causal, scale, float(layer.logit_cap or 0.0), os.environ.get("B200_EXTEND_FLAT"))
+            flat = md.flat_bytes.get(form)
+            if flat is None:
+                flat = md.flat_bytes[form] = self.lib.b200_extend_layer_flat_bytes(
+                    bs, md.max_extend_len, max_kv, hq, hkv, d, 1 if causal else 0, *form[6:8], lens)
+        if flat:
             try:
-                scratch = torch.empty(scratch_bytes, dtype=torch.uint8, device=q.device)
-            except torch.cuda.OutOfMemoryError:          # an FP8 pool's dense copy at least, or nothing
-                scratch_bytes = self.lib.b200_extend_layer_scratch_bytes(1, total_kv, bs, max_kv, hkv * d, 1) if fp8 else 0
-                scratch = torch.empty(scratch_bytes, dtype=torch.uint8, device=q.device) if fp8 else None
+                scratch = torch.empty(scratch_bytes + flat, dtype=torch.uint8, device=q.device)
+                scratch_bytes += flat
+            except torch.cuda.OutOfMemoryError:          # the other kernels need none; not asked for again in this forward
+                flat = md.flat_bytes[form] = 0
+        if scratch is None and scratch_bytes:
+            scratch = torch.empty(scratch_bytes, dtype=torch.uint8, device=q.device)
         kp = vp = kst = vst = locp = n_new = 0
         if rows is not None:
             k, v, loc = rows
             kp, vp, kst, vst, locp, n_new = k.data_ptr(), v.data_ptr(), k.stride(0), v.stride(0), loc.data_ptr(), loc.numel()
-        lens = md.host_lens.buffer_info()[0] if md.host_lens is not None and len(md.host_lens) == 2 * bs else 0
         args = _lib.EXTEND_LAYER_ARGS.pack(
             q.data_ptr(), q.stride(0), k_cache.data_ptr(), v_cache.data_ptr(), k_cache.stride(0), o.data_ptr(), o.stride(0),
             req_to_token.data_ptr(), req_to_token.stride(0), req_pool_indices.data_ptr(), seq_lens.data_ptr(),
@@ -403,7 +415,7 @@ class B200AttnBackend(AttentionBackend):
             0 if not fp8 else 2 if k_cache.dtype == torch.float8_e5m2 else 1, float(layer.scaling),
             float(layer.logit_cap or 0.0), 1.0 if ks is None else ks, 1.0 if vs is None else vs, 0 if ks is None else 1,
             _lib.current_stream())
-        _lib.check(self.lib.b200_extend_layer(args), "b200_attn_extend")
+        _lib.check(self.lib.b200_extend_layer_planned(args, 1 if flat else 0), "b200_attn_extend")
         return o
 
     @staticmethod
