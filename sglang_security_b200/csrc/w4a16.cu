@@ -29,6 +29,8 @@
 
 namespace b200 {
 
+static WaitCounter wait_counter_registered(tc::wait_counter());
+
 int w4a16_gemv_max_m(int N);                                   // w4a16_gemv.cu
 bool w4a16_gemv_supported(int M, int N, int K, int group);
 
@@ -176,6 +178,7 @@ struct W4GemmParams {
   int M, N, K, group;
   int raw_tma;              // 1: packed tiles by TMA (N % 32 == 0), 0: by the producer warp's lanes
   int kb_per_split;         // SWAP kernels launched as clusters: stages per cluster rank (split-K)
+  int* wait_error;          // tc::report_gave_up
 };
 
 constexpr int kW4PackedBytes = 64 * 64;  // one sub-block: 64 k rows x 16 int32 (= 128 output columns)
@@ -196,7 +199,7 @@ struct W4Cfg {
   static constexpr int ACC_COLS = BM;  // fp32 columns per accumulator set
   static constexpr int TMEM_COLS = 2 * ACC_COLS < 32 ? 32 : 2 * ACC_COLS;
   static constexpr int NBARS = 2 * ST + 2 * RAWS + 4;
-  static constexpr int SMEM = ST * STAGE_BYTES + RAWS * RAW_BYTES + NBARS * 8 + 16 + 1024;
+  static constexpr int SMEM = ST * STAGE_BYTES + RAWS * RAW_BYTES + NBARS * 8 + 16 + 1024;   // + tmem slot, gave up
   static_assert(SMEM <= 232448, "shared memory budget");
 };
 
@@ -219,7 +222,8 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
   auto rempty_bar = [&](int s) { return bars + 8u * (2 * ST + RAWS + s); };
   auto tfull_bar = [&](int a) { return bars + 8u * (2 * ST + 2 * RAWS + a); };
   auto tempty_bar = [&](int a) { return bars + 8u * (2 * ST + 2 * RAWS + 2 + a); };
-  const uint32_t tmem_slot = bars + 8u * C::NBARS;
+  const uint32_t tmem_slot = bars + 8u * C::NBARS, gave_up = tmem_slot + 4;
+  bool dead = false;
   volatile uint32_t* tmem_slot_ptr =
       reinterpret_cast<volatile uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
 
@@ -259,6 +263,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
       tc::mbar_init(tfull_bar(a), 1);
       tc::mbar_init(tempty_bar(a), 4);
     }
+    asm volatile("st.shared.u32 [%0], 0;\n" ::"r"(gave_up) : "memory");
     tc::fence_barrier_init();
   }
   if (warp == 1) {
@@ -278,7 +283,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     for (int tile = tile0; tile < num_tiles; tile += tile_step) {
       const int m_blk = tile % m_blocks;
       for (int kb = kb_begin; kb < kb_end; ++kb) {
-        tc::mbar_wait(empty_bar(stage), phase ^ 1u);
+        tc::mbar_wait_bounded(empty_bar(stage), phase ^ 1u, dead, gave_up);
         if (tc::elect_one()) {
           tc::mbar_arrive_expect_tx(full_bar(stage), C::X_BYTES);
 #pragma unroll
@@ -308,7 +313,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         const uint32_t zdst = dst + KS * kW4PackedBytes;
         if (p.raw_tma) {
           if (lane == 0) {
-            tc::mbar_wait(rempty_bar(rs), rphase ^ 1u);
+            tc::mbar_wait_bounded(rempty_bar(rs), rphase ^ 1u, dead, gave_up);
             tc::mbar_arrive_expect_tx(rfull_bar(rs),
                                       KS * (kW4PackedBytes + (zs_rows ? kW4ZsBytes : 0)));
             tc::tma_load_2d_hint(dst, &tmap_q, rfull_bar(rs), n_blk * (BN / 8), kb * KS * BK,
@@ -324,7 +329,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
           }
         } else {
           // rows whose pitch is not a multiple of 16 bytes: the 32 lanes copy the tile word by word
-          tc::mbar_wait(rempty_bar(rs), rphase ^ 1u);
+          tc::mbar_wait_bounded(rempty_bar(rs), rphase ^ 1u, dead, gave_up);
 #pragma unroll 1
           for (int j = 0; j < KS; ++j) {
             uint32_t v[32];
@@ -372,11 +377,11 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     int local = 0;
     for (int tile = tile0; tile < num_tiles; tile += tile_step, ++local) {
       const int acc = local & 1;
-      tc::mbar_wait(tempty_bar(acc), ((local >> 1) & 1u) ^ 1u);
+      tc::mbar_wait_bounded(tempty_bar(acc), ((local >> 1) & 1u) ^ 1u, dead, gave_up);
       tc::tc_fence_after();
       const uint32_t tmem_d = tmem_base + acc * C::ACC_COLS;
       for (int kb = kb_begin; kb < kb_end; ++kb) {
-        tc::mbar_wait(full_bar(stage), phase);
+        tc::mbar_wait_bounded(full_bar(stage), phase, dead, gave_up);
         tc::tc_fence_after();
         const uint32_t sx = smem_base + stage * C::STAGE_BYTES;
         // weight rows kk*16.. of a [64 k x 128 n] sub-tile; panels of 64 n are 64*128 B apart
@@ -419,7 +424,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     for (int tile = tile0; tile < num_tiles; tile += tile_step, ++local) {
       const int m_blk = tile % m_blocks, n_blk = tile / m_blocks;
       const int acc = local & 1;
-      tc::mbar_wait(tfull_bar(acc), (local >> 1) & 1u);
+      tc::mbar_wait_bounded(tfull_bar(acc), (local >> 1) & 1u, dead, gave_up);
       tc::tc_fence_after();
       if (SWAP) {
         // accumulator lanes = output columns, TMEM columns = tokens
@@ -552,6 +557,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     const uint32_t r_off = row0 * 64 + col * 4;
     int stage = grp, rs = grp;            // ring positions of this group's next stage
     uint32_t phase = 0, rphase = 0;
+    uint32_t polls = tc::kWaitPolls;      // (the clock form here: 256-row tiles 5 % slower, counted 1 to 2 %)
     int tile = tile0, kb = kb_begin + grp;
     while (true) {
       while (kb >= kb_end) {
@@ -563,8 +569,8 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
       // may land after those of the next one: a group that is ahead would take the phase before last of `full` for its own,
       // dequantise the words of an older stage and release the slot for the other group (wrong sums, or a ring that stands
       // still).  So the slot's last owner has to have released it, which is after its copies had landed.
-      if (RAWS % DG != 0) tc::mbar_wait(rempty_bar(rs), rphase ^ 1u);
-      tc::mbar_wait(rfull_bar(rs), rphase);
+      if (RAWS % DG != 0) tc::mbar_wait_counted(rempty_bar(rs), rphase ^ 1u, polls);
+      tc::mbar_wait_counted(rfull_bar(rs), rphase, polls);
       const uint32_t rsrc = raw_base + rs * C::RAW_BYTES;
       uint32_t q[KS][RPT];
       uint4 zb[KS], sc[KS];
@@ -603,8 +609,11 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
       if (zs_rows) {
         uint4 w[RPT];
 #pragma unroll
-        for (int i = 0; i < RPT; ++i) w[i] = dequant8<T>(q[0][i], zb[0], sc[0]);
-        tc::mbar_wait(empty_bar(stage), phase ^ 1u);
+        for (int i = 0; i < RPT; ++i) {
+          w[i] = dequant8<T>(q[0][i], zb[0], sc[0]);
+          asm volatile("" : "+r"(w[i].x), "+r"(w[i].y), "+r"(w[i].z), "+r"(w[i].w));   // before the wait, not behind it
+        }
+        tc::mbar_wait_counted(empty_bar(stage), phase ^ 1u, polls);
 #pragma unroll
         for (int j = 0; j < KS; ++j) {
 #pragma unroll
@@ -623,7 +632,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         const int cc = c < NC ? c : NC - 1;  // clamped: columns >= N are computed but never stored
         int g_cached = -1;
         uint4 zg = make_uint4(0, 0, 0, 0), sg = zg;
-        tc::mbar_wait(empty_bar(stage), phase ^ 1u);
+        tc::mbar_wait_counted(empty_bar(stage), phase ^ 1u, polls);
 #pragma unroll
         for (int j = 0; j < KS; ++j) {
 #pragma unroll
@@ -655,6 +664,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
       }
       kb += DG;
     }
+    if (polls == 0) tc::mark_gave_up(gave_up);
   }
 
   if (SWAP && S > 1 && (warp < 2 || warp >= 6)) {  // everyone but the epilogue warps (done above)
@@ -664,7 +674,10 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
   }
   tc::tc_fence_before();
   __syncthreads();
-  if (warp == 1) tc::tmem_dealloc(tmem_base, C::TMEM_COLS);
+  if (warp == 1) {
+    tc::report_gave_up(gave_up, p.wait_error);
+    tc::tmem_dealloc(tmem_base, C::TMEM_COLS);
+  }
 }
 
 // Tile selection.  M <= 64: swap-AB (tokens are the UMMA N dimension).  Otherwise 128-row tiles, or
@@ -692,7 +705,9 @@ template <typename T, int BM, bool SWAP, int DQ, int DG>
 static int launch_w4a16_gemm(const void* x, int64_t ldx, W4GemmParams p, cudaStream_t st) {
   using C = W4Cfg<BM, SWAP>;
   CUtensorMap tx, tq;
-  int rc = make_tmap_2d(&tx, x, p.M, p.K, ldx * 2, SWAP ? BM : 128, 64, 2, false);
+  int rc = wait_error_arm("w4a16_gemm", &p.wait_error);
+  if (rc) return rc;
+  rc = make_tmap_2d(&tx, x, p.M, p.K, ldx * 2, SWAP ? BM : 128, 64, 2, false);
   if (rc) return rc;
   p.raw_tma = (p.N % 32 == 0 && aligned16(p.qweight)) ? 1 : 0;
   if (p.raw_tma) {

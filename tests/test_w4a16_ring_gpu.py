@@ -72,3 +72,12 @@ def test_many_laps(m, n, k, variant, dtype, group):
     for _ in range(40):
         assert torch.equal(W.w4a16_gemm(x, q, z, s, group), first)
     _lib.check_waits()
+
+
+def test_every_wait_of_the_kernel_has_a_limit():
+    from pathlib import Path
+
+    source = (Path(W.__file__).resolve().parents[2] / "csrc" / "w4a16.cu").read_text()
+    assert "mbar_wait_bounded(" in source and "mbar_wait_counted(" in source
+    assert "mbar_wait(" not in source
+    assert "report_gave_up(" in source and "wait_error_arm(" in source
