@@ -12,8 +12,8 @@
 //   warp 1      MMA issuer: per 64 k four tcgen05.mma of 128 channels x bn tokens, A from tensor memory
 //   warps 2, 3  packed words, zeros and scales by cp.async: 4.5 KiB per 64 k, a deep ring
 //   warps 4-11  dequantisers, two groups on alternate stages: thread = channel; 8 words -> 32 pairs (w - z) * s, rounded as
-//               awq_dequant_kernel does -> tcgen05.st.  With several CTAs per SM: also the epilogue.
-//   warps 12-15 epilogue of the persistent form (one CTA per SM, two accumulators)
+//               awq_dequant_kernel does -> tcgen05.st; then the epilogue.
+// A CTA has one tile (a block of tokens x 128 channels, or a cluster rank's part of its K).
 //
 // A 16-channel x 64-k tile of the stream is 32 pieces of 16 bytes, piece 4 g + t = columns g and g + 8 at k = 8 t ..+7
 // of both 32-k halves.  It lands in shared memory as piece t of all g next to each other, so that the 16-byte reads of a
@@ -21,8 +21,8 @@
 //
 // Bound by the dequantisers: ~200 instructions a warp and stage, ~400 clocks of an SM per 128 channels x 64 k with two CTAs
 // on it (scales read from global memory by the dequantisers had cost 600).  us, w4a16.cu -> here (f16, Qwen2.5-32B at
-// TP 2, qkv / o / gate_up / down): 24 tokens 11.1 / 10.0 / 46.4 / 25.5 -> 8.8 / 7.1 / 30 / 20; 128 tokens 18.4 / 19.1 / 50.8 /
-// 35.6 -> 13.2 / 12.0 / 42.6 / 29.2.
+// TP 2, qkv / o / gate_up / down): 24 tokens 11.1 / 10.0 / 46.4 / 25.5 -> 8.6 / 7.4 / 29.4 / 19.4; 128 tokens 18.4 / 19.1 /
+// 50.8 / 35.6 -> 13.4 / 12.1 / 43.1 / 27.6.
 #include "gemm_tc.cuh"
 
 namespace b200 {
@@ -44,20 +44,24 @@ struct TsParams {
   int* wait_error;
 };
 
-constexpr int kTsMaxX = 8, kTsMaxR = 24, kTsMaxA = 4;   // ring limits
+constexpr int kTsMaxX = 8, kTsMaxR = 24, kTsMinR = 6, kTsMaxA = 4;   // ring limits
 constexpr int kTsWordBytes = 4096, kTsRowBytes = 256;
-constexpr int kTsBarBytes = (2 * kTsMaxX + 2 * kTsMaxR + 2 * kTsMaxA + 4) * 8 + 16;
+constexpr int kTsThreads = 384;
+constexpr int kTsBarBytes = (2 * kTsMaxX + 2 * kTsMaxR + 2 * kTsMaxA + 1) * 8 + 16;
 
 template <int CTAS>
 struct TsCfg {
-  static constexpr int WARPS = CTAS > 1 ? 12 : 16;
-  static constexpr int ND = CTAS > 1 ? 1 : 2;                  // accumulators
   static constexpr int NA = CTAS == 3 ? 2 : 4;                 // A buffers of 64 k (32 columns), NA / 2 per dequantising group
   static constexpr int MAX_BN = CTAS == 3 ? 64 : CTAS == 2 ? 128 : 192;
   static constexpr int D_COL = NA * 32;
   static constexpr int TMEM_COLS = CTAS == 3 ? 128 : CTAS == 2 ? 256 : 512;
   static constexpr int BUDGET = CTAS == 3 ? 75 * 1024 : CTAS == 2 ? 113 * 1024 : 225 * 1024;
-  static_assert(D_COL + ND * MAX_BN <= TMEM_COLS, "tensor memory");
+  static_assert(D_COL + MAX_BN <= TMEM_COLS, "tensor memory");
+  // The packed ring may have an odd number of slots, which then pass from one dequantising group to the other.  A group that
+  // waits for the words of stage i has stored stage i - 2, so the MMAs of stage i - 2 - NA are done, and with them the words
+  // of all stages up to that one had landed: a slot's phase before the one waited for is complete, and its parity is not
+  // taken for that of the phase before last.
+  static_assert(NA + 2 <= kTsMinR, "a group may not be a lap of the packed ring ahead");
 };
 
 template <typename T>
@@ -116,7 +120,7 @@ __device__ __forceinline__ uint32_t ts_ld_pair(uint32_t addr) {   // one 16-bit 
 }
 
 template <typename T, int CTAS>
-__global__ void __launch_bounds__(TsCfg<CTAS>::WARPS * 32, CTAS)
+__global__ void __launch_bounds__(kTsThreads, CTAS)
 w4a16_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsParams p) {
   using C = TsCfg<CTAS>;
   extern __shared__ uint8_t smem_raw[];
@@ -130,20 +134,19 @@ w4a16_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsParams p) {
   auto rempty = [&](int s) { return bars + 8u * (2 * kTsMaxX + kTsMaxR + s); };
   auto afull = [&](int s) { return bars + 8u * (2 * kTsMaxX + 2 * kTsMaxR + s); };
   auto aempty = [&](int s) { return bars + 8u * (2 * kTsMaxX + 2 * kTsMaxR + kTsMaxA + s); };
-  auto dfull = [&](int a) { return bars + 8u * (2 * kTsMaxX + 2 * kTsMaxR + 2 * kTsMaxA + a); };
-  auto dempty = [&](int a) { return bars + 8u * (2 * kTsMaxX + 2 * kTsMaxR + 2 * kTsMaxA + 2 + a); };
-  const uint32_t tmem_slot = bars + 8u * (2 * kTsMaxX + 2 * kTsMaxR + 2 * kTsMaxA + 4), gave_up = tmem_slot + 4;
+  const uint32_t dfull = bars + 8u * (2 * kTsMaxX + 2 * kTsMaxR + 2 * kTsMaxA);   // the accumulator is complete
+  const uint32_t tmem_slot = dfull + 8, gave_up = tmem_slot + 4;
 
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
   const int S = CTAS > 1 ? static_cast<int>(cluster_nctarank()) : 1;
   const int crank = S > 1 ? static_cast<int>(cluster_ctarank()) : 0;
   const int tok_blocks = ceil_div(p.M, p.bn);
-  const int num_tiles = tok_blocks * ceil_div(p.N, 128);
   const int KB = p.K >> 6;
   const int kb0 = S > 1 ? min(KB, crank * p.kb_per_split) : 0;
   const int kb1 = S > 1 ? min(KB, kb0 + p.kb_per_split) : KB;
-  const int tile0 = static_cast<int>(blockIdx.x) / S, tile_step = static_cast<int>(gridDim.x) / S;
+  const int tile = static_cast<int>(blockIdx.x) / S;
+  const int tok0 = (tile % tok_blocks) * p.bn, n0 = (tile / tok_blocks) * 128;
   bool dead = false;
 
   if (warp == 0 && lane == 0) {
@@ -160,10 +163,7 @@ w4a16_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsParams p) {
       tc::mbar_init(afull(s), 4);
       tc::mbar_init(aempty(s), 1);
     }
-    for (int a = 0; a < 2; ++a) {
-      tc::mbar_init(dfull(a), 1);
-      tc::mbar_init(dempty(a), 4);
-    }
+    tc::mbar_init(dfull, 1);
     asm volatile("st.shared.u32 [%0], 0;\n" ::"r"(gave_up) : "memory");
     tc::fence_barrier_init();
   }
@@ -186,71 +186,60 @@ w4a16_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsParams p) {
 
   if (warp == 0) {
     griddep_wait();                                // the activations are the previous kernel's
-    int s = 0;
     uint32_t phase = 0;
-    for (int tile = tile0; tile < num_tiles; tile += tile_step) {
-      const int tok0 = (tile % tok_blocks) * p.bn;
-      for (int kb = kb0; kb < kb1; ++kb) {
+    for (int kb = kb0; kb < kb1; phase ^= 1u) {    // a lap of the ring
+      const int lap_end = min(kb1, kb + p.nx);
+      for (int s = 0; kb < lap_end; ++kb, ++s) {
         tc::mbar_wait_bounded(xempty(s), phase ^ 1u, dead, gave_up);
         if (tc::elect_one()) {
           tc::mbar_arrive_expect_tx(xfull(s), x_bytes);
           tc::tma_load_2d(base + s * x_bytes, &tmap_x, xfull(s), kb * 64, tok0);
         }
         __syncwarp();
-        if (++s == p.nx) {
-          s = 0;
-          phase ^= 1u;
-        }
       }
     }
   } else if (warp == 1) {
     constexpr uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
     const uint32_t idesc = tc::make_idesc(fmt, fmt, 128, p.bn, 0, 0);
-    int s = 0, a = 0, local = 0;
+    const uint32_t tmem_d = tmem_base + C::D_COL;
+    int s = 0, a = 0;
     uint32_t phase = 0, aphase = 0;
-    for (int tile = tile0; tile < num_tiles; tile += tile_step, ++local) {
-      const int d = local % C::ND;
-      tc::mbar_wait_bounded(dempty(d), ((local / C::ND) & 1u) ^ 1u, dead, gave_up);
+    for (int kb = kb0; kb < kb1; ++kb) {
+      tc::mbar_wait_bounded(xfull(s), phase, dead, gave_up);
+      tc::mbar_wait_bounded(afull(a), aphase, dead, gave_up);
       tc::tc_fence_after();
-      const uint32_t tmem_d = tmem_base + C::D_COL + d * C::MAX_BN;
-      for (int kb = kb0; kb < kb1; ++kb) {
-        tc::mbar_wait_bounded(xfull(s), phase, dead, gave_up);
-        tc::mbar_wait_bounded(afull(a), aphase, dead, gave_up);
-        tc::tc_fence_after();
-        const uint64_t bdesc = tc::make_smem_desc_sw128(base + s * x_bytes, 1024, 16);
-        if (tc::elect_one()) {
+      const uint64_t bdesc = tc::make_smem_desc_sw128(base + s * x_bytes, 1024, 16);
+      if (tc::elect_one()) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k)              // 32 bytes of K further on: 2 in the address field
-            tc::mma_f16_ts(tmem_d, tmem_base + a * 32 + k * 8, bdesc + 2 * k, idesc, kb != kb0 || k != 0 ? 1u : 0u);
-          tc::mma_commit(xempty(s));
-          tc::mma_commit(aempty(a));
-        }
-        __syncwarp();
-        if (++s == p.nx) {
-          s = 0;
-          phase ^= 1u;
-        }
-        if (++a == C::NA) {
-          a = 0;
-          aphase ^= 1u;
-        }
+        for (int k = 0; k < 4; ++k)                // 32 bytes of K further on: 2 in the address field
+          tc::mma_f16_ts(tmem_d, tmem_base + a * 32 + k * 8, bdesc + 2 * k, idesc, kb != kb0 || k != 0 ? 1u : 0u);
+        tc::mma_commit(xempty(s));
+        tc::mma_commit(aempty(a));
       }
-      if (tc::elect_one()) tc::mma_commit(dfull(d));
       __syncwarp();
+      if (++s == p.nx) {
+        s = 0;
+        phase ^= 1u;
+      }
+      if (++a == C::NA) {
+        a = 0;
+        aphase ^= 1u;
+      }
     }
+    if (tc::elect_one()) tc::mma_commit(dfull);
+    __syncwarp();
   } else if (warp < 4) {
     // packed words: piece i of a stage = strip i / 32, piece i % 32 = 4 g + t of that tile -> strip * 512 + t * 128 + g * 16
     const int l = static_cast<int>(threadIdx.x) - 64;          // 0 .. 63
     const uint32_t dst0 = raw + (l >> 5) * 512 + (lane & 3) * 128 + (lane >> 2) * 16;
     const T* zeros = static_cast<const T*>(p.zeros);
     const T* scales = static_cast<const T*>(p.scales);
-    int s = 0;
+    const int strip0 = n0 / 16 + (l >> 5), col = n0 + (lane & 15) * 8;
+    const uint4* src = p.qw + static_cast<int64_t>(strip0) * KB * 32 + lane;
     uint32_t phase = 0;
-    for (int tile = tile0; tile < num_tiles; tile += tile_step) {
-      const int strip0 = (tile / tok_blocks) * 8 + (l >> 5);
-      const uint4* src = p.qw + static_cast<int64_t>(strip0) * KB * 32 + lane;
-      const int col = (tile / tok_blocks) * 128 + (lane & 15) * 8;
-      for (int kb = kb0; kb < kb1; ++kb) {
+    for (int kb = kb0; kb < kb1; phase ^= 1u) {    // a lap of the ring
+      const int lap_end = min(kb1, kb + p.nr);
+      for (int s = 0; kb < lap_end; ++kb, ++s) {
         tc::mbar_wait_bounded(rempty(s), phase ^ 1u, dead, gave_up);
 #pragma unroll
         for (int j = 0; j < 4; ++j)                // strips past N hold channels that are never stored
@@ -261,149 +250,114 @@ w4a16_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsParams p) {
         if (col < p.N && (l < 32 || p.group < 64))
           cp_async16(raw + s * p.raw_bytes + kTsWordBytes + (l >> 5) * (2 * kTsRowBytes) + lane * 16, (lane < 16 ? zeros : scales) + row);
         asm volatile("cp.async.mbarrier.arrive.noinc.shared.b64 [%0];\n" ::"r"(rfull(s)) : "memory");
-        if (++s == p.nr) {
-          s = 0;
-          phase ^= 1u;
-        }
       }
     }
     cp_async_commit();
     cp_async_wait<0>();
     griddep_launch_dependents();
-  } else if (warp < 12) {
+  } else {
     const int grp = (warp - 4) >> 2;
     const int r = (warp & 3) * 32 + lane;          // channel of the tile = lane of tensor memory
     const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const bool hi = (lane & 8) != 0;               // columns 8 .. 15 of a 16-channel tile
     const uint32_t src0 = raw + (r >> 4) * 512 + (lane & 7) * 16;
     const uint32_t sz0 = raw + kTsWordBytes + r * 2, sz1 = p.group < 64 ? sz0 + 2 * kTsRowBytes : sz0;
-    // this group's stages are every second one of the CTA's, which run on across tiles
-    int rs = grp, a = grp, skip = grp;
+    // this group's stages are every second one of the CTA's
+    int rs = grp, a = grp;
     uint32_t rphase = 0, aphase = 0;
-    for (int tile = tile0; tile < num_tiles; tile += tile_step) {
-      int kb = kb0 + skip;
-      for (; kb < kb1; kb += 2) {
-        tc::mbar_wait_bounded(rfull(rs), rphase, dead, gave_up);
-        const uint32_t at = rs * p.raw_bytes;
-        uint32_t w[8];
+    for (int kb = kb0 + grp; kb < kb1; kb += 2) {
+      tc::mbar_wait_bounded(rfull(rs), rphase, dead, gave_up);
+      const uint32_t at = rs * p.raw_bytes;
+      uint32_t w[8];
 #pragma unroll
-        for (int t = 0; t < 4; ++t) {
-          const uint4 v = lds128(src0 + at + t * 128);
-          w[t] = hi ? v.y : v.x;
-          w[4 + t] = hi ? v.w : v.z;
-        }
-        const uint32_t z2[2] = {ts_ld_pair(sz0 + at), ts_ld_pair(sz1 + at)};
-        const uint32_t s2[2] = {ts_ld_pair(sz0 + at + kTsRowBytes), ts_ld_pair(sz1 + at + kTsRowBytes)};
-        const uint32_t zh[2] = {ts_high_zero(z2[0]), ts_high_zero(z2[1])};
-        __syncwarp();
-        if (lane == 0) tc::mbar_arrive(rempty(rs));
-        uint32_t o[32];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) ts_dequant8<T>(w[i], z2[i >> 2], zh[i >> 2], s2[i >> 2], o + 4 * i);
-        tc::mbar_wait_bounded(aempty(a), aphase ^ 1u, dead, gave_up);
-        tc::tc_fence_after();
-        __syncwarp();
-        tc::tmem_st32(tmem_base + lane_addr + a * 32, o);
-        tc::tmem_st_wait();
-        tc::tc_fence_before();
-        __syncwarp();
-        if (lane == 0) tc::mbar_arrive(afull(a));
-        rs += 2;
-        if (rs >= p.nr) {
-          rs -= p.nr;
-          rphase ^= 1u;
-        }
-        if (C::NA == 4) a ^= 2;
-        if (a < 2) aphase ^= 1u;
+      for (int t = 0; t < 4; ++t) {
+        const uint4 v = lds128(src0 + at + t * 128);
+        w[t] = hi ? v.y : v.x;
+        w[4 + t] = hi ? v.w : v.z;
       }
-      skip = kb - kb1;
-    }
-    if (CTAS > 1) {
-      // the one tile's epilogue
-      griddep_wait();
-      const int tok0 = (tile0 % tok_blocks) * p.bn;
-      const int n = (tile0 / tok_blocks) * 128 + r;
-      const int toks = min(p.bn, p.M - tok0);
-      const float bias = p.bias && n < p.N ? to_float<T>(static_cast<const T*>(p.bias)[n]) : 0.f;
-      const uint32_t tmem_d = tmem_base + lane_addr + C::D_COL;
-      if (kb1 > kb0) tc::mbar_wait_bounded(dfull(0), 0, dead, gave_up);
+      const uint32_t z2[2] = {ts_ld_pair(sz0 + at), ts_ld_pair(sz1 + at)};
+      const uint32_t s2[2] = {ts_ld_pair(sz0 + at + kTsRowBytes), ts_ld_pair(sz1 + at + kTsRowBytes)};
+      const uint32_t zh[2] = {ts_high_zero(z2[0]), ts_high_zero(z2[1])};
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(rempty(rs));
+      uint32_t o[32];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) ts_dequant8<T>(w[i], z2[i >> 2], zh[i >> 2], s2[i >> 2], o + 4 * i);
+      tc::mbar_wait_bounded(aempty(a), aphase ^ 1u, dead, gave_up);
       tc::tc_fence_after();
       __syncwarp();
-      if (S == 1) {
-        for (int c = grp * 16; c < toks; c += 32) {
-          uint32_t v[16];
-          tc::tmem_ld16(tmem_d + c, v);
-          tc::tmem_ld_wait();
-          store16(reinterpret_cast<const float*>(v), tok0 + c, n, bias);
-        }
-      } else {
-        // fixed-order cluster reduction: token m of the partial goes to rank m % S, slot [rank][m / S][channel] of its
-        // idle rings; then each rank adds the slots of its own tokens in rank order
-        const int tpr = ceil_div(toks, S);
-        const uint32_t push = base + (crank * tpr * 128 + r) * 4;
-        cluster_sync_all();                        // every peer's rings are idle
-        for (int c = grp * 16; c < toks; c += 32) {
-          uint32_t v[16];
-          if (kb1 > kb0) {
-            tc::tmem_ld16(tmem_d + c, v);
-            tc::tmem_ld_wait();
-          } else {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = 0u;
-          }
-          int q = c % S, slot = c / S;
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            if (c + j < toks)
-              asm volatile("st.shared::cluster.u32 [%0], %1;\n" ::"r"(map_to_rank(push + slot * 512, q)), "r"(v[j]) : "memory");
-            if (++q == S) {
-              q = 0;
-              ++slot;
-            }
-          }
-        }
-        __syncwarp();
-        cluster_sync_all();                        // all partials have arrived
-        for (int j = grp; j < tpr; j += 2) {
-          const int m = j * S + crank;
-          if (m >= toks) break;
-          float sum = 0.f;
-          for (int q = 0; q < S; ++q) {
-            float x;
-            asm volatile("ld.shared.f32 %0, [%1];\n" : "=f"(x) : "r"(base + ((q * tpr + j) * 128 + r) * 4) : "memory");
-            sum += x;
-          }
-          if (n < p.N) out[static_cast<int64_t>(tok0 + m) * p.ldc + n] = from_float<T>(sum + bias);
-        }
+      tc::tmem_st32(tmem_base + lane_addr + a * 32, o);
+      tc::tmem_st_wait();
+      tc::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(afull(a));
+      rs += 2;
+      if (rs >= p.nr) {
+        rs -= p.nr;
+        rphase ^= 1u;
       }
+      if (C::NA == 4) a ^= 2;
+      if (a < 2) aphase ^= 1u;
     }
-  } else {
+    // ---- epilogue
     griddep_wait();
-    const int r = (warp & 3) * 32 + lane;
-    const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    int local = 0;
-    for (int tile = tile0; tile < num_tiles; tile += tile_step, ++local) {
-      const int d = local % C::ND;
-      const int tok0 = (tile % tok_blocks) * p.bn, n = (tile / tok_blocks) * 128 + r;
-      const int toks = min(p.bn, p.M - tok0);
-      const float bias = p.bias && n < p.N ? to_float<T>(static_cast<const T*>(p.bias)[n]) : 0.f;
-      tc::mbar_wait_bounded(dfull(d), (local / C::ND) & 1u, dead, gave_up);
-      tc::tc_fence_after();
-      __syncwarp();
-      const uint32_t tmem_d = tmem_base + lane_addr + C::D_COL + d * C::MAX_BN;
-      for (int c = 0; c < toks; c += 16) {
+    const int n = n0 + r;
+    const int toks = min(p.bn, p.M - tok0);
+    const float bias = p.bias && n < p.N ? to_float<T>(static_cast<const T*>(p.bias)[n]) : 0.f;
+    const uint32_t tmem_d = tmem_base + lane_addr + C::D_COL;
+    if (kb1 > kb0) tc::mbar_wait_bounded(dfull, 0, dead, gave_up);
+    tc::tc_fence_after();
+    __syncwarp();
+    if (S == 1) {
+      for (int c = grp * 16; c < toks; c += 32) {
         uint32_t v[16];
         tc::tmem_ld16(tmem_d + c, v);
         tc::tmem_ld_wait();
         store16(reinterpret_cast<const float*>(v), tok0 + c, n, bias);
       }
-      tc::tc_fence_before();
+    } else {
+      // fixed-order cluster reduction: token m of the partial goes to rank m % S, slot [rank][m / S][channel] of its
+      // idle rings; then each rank adds the slots of its own tokens in rank order
+      const int tpr = ceil_div(toks, S);
+      const uint32_t push = base + (crank * tpr * 128 + r) * 4;
+      cluster_sync_all();                          // every peer's rings are idle
+      for (int c = grp * 16; c < toks; c += 32) {
+        uint32_t v[16];
+        if (kb1 > kb0) {
+          tc::tmem_ld16(tmem_d + c, v);
+          tc::tmem_ld_wait();
+        } else {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) v[j] = 0u;
+        }
+        int q = c % S, slot = c / S;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          if (c + j < toks)
+            asm volatile("st.shared::cluster.u32 [%0], %1;\n" ::"r"(map_to_rank(push + slot * 512, q)), "r"(v[j]) : "memory");
+          if (++q == S) {
+            q = 0;
+            ++slot;
+          }
+        }
+      }
       __syncwarp();
-      if (lane == 0) tc::mbar_arrive(dempty(d));
+      cluster_sync_all();                          // all partials have arrived
+      for (int j = grp; j < tpr; j += 2) {
+        const int m = j * S + crank;
+        if (m >= toks) break;
+        float sum = 0.f;
+        for (int q = 0; q < S; ++q) {
+          float x;
+          asm volatile("ld.shared.f32 %0, [%1];\n" : "=f"(x) : "r"(base + ((q * tpr + j) * 128 + r) * 4) : "memory");
+          sum += x;
+        }
+        if (n < p.N) out[static_cast<int64_t>(tok0 + m) * p.ldc + n] = from_float<T>(sum + bias);
+      }
     }
   }
 
-  if (CTAS > 1 && S > 1 && warp < 4) {             // the two barriers of the reduction
+  if (S > 1 && warp < 4) {                         // the two barriers of the reduction
     __syncwarp();
     cluster_sync_all();
     cluster_sync_all();
@@ -424,7 +378,7 @@ template <int CTAS>
 static void ts_rings(TsPlan* pl, int raw) {
   using C = TsCfg<CTAS>;
   const int x = pl->bn * 128, room = C::BUDGET - kTsBarBytes - 1024;
-  const int nx = (room - 6 * raw) / x;
+  const int nx = (room - kTsMinR * raw) / x;
   pl->nx = nx > kTsMaxX ? kTsMaxX : nx;
   const int nr = (room - pl->nx * x) / raw;
   pl->nr = nr > kTsMaxR ? kTsMaxR : nr;
@@ -485,12 +439,11 @@ template <typename T, int CTAS>
 static int launch_ts(const TsPlan& pl, const CUtensorMap& tx, const TsParams& p, cudaStream_t st) {
   auto kern = w4a16_ts_kernel<T, CTAS>;
   B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, TsCfg<CTAS>::BUDGET));
-  const int tiles = ceil_div(p.M, p.bn) * ceil_div(p.N, 128), sms = device_sm_count();
-  const int grid = CTAS > 1 ? tiles * pl.S : (tiles < sms ? tiles : sms);
+  const int tiles = ceil_div(p.M, p.bn) * ceil_div(p.N, 128);
   note_variant("w4a16_ts ctas=%d bn=%d splits=%d nx=%d nr=%d tiles=%d", CTAS, p.bn, pl.S, p.nx, p.nr, tiles);
   {
     ScopedKernelTimer timer("w4a16_gemm", st);
-    B200_CUDA_OK(launch_kernel(kern, dim3(grid), dim3(TsCfg<CTAS>::WARPS * 32), pl.smem, st, pl.S,
+    B200_CUDA_OK(launch_kernel(kern, dim3(tiles * pl.S), dim3(kTsThreads), pl.smem, st, pl.S,
                                pdl_family(p.M, kPdlGemmSmall), tx, p));
   }
   B200_CHECK_LAUNCH("w4a16_ts_kernel");

@@ -1,4 +1,6 @@
 """Int4 linear with the dequantised weight in tensor memory (csrc/w4a16_ts.cu) at the edges of its tiles, splits and rings."""
+import re
+
 import pytest
 import torch
 
@@ -25,19 +27,29 @@ def _weight(n, k, group, dtype, g):
     return q, (z + magic).to(dtype), s, W.gemv_stream_repack(q), w16
 
 
-# N, K, group: a part-filled channel tile, one K block, groups of 32, a group over all of K, K splits of 2 .. 8 and ragged
-# ones, more tiles than SMs (three CTAs an SM up to 64 tokens), tiles of 192 tokens (one CTA an SM, several tiles each)
+# N, K, group -> (CTAs an SM, K splits) of the token counts below: a part-filled channel tile, one K block, groups of 32, a
+# group over all of K, K splits of 2 .. 8 and ragged ones, more tiles than SMs (three CTAs an SM up to 64 tokens), tiles of
+# up to 192 tokens (one CTA an SM)
 @pytest.mark.gpu
-@pytest.mark.parametrize("n,k,group", [(16, 64, 64), (144, 192, 64), (272, 2048, 32), (512, 1024, 1024), (1536, 4096, 128),
-                                       (3584, 5120, 128), (5120, 13824, 128), (24576, 512, 128), (19200, 576, 64)])
+@pytest.mark.parametrize("n,k,group,forms", [
+    (16, 64, 64, {(2, 1)}),
+    (144, 192, 64, {(2, 1)}),
+    (272, 2048, 32, {(2, 8)}),
+    (512, 1024, 1024, {(2, 4), (2, 1)}),
+    (1536, 4096, 128, {(2, 8), (2, 6), (2, 4), (2, 3)}),
+    (3584, 5120, 128, {(2, 5), (2, 4), (2, 2), (2, 1)}),
+    (5120, 13824, 128, {(2, 6), (2, 3), (2, 1), (1, 1)}),
+    (24576, 512, 128, {(3, 2), (2, 1)}),
+    (19200, 576, 64, {(3, 2), (2, 1)}),
+])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
-def test_matches_a_dense_product(n, k, group, dtype):
+def test_matches_a_dense_product(n, k, group, forms, dtype):
     g = torch.Generator(device="cuda").manual_seed(n + k)
     q, z, s, stream, w16 = _weight(n, k, group, dtype, g)
     # rounding of the result to 16 bits, 2-norm: 2^-11 / sqrt(3) (f16), 2^-8 / sqrt(3) (bf16); sums of at most 13824
     # products in 32 bits add 1e-5 at most
     limit = 1.2 * (2 ** -11 if dtype == torch.float16 else 2 ** -8) / 3 ** 0.5 + 1e-5
-    taken = 0
+    taken, seen = 0, set()
     for m in (17, 31, 32, 33, 64, 65, 112, 128, 129, 192, 256, 300, 385, 512):
         if not W.ts_takes(m, n, k, group):
             continue
@@ -48,11 +60,12 @@ def test_matches_a_dense_product(n, k, group, dtype):
         out = W.w4a16_gemm_ts(x, stream, z, s, group, bias)
         again = W.w4a16_gemm_ts(x, stream, z, s, group, bias)
         assert _lib.last_variant().startswith("w4a16_ts"), _lib.last_variant()
+        seen.add(tuple(int(re.search(rf"{name}=(\d+)", _lib.last_variant())[1]) for name in ("ctas", "splits")))
         ref = x.double() @ w16.double() + (0 if bias is None else bias.double())
         err = ((out.double() - ref).norm() / ref.norm()).item()
         assert err <= limit, (m, err, limit, _lib.last_variant())
         assert torch.equal(out, again)                      # sums of split K in rank order
-    assert taken >= 6
+    assert taken >= 6 and seen == forms
     _lib.check_waits()
 
 
