@@ -389,8 +389,8 @@ static void ts_rings(TsPlan* pl, int raw) {
 // Measured (f16, us): a 64-k stage takes 0.22 + 0.0004 bn of a CTA alone on its SM, 0.19 + 0.0007 bn times their number where
 // several share one; a split 2 + 0.02 bn for the exchange of the partials.
 // At most 1.63 CTAs an SM (241 of 148).  Every split of 19 to 74 tiles timed (K 2560, 5120 and 13824; 24, 64 and 128 tokens):
-// up to 1.75 an SM the clusters run in one wave, beyond that those of six to eight CTAs take two (5120 deep, 64 tokens: 264
-// CTAs in sixes 13.1 us, 276 20.2).  Between 1.63 and 1.75 the picks would be 4 % faster on average (13824 deep, 42 tiles, 64
+// up to 1.75 an SM all clusters run in one wave, then soon in two (5120 deep, 64 tokens: 264 CTAs in sixes 13.1 us, 276 20.2;
+// 256 in eights 10.9, 272 16.1).  Between 1.63 and 1.75 the picks would be 4 % faster on average (13824 deep, 42 tiles, 64
 // tokens: three parts 25.1 / six 22.4), but up to 11 % slower where K is short and the exchange counts (2560 deep, 32 tiles, 24
 // tokens: four parts 6.6 / eight 7.3).  Three CTAs an SM, each half of K, only where that fills them and two would leave every second SM
 // half idle (27648 x 5120, 16 / 64 tokens: 34.6 / 38.6 with two, 29.9 / 34.9 with three).

@@ -4,6 +4,7 @@ import pytest
 import torch
 
 from sglang_security_b200 import _lib
+from sglang_security_b200.layers.radix_attention import AttentionType
 from test_extend_layer_gpu import _batch
 
 pytestmark = pytest.mark.gpu
@@ -67,3 +68,42 @@ def test_without_workspace_and_with_many_requests():
     assert "flat" not in _lib.last_variant()
     ref = _exact(fb, q, k, v, 8, 2, 64, torch.bfloat16)
     assert (o.double() - ref).norm() <= 6e-3 * ref.norm()
+
+
+# what the batches above leave out: several tiles of heads a kv head (groups of 5, 7, 3, 6), f16, e5m2, pools with scales (they
+# ride on the scores and on both stores of the output), no causal mask
+@pytest.mark.parametrize("hq,hkv,d", [(20, 4, 128), (14, 2, 64), (12, 4, 128), (12, 2, 64)])
+@pytest.mark.parametrize("act,pool_dtype,scales", [
+    (torch.bfloat16, torch.bfloat16, None), (torch.float16, torch.float16, None),
+    (torch.float16, torch.float8_e4m3fn, (0.5, 1.25)), (torch.bfloat16, torch.float8_e5m2, (0.75, 0.5)),
+])
+@pytest.mark.parametrize("causal", [True, False])
+def test_head_tiles_types_scales_and_masks(hq, hkv, d, act, pool_dtype, scales, causal, monkeypatch):
+    monkeypatch.setenv("B200_EXTEND_FLAT", "1")
+    prefix, new = [1500, 5, 0, 2000], [400, 257, 1, 900]
+    backend, layer, fb, (q, k, v) = _batch(4, prefix, new, hq, hkv, d, pool_dtype, act, hq)
+    if scales:
+        layer.k_scale_float, layer.v_scale_float = scales
+    if not causal:
+        layer.attn_type = AttentionType.ENCODER_ONLY
+    backend.init_forward_metadata(fb)
+    o = layer(q, k, v, fb)
+    assert "flat" in _lib.last_variant(), _lib.last_variant()
+    assert torch.equal(layer(q, k, v, fb), o)
+    _lib.check_waits()
+    pool, rtt = fb.token_to_kv_pool, fb.req_to_token_pool.req_to_token
+    ks, vs = scales or (1.0, 1.0)
+    kc, vc = (b[0].view(pool_dtype) for b in (pool.k_buffer, pool.v_buffer))
+    at = 0
+    for b, (p, n) in enumerate(zip(prefix, new)):
+        idx = rtt[b, :p + n].long()
+        kb, vb = (c[idx].double().transpose(0, 1).repeat_interleave(hq // hkv, 0) for c in (kc, vc))
+        s = q[at:at + n].double().view(n, hq, d).transpose(0, 1) @ kb.transpose(1, 2) * (d ** -0.5 * ks)
+        if causal:
+            s.masked_fill_(torch.arange(p + n, device="cuda")[None] > torch.arange(p, p + n, device="cuda")[:, None], float("-inf"))
+        ref = (s.softmax(-1) @ vb * vs).transpose(0, 1).reshape(n, hq * d)
+        # weights and result rounded to 16 bits: 2^-9 (bf16) or 2^-12 (f16) relative each, 2-norm 1.6e-3 and 2e-4; about four
+        # times that, as above
+        limit = 6e-3 if act == torch.bfloat16 else 7.5e-4
+        assert (o[at:at + n].double() - ref).norm() <= limit * ref.norm(), b
+        at += n
