@@ -49,10 +49,6 @@ __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity) {
 // caller run to its end; once `dead`, a thread's later waits only poll, so a lost signal costs one limit and not one
 // per wait.
 static __device__ unsigned g_wait_timeouts;
-__device__ __forceinline__ void mark_gave_up(uint32_t gave_up) {
-  atomicAdd(&g_wait_timeouts, 1u);
-  asm volatile("st.shared.u32 [%0], 1;\n" ::"r"(gave_up) : "memory");
-}
 __device__ __forceinline__ void mbar_wait_bounded(uint32_t bar, uint32_t parity, bool& dead, uint32_t gave_up,
                                                   long long limit = 1ll << 32) {
   if (mbar_try_wait(bar, parity)) return;
@@ -61,7 +57,8 @@ __device__ __forceinline__ void mbar_wait_bounded(uint32_t bar, uint32_t parity,
     if (mbar_try_wait(bar, parity)) return;
     if (clock64() - t0 > limit) {
       dead = true;
-      mark_gave_up(gave_up);
+      atomicAdd(&g_wait_timeouts, 1u);
+      asm volatile("st.shared.u32 [%0], 1;\n" ::"r"(gave_up) : "memory");
     }
   }
 }
@@ -72,6 +69,10 @@ __device__ __forceinline__ void mbar_wait_bounded(uint32_t bar, uint32_t parity,
 constexpr uint32_t kWaitPolls = 1u << 22;
 __device__ __forceinline__ void mbar_wait_counted(uint32_t bar, uint32_t parity, uint32_t& polls) {
   while (!mbar_try_wait(bar, parity) && polls != 0) --polls;
+}
+__device__ __forceinline__ void mark_gave_up(uint32_t gave_up) {
+  atomicAdd(&g_wait_timeouts, 1u);
+  asm volatile("st.shared.u32 [%0], 1;\n" ::"r"(gave_up) : "memory");
 }
 // The end of a block with bounded waits, by one thread after the block has met: where a wait ran out, a millisecond
 // for the copies and MMAs that may still be in flight, and the host's error word (wait_error_word()) is marked, which
