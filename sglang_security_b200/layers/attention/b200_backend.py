@@ -9,8 +9,8 @@ and calls the sm_100a kernels through the C-ABI (include/b200_hotpath.h):
   forward_decode : b200_kv_write -> b200_attn_decode_fused (split-KV gather kernel whose last CTA per
                    request merges the splits and, on request, quantises the row for o_proj);
                    B200_ATTN_FUSED_TAIL=0 restores split kernel + merge kernel
-  forward_extend : b200_extend_layer: pool write, 16-bit copy of an FP8 pool's rows, attention (tcgen05 prefix
-                   rectangle + causal triangle) in one native call.  Short extends are bound by the host: 64 fresh
+  forward_extend : b200_extend_layer_planned: pool write, 16-bit copy of an FP8 pool's rows, attention (tcgen05
+                   prefix rectangle + causal triangle) in one native call.  Short extends are bound by the host: 64 fresh
                    tokens took 62 us a call in three native calls with torch's Stream objects, 37 in one; behind an
                    FP8 pool, whose prefix sum and row table were torch operations, 146, now 46.
 
@@ -383,7 +383,6 @@ class B200AttnBackend(AttentionBackend):
                 raise _lib.B200Error("forward_extend: k_scale and v_scale must be given together")
             total_kv, max_kv = md.kv_extent(forward_batch, seq_lens)
             scratch_bytes = self.lib.b200_extend_layer_dense_bytes(total_kv, bs, max_kv, hkv, d)
-        lens = md.host_lens.buffer_info()[0] if md.host_lens is not None and len(md.host_lens) == 2 * bs else 0
         flat = 0
         if max_kv >= 1024:
             # whether the persistent kernel takes it, and its workspace: once per forward, not in every layer
@@ -391,6 +390,7 @@ class B200AttnBackend(AttentionBackend):
             form = (bs, max_kv, hq, hkv, d, causal, scale, float(layer.logit_cap or 0.0), os.environ.get("B200_EXTEND_FLAT"))
             flat = md.flat_bytes.get(form)
             if flat is None:
+                lens = md.host_lens.buffer_info()[0] if md.host_lens is not None and len(md.host_lens) == 2 * bs else 0
                 flat = md.flat_bytes[form] = self.lib.b200_extend_layer_flat_bytes(
                     bs, md.max_extend_len, max_kv, hq, hkv, d, 1 if causal else 0, *form[6:8], lens)
         if flat:
@@ -409,7 +409,7 @@ class B200AttnBackend(AttentionBackend):
             q.data_ptr(), q.stride(0), k_cache.data_ptr(), v_cache.data_ptr(), k_cache.stride(0), o.data_ptr(), o.stride(0),
             req_to_token.data_ptr(), req_to_token.stride(0), req_pool_indices.data_ptr(), seq_lens.data_ptr(),
             prefix_lens.data_ptr(), extend_lens.data_ptr(), md.qo_indptr.data_ptr(), kp, vp, kst, vst, locp, n_new,
-            0 if scratch is None else scratch.data_ptr(), scratch_bytes, total_kv, lens, bs,
+            0 if scratch is None else scratch.data_ptr(), scratch_bytes, total_kv, 0, bs,
             md.max_extend_len, max_kv, hq, hkv, d, dv,
             1 if causal else 0, _lib.dtype_code(q.dtype),
             0 if not fp8 else 2 if k_cache.dtype == torch.float8_e5m2 else 1, float(layer.scaling),
