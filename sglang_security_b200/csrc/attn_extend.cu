@@ -651,8 +651,9 @@ struct ExtendHost {
   const int32_t* lens = nullptr;    // new tokens and prefix of every request, or null
   int flat = -1;                    // the persistent kernel: chosen before the call (1), not (0), to be chosen in the call (-1)
 };
-// When the two-tile kernel's last CTA ends: its CTAs in the order of the grid, each to the SM that is free first.  From 68
-// calls timed (within 6 %, head size 64 2 %; without the requests' lengths, and so the order, 20 %).
+// When the two-tile kernel's last CTA ends: its CTAs in the order of the grid, each to the SM that is free first.  Fitted to 68
+// calls timed one by one (within 6 %; without the requests' lengths, and so the order, 20 %); calls timed in rows of 8
+// (profiles/extend_flat_calls.json) take 6 % longer at the median, one in twenty 21 %.
 constexpr int kFlatMaxSms = 256;
 static double wide_last_us(int D, const ExtendParams& p, int bs, int max_extend_len, const int32_t* lens) {
   const int sms = device_sm_count(), tok_cta = 256 / p.pack, heads = p.Hkv * p.head_tiles, blocks = ceil_div(max_extend_len, tok_cta);
@@ -674,10 +675,12 @@ static double wide_last_us(int D, const ExtendParams& p, int bs, int max_extend_
 // sizes 64 and 128, 1 to 30 equal and ragged requests of 64 to 8192 new tokens behind 0 to 8000).  Its time is a fixed part
 // (the plan, the first loads, the last store, the merge) and every SM's equal share of items and key tiles (within 6 %); it
 // has to be a twentieth less than the others'.  Not above four waves of the two-tile kernel's CTAs, whose last one is a
-// small part there (2 x 8192 fresh tokens 944 us there, 1052 here), which also bounds the work of this estimate (~8 us:
+// small part there (2 x 8192 fresh tokens 972 us there, 1155 here), which also bounds the work of this estimate (~8 us:
 // callers with many layers of one batch ask b200_extend_layer_flat_bytes once).
-// 48 of the calls come here, 12 % faster on average, 4 % slower at worst (us, there / here: groups of 4, 8 x 512 behind 1536
-// 115 / 109, behind 4000 211 / 189, 3 x 100 behind 7000 146 / 61; head size 64, 2 x 1000 behind 7000 113 / 76).
+// Of 120 other calls, timed in rows of 8 (profiles/extend_flat_calls.json), 26 come here, 12 % faster on average (us, there /
+// here: groups of 4, 8 x up to 512 behind 1536 121 / 114; groups of 5, 4 x 512 behind 8000 290 / 202; head size 64, 2 x 1000
+// behind 7000 140 / 126); the one that loses most beyond 60 us, below which the host is the limit, is 8 x 512 behind 4000,
+// 298 / 311.
 static bool flat_pays(int D, const ExtendParams& p, int bs, int max_extend_len, int64_t ctas, int splits, double wide, double narrow,
                       const int32_t* lens) {
   const int sms = device_sm_count(), tok_cta = 256 / p.pack;

@@ -14,9 +14,11 @@
 // (deterministic); who begins an item writes how many go on with it.
 //
 // Bound by the softmax chain of a key tile as that kernel is (2.0 us a pair of tiles), by ~8 us an item that the next item's
-// loads hide in part, and ~28 us once (plan, first loads, partial results through L2, merge).  us, two-tile kernel / this (head
-// size 128, groups of 4, ragged): 8 x 512 behind 1536 115 / 109, behind 4000 211 / 189; 3 x 100 behind 7000 146 / 61; fresh
-// 2 x 8192 944 / 1052: flat_pays in attn_extend.cu chooses.
+// loads hide in part, and ~28 us once (plan, first loads, partial results through L2, merge).  us, other kernels / this (in rows
+// of 8 calls, profiles/extend_flat_calls.json): groups of 4, 8 x up to 512 behind 1536 121 / 114, 2 x up to 390 behind 4192 84 /
+// 70; groups of 5, 4 x 512 behind 8000 290 / 202; head size 64, 4 x up to 1000 behind 6000 205 / 150; but fresh 2 x 8192 972 /
+// 1155: flat_pays in attn_extend.cu chooses.  Counters (the first of these): tensor pipe 40 %, exponential unit 41 % of the
+// active clocks, 0.34 instructions a clock; the merge 12 us of 111, bound by reading its 39 MB.
 //
 // Warps, shared and tensor memory as in attn_extend_wide.cuh; three barriers more: Q is free, O of a tile is free.
 #pragma once

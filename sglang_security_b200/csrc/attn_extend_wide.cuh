@@ -19,8 +19,9 @@
 // Shared memory per 128 keys: Q and K of two QK (128 KiB), V of two PV (64), the gather (64) = 2048 clocks at
 // 128 B/clk, as long as the tensor work and the 32768 exponentials take: the three bound it together (D 128: 3450
 // clocks measured, 2980 without the exponentials).  64-key tiles with two score buffers, which take the softmax
-// off the chain, read Q twice as often and were slower: 2 x 8192 tokens 1055 us against 907.  Llama-3.1-8B heads,
-// us before -> now: 2 x 8192 fresh tokens 1524 -> 907, 8 turns of up to 512 behind 1536 cached 153 -> 101.
+// off the chain, read Q twice as often and were slower: 2 x 8192 tokens 1055 us against 907, both in a burst.
+// Llama-3.1-8B heads, us before -> now: 2 x 8192 fresh tokens 1516 -> 920 in a burst, 1600 -> 1100 where the power cap holds
+// the clock down; 8 turns of up to 512 behind 1536 cached 155 -> 115.
 #pragma once
 
 namespace b200 {
@@ -29,7 +30,8 @@ constexpr int kWideThreads = 384;
 constexpr int kWideTile = 128;                     // keys
 constexpr int kWideMinKeys = 1024;                 // shorter requests: attn_extend_kernel
 constexpr int kWideLoaders = 96;
-constexpr int kWideSoftmaxRegs = 192, kWideOtherRegs = 120;   // 256 x 192 + 128 x 120 <= 384 x 168 at launch; no spills
+constexpr int kWideSoftmaxRegs = 192, kWideOtherRegs = 120;   // 256 x 192 + 128 x 120 <= 384 x 168 at launch
+// (spilled: 4 bytes by the cluster instances of head size 64, 8 by attn_extend_flat_kernel, nothing by the others)
 
 template <int D>
 struct WideCfg {

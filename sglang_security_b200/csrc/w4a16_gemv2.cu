@@ -141,6 +141,7 @@ __device__ __forceinline__ uint32_t g2_hmul2(uint32_t a, uint32_t b) {
 // long as before fits: for grids that end a wave earlier with them (us, two / three a SM, f16, 9 and 16 tokens, Qwen2.5-32B
 // at TP 2, all four linears: 86.3 / 70.1 and 89.5 / 73.3; Llama-3.1-8B bf16 65.1 / 59.7 and 76.9 / 67.9; where both take
 // one wave, at TP 4, 35.0 / 36.6).
+// 80 registers a thread with three: seven of the eight instances spill 4 to 32 bytes.
 //  SPG = 32-k steps per quantisation group
 // known at compile time (1, 2, 4 = groups of 32, 64, 128: the fold sits at fixed places of the
 // unrolled round, no counters) or 0 = any other group size (run-time step counter).
