@@ -696,7 +696,7 @@ static bool flat_pays(int D, const ExtendParams& p, int bs, int max_extend_len, 
   if (flat >= 0.95 * narrow) return false;
   return flat < 0.95 * (splits > 1 ? wide : wide_last_us(D, p, bs, max_extend_len, lens));
 }
-// B200_EXTEND_FLAT: 0 never, 1 wherever it can (read per launch, for tests and A/B); else -1: by the estimates
+// B200_EXTEND_FLAT: 0 never, 1 wherever it can (read per launch and per choice, for tests and A/B); else -1: by the estimates
 static int extend_flat_choice() {
   const char* e = std::getenv("B200_EXTEND_FLAT");
   return e && (e[0] == '0' || e[0] == '1') ? e[0] - '0' : -1;

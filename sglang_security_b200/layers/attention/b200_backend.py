@@ -31,6 +31,8 @@ from ... import _lib
 from ...mem_cache.memory_pool import MHATokenToKVPool, kv_write
 from .base_attn_backend import AttentionBackend
 
+_ROW_TYPES = (torch.bfloat16, torch.float16)   # of the new rows that b200_extend_layer stores
+
 
 @dataclass
 class ForwardMetadata:
@@ -386,13 +388,13 @@ class B200AttnBackend(AttentionBackend):
         flat = 0
         if max_kv >= 1024:
             # whether the persistent kernel takes it, and its workspace: once per forward, not in every layer
-            scale = float(layer.scaling) * (1.0 if ks is None else ks)
-            form = (bs, max_kv, hq, hkv, d, causal, scale, float(layer.logit_cap or 0.0), os.environ.get("B200_EXTEND_FLAT"))
+            form = (hq, hkv, d, causal, layer.scaling, layer.logit_cap, ks)
             flat = md.flat_bytes.get(form)
             if flat is None:
                 lens = md.host_lens.buffer_info()[0] if md.host_lens is not None and len(md.host_lens) == 2 * bs else 0
                 flat = md.flat_bytes[form] = self.lib.b200_extend_layer_flat_bytes(
-                    bs, md.max_extend_len, max_kv, hq, hkv, d, 1 if causal else 0, *form[6:8], lens)
+                    bs, md.max_extend_len, max_kv, hq, hkv, d, 1 if causal else 0,
+                    float(layer.scaling) * (1.0 if ks is None else ks), float(layer.logit_cap or 0.0), lens)
         if flat:
             try:
                 scratch = torch.empty(scratch_bytes + flat, dtype=torch.uint8, device=q.device)
@@ -415,7 +417,8 @@ class B200AttnBackend(AttentionBackend):
             0 if not fp8 else 2 if k_cache.dtype == torch.float8_e5m2 else 1, float(layer.scaling),
             float(layer.logit_cap or 0.0), 1.0 if ks is None else ks, 1.0 if vs is None else vs, 0 if ks is None else 1,
             _lib.current_stream())
-        _lib.check(self.lib.b200_extend_layer_planned(args, 1 if flat else 0), "b200_attn_extend")
+        # (without the workspace the call takes one of the other kernels)
+        _lib.check(self.lib.b200_extend_layer_planned(args, 1) if flat else self.lib.b200_extend_layer(args), "b200_attn_extend")
         return o
 
     @staticmethod
@@ -426,10 +429,11 @@ class B200AttnBackend(AttentionBackend):
         bytes that are in the pool's FP8 type already, 32 bits) are not for it."""
         if not (k.is_cuda and loc.dtype == torch.int64 and loc.is_contiguous()):
             return None
-        if q_dtype not in (torch.bfloat16, torch.float16) or k.dtype != q_dtype or v.dtype != q_dtype:
+        if k.dtype != q_dtype or v.dtype != q_dtype or q_dtype not in _ROW_TYPES:
             return None
-        if v_cache.dtype != k_cache.dtype or (k_cache.dtype != q_dtype and not (
-                type(pool) is MHATokenToKVPool and _lib.is_fp8_kv(k_cache.dtype))):
+        pool_dtype = k_cache.dtype
+        if v_cache.dtype != pool_dtype or (pool_dtype != q_dtype and not (
+                type(pool) is MHATokenToKVPool and _lib.is_fp8_kv(pool_dtype))):
             return None
         n = loc.numel()
         if n == 0 or not (k_cache.is_contiguous() and v_cache.is_contiguous()):

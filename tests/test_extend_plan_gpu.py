@@ -84,6 +84,7 @@ def test_without_memory_for_the_workspace_the_other_kernels_run(pool_dtype, monk
     want = layer(q, k, v, fb)
     assert "flat" not in _lib.last_variant()
     monkeypatch.delenv("B200_EXTEND_FLAT")
+    backend.init_forward_metadata(fb)
     dense = _lib.load().b200_extend_layer_dense_bytes(sum(map(sum, TURNS)), 6, 3640, 8, 128)   # the FP8 pool's copy
     empty, refused = torch.empty, []
 
