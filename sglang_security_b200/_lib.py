@@ -453,10 +453,16 @@ def dtype_code(torch_dtype) -> int:
     return _dtype_codes[torch_dtype]
 
 
-def is_fp8_kv(torch_dtype) -> bool:
-    import torch
+_fp8_kv_dtypes = ()
 
-    return torch_dtype in (torch.float8_e4m3fn, torch.float8_e5m2)
+
+def is_fp8_kv(torch_dtype) -> bool:
+    global _fp8_kv_dtypes
+    if not _fp8_kv_dtypes:
+        import torch
+
+        _fp8_kv_dtypes = (torch.float8_e4m3fn, torch.float8_e5m2)
+    return torch_dtype in _fp8_kv_dtypes
 
 
 def kv_dtype_code(act_dtype, pool_dtype) -> int:
