@@ -37,6 +37,7 @@
 namespace b200 {
 
 constexpr int kG2Threads = 256;
+constexpr int kG2Smem3 = 72 * 1024;  // shared memory of a CTA with three an SM
 
 struct Gemv2Params {
   const void* x;
@@ -376,17 +377,17 @@ w4a16_gemv2_kernel(const Gemv2Params p) {
   if (S > 1) g2_cluster_sync();
   else __syncthreads();
   {
-    const int cpr = 128 / static_cast<int>(S);  // columns reduced by this rank (S is a power of two)
-    const int cshift = 31 - __clz(cpr);
+    const int cpr = ceil_div(128, static_cast<int>(S));  // columns reduced by this rank (the last may have fewer)
+    const int cshift = 32 - __clz(cpr - 1);
     T* o = static_cast<T*>(p.out);
     const T* bias = static_cast<const T*>(p.bias);
-    // kG2Threads is a multiple of cpr: a thread keeps the same column for all of its items, so its
-    // bias is loaded once (inside the loop the load would wait behind the previous output store)
-    const int c = static_cast<int>(rank) * cpr + (threadIdx.x & (cpr - 1));
+    // a thread keeps one column for all of its tokens, so its bias is loaded once (inside the loop the load would wait
+    // behind the previous output store)
+    const int i = threadIdx.x & ((1 << cshift) - 1);
+    const int c = static_cast<int>(rank) * cpr + i;
     const int n = n_grp * 128 + c;
-    const float bias_n = (bias && n < p.N) ? to_float<T>(bias[n]) : 0.f;
-    for (int item = threadIdx.x; item < p.M * cpr; item += kG2Threads) {
-      const int m = item >> cshift;
+    const float bias_n = (bias && c < 128 && n < p.N) ? to_float<T>(bias[n]) : 0.f;
+    for (int m = i < cpr && c < 128 ? threadIdx.x >> cshift : p.M; m < p.M; m += kG2Threads >> cshift) {
       const uint32_t local = sbase + part_off + (m * 128 + c) * 4;
       float sum = 0.f;
       if (S == 1) {
@@ -441,6 +442,41 @@ static bool gemv2_shape_ok(int M, int N, int K, int group) {
          (group == 32 || group % 64 == 0);
 }
 
+// Clusters of S CTAs that are resident at once, three CTAs an SM with the most shared memory that a plan gives them.
+static int gemv2_clusters(int S) {
+  static std::atomic<int> cached[64][9];
+  auto kern = w4a16_gemv2_kernel<__half, 1, 4, 3>;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
+    (void)cudaGetLastError();
+    return 0;
+  }
+  int n = cached[dev][S].load(std::memory_order_relaxed);
+  if (n == 0) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(S * 8);
+    cfg.blockDim = dim3(kG2Threads);
+    cfg.dynamicSmemBytes = kG2Smem3;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = S;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaFuncAttributes fa;
+    if (cudaFuncGetAttributes(&fa, kern) != cudaSuccess ||
+        (fa.maxDynamicSharedSizeBytes < kG2Smem3 &&
+         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kG2Smem3) != cudaSuccess) ||
+        cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) {
+      (void)cudaGetLastError();
+      n = -1;
+    }
+    cached[dev][S].store(n, std::memory_order_relaxed);
+  }
+  return n > 0 ? n : 0;
+}
+
 struct Gemv2Plan {
   int ctas, S, kb_per_rank, xs_stride, sz_off, sum_off, part_off, smem;
 };
@@ -463,12 +499,24 @@ static bool gemv2_plan(int M, int N, int K, int group, Gemv2Plan* pl) {
   } else {
     // at least two CTAs per SM, at least two slice units per rank
     const int sms = device_sm_count();
-    while (n_groups * S < 2 * sms && S < 8 && units >= 4 * S) S *= 2;
+    while (n_groups * S < 2 * sms && S < 8 &&
+           (units >= 4 * S || (MT == 1 && ceil_div(units, 2 * S) == 2 && (2 * S - 1) * 2 < units)))
+      S *= 2;
+    // One token tile: where the clusters are not all resident at three CTAs an SM, a smaller one that is and that still
+    // gives every SM two, since a second wave of a few CTAs costs as much as the first (f16, one token, us: 7168 x 4096 in
+    // 8 slices, 448 CTAs for 444 places, 10.9, in 6 7.5; 8192 x 28672 in 8 / 6 35.4 / 30.3; and 896 x 896 in 2 / 4
+    // 3.9 / 3.2).  Fewer than two leave the balance to chance: 28672 x 4096 whole 25, in 2 slices 20.
+    if (MT == 1 && n_groups > gemv2_clusters(S)) {
+      for (int c = S - 2; c > 0 && n_groups * c >= 2 * sms; c -= 2)
+        if (n_groups <= gemv2_clusters(c)) {
+          S = c;
+          break;
+        }
+    }
   }
   if (S > units) S = units;
   if (S < 1) S = 1;
-  while (S & (S - 1)) S &= S - 1;  // the reduce splits 128 columns over the ranks: power of two
-  for (;; S *= 2) {
+  for (;; S = MT == 1 ? S + 1 : 2 * S) {
     const int kb_per_rank = ceil_div(units, S) * upg;
     const int xs_stride = kb_per_rank * 128 + 64;  // +64: conflict-free LDS.128 across token rows
     const int ng = ceil_div(kb_per_rank * 64, group) + 1;
@@ -479,7 +527,7 @@ static bool gemv2_plan(int M, int N, int K, int group, Gemv2Plan* pl) {
     pl->sum_off = pl->sz_off + ng * 1024;
     pl->part_off = pl->sum_off + ng * 2 * MT * 8 * 4;
     pl->smem = pl->part_off + MT * 8 * 128 * 4;
-    if (pl->smem <= 72 * 1024 || S >= 8) break;  // keep >= 3 CTAs per SM when K allows
+    if (pl->smem <= kG2Smem3 || S >= 8) break;  // keep >= 3 CTAs per SM when K allows
   }
   pl->ctas = MT == 1 ? 3 : 2;
   if (MT == 2 && pl->part_off <= 75 * 1024) {

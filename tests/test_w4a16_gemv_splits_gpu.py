@@ -1,0 +1,39 @@
+"""Stream GEMV with K split over clusters whose size is no power of two (a rank then reduces ceil(128 / size) columns, the
+last one fewer): unit scales and activations in {-1, 0, 1}, so every sum is a whole number below 2^24 and the result is the
+exact one, rounded once."""
+import pytest
+import torch
+from oracle import int4 as O
+from test_w4a16_gpu import _prep, _rand_i32, gemv2_cfg  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(m, n, k, group, dtype):
+    from sglang_security_b200.layers.quantization.w4a16_kernel import gemv_stream_repack, w4a16_gemv_v2
+
+    qweight, qzeros = _rand_i32((k, n // 8), n + m), _rand_i32((k // group, n // 8), k)
+    x = torch.randint(-1, 2, (m, k), generator=torch.Generator().manual_seed(m)).to(dtype)
+    bias = torch.randint(-8, 9, (n,), generator=torch.Generator().manual_seed(n)).to(dtype)
+    w = O.unpack_awq_int4(qweight).float() - O.unpack_awq_int4(qzeros).float().repeat_interleave(group, 0)
+    qw, zb, sc = _prep(qweight, torch.ones((k // group, n), dtype=dtype), qzeros, dtype)
+    out = w4a16_gemv_v2(x.cuda(), gemv_stream_repack(qw), zb, sc, group, bias.cuda())
+    exact = (x.float() @ w + bias.float()).to(dtype)
+    assert torch.equal(out.cpu(), exact)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("m", [1, 5, 8, 13, 16])
+@pytest.mark.parametrize("splits", [3, 5, 6, 7])
+def test_cluster_sizes(splits, m, dtype, gemv2_cfg):  # noqa: F811
+    gemv2_cfg(splits)
+    _run(m, 288, 2560, 64, dtype)
+
+
+@pytest.mark.parametrize("m,n,k,splits", [(1, 7168, 4096, 6), (8, 7168, 4096, 6), (1, 896, 896, 4), (1, 28672, 1024, 2)])
+def test_default_sizes(m, n, k, splits):
+    """7168 channels: eight slices are more clusters than are resident at once."""
+    from sglang_security_b200 import _lib
+
+    _run(m, n, k, 128, torch.float16)
+    assert f"splits={splits} " in _lib.last_variant()
