@@ -141,6 +141,26 @@ int b200_attn_decode(const void* q, int64_t q_stride, const void* k_cache, const
                      int Hkv, int D, int Dv, float scale, float logit_cap, int dtype,
                      void* workspace, size_t workspace_bytes, int num_splits, void* stream);
 
+/* A layer's decode in one call: entry b's new K/V row (k, v [bs, Hkv, D] in the dtype of q, token strides in elements) goes
+ * to slot loc[b] of the pool, then attention as b200_attn_decode / _fused (tickets, q_out and q_scales may be NULL).  The
+ * split kernel stores the rows itself, so a request's page table may name its own new slot but none that another request
+ * of the batch is given in this call.  _fp8kv_: rows quantised as b200_kv_write_fp8 does (divided by the scales where
+ * has_scale), then b200_attn_decode_fp8kv / _fused. */
+int b200_attn_decode_layer(const void* k, int64_t k_stride, const void* v, int64_t v_stride, const int64_t* loc,
+                           const void* q, int64_t q_stride, void* k_cache, void* v_cache, int64_t kv_row_stride, void* o,
+                           int64_t o_stride, const int32_t* req_to_token, int64_t req_to_token_stride,
+                           const int64_t* req_pool_indices, const int64_t* seq_lens, int bs, int Hq, int Hkv, int D, int Dv,
+                           float scale, float logit_cap, int dtype, void* workspace, size_t workspace_bytes, int num_splits,
+                           void* tickets, size_t ticket_bytes, void* q_out, int64_t q_out_stride, float* q_scales,
+                           void* stream);
+int b200_attn_decode_fp8kv_layer(const void* k, int64_t k_stride, const void* v, int64_t v_stride, const int64_t* loc,
+                                 int has_scale, const void* q, int64_t q_stride, void* k_cache, void* v_cache,
+                                 int64_t kv_row_stride, void* o, int64_t o_stride, const int32_t* req_to_token,
+                                 int64_t req_to_token_stride, const int64_t* req_pool_indices, const int64_t* seq_lens, int bs,
+                                 int Hq, int Hkv, int D, int Dv, float scale, float logit_cap, float k_scale, float v_scale,
+                                 int dtype, void* workspace, size_t workspace_bytes, int num_splits, void* tickets,
+                                 size_t ticket_bytes, void* q_out, int64_t q_out_stride, float* q_scales, void* stream);
+
 /* b200_attn_decode for callers that cannot allocate device memory (CUDA graph capture, tight serving
  * loops, harnesses that forbid cudaMalloc).  NO COUNTERPART IN THE REFERENCE: added at the request
  * of the run's operators.  Same operands, math and kernels as b200_attn_decode, minus the workspace:

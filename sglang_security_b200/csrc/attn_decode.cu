@@ -58,6 +58,14 @@ struct DecodeParams {
   // optional output gate [rows, gate_stride] in T: o is multiplied by sigmoid(gate[row, head * D + d])
   const void* gate;
   int64_t gate_stride;
+  // b200_attn_decode_layer: entry b's new K/V row [Hkv, D] in T, stored to slot loc[b] of the pool before it is read
+  // (null: the pool holds it already)
+  const void* new_k;
+  const void* new_v;
+  int64_t new_k_stride, new_v_stride;
+  const int64_t* loc;
+  float k_scale_w, v_scale_w;   // FP8 pool: divisors of the stored rows, where scale_new
+  int scale_new;
 };
 
 constexpr float kLog2e = 1.4426950408889634f;
@@ -147,6 +155,39 @@ __device__ __forceinline__ uint32_t pack2<__half>(float lo, float hi) {
   return r;
 }
 
+
+// One warp stores entry b's new K and V rows of one kv head to the pool, 16 bytes of the source a lane and pass.  The caller
+// synchronises the warp before it requests the tile that holds the new token; other CTAs read other slots (a request's page
+// table names no slot that another request of the batch is being given).
+// A KV write launch of its own cost a dependent launch of ~2 us in front of every layer's attention, with 1 to 64 requests
+// (us, 32 / 8 heads of 128, bf16: 1 x 1000 10.4 -> 8.4, 8 x 1000 14.4 -> 12.4, 64 x 300 14.5 -> 12.4, 64 x 3000 101.3 ->
+// 100.5; 1.086 x over 110 batches, none slower).  The store's latency hides beside the page table's.
+template <typename T, int D, bool FP8, bool E5M2>
+__device__ __forceinline__ void store_new_rows(const DecodeParams& p, int b, int kvh, int lane) {
+  constexpr int CPR = D / 8;
+  const int64_t slot = p.loc[b];
+#pragma unroll
+  for (int i = lane; i < 2 * CPR; i += 32) {
+    const bool is_v = i >= CPR;
+    const int c = i - (is_v ? CPR : 0);
+    const T* src = static_cast<const T*>(is_v ? p.new_v : p.new_k) + b * (is_v ? p.new_v_stride : p.new_k_stride) + kvh * D + c * 8;
+    char* dst = const_cast<char*>(static_cast<const char*>(is_v ? p.v_cache : p.k_cache));
+    const uint4 raw = *reinterpret_cast<const uint4*>(src);
+    if (FP8) {
+      const T* e = reinterpret_cast<const T*>(&raw);
+      const float scale = is_v ? p.v_scale_w : p.k_scale_w;
+      uint32_t lo = 0, hi = 0;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        lo |= to_fp8_torch<T>(e[j], scale, p.scale_new != 0, E5M2) << (8 * j);
+        hi |= to_fp8_torch<T>(e[4 + j], scale, p.scale_new != 0, E5M2) << (8 * j);
+      }
+      *reinterpret_cast<uint2*>(dst + slot * p.kv_row_stride + kvh * D + c * 8) = make_uint2(lo, hi);
+    } else {
+      *reinterpret_cast<uint4*>(dst + (slot * p.kv_row_stride + kvh * D + c * 8) * 2) = raw;
+    }
+  }
+}
 
 // ---- fused tail: merge of the split partials (+ per-token FP8 quantisation) inside the kernel ----
 // Two levels of ticket counters (threadFenceReduction pattern; bar.sync + one gpu-scope acq_rel
@@ -309,7 +350,11 @@ attn_decode_mma_kernel(const DecodeParams p) {
   const int len = static_cast<int>(p.seq_lens[b]);
   const int chunk = split_chunk(len, p.num_splits, C::ALIGN);
   const int start = split * chunk;
-  if (start >= len) return;
+  constexpr bool NEW = !TAIL && !ROWS;
+  if (start >= len) {
+    if (NEW && p.new_k && len <= 0 && split == 0 && warp == 0) store_new_rows<T, D, false, false>(p, b, kvh, lane);
+    return;
+  }
   const int end = min(len, start + chunk);
   const int ntiles = ceil_div(end - start, NT);
   const int n_my = warp < ntiles ? (ntiles - warp + NW - 1) / NW : 0;
@@ -381,6 +426,10 @@ attn_decode_mma_kernel(const DecodeParams p) {
   };
 
   load_slots(0);
+  if (NEW && p.new_k && end == len && warp == (ntiles - 1) % NW) {   // this warp's last tile holds the new token
+    store_new_rows<T, D, false, false>(p, b, kvh, lane);
+    __syncwarp();
+  }
 #pragma unroll
   for (int s = 0; s < STAGES - 1; ++s) {
     issue_tile(s);
@@ -941,6 +990,42 @@ struct DecodeTail {
   float* q_scales;
 };
 
+// New rows of b200_attn_decode_layer / _fp8kv_layer.
+struct DecodeNewRows {
+  const void* k;
+  const void* v;
+  int64_t k_stride, v_stride;
+  const int64_t* loc;
+  int has_scale;
+};
+
+// The split kernel stores the rows itself where 16-byte pieces of a head fit them and it is not the instance with the
+// in-kernel tail; else they are written by a launch of their own before it.
+static int apply_new_rows(DecodeParams& p, const DecodeNewRows* rows, int D, int dtype, bool fp8, int e5m2, float k_scale,
+                          float v_scale, void* stream, const char* who) {
+  if (!rows) return 0;
+  B200_REQUIRE(rows->k && rows->v && rows->loc, "%s: null pointer", who);
+  if (!p.tickets && aligned16(rows->k) && aligned16(rows->v) && rows->k_stride % 8 == 0 && rows->v_stride % 8 == 0) {
+    p.new_k = rows->k;
+    p.new_v = rows->v;
+    p.new_k_stride = rows->k_stride;
+    p.new_v_stride = rows->v_stride;
+    p.loc = rows->loc;
+    p.k_scale_w = k_scale;
+    p.v_scale_w = v_scale;
+    p.scale_new = rows->has_scale;
+    return 0;
+  }
+  B200_REQUIRE(p.kv_row_stride == static_cast<int64_t>(p.Hkv) * D, "%s: pool rows of %lld elements for %d heads", who,
+               static_cast<long long>(p.kv_row_stride), p.Hkv);
+  void *kc = const_cast<void*>(p.k_cache), *vc = const_cast<void*>(p.v_cache);
+  const int row = p.Hkv * D;
+  if (fp8)
+    return b200_kv_write_fp8(rows->k, rows->v, rows->k_stride, rows->v_stride, kc, vc, rows->loc, p.bs, row, k_scale, v_scale,
+                             rows->has_scale, dtype | e5m2, stream);
+  return b200_kv_write(rows->k, rows->v, rows->k_stride * 2, rows->v_stride * 2, kc, vc, rows->loc, p.bs, row * 2, row * 2, stream);
+}
+
 static int apply_tail(DecodeParams& p, const DecodeTail* tail, int D, const char* who) {
   p.tickets = nullptr;
   p.q_out = nullptr;
@@ -1086,7 +1171,8 @@ static int attn_decode_impl(const void* q, int64_t q_stride, const void* k_cache
                             int Hq, int Hkv, int D, int Dv, float scale, float logit_cap, int dtype,
                             void* workspace, size_t workspace_bytes, int num_splits, void* stream,
                             const b200::DecodeTail* tail, const int32_t* row_list = nullptr,
-                            const void* gate = nullptr, int64_t gate_stride = 0) {
+                            const void* gate = nullptr, int64_t gate_stride = 0,
+                            const b200::DecodeNewRows* rows = nullptr) {
   using namespace b200;
   if (bs == 0) return 0;
   B200_REQUIRE(q && k_cache && v_cache && o && req_to_token && req_pool_indices && seq_lens,
@@ -1138,6 +1224,7 @@ static int attn_decode_impl(const void* q, int64_t q_stride, const void* k_cache
   p.part_lse = p.part_o ? p.part_o + static_cast<size_t>(bs) * Hq * num_splits * Dv : nullptr;
 
   if (int rc = apply_tail(p, tail, D, "b200_attn_decode_fused")) return rc;
+  if (int rc = apply_new_rows(p, rows, D, dtype, false, 0, 1.f, 1.f, stream, "b200_attn_decode_layer")) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int rc = dtype == B200_BF16 ? dispatch_decode<__nv_bfloat16>(p, D, G, st)
                               : dispatch_decode<__half>(p, D, G, st);
@@ -1205,7 +1292,8 @@ static int attn_decode_fp8kv_impl(const void* q, int64_t q_stride, const void* k
                                   const int64_t* seq_lens, int bs, int Hq, int Hkv, int D, int Dv,
                                   float scale, float logit_cap, float k_scale, float v_scale,
                                   int dtype, void* workspace, size_t workspace_bytes, int num_splits,
-                                  void* stream, const b200::DecodeTail* tail) {
+                                  void* stream, const b200::DecodeTail* tail,
+                                  const b200::DecodeNewRows* rows = nullptr) {
   using namespace b200;
   if (bs == 0) return 0;
   const bool e5m2 = (dtype & B200_KV_FP8_E5M2) != 0;
@@ -1261,6 +1349,9 @@ static int attn_decode_fp8kv_impl(const void* q, int64_t q_stride, const void* k
   p.part_o = static_cast<float*>(workspace);
   p.part_lse = p.part_o ? p.part_o + static_cast<size_t>(bs) * Hq * num_splits * Dv : nullptr;
   if (int rc = apply_tail(p, tail, D, "b200_attn_decode_fp8kv_fused")) return rc;
+  if (int rc = apply_new_rows(p, rows, D, dtype, true, e5m2 ? B200_KV_FP8_E5M2 : 0, k_scale, v_scale, stream,
+                              "b200_attn_decode_fp8kv_layer"))
+    return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int rc = dtype == B200_BF16 ? dispatch_decode_fp8kv<__nv_bfloat16>(p, D, G, e5m2, st)
                                     : dispatch_decode_fp8kv<__half>(p, D, G, e5m2, st);
@@ -1301,6 +1392,34 @@ int b200_attn_decode_fp8kv_fused(const void* q, int64_t q_stride, const void* k_
                                 req_to_token, req_to_token_stride, req_pool_indices, seq_lens, bs, Hq,
                                 Hkv, D, Dv, scale, logit_cap, k_scale, v_scale, dtype, workspace,
                                 workspace_bytes, num_splits, stream, &tail);
+}
+
+int b200_attn_decode_layer(const void* k, int64_t k_stride, const void* v, int64_t v_stride, const int64_t* loc,
+                           const void* q, int64_t q_stride, void* k_cache, void* v_cache, int64_t kv_row_stride, void* o,
+                           int64_t o_stride, const int32_t* req_to_token, int64_t req_to_token_stride,
+                           const int64_t* req_pool_indices, const int64_t* seq_lens, int bs, int Hq, int Hkv, int D, int Dv,
+                           float scale, float logit_cap, int dtype, void* workspace, size_t workspace_bytes, int num_splits,
+                           void* tickets, size_t ticket_bytes, void* q_out, int64_t q_out_stride, float* q_scales,
+                           void* stream) {
+  const b200::DecodeTail tail = {tickets, ticket_bytes, q_out, q_out_stride, q_scales};
+  const b200::DecodeNewRows rows = {k, v, k_stride, v_stride, loc, 0};
+  return attn_decode_impl(q, q_stride, k_cache, v_cache, kv_row_stride, o, o_stride, req_to_token, req_to_token_stride,
+                          req_pool_indices, seq_lens, bs, Hq, Hkv, D, Dv, scale, logit_cap, dtype, workspace, workspace_bytes,
+                          num_splits, stream, tickets || q_out ? &tail : nullptr, nullptr, nullptr, 0, &rows);
+}
+
+int b200_attn_decode_fp8kv_layer(const void* k, int64_t k_stride, const void* v, int64_t v_stride, const int64_t* loc,
+                                 int has_scale, const void* q, int64_t q_stride, void* k_cache, void* v_cache,
+                                 int64_t kv_row_stride, void* o, int64_t o_stride, const int32_t* req_to_token,
+                                 int64_t req_to_token_stride, const int64_t* req_pool_indices, const int64_t* seq_lens, int bs,
+                                 int Hq, int Hkv, int D, int Dv, float scale, float logit_cap, float k_scale, float v_scale,
+                                 int dtype, void* workspace, size_t workspace_bytes, int num_splits, void* tickets,
+                                 size_t ticket_bytes, void* q_out, int64_t q_out_stride, float* q_scales, void* stream) {
+  const b200::DecodeTail tail = {tickets, ticket_bytes, q_out, q_out_stride, q_scales};
+  const b200::DecodeNewRows rows = {k, v, k_stride, v_stride, loc, has_scale};
+  return attn_decode_fp8kv_impl(q, q_stride, k_cache, v_cache, kv_row_stride, o, o_stride, req_to_token, req_to_token_stride,
+                                req_pool_indices, seq_lens, bs, Hq, Hkv, D, Dv, scale, logit_cap, k_scale, v_scale, dtype,
+                                workspace, workspace_bytes, num_splits, stream, tickets || q_out ? &tail : nullptr, &rows);
 }
 
 int b200_attn_decode_split_align(int D, int group) {

@@ -96,7 +96,10 @@ attn_decode_fp8kv_kernel(const DecodeParams p) {
   const int len = static_cast<int>(p.seq_lens[b]);
   const int chunk = split_chunk(len, p.num_splits, C::ALIGN);
   const int start = split * chunk;
-  if (start >= len) return;
+  if (start >= len) {
+    if (!TAIL && p.new_k && len <= 0 && split == 0 && warp == 0) store_new_rows<T, D, true, E5M2>(p, b, kvh, lane);
+    return;
+  }
   const int end = min(len, start + chunk);
   const int ntiles = ceil_div(end - start, NT);
   const int n_my = warp < ntiles ? (ntiles - warp + NW - 1) / NW : 0;
@@ -165,6 +168,10 @@ attn_decode_fp8kv_kernel(const DecodeParams p) {
   };
 
   load_slots(0);
+  if (!TAIL && p.new_k && end == len && warp == (ntiles - 1) % NW) {   // this warp's last tile holds the new token
+    store_new_rows<T, D, true, E5M2>(p, b, kvh, lane);
+    __syncwarp();
+  }
 #pragma unroll
   for (int s = 0; s < STAGES - 1; ++s) {
     issue_tile(s);

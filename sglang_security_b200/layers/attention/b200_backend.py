@@ -275,11 +275,15 @@ class B200AttnBackend(AttentionBackend):
         bs = q.shape[0]
         o = q.new_empty((bs, hq * dv))
         pool = forward_batch.token_to_kv_pool
+        k_cache = pool.get_key_buffer(layer.layer_id)
+        v_cache = pool.get_value_buffer(layer.layer_id)
+        rows = None
         if save_kv_cache:
-            k_cache, v_cache = self._save_kv(layer, forward_batch, k, v)
-        else:
-            k_cache = pool.get_key_buffer(layer.layer_id)
-            v_cache = pool.get_value_buffer(layer.layer_id)
+            # one new row a request: the attention kernel stores it itself
+            if bs and forward_batch.out_cache_loc.numel() == bs:
+                rows = self._new_rows(q.dtype, k, v, k_cache, v_cache, pool, forward_batch.out_cache_loc, hkv, d)
+            if rows is None:
+                self._save_kv(layer, forward_batch, k, v)
         if bs == 0:
             return self._maybe_quant(o, fp8_out)
         self._check_layer(layer)
@@ -299,11 +303,19 @@ class B200AttnBackend(AttentionBackend):
                   k_cache.stride(0), o.data_ptr(), o.stride(0), req_to_token.data_ptr(),
                   req_to_token.stride(0), req_pool_indices.data_ptr(), seq_lens.data_ptr(), bs, hq,
                   hkv, d, dv, float(layer.scaling), float(layer.logit_cap or 0.0))
+        new = None
+        if rows is not None:
+            new = (rows[0].data_ptr(), rows[0].stride(0), rows[1].data_ptr(), rows[1].stride(0), rows[2].data_ptr())
         if fp8kv:
             ks, vs = self._kv_scales(layer)
             common = common + (1.0 if ks is None else ks, 1.0 if vs is None else vs)
+            if new is not None:
+                if (ks is None) != (vs is None):
+                    raise _lib.B200Error("forward_decode: k_scale and v_scale must be given together")
+                new = new + (0 if ks is None else 1,)
         common = common + (_lib.kv_dtype_code(q.dtype, k_cache.dtype), _lib.ptr(ws),
                            0 if ws is None else ws.numel(), md.num_splits)
+        layer_fn = self.lib.b200_attn_decode_fp8kv_layer if fp8kv else self.lib.b200_attn_decode_layer
         # the tail only pays when it replaces a launch: the merge (splits > 1) or the quantiser
         fused = self.fused_tail and (md.num_splits > 1 or fp8_out) and (hq * dv) % 8 == 0
         if fused:
@@ -313,17 +325,23 @@ class B200AttnBackend(AttentionBackend):
                 sa = torch.empty((bs, 1), dtype=torch.float32, device=q.device)
             fn = self.lib.b200_attn_decode_fp8kv_fused if fp8kv else self.lib.b200_attn_decode_fused
             tickets = self._ticket_buffer(bs) if bs <= self.tail_in_kernel_max_bs else None
-            rc = fn(*common, _lib.ptr(tickets), 0 if tickets is None else tickets.numel() * 4,
-                    _lib.ptr(qa), 0 if qa is None else qa.stride(0), _lib.ptr(sa),
-                    _lib.current_stream())
+            tail = (_lib.ptr(tickets), 0 if tickets is None else tickets.numel() * 4,
+                    _lib.ptr(qa), 0 if qa is None else qa.stride(0), _lib.ptr(sa))
+            if new is None:
+                rc = fn(*common, *tail, _lib.current_stream())
+            else:
+                rc = layer_fn(*new, *common, *tail, _lib.current_stream())
             _lib.check(rc, "b200_attn_decode_fused")
             if fp8_out:
                 from ..quantization.fp8_utils import QuantizedActivation
 
                 return QuantizedActivation(qa, sa, q.dtype)
             return o
-        fn = self.lib.b200_attn_decode_fp8kv if fp8kv else self.lib.b200_attn_decode
-        rc = fn(*common, _lib.current_stream())
+        if new is None:
+            fn = self.lib.b200_attn_decode_fp8kv if fp8kv else self.lib.b200_attn_decode
+            rc = fn(*common, _lib.current_stream())
+        else:
+            rc = layer_fn(*new, *common, None, 0, None, 0, None, _lib.current_stream())
         _lib.check(rc, "b200_attn_decode")
         return self._maybe_quant(o, fp8_out)
 

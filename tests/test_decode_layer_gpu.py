@@ -1,0 +1,78 @@
+"""Decode whose split kernel stores the new K/V rows itself: output and pools are the same bytes as with a KV write of its
+own before it, for page tables in any order, splits, several head tiles, entries without tokens, FP8 pools with and without
+scales, and rows that 16-byte loads do not fit (those are written by a launch before)."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from sglang_security_b200.layers.attention.b200_backend import B200AttnBackend
+from sglang_security_b200.layers.radix_attention import RadixAttention
+from sglang_security_b200.mem_cache.memory_pool import MHATokenToKVPool, ReqToTokenPool
+from sglang_security_b200.model_executor.forward_batch_info import ForwardBatch, ForwardMode
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _run(monkeypatch, own, heads, act, pool_dtype, lens, splits, scales, pad):
+    from sglang_security_b200 import _lib
+
+    hq, hkv, d = heads
+    g = torch.Generator(device=DEV).manual_seed(7)
+    bs, total = len(lens), sum(lens) + len(lens)
+    rtp = ReqToTokenPool(bs + 1, max(lens) + 9, DEV)
+    kvp = MHATokenToKVPool(total + 16, 1, pool_dtype, hkv, d, 1, DEV)
+    for buf in (kvp.k_buffer[0], kvp.v_buffer[0]):
+        rows = torch.randn(buf.shape, device=DEV, generator=g)
+        buf.copy_(rows.to(pool_dtype).view(torch.uint8) if pool_dtype.itemsize == 1 else rows)
+    slots = torch.randperm(total, device=DEV, generator=g) + 1
+    loc, at = [], 0
+    for b, n in enumerate(lens):
+        rtp.req_to_token[b, :n] = slots[at:at + n].to(torch.int32)
+        loc.append(slots[at + max(n - 1, 0)])          # an entry without tokens has a slot too
+        at += n + 1
+    width = (hq + 2 * hkv) * d
+    qkv = torch.randn(bs, width + pad, device=DEV, generator=g).to(act)[:, :width]
+    q, k, v = qkv.split([hq * d, hkv * d, hkv * d], dim=-1)
+    q = q.contiguous()
+    cfg = SimpleNamespace(num_attention_heads=hq, context_len=rtp.max_context_len, get_num_kv_heads=lambda tp: hkv)
+    backend = B200AttnBackend(SimpleNamespace(device=DEV, req_to_token_pool=rtp, token_to_kv_pool=kvp, model_config=cfg,
+                                              tp_size=1, server_args=SimpleNamespace(triton_attention_num_kv_splits=splits)))
+    monkeypatch.setattr(backend, "_num_splits", lambda *a: splits)
+    if not own:
+        monkeypatch.setattr(backend, "_new_rows", lambda *a: None)
+    layer = RadixAttention(hq, d, d ** -0.5, hkv, 0)
+    if scales:
+        layer.k_scale_float, layer.v_scale_float = scales
+    t = torch.tensor(lens, dtype=torch.int64)
+    fb = ForwardBatch(forward_mode=ForwardMode.DECODE, batch_size=bs,
+                      req_pool_indices=torch.arange(bs, dtype=torch.int64, device=DEV), seq_lens=t.to(DEV),
+                      out_cache_loc=torch.stack(loc), seq_lens_sum=sum(lens), seq_lens_cpu=t, req_to_token_pool=rtp,
+                      token_to_kv_pool=kvp, attn_backend=backend)
+    backend.init_forward_metadata(fb)
+    n0 = _lib.load().b200_launch_count()
+    o = layer(q, k, v, fb)
+    launches = _lib.load().b200_launch_count() - n0
+    live = torch.tensor([n > 0 for n in lens], device=DEV)
+    return o[live].clone(), kvp.k_buffer[0].clone(), kvp.v_buffer[0].clone(), launches
+
+
+@pytest.mark.parametrize("splits", [1, 5])
+@pytest.mark.parametrize("heads,act,pool,scales,pad", [
+    ((32, 8, 128), torch.bfloat16, torch.bfloat16, None, 0),
+    ((14, 2, 64), torch.float16, torch.float16, None, 8),
+    ((48, 2, 128), torch.bfloat16, torch.bfloat16, None, 0),             # three head tiles of a kv head
+    ((8, 2, 64), torch.bfloat16, torch.bfloat16, None, 3),               # rows that do not start on 16 bytes
+    ((32, 8, 128), torch.bfloat16, torch.float8_e4m3fn, None, 0),
+    ((20, 4, 128), torch.float16, torch.float8_e4m3fn, (0.5, 1.5), 0),
+    ((14, 2, 64), torch.bfloat16, torch.float8_e5m2, (0.25, 2.0), 16),
+    ((40, 2, 64), torch.bfloat16, torch.float8_e4m3fn, None, 0),
+])
+def test_same_bytes_as_a_write_before(heads, act, pool, scales, pad, splits, monkeypatch):
+    lens = [1, 0, 17, 48, 49, 300, 96, 97, 3]
+    got = _run(monkeypatch, True, heads, act, pool, lens, splits, scales, pad)
+    ref = _run(monkeypatch, False, heads, act, pool, lens, splits, scales, pad)
+    for a, b in zip(got[:3], ref[:3]):
+        assert torch.equal(a.view(torch.uint8), b.view(torch.uint8))
+    assert got[3] == ref[3] - (pad != 3)
