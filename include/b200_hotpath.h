@@ -145,21 +145,26 @@ int b200_attn_decode(const void* q, int64_t q_stride, const void* k_cache, const
  * to slot loc[b] of the pool, then attention as b200_attn_decode / _fused (tickets, q_out and q_scales may be NULL).  The
  * split kernel stores the rows itself, so a request's page table may name its own new slot but none that another request
  * of the batch is given in this call.  _fp8kv_: rows quantised as b200_kv_write_fp8 does (divided by the scales where
- * has_scale), then b200_attn_decode_fp8kv / _fused. */
+ * has_scale), then b200_attn_decode_fp8kv / _fused.  k NULL: the rows are in the pool.
+ * pieces > 0 (at least bs, at most 128 requests, no tail): the batch is cut into that many pieces at most, of about equal
+ * length, instead of num_splits a request (b200_attn_decode_pieces: how many, 0 where splits serve the batch); workspace from b200_attn_decode_pieces_workspace_bytes, 16-byte aligned. */
 int b200_attn_decode_layer(const void* k, int64_t k_stride, const void* v, int64_t v_stride, const int64_t* loc,
                            const void* q, int64_t q_stride, void* k_cache, void* v_cache, int64_t kv_row_stride, void* o,
                            int64_t o_stride, const int32_t* req_to_token, int64_t req_to_token_stride,
                            const int64_t* req_pool_indices, const int64_t* seq_lens, int bs, int Hq, int Hkv, int D, int Dv,
                            float scale, float logit_cap, int dtype, void* workspace, size_t workspace_bytes, int num_splits,
-                           void* tickets, size_t ticket_bytes, void* q_out, int64_t q_out_stride, float* q_scales,
+                           int pieces, void* tickets, size_t ticket_bytes, void* q_out, int64_t q_out_stride, float* q_scales,
                            void* stream);
 int b200_attn_decode_fp8kv_layer(const void* k, int64_t k_stride, const void* v, int64_t v_stride, const int64_t* loc,
                                  int has_scale, const void* q, int64_t q_stride, void* k_cache, void* v_cache,
                                  int64_t kv_row_stride, void* o, int64_t o_stride, const int32_t* req_to_token,
                                  int64_t req_to_token_stride, const int64_t* req_pool_indices, const int64_t* seq_lens, int bs,
                                  int Hq, int Hkv, int D, int Dv, float scale, float logit_cap, float k_scale, float v_scale,
-                                 int dtype, void* workspace, size_t workspace_bytes, int num_splits, void* tickets,
-                                 size_t ticket_bytes, void* q_out, int64_t q_out_stride, float* q_scales, void* stream);
+                                 int dtype, void* workspace, size_t workspace_bytes, int num_splits, int pieces,
+                                 void* tickets, size_t ticket_bytes, void* q_out, int64_t q_out_stride, float* q_scales,
+                                 void* stream);
+int b200_attn_decode_pieces(int bs, int Hkv, int group, int64_t total_len, int64_t max_len, int num_sms);
+size_t b200_attn_decode_pieces_workspace_bytes(int bs, int Hq, int Dv, int pieces);
 
 /* b200_attn_decode for callers that cannot allocate device memory (CUDA graph capture, tight serving
  * loops, harnesses that forbid cudaMalloc).  NO COUNTERPART IN THE REFERENCE: added at the request
@@ -169,7 +174,7 @@ int b200_attn_decode_fp8kv_layer(const void* k, int64_t k_stride, const void* v,
  * Limit: b200_attn_decode_workspace_bytes(bs, Hq, Dv, num_splits) must not exceed
  * B200_ATTN_DECODE_NOALLOC_SCRATCH_BYTES (8 MiB: e.g. 64 requests x 32 heads x 7 splits at Dv 128);
  * larger requests are rejected with an error (status 1, b200_last_error()), nothing is launched.
- * The device that owns `stream` must be current.  Every call on a device shares the scratch and
+ * The device that owns `stream` must be current.  Every call on a device pieces the scratch and
  * finds the previous call's contents in it (none of it has to be zero); calls that overlap on the
  * GPU (different streams, concurrent graph launches) race on it - serialise them on one stream.  */
 #define B200_ATTN_DECODE_NOALLOC_SCRATCH_BYTES (8u << 20)

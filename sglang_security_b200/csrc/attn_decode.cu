@@ -66,6 +66,9 @@ struct DecodeParams {
   const int64_t* loc;
   float k_scale_w, v_scale_w;   // FP8 pool: divisors of the stored rows, where scale_new
   int scale_new;
+  // PIECES instances: the batch is cut into this many pieces at most (decode_piece); grid.x is the piece
+  int pieces;
+  int2* plan;                   // [bs] first partial row and count of a request, for the merge
 };
 
 constexpr float kLog2e = 1.4426950408889634f;
@@ -155,6 +158,75 @@ __device__ __forceinline__ uint32_t pack2<__half>(float lo, float hi) {
   return r;
 }
 
+
+// ---- pieces of equal length, for batches of unequal requests --------------------------------------------------------
+// A split count for all requests cuts the long ones into long pieces and the short ones into short ones, and the long
+// pieces run alone at the end.  Here the batch is cut into at most `pieces` pieces of about equal length, one wave of CTAs:
+// the least length T (in ALIGN tokens) that gives no more than that, found by bisection over the lengths in the warp's
+// registers, then a prefix sum over the requests' piece counts.  Every warp of every CTA does it for itself (~0.5 us) from
+// the lengths on the device, so a captured launch follows them.  us, splits / pieces (random lengths, 32 / 8 heads of 128):
+// bf16 16 x up to 6000 51.2 -> 43.0, 32 x up to 1000 20.2 -> 16.0; e4m3 27 x up to 6000 46.8 -> 42.8, 32 x up to 3000 35.2
+// -> 28.7.  Tried: exact equal pieces, ranges that begin and end inside requests; a CTA then starts on up to two requests,
+// which costs what the even end gives below ~1000 tokens a CTA (e4m3 48 x up to 1500: splits 27.2, pieces 21.3, pieces 25.0).
+constexpr int kPieceMaxBatch = 128;
+struct DecodePiece {
+  int b, start, end, len, count;   // b < 0: no such piece
+};
+__device__ __forceinline__ DecodePiece decode_piece(const int64_t* seq_lens, int bs, int pieces, int x, int align, int lane) {
+  constexpr int R = kPieceMaxBatch / 32;
+  int u[R];
+  int total = 0, longest = 1;
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int i = r * 32 + lane;
+    const int len = i < bs ? static_cast<int>(seq_lens[i]) : 0;
+    u[r] = len > 0 ? (len + align - 1) / align : 0;
+    total += u[r];
+    longest = max(longest, u[r]);
+  }
+  total = __reduce_add_sync(0xffffffffu, total);
+  longest = __reduce_max_sync(0xffffffffu, longest);
+  // ceil(a / T) for a >= 1: (a - 0.5) / T never rounds across a whole number below 2^22
+  auto count_of = [](int a, float inv) { return a ? static_cast<int>((static_cast<float>(a) - 0.5f) * inv) + 1 : 0; };
+  int lo = max(1, total / pieces), hi = longest;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    const float inv = 1.0f / static_cast<float>(mid);
+    int n = 0;
+#pragma unroll
+    for (int r = 0; r < R; ++r) n += count_of(u[r], inv);
+    if (__reduce_add_sync(0xffffffffu, n) <= pieces) hi = mid;
+    else lo = mid + 1;
+  }
+  const float inv = 1.0f / static_cast<float>(lo);
+  DecodePiece out = {-1, 0, 0, 0, 0};
+  int before = 0;
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    if (r * 32 >= bs) break;
+    const int n = count_of(u[r], inv);
+    int incl = n;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, incl, off);
+      if (lane >= off) incl += t;
+    }
+    const unsigned hit = __ballot_sync(0xffffffffu, x < before + incl);
+    if (out.b < 0 && hit) {
+      const int src = __ffs(hit) - 1;
+      const int units = __shfl_sync(0xffffffffu, u[r], src);
+      out.count = __shfl_sync(0xffffffffu, n, src);
+      const int j = x - before - (__shfl_sync(0xffffffffu, incl, src) - out.count);
+      out.b = r * 32 + src;
+      out.len = static_cast<int>(seq_lens[out.b]);
+      const int chunk = (units + out.count - 1) / out.count * align;   // gives `count` pieces again, none empty
+      out.start = j * chunk;
+      out.end = min(out.len, out.start + chunk);
+    }
+    before += __shfl_sync(0xffffffffu, incl, 31);
+  }
+  return out;
+}
 
 // One warp stores entry b's new K and V rows of one kv head to the pool, 16 bytes of the source a lane and pass.  The caller
 // synchronises the warp before it requests the tile that holds the new token; other CTAs read other slots (a request's page
@@ -325,7 +397,7 @@ namespace b200 {
 
 // HI: the tile holds more than 8 heads (rows 8..15 of the MMA are live).  ROWS: the row list and the output gate
 // of b200_attn_decode_rows (an instance of its own: the others stay at their register limit without spills).
-template <typename T, int D, int NT, int STAGES, int NW, bool HI, bool TAIL, bool ROWS = false>
+template <typename T, int D, int NT, int STAGES, int NW, bool HI, bool TAIL, bool ROWS = false, bool PIECES = false>
 __global__ void __launch_bounds__(NW * 32, TAIL ? 4 : 0)
 attn_decode_mma_kernel(const DecodeParams p) {
   using C = MmaCfg<D, NT, STAGES, NW>;
@@ -343,19 +415,37 @@ attn_decode_mma_kernel(const DecodeParams p) {
   const int split = blockIdx.x;
   const int kvh = blockIdx.y / p.head_tiles;
   const int ht = blockIdx.y - kvh * p.head_tiles;
-  const int b = blockIdx.z;
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
-
-  const int len = static_cast<int>(p.seq_lens[b]);
-  const int chunk = split_chunk(len, p.num_splits, C::ALIGN);
-  const int start = split * chunk;
   constexpr bool NEW = !TAIL && !ROWS;
-  if (start >= len) {
-    if (NEW && p.new_k && len <= 0 && split == 0 && warp == 0) store_new_rows<T, D, false, false>(p, b, kvh, lane);
-    return;
+  int b = blockIdx.z, len, chunk = 0, start, end;
+  bool whole = false;                    // PIECES: writes the output row, not a partial one
+  if constexpr (PIECES) {
+    const DecodePiece piece = decode_piece(p.seq_lens, p.bs, p.pieces, split, C::ALIGN, lane);
+    if (split == 0 && warp == 0) {       // entries without tokens
+      for (int i = 0; i < p.bs; ++i) {
+        if (p.seq_lens[i] > 0) continue;
+        if (p.new_k) store_new_rows<T, D, false, false>(p, i, kvh, lane);
+        if (blockIdx.y == 0 && lane == 0) p.plan[i] = make_int2(0, 0);
+      }
+    }
+    if (piece.b < 0) return;
+    b = piece.b;
+    len = piece.len;
+    start = piece.start;
+    end = piece.end;
+    whole = piece.count == 1;
+    if (start == 0 && blockIdx.y == 0 && threadIdx.x == 0) p.plan[b] = make_int2(split, piece.count);
+  } else {
+    len = static_cast<int>(p.seq_lens[b]);
+    chunk = split_chunk(len, p.num_splits, C::ALIGN);
+    start = split * chunk;
+    if (start >= len) {
+      if (NEW && p.new_k && len <= 0 && split == 0 && warp == 0) store_new_rows<T, D, false, false>(p, b, kvh, lane);
+      return;
+    }
+    end = min(len, start + chunk);
   }
-  const int end = min(len, start + chunk);
   const int ntiles = ceil_div(end - start, NT);
   const int n_my = warp < ntiles ? (ntiles - warp + NW - 1) / NW : 0;
 
@@ -599,12 +689,13 @@ attn_decode_mma_kernel(const DecodeParams p) {
     }
     float out = num / den;
     const int hq = kvh * p.group + head0 + h;
-    if (p.num_splits == 1) {
+    if (PIECES ? whole : p.num_splits == 1) {
       const int64_t row = ROWS && p.row_list ? p.row_list[b] : b;
       if (ROWS && p.gate) out *= sigmoid_f(to_float<T>(static_cast<const T*>(p.gate)[row * p.gate_stride + hq * D + d]));
       static_cast<T*>(p.o)[row * p.o_stride + hq * D + d] = from_float<T>(out);
     } else {
-      const int64_t pidx = (static_cast<int64_t>(b) * p.Hq + hq) * p.num_splits + split;
+      const int64_t pidx = PIECES ? static_cast<int64_t>(split) * p.Hq + hq
+                                  : (static_cast<int64_t>(b) * p.Hq + hq) * p.num_splits + split;
       p.part_o[pidx * D + d] = out;
       if (d == 0) p.part_lse[pidx] = M + log2f(den);
     }
@@ -621,7 +712,7 @@ attn_decode_mma_kernel(const DecodeParams p) {
 // Sums run over the splits in order, as in attn_merge_quant_kernel: same bytes.
 constexpr int kMergeWarps = 4;
 
-// V columns per lane: 4, or 1 for rows that 16-byte loads do not fit
+// V columns per lane: 4 (2: half-width rows), or 1 for rows that 16-byte loads do not fit
 template <int V>
 __device__ __forceinline__ void merge_load(float (&x)[V], const float* p) {
   if constexpr (V == 4) {
@@ -630,6 +721,10 @@ __device__ __forceinline__ void merge_load(float (&x)[V], const float* p) {
     x[1] = f.y;
     x[2] = f.z;
     x[3] = f.w;
+  } else if constexpr (V == 2) {
+    const float2 f = __ldcg(reinterpret_cast<const float2*>(p));
+    x[0] = f.x;
+    x[1] = f.y;
   } else {
     x[0] = __ldcg(p);
   }
@@ -699,6 +794,62 @@ attn_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ pa
       dst[e] = from_float<T>(y);
     }
   }
+}
+
+// Merge behind the PIECES instances: one warp per head, piece s of request b in row first + s of the partials.  A request
+// in one piece was written by the split kernel.  Sums run over the pieces in order.
+template <typename T, int D>
+__global__ void __launch_bounds__(kMergeWarps * 32)
+attn_merge_pieces_kernel(const float* __restrict__ part_o, const float* __restrict__ part_lse, T* __restrict__ o,
+                         int64_t o_stride, const int2* __restrict__ plan, int Hq) {
+  constexpr int V = D / 32, AHEAD = 8;
+  griddep_wait();
+  griddep_launch_dependents();
+  const int lane = threadIdx.x & 31, b = blockIdx.y;
+  const int hq = blockIdx.x * kMergeWarps + (threadIdx.x >> 5);
+  if (hq >= Hq) return;
+  const int2 pc = __ldcg(plan + b);
+  const int count = pc.y;
+  if (count <= 1) return;
+  const float* lse = part_lse + static_cast<int64_t>(pc.x) * Hq + hq;
+  const float* po = part_o + (static_cast<int64_t>(pc.x) * Hq + hq) * D + lane * V;
+  const int64_t step = static_cast<int64_t>(Hq) * D;
+  float x[AHEAD][V];
+#pragma unroll
+  for (int i = 0; i < AHEAD; ++i)
+    if (i < count) merge_load<V>(x[i], po + i * step);
+  const float lse0 = lane < count ? __ldcg(lse + static_cast<int64_t>(lane) * Hq) : -INFINITY;
+  float M = lse0;
+  for (int s = 32 + lane; s < count; s += 32) M = fmaxf(M, __ldcg(lse + static_cast<int64_t>(s) * Hq));
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, off));
+  float den = 0.f, num[V];
+#pragma unroll
+  for (int e = 0; e < V; ++e) num[e] = 0.f;
+  for (int s0 = 0; s0 < count; s0 += 32) {
+    const float l = s0 == 0 ? lse0 : (s0 + lane < count ? __ldcg(lse + static_cast<int64_t>(s0 + lane) * Hq) : -INFINITY);
+    const float w_lane = s0 + lane < count ? fast_exp2(l - M) : 0.f;
+    for (int s1 = s0; s1 < min(count, s0 + 32); s1 += AHEAD) {
+      if (s1 > 0) {
+#pragma unroll
+        for (int i = 0; i < AHEAD; ++i)
+          if (s1 + i < count) merge_load<V>(x[i], po + (s1 + i) * step);
+      }
+#pragma unroll
+      for (int i = 0; i < AHEAD; ++i) {
+        const float w = __shfl_sync(0xffffffffu, w_lane, (s1 + i) & 31);
+        if (s1 + i < count) {
+          den += w;
+#pragma unroll
+          for (int e = 0; e < V; ++e) num[e] += w * x[i][e];
+        }
+      }
+    }
+  }
+  const float inv = 1.f / den;
+  T* dst = o + static_cast<int64_t>(b) * o_stride + hq * D + lane * V;
+#pragma unroll
+  for (int e = 0; e < V; ++e) dst[e] = from_float<T>(num[e] * inv);
 }
 
 // Merge of split partials for ALL heads of a request + per-token FP8 quantisation of the merged
@@ -856,7 +1007,7 @@ static int launch_decode_any(void (*kern)(const DecodeParams), const DecodeParam
                                       C::SMEM_BYTES));
     if (n_configured < 64) configured[n_configured++] = kern;
   }
-  dim3 grid(p.num_splits, p.Hkv * p.head_tiles, p.bs);
+  const dim3 grid = p.pieces ? dim3(p.pieces, p.Hkv * p.head_tiles) : dim3(p.num_splits, p.Hkv * p.head_tiles, p.bs);
   {
     ScopedKernelTimer timer(timer_name, st);
     B200_CUDA_OK(launch_kernel(kern, grid, dim3(C::THREADS), C::SMEM_BYTES, st, 1,
@@ -879,6 +1030,9 @@ static int launch_decode(const DecodeParams& p, cudaStream_t st) {
                                              "attn_decode_split", "attn_decode_mma_kernel");
   if (p.row_list || p.gate)
     return launch_decode_any<C>(attn_decode_mma_kernel<T, D, kNT, kStages, kNW, HI, false, true>, p, st,
+                                "attn_decode_split", "attn_decode_mma_kernel");
+  if (p.pieces)
+    return launch_decode_any<C>(attn_decode_mma_kernel<T, D, kNT, kStages, kNW, HI, false, false, true>, p, st,
                                 "attn_decode_split", "attn_decode_mma_kernel");
   auto kern = attn_decode_mma_kernel<T, D, kNT, kStages, kNW, HI, false>;
   static bool attr_done = false;
@@ -922,6 +1076,8 @@ static int launch_decode_fp8kv_st(const DecodeParams& p, cudaStream_t st) {
   using C = Fp8KvCfg<D, kNT8, ST, kNW>;
   if (p.tickets) return launch_decode_any<C>(attn_decode_fp8kv_kernel<T, D, kNT8, ST, kNW, HI, true>, p, st,
                                              "attn_decode_fp8kv", "attn_decode_fp8kv_kernel");
+  if (p.pieces) return launch_decode_any<C>(attn_decode_fp8kv_kernel<T, D, kNT8, ST, kNW, HI, false, false, true>, p, st,
+                                            "attn_decode_fp8kv", "attn_decode_fp8kv_kernel");
   auto kern = attn_decode_fp8kv_kernel<T, D, kNT8, ST, kNW, HI, false>;
   static bool attr_done = false;
   if (!attr_done) {
@@ -950,6 +1106,8 @@ static int launch_decode_fp8kv(const DecodeParams& p, cudaStream_t st) {
 template <typename T, int D, bool HI>
 static int launch_decode_e5m2kv(const DecodeParams& p, cudaStream_t st) {
   using C = Fp8KvCfg<D, kNT8, 2, kNW>;
+  if (p.pieces) return launch_decode_any<C>(attn_decode_fp8kv_kernel<T, D, kNT8, 2, kNW, HI, false, true, true>, p, st,
+                                            "attn_decode_fp8kv", "attn_decode_fp8kv_kernel<e5m2>");
   auto kern = attn_decode_fp8kv_kernel<T, D, kNT8, 2, kNW, HI, false, true>;
   static bool attr_done = false;
   if (!attr_done) {
@@ -1126,6 +1284,63 @@ int b200_attn_decode_num_splits_ragged(int bs, int Hkv, int group, int D, int64_
   return decode_num_splits(bs, Hkv, group, D, avg_len, max_len, num_sms);
 }
 
+static size_t pieces_plan_offset(int Hq, int Dv, int pieces) {
+  return (b200_attn_decode_workspace_bytes(1, Hq, Dv, pieces < 2 ? 2 : pieces) + 15) / 16 * 16;
+}
+
+size_t b200_attn_decode_pieces_workspace_bytes(int bs, int Hq, int Dv, int pieces) {
+  if (pieces <= 0 || bs <= 0) return 0;
+  return pieces_plan_offset(Hq, Dv, pieces) + static_cast<size_t>(bs) * sizeof(int2);
+}
+
+static int use_pieces(b200::DecodeParams& p, int pieces, int Dv, void* workspace, size_t bytes, const char* who) {
+  using namespace b200;
+  B200_REQUIRE(pieces >= p.bs && p.bs <= kPieceMaxBatch && pieces <= 65535, "%s: %d pieces for %d requests", who, pieces, p.bs);
+  B200_REQUIRE(workspace && aligned16(workspace) && bytes >= b200_attn_decode_pieces_workspace_bytes(p.bs, p.Hq, Dv, pieces),
+               "%s: workspace too small for %d pieces", who, pieces);
+  p.pieces = pieces;
+  p.part_o = static_cast<float*>(workspace);
+  p.part_lse = p.part_o + static_cast<size_t>(pieces) * p.Hq * Dv;
+  p.plan = reinterpret_cast<int2*>(static_cast<char*>(workspace) + pieces_plan_offset(p.Hq, Dv, pieces));
+  return 0;
+}
+
+static int merge_pieces(const b200::DecodeParams& p, int D, int dtype, void* stream) {
+  using namespace b200;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const dim3 grid(ceil_div(p.Hq, kMergeWarps), p.bs);
+  ScopedKernelTimer timer("attn_merge", st);
+#define MERGE_PIECES(T, D_)                                                                                                \
+  B200_CUDA_OK(launch_kernel(attn_merge_pieces_kernel<T, D_>, grid, dim3(kMergeWarps * 32), 0, st, 1,                      \
+                             pdl_family(p.bs, kPdlMerge), p.part_o, p.part_lse, static_cast<T*>(p.o), p.o_stride, p.plan, p.Hq))
+  if (dtype == B200_BF16) {
+    if (D == 128) MERGE_PIECES(__nv_bfloat16, 128);
+    else MERGE_PIECES(__nv_bfloat16, 64);
+  } else {
+    if (D == 128) MERGE_PIECES(__half, 128);
+    else MERGE_PIECES(__half, 64);
+  }
+#undef MERGE_PIECES
+  B200_CHECK_LAUNCH("attn_merge_pieces_kernel");
+  return 0;
+}
+
+/* How many pieces a decode batch of unequal requests is cut into, or 0 where a split count for all serves it. */
+int b200_attn_decode_pieces(int bs, int Hkv, int group, int64_t total_len, int64_t max_len, int num_sms) {
+  using namespace b200;
+  if (bs < 2 || bs > kPieceMaxBatch || Hkv <= 0 || group <= 0) return 0;
+  if (num_sms <= 0) num_sms = 148;
+  // One wave at four CTAs an SM (two and three waves were slower in every batch timed).  Not where the longest request is
+  // within an eighth of the average; from 1.5 pieces a request on (64 x up to 1500 tokens, 1.2 pieces a request: 50.1 us in
+  // splits, 53.0 in pieces); up to 16 (4 x up to 4000, 18 a request: 10.3 / 11.4, where splits of every request fill the
+  // wave as well); and from 250 tokens a piece on (8 x up to 2000, 135 a piece: 11.6 / 12.1; 16 x up to 2000, 270: 17.5 /
+  // 15.2), below which the plan and the merge cost what the even end gives.
+  const int64_t pieces = static_cast<int64_t>(num_sms) * 4 / (Hkv * ceil_div(group, tile_heads(group)));
+  const bool unequal = max_len * 8 * bs > total_len * 9;
+  if (!unequal || 2 * pieces < 3 * bs || pieces > 16 * bs || total_len < 250 * pieces || pieces > 65535) return 0;
+  return static_cast<int>(pieces);
+}
+
 static int attn_merge_impl(const float* part_o, const float* part_lse, void* o, int64_t o_stride,
                            const int64_t* seq_lens, int bs, int Hq, int Dv, int num_splits,
                            int split_align, const int32_t* row_list, const void* gate,
@@ -1172,7 +1387,7 @@ static int attn_decode_impl(const void* q, int64_t q_stride, const void* k_cache
                             void* workspace, size_t workspace_bytes, int num_splits, void* stream,
                             const b200::DecodeTail* tail, const int32_t* row_list = nullptr,
                             const void* gate = nullptr, int64_t gate_stride = 0,
-                            const b200::DecodeNewRows* rows = nullptr) {
+                            const b200::DecodeNewRows* rows = nullptr, int pieces = 0) {
   using namespace b200;
   if (bs == 0) return 0;
   B200_REQUIRE(q && k_cache && v_cache && o && req_to_token && req_pool_indices && seq_lens,
@@ -1191,7 +1406,7 @@ static int attn_decode_impl(const void* q, int64_t q_stride, const void* k_cache
                "b200_attn_decode: q/k_cache/v_cache must be 16-byte aligned with strides %% 8 == 0");
   B200_REQUIRE(bs <= 65535 && Hkv * 8 <= 65535, "b200_attn_decode: grid too large");
   const size_t need = b200_attn_decode_workspace_bytes(bs, Hq, Dv, num_splits);
-  B200_REQUIRE(num_splits == 1 || (workspace && workspace_bytes >= need),
+  B200_REQUIRE(num_splits == 1 || pieces > 0 || (workspace && workspace_bytes >= need),
                "b200_attn_decode: workspace too small (%zu < %zu)", workspace_bytes, need);
 
   DecodeParams p = {};
@@ -1225,10 +1440,15 @@ static int attn_decode_impl(const void* q, int64_t q_stride, const void* k_cache
 
   if (int rc = apply_tail(p, tail, D, "b200_attn_decode_fused")) return rc;
   if (int rc = apply_new_rows(p, rows, D, dtype, false, 0, 1.f, 1.f, stream, "b200_attn_decode_layer")) return rc;
+  if (pieces > 0) {
+    B200_REQUIRE(!tail && !row_list && !gate, "b200_attn_decode_layer: pieces take no fused tail");
+    if (int rc = use_pieces(p, pieces, Dv, workspace, workspace_bytes, "b200_attn_decode_layer")) return rc;
+  }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int rc = dtype == B200_BF16 ? dispatch_decode<__nv_bfloat16>(p, D, G, st)
                               : dispatch_decode<__half>(p, D, G, st);
   if (rc) return rc;
+  if (pieces > 0) return merge_pieces(p, D, dtype, stream);
   if (tail && !tail->tickets && tail->q_out)
     return dtype == B200_BF16 ? launch_merge_quant<__nv_bfloat16>(p, Dv, decode_align(), st)
                               : launch_merge_quant<__half>(p, Dv, decode_align(), st);
@@ -1293,7 +1513,7 @@ static int attn_decode_fp8kv_impl(const void* q, int64_t q_stride, const void* k
                                   float scale, float logit_cap, float k_scale, float v_scale,
                                   int dtype, void* workspace, size_t workspace_bytes, int num_splits,
                                   void* stream, const b200::DecodeTail* tail,
-                                  const b200::DecodeNewRows* rows = nullptr) {
+                                  const b200::DecodeNewRows* rows = nullptr, int pieces = 0) {
   using namespace b200;
   if (bs == 0) return 0;
   const bool e5m2 = (dtype & B200_KV_FP8_E5M2) != 0;
@@ -1321,7 +1541,7 @@ static int attn_decode_fp8kv_impl(const void* q, int64_t q_stride, const void* k
   B200_REQUIRE(bs <= 65535 && Hkv * 8 <= 65535, "b200_attn_decode_fp8kv: grid too large");
   B200_REQUIRE(k_scale > 0.f && v_scale > 0.f, "b200_attn_decode_fp8kv: scales must be positive");
   const size_t need = b200_attn_decode_workspace_bytes(bs, Hq, Dv, num_splits);
-  B200_REQUIRE(num_splits == 1 || (workspace && workspace_bytes >= need),
+  B200_REQUIRE(num_splits == 1 || pieces > 0 || (workspace && workspace_bytes >= need),
                "b200_attn_decode_fp8kv: workspace too small (%zu < %zu)", workspace_bytes, need);
   DecodeParams p = {};
   p.q = q;
@@ -1352,10 +1572,15 @@ static int attn_decode_fp8kv_impl(const void* q, int64_t q_stride, const void* k
   if (int rc = apply_new_rows(p, rows, D, dtype, true, e5m2 ? B200_KV_FP8_E5M2 : 0, k_scale, v_scale, stream,
                               "b200_attn_decode_fp8kv_layer"))
     return rc;
+  if (pieces > 0) {
+    B200_REQUIRE(!tail, "b200_attn_decode_fp8kv_layer: pieces take no fused tail");
+    if (int rc = use_pieces(p, pieces, Dv, workspace, workspace_bytes, "b200_attn_decode_fp8kv_layer")) return rc;
+  }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int rc = dtype == B200_BF16 ? dispatch_decode_fp8kv<__nv_bfloat16>(p, D, G, e5m2, st)
                                     : dispatch_decode_fp8kv<__half>(p, D, G, e5m2, st);
   if (rc) return rc;
+  if (pieces > 0) return merge_pieces(p, D, dtype, stream);
   if (tail && !tail->tickets && tail->q_out)
     return dtype == B200_BF16 ? launch_merge_quant<__nv_bfloat16>(p, Dv, decode_align_fp8kv(), st)
                               : launch_merge_quant<__half>(p, Dv, decode_align_fp8kv(), st);
@@ -1399,13 +1624,13 @@ int b200_attn_decode_layer(const void* k, int64_t k_stride, const void* v, int64
                            int64_t o_stride, const int32_t* req_to_token, int64_t req_to_token_stride,
                            const int64_t* req_pool_indices, const int64_t* seq_lens, int bs, int Hq, int Hkv, int D, int Dv,
                            float scale, float logit_cap, int dtype, void* workspace, size_t workspace_bytes, int num_splits,
-                           void* tickets, size_t ticket_bytes, void* q_out, int64_t q_out_stride, float* q_scales,
+                           int pieces, void* tickets, size_t ticket_bytes, void* q_out, int64_t q_out_stride, float* q_scales,
                            void* stream) {
   const b200::DecodeTail tail = {tickets, ticket_bytes, q_out, q_out_stride, q_scales};
   const b200::DecodeNewRows rows = {k, v, k_stride, v_stride, loc, 0};
   return attn_decode_impl(q, q_stride, k_cache, v_cache, kv_row_stride, o, o_stride, req_to_token, req_to_token_stride,
                           req_pool_indices, seq_lens, bs, Hq, Hkv, D, Dv, scale, logit_cap, dtype, workspace, workspace_bytes,
-                          num_splits, stream, tickets || q_out ? &tail : nullptr, nullptr, nullptr, 0, &rows);
+                          num_splits, stream, tickets || q_out ? &tail : nullptr, nullptr, nullptr, 0, k ? &rows : nullptr, pieces);
 }
 
 int b200_attn_decode_fp8kv_layer(const void* k, int64_t k_stride, const void* v, int64_t v_stride, const int64_t* loc,
@@ -1413,13 +1638,14 @@ int b200_attn_decode_fp8kv_layer(const void* k, int64_t k_stride, const void* v,
                                  int64_t kv_row_stride, void* o, int64_t o_stride, const int32_t* req_to_token,
                                  int64_t req_to_token_stride, const int64_t* req_pool_indices, const int64_t* seq_lens, int bs,
                                  int Hq, int Hkv, int D, int Dv, float scale, float logit_cap, float k_scale, float v_scale,
-                                 int dtype, void* workspace, size_t workspace_bytes, int num_splits, void* tickets,
-                                 size_t ticket_bytes, void* q_out, int64_t q_out_stride, float* q_scales, void* stream) {
+                                 int dtype, void* workspace, size_t workspace_bytes, int num_splits, int pieces,
+                                 void* tickets, size_t ticket_bytes, void* q_out, int64_t q_out_stride, float* q_scales,
+                                 void* stream) {
   const b200::DecodeTail tail = {tickets, ticket_bytes, q_out, q_out_stride, q_scales};
   const b200::DecodeNewRows rows = {k, v, k_stride, v_stride, loc, has_scale};
   return attn_decode_fp8kv_impl(q, q_stride, k_cache, v_cache, kv_row_stride, o, o_stride, req_to_token, req_to_token_stride,
                                 req_pool_indices, seq_lens, bs, Hq, Hkv, D, Dv, scale, logit_cap, k_scale, v_scale, dtype,
-                                workspace, workspace_bytes, num_splits, stream, tickets || q_out ? &tail : nullptr, &rows);
+                                workspace, workspace_bytes, num_splits, stream, tickets || q_out ? &tail : nullptr, k ? &rows : nullptr, pieces);
 }
 
 int b200_attn_decode_split_align(int D, int group) {

@@ -71,7 +71,7 @@ __device__ __forceinline__ void q4_to_f16<__nv_bfloat16>(const __nv_bfloat16* q,
   hi = *reinterpret_cast<const uint32_t*>(&hb);
 }
 
-template <typename T, int D, int NT, int STAGES, int NW, bool HI, bool TAIL, bool E5M2 = false>
+template <typename T, int D, int NT, int STAGES, int NW, bool HI, bool TAIL, bool E5M2 = false, bool PIECES = false>
 __global__ void __launch_bounds__(NW * 32, TAIL ? 4 : 0)
 attn_decode_fp8kv_kernel(const DecodeParams p) {
   using C = Fp8KvCfg<D, NT, STAGES, NW>;
@@ -89,18 +89,37 @@ attn_decode_fp8kv_kernel(const DecodeParams p) {
   const int split = blockIdx.x;
   const int kvh = blockIdx.y / p.head_tiles;
   const int ht = blockIdx.y - kvh * p.head_tiles;
-  const int b = blockIdx.z;
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
-
-  const int len = static_cast<int>(p.seq_lens[b]);
-  const int chunk = split_chunk(len, p.num_splits, C::ALIGN);
-  const int start = split * chunk;
-  if (start >= len) {
-    if (!TAIL && p.new_k && len <= 0 && split == 0 && warp == 0) store_new_rows<T, D, true, E5M2>(p, b, kvh, lane);
-    return;
+  constexpr bool NEW = !TAIL;
+  int b = blockIdx.z, len, chunk = 0, start, end;
+  bool whole = false;                    // PIECES: writes the output row, not a partial one
+  if constexpr (PIECES) {
+    const DecodePiece piece = decode_piece(p.seq_lens, p.bs, p.pieces, split, C::ALIGN, lane);
+    if (split == 0 && warp == 0) {       // entries without tokens
+      for (int i = 0; i < p.bs; ++i) {
+        if (p.seq_lens[i] > 0) continue;
+        if (p.new_k) store_new_rows<T, D, true, E5M2>(p, i, kvh, lane);
+        if (blockIdx.y == 0 && lane == 0) p.plan[i] = make_int2(0, 0);
+      }
+    }
+    if (piece.b < 0) return;
+    b = piece.b;
+    len = piece.len;
+    start = piece.start;
+    end = piece.end;
+    whole = piece.count == 1;
+    if (start == 0 && blockIdx.y == 0 && threadIdx.x == 0) p.plan[b] = make_int2(split, piece.count);
+  } else {
+    len = static_cast<int>(p.seq_lens[b]);
+    chunk = split_chunk(len, p.num_splits, C::ALIGN);
+    start = split * chunk;
+    if (start >= len) {
+      if (NEW && p.new_k && len <= 0 && split == 0 && warp == 0) store_new_rows<T, D, true, E5M2>(p, b, kvh, lane);
+      return;
+    }
+    end = min(len, start + chunk);
   }
-  const int end = min(len, start + chunk);
   const int ntiles = ceil_div(end - start, NT);
   const int n_my = warp < ntiles ? (ntiles - warp + NW - 1) / NW : 0;
 
@@ -168,7 +187,7 @@ attn_decode_fp8kv_kernel(const DecodeParams p) {
   };
 
   load_slots(0);
-  if (!TAIL && p.new_k && end == len && warp == (ntiles - 1) % NW) {   // this warp's last tile holds the new token
+  if (NEW && p.new_k && end == len && warp == (ntiles - 1) % NW) {   // this warp's last tile holds the new token
     store_new_rows<T, D, true, E5M2>(p, b, kvh, lane);
     __syncwarp();
   }
@@ -358,10 +377,11 @@ attn_decode_fp8kv_kernel(const DecodeParams p) {
     }
     const float out = num / den * p.v_scale;
     const int hq = kvh * p.group + head0 + h;
-    if (p.num_splits == 1) {
+    if (PIECES ? whole : p.num_splits == 1) {
       static_cast<T*>(p.o)[static_cast<int64_t>(b) * p.o_stride + hq * D + d] = from_float<T>(out);
     } else {
-      const int64_t pidx = (static_cast<int64_t>(b) * p.Hq + hq) * p.num_splits + split;
+      const int64_t pidx = PIECES ? static_cast<int64_t>(split) * p.Hq + hq
+                                  : (static_cast<int64_t>(b) * p.Hq + hq) * p.num_splits + split;
       p.part_o[pidx * D + d] = out;
       if (d == 0) p.part_lse[pidx] = M + log2f(den);
     }

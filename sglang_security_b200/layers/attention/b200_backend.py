@@ -37,6 +37,7 @@ _ROW_TYPES = (torch.bfloat16, torch.float16)   # of the new rows that b200_exten
 @dataclass
 class ForwardMetadata:
     num_splits: int = 1
+    pieces: int = 0              # decode: > 0 where the batch is cut into pieces of equal length, not splits of a request
     workspace: Optional[torch.Tensor] = None
     # extend only
     qo_indptr: Optional[torch.Tensor] = None
@@ -122,9 +123,11 @@ class B200AttnBackend(AttentionBackend):
             bs, self.num_kv_head, self.num_head // self.num_kv_head, head_dim, int(avg_len),
             max(int(avg_len), int(max_len)), self.num_sms)
 
-    def _ensure_workspace(self, bs: int, num_splits: int) -> Optional[torch.Tensor]:
+    def _ensure_workspace(self, bs: int, num_splits: int, pieces: int = 0) -> Optional[torch.Tensor]:
         need = self.lib.b200_attn_decode_workspace_bytes(bs, self.num_head, self.v_head_dim,
                                                          num_splits)
+        if pieces:
+            need = max(need, self.lib.b200_attn_decode_pieces_workspace_bytes(bs, self.num_head, self.v_head_dim, pieces))
         if need == 0:
             return None
         if self._workspace is None or self._workspace.numel() < need:
@@ -142,8 +145,12 @@ class B200AttnBackend(AttentionBackend):
             lens = getattr(forward_batch, "seq_lens_cpu", None)   # host copy, where the scheduler keeps one
             longest = int(lens.max()) if torch.is_tensor(lens) and not lens.is_cuda and lens.numel() else 0
             s = self._num_splits(bs, head_dim, max(1, total // bs), longest)
-            self.forward_metadata = ForwardMetadata(num_splits=s,
-                                                    workspace=self._ensure_workspace(bs, s))
+            pieces = 0
+            if longest and self.fixed_num_kv_splits <= 0:
+                pieces = self.lib.b200_attn_decode_pieces(bs, self.num_kv_head, self.num_head // self.num_kv_head, int(total),
+                                                          longest, self.num_sms)
+            self.forward_metadata = ForwardMetadata(num_splits=s, pieces=pieces,
+                                                    workspace=self._ensure_workspace(bs, s, pieces))
         else:
             self.forward_metadata = self._init_extend_metadata(forward_batch)
 
@@ -317,7 +324,8 @@ class B200AttnBackend(AttentionBackend):
                            0 if ws is None else ws.numel(), md.num_splits)
         layer_fn = self.lib.b200_attn_decode_fp8kv_layer if fp8kv else self.lib.b200_attn_decode_layer
         # the tail only pays when it replaces a launch: the merge (splits > 1) or the quantiser
-        fused = self.fused_tail and (md.num_splits > 1 or fp8_out) and (hq * dv) % 8 == 0
+        pieces = 0 if fp8_out else md.pieces
+        fused = self.fused_tail and not pieces and (md.num_splits > 1 or fp8_out) and (hq * dv) % 8 == 0
         if fused:
             qa = sa = None
             if fp8_out:
@@ -330,18 +338,20 @@ class B200AttnBackend(AttentionBackend):
             if new is None:
                 rc = fn(*common, *tail, _lib.current_stream())
             else:
-                rc = layer_fn(*new, *common, *tail, _lib.current_stream())
+                rc = layer_fn(*new, *common, 0, *tail, _lib.current_stream())
             _lib.check(rc, "b200_attn_decode_fused")
             if fp8_out:
                 from ..quantization.fp8_utils import QuantizedActivation
 
                 return QuantizedActivation(qa, sa, q.dtype)
             return o
-        if new is None:
+        if new is None and not pieces:
             fn = self.lib.b200_attn_decode_fp8kv if fp8kv else self.lib.b200_attn_decode
             rc = fn(*common, _lib.current_stream())
         else:
-            rc = layer_fn(*new, *common, None, 0, None, 0, None, _lib.current_stream())
+            if new is None:
+                new = (None, 0, None, 0, None, 0) if fp8kv else (None, 0, None, 0, None)
+            rc = layer_fn(*new, *common, pieces, None, 0, None, 0, None, _lib.current_stream())
         _lib.check(rc, "b200_attn_decode")
         return self._maybe_quant(o, fp8_out)
 

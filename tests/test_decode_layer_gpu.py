@@ -15,7 +15,7 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda"
 
 
-def _run(monkeypatch, own, heads, act, pool_dtype, lens, splits, scales, pad):
+def _run(monkeypatch, own, heads, act, pool_dtype, lens, splits, scales, pad, pieces=0):
     from sglang_security_b200 import _lib
 
     hq, hkv, d = heads
@@ -51,6 +51,10 @@ def _run(monkeypatch, own, heads, act, pool_dtype, lens, splits, scales, pad):
                       out_cache_loc=torch.stack(loc), seq_lens_sum=sum(lens), seq_lens_cpu=t, req_to_token_pool=rtp,
                       token_to_kv_pool=kvp, attn_backend=backend)
     backend.init_forward_metadata(fb)
+    if pieces:
+        backend.forward_metadata.pieces = pieces
+        backend.forward_metadata.workspace = backend._ensure_workspace(bs, splits, pieces)
+        backend.forward_metadata.workspace.fill_(0xff)       # NaN in every partial row
     n0 = _lib.load().b200_launch_count()
     o = layer(q, k, v, fb)
     launches = _lib.load().b200_launch_count() - n0
@@ -76,3 +80,41 @@ def test_same_bytes_as_a_write_before(heads, act, pool, scales, pad, splits, mon
     for a, b in zip(got[:3], ref[:3]):
         assert torch.equal(a.view(torch.uint8), b.view(torch.uint8))
     assert got[3] == ref[3] - (pad != 3)
+
+
+@pytest.mark.parametrize("heads,act,pool,scales", [
+    ((32, 8, 128), torch.bfloat16, torch.bfloat16, None), ((14, 2, 64), torch.float16, torch.float16, None),
+    ((48, 2, 128), torch.bfloat16, torch.bfloat16, None), ((20, 4, 128), torch.float16, torch.float8_e4m3fn, (0.5, 1.5)),
+    ((40, 2, 64), torch.bfloat16, torch.float8_e4m3fn, None), ((8, 2, 64), torch.bfloat16, torch.float8_e5m2, None),
+])
+@pytest.mark.parametrize("lens,pieces", [
+    ([1, 0, 17, 48, 49, 300, 96, 97, 3], 9),                     # a piece a request at most
+    ([1, 0, 17, 48, 49, 300, 96, 97, 3], 14),
+    ([0, 5000, 1, 0, 700, 0], 40),                               # a request in many pieces; the last entries are empty
+    ([7 + 37 * i % 911 for i in range(128)], 148),               # the largest batch
+    ([2000, 96, 96], 64),                                        # more pieces than tiles need
+    ([33], 1),
+])
+def test_pieces_of_equal_length(heads, act, pool, scales, lens, pieces, monkeypatch):
+    """Against one split a request, which sums the same terms in another order: the probabilities are rounded once to 16
+    bits (f16 or bf16: 2^-9 of each) and the output once, so the outputs differ by 2^-8 in the 2-norm and no element by more
+    than that of the largest |v| (6 at most here, times the scale)."""
+    got = _run(monkeypatch, True, heads, act, pool, lens, 1, scales, 0, pieces)
+    ref = _run(monkeypatch, True, heads, act, pool, lens, 1, scales, 0)
+    for a, b in zip(got[1:3], ref[1:3]):
+        assert torch.equal(a.view(torch.uint8), b.view(torch.uint8))
+    a, b = got[0].double(), ref[0].double()
+    assert bool(a.isfinite().all())
+    assert (a - b).norm() <= 2.0 ** -8 * b.norm()
+    assert (a - b).abs().max() <= 2.0 ** -8 * 6 * (scales[1] if scales else 1.0)
+
+
+def test_rule_of_the_pieces():
+    from sglang_security_b200 import _lib
+
+    lib = _lib.load()
+    f = lambda bs, total, longest, hkv=8, group=4: lib.b200_attn_decode_pieces(bs, hkv, group, total, longest, 148)  # noqa: E731
+    assert f(27, 27 * 3750, 6000) == 74 and f(16, 20000, 2000) == 74
+    assert f(27, 27 * 4096, 4096) == 0                           # equal requests
+    assert f(64, 64 * 1000, 1500) == 0 and f(4, 10000, 4000) == 0 and f(8, 10000, 2000) == 0 and f(129, 10 ** 6, 10 ** 5) == 0
+    assert f(40, 40 * 1915, 3064, 4, 5) == 148 and f(27, 27 * 3750, 6000, 2, 24) == 148
