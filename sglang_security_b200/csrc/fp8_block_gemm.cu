@@ -490,7 +490,7 @@ static int launch_block_pair(const void* a, int64_t lda, const void* b, int64_t 
   p.vec_ok = p.ldc % 8 == 0 && aligned16(p.out);
   p.splits = 1;
   p.kb_per_split = ceil_div(p.K, 128);
-  note_variant("fp8_block_gemm pair tiles=%d", tiles);
+  note_variant("fp8_block_gemm bn=256 pair tiles=%d", tiles);
   {
     ScopedKernelTimer timer("fp8_block_gemm", st);
     B200_CUDA_OK(launch_kernel(fp8_block_pair_kernel<OutT>, dim3(2 * (tiles < pairs ? tiles : pairs)), dim3(kBlkThreads),
@@ -512,6 +512,8 @@ static int launch_block_gemm(const void* a, int64_t lda, const void* b, int64_t 
   const double narrow = ceil_div(mb * ceil_div(p.N, 128), sms) * (0.28 * num_kb + 2.7) + 3.7;
   const double wide = ceil_div(mb * nb, sms) * (0.41 * num_kb + 6.0) + 2.9;
   const double pair = pairs > 0 ? ceil_div(ceil_div(p.M, 256) * nb, pairs) * (0.37 * num_kb + 5.5) + 2.8 : wide;
+  // a short K leaves little for wide tiles to save: only where there are 1.5 of them an SM
+  if (num_kb < 12 && 2 * mb * nb < 3 * sms) return launch_block_gemm_bn<OutT, 128>(a, lda, b, ldb, p, st);
   if (pair < wide && pair < narrow) return launch_block_pair<OutT>(a, lda, b, ldb, p, pairs, st);
   if (wide < narrow) return launch_block_gemm_bn<OutT, 256>(a, lda, b, ldb, p, st);
   return launch_block_gemm_bn<OutT, 128>(a, lda, b, ldb, p, st);
