@@ -152,7 +152,7 @@ fp8_quant_row_kernel(const T* __restrict__ x, int64_t ldx, uint8_t* __restrict__
   }
 }
 
-// 16 lanes per 128-element group (8 elements per lane), 2 groups per warp, GPT groups per lane.
+// 16 lanes per 128-element group (8 elements per lane), 2 groups per warp.
 // scales[m * s_row + g * s_col]: row-major (s_row = K/128, s_col = 1) or column-major / TMA
 // aligned (s_row = 1, s_col = padded M).
 // x / scale is a true division.  With r = 1 / scale rounded to nearest, q = x r and one remainder step
@@ -160,10 +160,9 @@ fp8_quant_row_kernel(const T* __restrict__ x, int64_t ldx, uint8_t* __restrict__
 // division's for every significand of x and of the maximum is checked exhaustively by the tests.  That holds while
 // the remainder is exact: a quotient that is not rounded to zero is at least 2^-11, so its product with the scale is
 // a multiple of 2^-57 scale, which fp32 holds from a scale of 2^-92 on.  Smaller scales (a caller's eps; below 3e-39
-// their reciprocal is infinite) and infinite ones are divided by.  The compiler's division and one load in flight per lane bound the kernel: 3001 x 14336 bf16 took 46.5 us, now 32.5, of 20 us
-// of HBM time; 2048 x 4096 10.9, now 8.8.
+// their reciprocal is infinite) and infinite ones are divided by.  The compiler's division and one load in flight per lane bound the kernel.
 constexpr float kReciprocalMin = 0x1p-90f;
-template <typename T, int GPT>
+template <typename T>
 __global__ void __launch_bounds__(256)
 fp8_quant_group128_kernel(const T* __restrict__ x, int64_t ldx, uint8_t* __restrict__ q,
                           int64_t ldq, float* __restrict__ scales, int64_t s_row, int64_t s_col,
@@ -172,51 +171,151 @@ fp8_quant_group128_kernel(const T* __restrict__ x, int64_t ldx, uint8_t* __restr
   griddep_launch_dependents();
   const int lane = threadIdx.x & 15;
   const unsigned total = static_cast<unsigned>(M) * groups_per_row;   // below 2^31: the launcher cuts the rows
-  const unsigned gid0 = blockIdx.x * (16u * GPT) + (threadIdx.x >> 4);
-  uint4 raw[GPT];
-  int64_t m[GPT];
-  int g[GPT];
+  const unsigned gid = blockIdx.x * 16u + (threadIdx.x >> 4);
+  const unsigned row = gid / static_cast<unsigned>(groups_per_row);
+  const int64_t m = row;
+  const int g = static_cast<int>(gid - row * groups_per_row);
+  const uint4 raw = gid < total ? *reinterpret_cast<const uint4*>(x + m * ldx + g * 128 + lane * 8) : make_uint4(0, 0, 0, 0);
+  const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+  float2 f[4];
+  float amax = eps;
 #pragma unroll
-  for (int i = 0; i < GPT; ++i) {
-    const unsigned gid = gid0 + i * 16;
-    const unsigned row = gid / static_cast<unsigned>(groups_per_row);
-    m[i] = gid < total ? static_cast<int64_t>(row) : -1;
-    g[i] = static_cast<int>(gid - row * groups_per_row);
-    raw[i] = m[i] >= 0 ? *reinterpret_cast<const uint4*>(x + m[i] * ldx + g[i] * 128 + lane * 8) : make_uint4(0, 0, 0, 0);
+  for (int e = 0; e < 4; ++e) {
+    f[e] = unpack2<T>(w[e]);
+    amax = fmaxf(amax, fmaxf(fabsf(f[e].x), fabsf(f[e].y)));
   }
 #pragma unroll
-  for (int i = 0; i < GPT; ++i) {
-    const uint32_t w[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
-    float2 f[4];
-    float amax = eps;
+  for (int off = 8; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
+  if (gid >= total) return;
+  const float s = amax / kFp8Max;
+  if (lane == 0) scales[m * s_row + g * s_col] = s;
+  if (s >= kReciprocalMin && s < INFINITY) {
+    const float r = 1.0f / s;
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      f[e] = unpack2<T>(w[e]);
-      amax = fmaxf(amax, fmaxf(fabsf(f[e].x), fabsf(f[e].y)));
+      const float qx = f[e].x * r, qy = f[e].y * r;
+      f[e].x = copysignf(fmaf(fmaf(-qx, s, f[e].x), r, qx), qx);   // -0 stays -0
+      f[e].y = copysignf(fmaf(fmaf(-qy, s, f[e].y), r, qy), qy);
     }
+  } else {
 #pragma unroll
-    for (int off = 8; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
-    if (m[i] < 0) continue;
-    const float s = amax / kFp8Max;
-    if (lane == 0) scales[m[i] * s_row + g[i] * s_col] = s;
-    if (s >= kReciprocalMin && s < INFINITY) {
-      const float r = 1.0f / s;
+    for (int e = 0; e < 4; ++e) f[e] = make_float2(f[e].x / s, f[e].y / s);
+  }
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    f[e].x = fminf(fmaxf(f[e].x, -kFp8Max), kFp8Max);
+    f[e].y = fminf(fmaxf(f[e].y, -kFp8Max), kFp8Max);
+  }
+  *reinterpret_cast<uint2*>(q + m * ldq + g * 128 + lane * 8) = make_uint2(e4m3x4(f[0], f[1]), e4m3x4(f[2], f[3]));
+}
+
+// The same for 8192 groups or more: 8 lanes x 16 elements a group, 32 rows a block, GPT groups a lane along K.  Half as many
+// lanes share the group's maximum, division and reciprocal; products and remainder steps are packed; groups without a NaN
+// (nearly all) need no clamp, since the conversion saturates; the general rules are a function of their own, so that six
+// or eight blocks fit an SM.  Issue slots and, with fewer blocks, bytes in flight bounded the kernel above: 3001 x 14336
+// bf16 32.7 -> 22.0 us (19.7 of HBM time), 2048 x 4096 9.5 -> 7.0, 512 x 4096 3.2 -> 2.4.  Two groups a lane from 65536 on
+// (3001 x 14336 one / two / four 23.9 / 22.0 / 29.6; 1024 x 4096 4.4 / 5.0).
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;\n" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+// One group by the general rules (NaN, infinities, tiny scales: a true division, clamped), 8 lanes of a full warp.
+template <typename T>
+__device__ __noinline__ void quant_group_general(const T* src, uint8_t* out, float* scale, bool store, bool lane0, float eps) {
+  float2 f[8];
+  float amax = eps;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const uint4 raw = *reinterpret_cast<const uint4*>(src + h * 64);
+    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      f[h * 4 + e] = unpack2<T>(w[e]);
+      amax = fmaxf(amax, fmaxf(fabsf(f[h * 4 + e].x), fabsf(f[h * 4 + e].y)));
+    }
+  }
+#pragma unroll
+  for (int off = 4; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
+  const float s = amax / kFp8Max;
+  if (s >= kReciprocalMin && s < INFINITY) {
+    const float r = 1.0f / s;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const float qx = f[e].x * r, qy = f[e].y * r;
+      f[e].x = copysignf(fmaf(fmaf(-qx, s, f[e].x), r, qx), qx);   // -0 stays -0
+      f[e].y = copysignf(fmaf(fmaf(-qy, s, f[e].y), r, qy), qy);
+    }
+  } else {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) f[e] = make_float2(f[e].x / s, f[e].y / s);
+  }
+  if (!store) return;
+  if (lane0) *scale = s;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    f[e].x = fminf(fmaxf(f[e].x, -kFp8Max), kFp8Max);
+    f[e].y = fminf(fmaxf(f[e].y, -kFp8Max), kFp8Max);
+  }
+  *reinterpret_cast<uint2*>(out) = make_uint2(e4m3x4(f[0], f[1]), e4m3x4(f[2], f[3]));
+  *reinterpret_cast<uint2*>(out + 64) = make_uint2(e4m3x4(f[4], f[5]), e4m3x4(f[6], f[7]));
+}
+
+template <typename T, int GPT>
+__global__ void __launch_bounds__(256, GPT == 1 ? 8 : 6)
+fp8_quant_group128_rows_kernel(const T* __restrict__ x, int64_t ldx, uint8_t* __restrict__ q, int64_t ldq,
+                               float* __restrict__ scales, int64_t s_row, int64_t s_col, int M, int groups_per_row, float eps) {
+  griddep_wait();
+  griddep_launch_dependents();
+  const int lane = threadIdx.x & 7;
+  const unsigned along = static_cast<unsigned>(ceil_div(groups_per_row, GPT));
+  const int m = static_cast<int>(blockIdx.x / along) * 32 + (threadIdx.x >> 3);
+  const int g0 = static_cast<int>(blockIdx.x % along) * GPT;
+  const bool row_ok = m < M;
+  const T* src = x + static_cast<int64_t>(row_ok ? m : M - 1) * ldx + g0 * 128 + lane * 8;
+  uint8_t* out = q + m * ldq + g0 * 128 + lane * 8;
+  float* sc = scales + m * s_row + g0 * s_col;
+  uint4 raw[GPT][2];
+#pragma unroll
+  for (int i = 0; i < GPT; ++i)
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      raw[i][h] = g0 + i < groups_per_row ? *reinterpret_cast<const uint4*>(src + i * 128 + h * 64) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+  for (int i = 0; i < GPT; ++i) {
+    if (g0 + i >= groups_per_row) break;
+    float2 f[8];
+    float a0 = 0.f, a1 = 0.f;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const uint32_t w[4] = {raw[i][h].x, raw[i][h].y, raw[i][h].z, raw[i][h].w};
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const float qx = f[e].x * r, qy = f[e].y * r;
-        f[e].x = copysignf(fmaf(fmaf(-qx, s, f[e].x), r, qx), qx);   // -0 stays -0
-        f[e].y = copysignf(fmaf(fmaf(-qy, s, f[e].y), r, qy), qy);
+        f[h * 4 + e] = unpack2<T>(w[e]);
+        a0 = max_nan(a0, fabsf(f[h * 4 + e].x));
+        a1 = max_nan(a1, fabsf(f[h * 4 + e].y));
       }
-    } else {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) f[e] = make_float2(f[e].x / s, f[e].y / s);
     }
+    a0 = max_nan(a0, a1);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      f[e].x = fminf(fmaxf(f[e].x, -kFp8Max), kFp8Max);
-      f[e].y = fminf(fmaxf(f[e].y, -kFp8Max), kFp8Max);
+    for (int off = 4; off > 0; off >>= 1) a0 = max_nan(a0, __shfl_xor_sync(0xffffffffu, a0, off));
+    const float s = fmaxf(a0, eps) / kFp8Max;
+    if (__any_sync(0xffffffffu, !(a0 == a0 && s >= kReciprocalMin && s < INFINITY))) {
+      quant_group_general(src + i * 128, out + i * 128, sc + i * s_col, row_ok, lane == 0, eps);
+      continue;
     }
-    *reinterpret_cast<uint2*>(q + m[i] * ldq + g[i] * 128 + lane * 8) = make_uint2(e4m3x4(f[0], f[1]), e4m3x4(f[2], f[3]));
+    const float r = 1.0f / s;
+    const float2 r2 = make_float2(r, r), ns = make_float2(-s, -s);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const float2 qe = fmul2(f[e], r2);
+      const float2 y = ffma2(ffma2(qe, ns, f[e]), r2, qe);
+      f[e] = make_float2(copysignf(y.x, qe.x), copysignf(y.y, qe.y));
+    }
+    if (!row_ok) continue;
+    if (lane == 0) sc[i * s_col] = s;
+    *reinterpret_cast<uint2*>(out + i * 128) = make_uint2(e4m3x4(f[0], f[1]), e4m3x4(f[2], f[3]));
+    *reinterpret_cast<uint2*>(out + i * 128 + 64) = make_uint2(e4m3x4(f[4], f[5]), e4m3x4(f[6], f[7]));
   }
 }
 
@@ -301,22 +400,33 @@ int b200_fp8_quant_group128(const void* x, int64_t ldx, void* q, int64_t ldq, fl
   for (int m0 = 0; m0 < M; m0 += step) {
     const int rows = M - m0 < step ? M - m0 : step;
     const unsigned total = static_cast<unsigned>(rows) * gpr;
+    const int64_t xo = static_cast<int64_t>(m0) * ldx, qo = static_cast<int64_t>(m0) * ldq;
+    float* sc = scales + static_cast<int64_t>(m0) * scale_row_stride;
     // four groups per lane once that still leaves every SM its eight blocks, one where blocks are scarce
     const bool many = total >= static_cast<unsigned>(device_sm_count()) * 8u * 64u;
     const unsigned blocks = (total + (many ? 63u : 15u)) / (many ? 64u : 16u);
-    const int64_t xo = static_cast<int64_t>(m0) * ldx, qo = static_cast<int64_t>(m0) * ldq;
-    float* sc = scales + static_cast<int64_t>(m0) * scale_row_stride;
-#define LAUNCH_GROUP(T, GPT)                                                                                          \
-  B200_CUDA_OK(launch_kernel(fp8_quant_group128_kernel<T, GPT>, dim3(blocks), dim3(256), 0, st, 1,                    \
-                             pdl_family(M, kPdlQuant), static_cast<const T*>(x) + xo, ldx,                            \
-                             static_cast<uint8_t*>(q) + qo, ldq, sc, scale_row_stride, scale_col_stride, rows, gpr, eps))
-    if (dtype == B200_BF16) {
-      if (many) LAUNCH_GROUP(__nv_bfloat16, 4);
-      else LAUNCH_GROUP(__nv_bfloat16, 1);
-    } else {
-      if (many) LAUNCH_GROUP(__half, 4);
-      else LAUNCH_GROUP(__half, 1);
+    const char* ev = getenv("GQ");
+    if (ev && *ev != '0' && rows <= 65535 * 32) {
+      const int gpt = *ev - '0';
+#define LAUNCH_ROWS(T, GPT)                                                                                                 \
+  B200_CUDA_OK(launch_kernel(fp8_quant_group128_rows_kernel<T, GPT>, dim3(ceil_div(gpr, GPT), ceil_div(rows, 32)), dim3(256), 0, \
+                             st, 1, getenv("GP") ? kPdlQuant : pdl_family(M, kPdlQuant), static_cast<const T*>(x) + xo, ldx, static_cast<uint8_t*>(q) + qo, \
+                             ldq, sc, scale_row_stride, scale_col_stride, rows, gpr, eps))
+      if (dtype == B200_BF16) { if (gpt == 1) LAUNCH_ROWS(__nv_bfloat16, 1); else if (gpt == 2) LAUNCH_ROWS(__nv_bfloat16, 2); else LAUNCH_ROWS(__nv_bfloat16, 4); }
+      else { if (gpt == 1) LAUNCH_ROWS(__half, 1); else if (gpt == 2) LAUNCH_ROWS(__half, 2); else LAUNCH_ROWS(__half, 4); }
+      continue;
     }
+#define LAUNCH_GROUP(KERNEL, BLOCKS)                                                                                  \
+  B200_CUDA_OK(launch_kernel(KERNEL, dim3(BLOCKS), dim3(256), 0, st, 1, pdl_family(M, kPdlQuant), static_cast<const T*>(x) + xo, ldx,       \
+                             static_cast<uint8_t*>(q) + qo, ldq, sc, scale_row_stride, scale_col_stride, rows, gpr, eps))
+    auto launch = [&](auto type) -> int {
+      using T = decltype(type);
+      if (total >= 65536) LAUNCH_GROUP((fp8_quant_group128_rows_kernel<T, 2>), ceil_div(gpr, 2) * ceil_div(rows, 32));
+      else if (total >= 8192) LAUNCH_GROUP((fp8_quant_group128_rows_kernel<T, 1>), gpr * ceil_div(rows, 32));
+      else LAUNCH_GROUP(fp8_quant_group128_kernel<T>, (total + 15) / 16);
+      return 0;
+    };
+    if (int rc = dtype == B200_BF16 ? launch(__nv_bfloat16()) : launch(__half())) return rc;
 #undef LAUNCH_GROUP
   }
   B200_CHECK_LAUNCH("fp8_quant_group128_kernel");
