@@ -82,7 +82,8 @@ def apply_w8a8_block_fp8_linear(input: torch.Tensor, weight: torch.Tensor, block
     if input_2d.stride(-1) != 1:
         input_2d = input_2d.contiguous()
     output_shape = [*input.shape[:-1], weight.shape[0]]
-    q_input, x_scale = per_token_group_quant_fp8(input_2d, block_size[1], column_major_scales=False)
+    # scales by K block: a block's token scales are then consecutive for the GEMM that reads them block by block
+    q_input, x_scale = per_token_group_quant_fp8(input_2d, block_size[1], column_major_scales=True)
     output = fp8_blockwise_scaled_mm(q_input, weight, x_scale, weight_scale, out_dtype=input.dtype,
                                      bias=bias, comm=comm)
     return output.view(*output_shape)
