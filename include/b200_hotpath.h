@@ -410,6 +410,26 @@ int b200_fp8_gemm_block128(const void* a, int64_t lda, const void* b, int64_t ld
                            int64_t bs_row_stride, const void* bias, void* out, int64_t ldc, int M,
                            int N, int K, int out_dtype, void* stream);
 
+/* A linear layer over a 16-bit activation in one call: the activation's quantiser, then the GEMM.  Eight-byte fields.
+ * block == 0: b200_fp8_quant_per_token and b200_fp8_gemm_rowcol (w_scale_stride 1 per channel, 0 one for all);
+ * block != 0: b200_fp8_quant_group128 (eps 1e-10, scales by K block) and b200_fp8_gemm_block128 (w_scale_stride between
+ * rows of 128 channels).  scratch, 256-byte aligned: M K bytes rounded up to 256, then M (block: M K / 128) floats. */
+typedef struct {
+  const void* x;
+  int64_t ldx;
+  const void* w;
+  int64_t ldw;
+  const float* w_scale;
+  int64_t w_scale_stride;
+  const void* bias;
+  void* out;
+  int64_t ldc;
+  void* scratch;
+  int64_t M, N, K, dtype, block;
+  void* stream;
+} b200_fp8_linear_args;
+int b200_fp8_linear(const b200_fp8_linear_args* args);
+
 /* ---- dense 16-bit GEMM (unquantised layers, lm_head) ------------------------------------------ */
 /* out[M,N] = x[M,K] . w[N,K]^T (+ bias[N]); bf16 / f16 operands and output, fp32 accumulation on
  * tcgen05 (same persistent TMA kernel as the FP8 path, kind::f16).  Replaces F.linear in

@@ -21,6 +21,9 @@ KV_FP8_E5M2 = 0x100  # B200_KV_FP8_E5M2: flag on the dtype argument of the FP8-K
 # b200_extend_layer_args: 8-byte fields in the order of the header
 EXTEND_LAYER_ARGS = struct.Struct("=Pq2PqPqPq2P3P2P2qPqP2qP7q3q4dqP".replace("P", "Q"))
 
+# b200_fp8_linear_args, likewise
+FP8_LINEAR_ARGS = struct.Struct("=QqQqQqQQqQ5qQ")
+
 _SIGNATURES = {
     "b200_version": (c_int, []),
     "b200_last_error": (c_char_p, []),
@@ -51,6 +54,7 @@ _SIGNATURES = {
     "b200_attn_extend_known": (c_int, [c_void_p, c_int64, c_void_p, c_void_p, c_int64, c_void_p, c_int64, c_void_p,
                                        c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                                        c_int, c_int, c_int, c_int, c_float, c_float, c_float, c_int, c_int, c_void_p]),
+    "b200_fp8_linear": (c_int, [c_char_p]),
     "b200_extend_layer": (c_int, [c_char_p]),
     "b200_extend_layer_planned": (c_int, [c_char_p, c_int]),
     "b200_extend_layer_dense_bytes": (c_size_t, [c_int64, c_int64, c_int64, c_int64, c_int64]),

@@ -597,4 +597,25 @@ int b200_fp8_gemm_block128_ar(void* comm, const void* a, int64_t lda, const void
                                 bias, out, ldc, M, N, K, out_dtype, stream, comm);
 }
 
+int b200_fp8_linear(const b200_fp8_linear_args* a) {
+  using namespace b200;
+  B200_REQUIRE(a, "b200_fp8_linear: null pointer");
+  B200_REQUIRE(a->M >= 0 && a->M <= 0x7fffffff && a->N >= 0 && a->N <= 0x7fffffff && a->K > 0 && a->K <= 0x7fffffff,
+               "b200_fp8_linear: bad shape %lldx%lldx%lld", static_cast<long long>(a->M), static_cast<long long>(a->N),
+               static_cast<long long>(a->K));
+  if (a->M == 0 || a->N == 0) return 0;
+  B200_REQUIRE(a->scratch && (reinterpret_cast<uintptr_t>(a->scratch) & 255u) == 0, "b200_fp8_linear: scratch");
+  const int M = static_cast<int>(a->M), N = static_cast<int>(a->N), K = static_cast<int>(a->K), dtype = static_cast<int>(a->dtype);
+  char* q = static_cast<char*>(a->scratch);
+  float* scales = reinterpret_cast<float*>(q + (a->M * a->K + 255) / 256 * 256);
+  if (a->block) {
+    const int rc = b200_fp8_quant_group128(a->x, a->ldx, q, K, scales, 1, M, M, K, 1e-10f, dtype, a->stream);
+    return rc ? rc : b200_fp8_gemm_block128(q, K, a->w, a->ldw, scales, 1, M, a->w_scale, a->w_scale_stride, a->bias, a->out,
+                                            a->ldc, M, N, K, dtype, a->stream);
+  }
+  const int rc = b200_fp8_quant_per_token(a->x, a->ldx, q, K, scales, nullptr, M, K, 0, 0.f, dtype, a->stream);
+  return rc ? rc : b200_fp8_gemm_rowcol(q, K, a->w, a->ldw, scales, M > 1 ? 1 : 0, a->w_scale, static_cast<int>(a->w_scale_stride),
+                                        a->bias, a->out, a->ldc, M, N, K, dtype, a->stream);
+}
+
 }  // extern "C"
