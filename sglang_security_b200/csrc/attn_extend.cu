@@ -142,6 +142,7 @@ attn_extend_kernel(const ExtendParams p) {
   const int lane = threadIdx.x & 31;
 
   // ---- work assignment ---------------------------------------------------------------------
+  griddep_wait();
   const int b = blockIdx.z;
   const int ext = p.extend_lens[b];
   const int prefix = p.prefix_lens[b];
@@ -587,7 +588,7 @@ static int launch_extend_inst(const ExtendParams& p, int bs, int max_extend_len,
   dim3 grid(ceil_div(max_extend_len, tok_per_tile), p.Hkv * p.head_tiles, bs);
   {
     ScopedKernelTimer timer("attn_extend", st);
-    kern<<<grid, kExtThreads, C::SMEM_BYTES, st>>>(p);
+    B200_CUDA_OK(launch_kernel(kern, grid, dim3(kExtThreads), C::SMEM_BYTES, st, 1, extend_pdl(), p));
   }
   B200_CHECK_LAUNCH("attn_extend_kernel");
   return 0;

@@ -166,6 +166,7 @@ attn_extend_flat_kernel(const ExtendParams p, int bs, float* ws) {
     tc::tmem_alloc(tmem_slot, 512);
     tc::tmem_relinquish();
   }
+  griddep_wait();                                  // lengths, pages, new rows and the workspace are the launch's before
   // ---- the plan: weight of one head of every request, then this CTA's first position
   {
     int64_t* wsum = reinterpret_cast<int64_t*>(smem);
@@ -649,7 +650,7 @@ static int launch_extend_flat(const ExtendParams& p_in, int bs, float* ws, size_
   note_variant("attn_extend_wide flat d=%d ctas=%d", D, ctas);
   {
     ScopedKernelTimer timer("attn_extend", st);
-    B200_CUDA_OK(launch_kernel(attn_extend_flat_kernel<T, D>, dim3(ctas), dim3(kWideThreads), SMEM, st, 1, 0, p, bs, ws));
+    B200_CUDA_OK(launch_kernel(attn_extend_flat_kernel<T, D>, dim3(ctas), dim3(kWideThreads), SMEM, st, 1, extend_pdl(), p, bs, ws));
     B200_CHECK_LAUNCH("attn_extend_flat_kernel");
     B200_CUDA_OK(launch_kernel(attn_extend_flat_merge_kernel<T, D>, dim3(ctas, D / 16), dim3(256), 0, st, 1, kPdlMerge, p,
                                static_cast<const float*>(ws), ctas));

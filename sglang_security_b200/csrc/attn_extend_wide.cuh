@@ -26,6 +26,9 @@
 
 namespace b200 {
 
+// Extend kernels are launched as dependents of the KV write before them (or what else stands there): their CTAs are placed,
+// and the persistent kernel's barriers and tensor memory ready, when it ends.
+inline int extend_pdl() { return pdl_gemm_family(1 << 20, kPdlAttn); }
 constexpr int kWideThreads = 384;
 constexpr int kWideTile = 128;                     // keys
 constexpr int kWideMinKeys = 1024;                 // shorter requests: attn_extend_kernel
@@ -58,6 +61,7 @@ attn_extend_wide_kernel(const ExtendParams p) {
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
 
+  griddep_wait();
   const int b = blockIdx.z;
   const int S = SPLIT ? p.kv_splits : 1;           // cluster size; every CTA of a cluster has the same query tiles
   const int rank = S > 1 ? static_cast<int>(cluster_ctarank()) : 0;
@@ -494,9 +498,9 @@ static int launch_extend_wide(const ExtendParams& p_in, int bs, int max_extend_l
   {
     ScopedKernelTimer timer("attn_extend", st);
     if (p.kv_splits > 1)
-      B200_CUDA_OK(launch_kernel(attn_extend_wide_kernel<T, D, true>, grid, dim3(kWideThreads), C::SMEM_BYTES, st, p.kv_splits, 0, p));
+      B200_CUDA_OK(launch_kernel(attn_extend_wide_kernel<T, D, true>, grid, dim3(kWideThreads), C::SMEM_BYTES, st, p.kv_splits, extend_pdl(), p));
     else
-      B200_CUDA_OK(launch_kernel(attn_extend_wide_kernel<T, D, false>, grid, dim3(kWideThreads), C::SMEM_BYTES, st, 1, 0, p));
+      B200_CUDA_OK(launch_kernel(attn_extend_wide_kernel<T, D, false>, grid, dim3(kWideThreads), C::SMEM_BYTES, st, 1, extend_pdl(), p));
   }
   B200_CHECK_LAUNCH("attn_extend_wide_kernel");
   return 0;

@@ -185,7 +185,7 @@ int b200_kv_write(const void* k, const void* v, int64_t k_token_stride_bytes,
     if (blocks > 148 * 16) blocks = 148 * 16;
     if (blocks < 1) blocks = 1;
     dim3 grid(static_cast<unsigned>(blocks), 2);
-    lerr = launch_kernel(kv_write_kernel<Vec>, grid, dim3(threads), 0, st, 1, pdl_family(num_tokens, kPdlOther),
+    lerr = launch_kernel(kv_write_kernel<Vec>, grid, dim3(threads), 0, st, 1, pdl_gemm_family(num_tokens, kPdlOther),
                          static_cast<const char*>(k), static_cast<const char*>(v),
                          k_token_stride_bytes, v_token_stride_bytes, static_cast<char*>(k_cache),
                          static_cast<char*>(v_cache), loc, num_tokens, k_row_bytes, v_row_bytes);
@@ -228,13 +228,13 @@ int b200_kv_write_fp8(const void* k, const void* v, int64_t k_token_stride,
   cudaError_t lerr;
   if (dtype == B200_BF16)
     lerr = launch_kernel(kv_write_fp8_kernel<__nv_bfloat16>, grid, dim3(256), 0, st, 1,
-                         pdl_family(num_tokens, kPdlOther), static_cast<const __nv_bfloat16*>(k),
+                         pdl_gemm_family(num_tokens, kPdlOther), static_cast<const __nv_bfloat16*>(k),
                          static_cast<const __nv_bfloat16*>(v), k_token_stride, v_token_stride,
                          static_cast<uint8_t*>(k_cache), static_cast<uint8_t*>(v_cache), loc,
                          num_tokens, row_elems, k_scale, v_scale, has_scale, e5m2);
   else
     lerr = launch_kernel(kv_write_fp8_kernel<__half>, grid, dim3(256), 0, st, 1,
-                         pdl_family(num_tokens, kPdlOther), static_cast<const __half*>(k),
+                         pdl_gemm_family(num_tokens, kPdlOther), static_cast<const __half*>(k),
                          static_cast<const __half*>(v), k_token_stride, v_token_stride,
                          static_cast<uint8_t*>(k_cache), static_cast<uint8_t*>(v_cache), loc,
                          num_tokens, row_elems, k_scale, v_scale, has_scale, e5m2);
