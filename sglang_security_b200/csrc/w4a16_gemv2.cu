@@ -137,12 +137,14 @@ __device__ __forceinline__ uint32_t g2_hmul2(uint32_t a, uint32_t b) {
   return r;
 }
 
-// MT = number of 8-token tiles (1: M <= 8, 2: M <= 16).  CTAS = CTAs per SM.  With two tiles, two CTAs keep six loads a
-// lane in flight (512 bytes each a warp); three keep four, and the partial tile takes the place of x, so that a K slice as
-// long as before fits: for grids that end a wave earlier with them (us, two / three a SM, f16, 9 and 16 tokens, Qwen2.5-32B
-// at TP 2, all four linears: 86.3 / 70.1 and 89.5 / 73.3; Llama-3.1-8B bf16 65.1 / 59.7 and 76.9 / 67.9; where both take
-// one wave, at TP 4, 35.0 / 36.6).
-// 80 registers a thread with three: seven of the eight instances spill 4 to 32 bytes.
+// MT = number of 8-token tiles (1: M <= 8, 2: M <= 16).  CTAS = CTAs per SM: three with one tile; with two tiles two, or
+// three with the partial tile in the place of x, so that a K slice as long as before fits: for grids that end a wave earlier
+// with them (us, two / three a SM, f16, 9 and 16 tokens, Qwen2.5-32B at TP 2, all four linears: 86.3 / 70.1 and 89.5 / 73.3;
+// Llama-3.1-8B bf16 65.1 / 59.7 and 76.9 / 67.9; where both take one wave, at TP 4, 35.0 / 36.6).
+// DEPTH: loads a lane in flight (512 bytes each a warp).  Four, not six: a branch a tile costs more than the depth gives
+// (checks on every tile, all the way: 47 -> 61 us), and a round of four leaves, with groups of 128, nothing or two tiles
+// that need none.  Four linears, us, six and a tail of up to two rounds with checks / this: Qwen2.5-32B at TP 2, f16, 1
+// token 47.2 / 41.2, 8 49.9 / 45.2, 16 73.4 / 71.5; Llama-3.1-8B 45.4 / 41.1, 49.0 / 44.4, 69.8 / 66.8.  Two: 49.9.
 //  SPG = 32-k steps per quantisation group
 // known at compile time (1, 2, 4 = groups of 32, 64, 128: the fold sits at fixed places of the
 // unrolled round, no counters) or 0 = any other group size (run-time step counter).
@@ -150,7 +152,7 @@ template <typename T, int MT, int SPG, int CTAS>
 __global__ void __launch_bounds__(kG2Threads, CTAS)
 w4a16_gemv2_kernel(const Gemv2Params p) {
   using MG = G2Magic<T>;
-  constexpr int DEPTH = MT == 2 && CTAS == 3 ? 4 : 6;
+  constexpr int DEPTH = 4;
   extern __shared__ __align__(128) uint8_t smem[];
   const uint32_t sbase = smem_u32(smem);
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
@@ -340,27 +342,38 @@ w4a16_gemv2_kernel(const Gemv2Params p) {
     int base = 0;
     const uint4* wq = wp + DEPTH * 32;  // the tile DEPTH ahead of the round's first
     uint32_t xround = 0;
-    // steady state: every tile of this round has a successor DEPTH tiles ahead
+    if constexpr (MT == 1) {
+      // steady state: every tile of this round has a successor DEPTH tiles ahead (two token tiles: 1 to 3 % slower with it)
 #pragma unroll 1
-    for (; base + 2 * DEPTH <= nkb; base += DEPTH, wq += DEPTH * 32, xround += DEPTH * 128) {
+      for (; base + 2 * DEPTH <= nkb; base += DEPTH, wq += DEPTH * 32, xround += DEPTH * 128) {
 #pragma unroll
-      for (int j = 0; j < DEPTH; ++j) {
-        const uint4 w = buf[j];
-        buf[j] = g2_ldg_stream(wq + j * 32);
-        tile(w, j, xround);
-      }
-    }
-    // tail: at most two rounds, loads predicated
-#pragma unroll 1
-    for (; base < nkb; base += DEPTH, wq += DEPTH * 32, xround += DEPTH * 128) {
-#pragma unroll
-      for (int j = 0; j < DEPTH; ++j) {
-        if (base + j < nkb) {
+        for (int j = 0; j < DEPTH; ++j) {
           const uint4 w = buf[j];
-          if (base + j + DEPTH < nkb) buf[j] = g2_ldg_stream(wq + j * 32);
+          buf[j] = g2_ldg_stream(wq + j * 32);
           tile(w, j, xround);
         }
       }
+    }
+    // whole rounds: only the loads look at the end
+#pragma unroll 1
+    for (; base + DEPTH <= nkb; base += DEPTH, wq += DEPTH * 32, xround += DEPTH * 128) {
+#pragma unroll
+      for (int j = 0; j < DEPTH; ++j) {
+        const uint4 w = buf[j];
+        if (base + j + DEPTH < nkb) buf[j] = g2_ldg_stream(wq + j * 32);
+        tile(w, j, xround);
+      }
+    }
+    // what is left of a round: two tiles with groups of 128 (a slice is whole groups), else up to DEPTH - 1
+    if constexpr (SPG == 4) {
+      if (base < nkb) {
+        tile(buf[0], 0, xround);
+        tile(buf[1], 1, xround);
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < DEPTH - 1; ++j)
+        if (base + j < nkb) tile(buf[j], j, xround);
     }
   }
   griddep_launch_dependents();

@@ -37,3 +37,15 @@ def test_default_sizes(m, n, k, splits):
 
     _run(m, n, k, 128, torch.float16)
     assert f"splits={splits} " in _lib.last_variant()
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("m", [1, 9])
+@pytest.mark.parametrize("group", [32, 64, 128, 320])
+@pytest.mark.parametrize("blocks", [5, 10, 15, 20, 25, 30, 35, 45])
+def test_ends_of_a_slice(blocks, group, m, dtype, gemv2_cfg):  # noqa: F811
+    """Slices of every length around a round of four 64-k tiles, one and two ranks (a group is whole in a slice)."""
+    for splits in (1, 2):
+        gemv2_cfg(splits)
+        k = blocks * 64 if group != 128 else blocks * 128
+        _run(m, 144, k, group, dtype)
