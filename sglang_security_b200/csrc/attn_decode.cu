@@ -21,6 +21,7 @@
 //   Warps are merged once through shared memory; partials (normalised O, log2-domain LSE) go to
 //   the workspace and are merged by attn_merge_kernel.
 #include <cstdlib>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -486,10 +487,11 @@ attn_decode_mma_kernel(const DecodeParams p) {
   const bool rtt_vec = (p.rtt_stride & 3) == 0 && (reinterpret_cast<uintptr_t>(p.req_to_token) & 15) == 0;
 
   int slot[RPG];
-  auto load_slots = [&](int k) {
-    if (k >= n_my) return;
+  // SAFE: tile k exists and is a whole one, and the page table takes 16-byte loads
+  auto load_slots = [&](int k, auto safe) {
+    if (!safe.value && k >= n_my) return;
     const int pos = start + (warp + k * NW) * NT + crow0;
-    if (rtt_vec && pos + RPG <= end) {
+    if (safe.value || (rtt_vec && pos + RPG <= end)) {
 #pragma unroll
       for (int i = 0; i < RPG / 4; ++i) {
         const int4 v = __ldg(reinterpret_cast<const int4*>(rtt + pos) + i);
@@ -500,8 +502,8 @@ attn_decode_mma_kernel(const DecodeParams p) {
       for (int i = 0; i < RPG; ++i) slot[i] = pos + i < end ? __ldg(rtt + pos + i) : 0;
     }
   };
-  auto issue_tile = [&](int k) {
-    if (k < n_my) {
+  auto issue_tile = [&](int k, auto safe) {
+    if (safe.value || k < n_my) {
       const uint32_t sk = ring + (k % STAGES) * STAGE_BYTES;
 #pragma unroll
       for (int i = 0; i < RPG; ++i) {
@@ -515,15 +517,15 @@ attn_decode_mma_kernel(const DecodeParams p) {
     cp_async_commit();
   };
 
-  load_slots(0);
+  load_slots(0, std::false_type{});
   if (NEW && p.new_k && end == len && warp == (ntiles - 1) % NW) {   // this warp's last tile holds the new token
     store_new_rows<T, D, false, false>(p, b, kvh, lane);
     __syncwarp();
   }
 #pragma unroll
   for (int s = 0; s < STAGES - 1; ++s) {
-    issue_tile(s);
-    load_slots(s + 1);
+    issue_tile(s, std::false_type{});
+    load_slots(s + 1, std::false_type{});
   }
 
   const bool capped = p.logit_cap > 0.f;
@@ -539,9 +541,9 @@ attn_decode_mma_kernel(const DecodeParams p) {
   const uint32_t v_row_off = (((lane >> 3) & 1) * 8 + lx) * ROW_BYTES;  // + kt * 16 * ROW_BYTES
   const int v_y = (lane >> 4) ^ lx;
 
-  for (int it = 0; it < n_my; ++it) {
-    issue_tile(it + STAGES - 1);
-    load_slots(it + STAGES);
+  auto step = [&](int it, auto safe) {
+    issue_tile(it + STAGES - 1, safe);
+    load_slots(it + STAGES, safe);
     cp_async_wait<STAGES - 1>();
     __syncwarp();
 
@@ -568,7 +570,7 @@ attn_decode_mma_kernel(const DecodeParams p) {
 #pragma unroll
         for (int e = 0; e < 4; ++e) s[nt][e] = cap_log2 * exact_tanh_log2(s[nt][e] * inv_cap);
     }
-    if (tok0 + NT > end) {  // tail tile: mask tokens past the end (warp-uniform branch)
+    if (!safe.value && tok0 + NT > end) {  // tail tile: mask tokens past the end (warp-uniform branch)
 #pragma unroll
       for (int nt = 0; nt < NS; ++nt) {
         const int t = tok0 + nt * 8 + (lane & 3) * 2;
@@ -639,7 +641,13 @@ attn_decode_mma_kernel(const DecodeParams p) {
       }
     }
     __syncwarp();  // stage may be refilled by the next iteration's issue
-  }
+  };
+  // Tiles whose successors are whole ones run a copy of the step without their checks (us: 64 x 4096 bf16 166.8 -> 160.9,
+  // 32 x up to 4000 of head size 64 15.6 -> 13.9, 1 x 1500 7.0 -> 6.6; e4m3 64 x 4096 100.3 -> 99.1).
+  int it = 0;
+  if (rtt_vec)
+    for (; it + STAGES + 1 < n_my; ++it) step(it, std::true_type{});
+  for (; it < n_my; ++it) step(it, std::false_type{});
   cp_async_wait<0>();
   if (p.pdl_late) griddep_launch_dependents();
 
