@@ -4,11 +4,36 @@
 //   out[M, N] = x[M, K] . w[N, K]^T (+ bias[N]),  bf16 / f16 operands, fp32 accumulation in TMEM.
 // Same CTA-pair TMA + tcgen05 kernel as the FP8 path (gemm_pair.cuh) with kind::f16; K-major
 // operands, so the reference's [N, K] weight is used as stored.
+#include "fp8_gemm_smallm.cuh"
 #include "gemm_pair.cuh"
 
 namespace b200 {
 
 static WaitCounter wait_counter_registered(tc::wait_counter());
+
+// Decode sizes: the swap-AB kernel with K split over a cluster (fp8_gemm_smallm.cuh), two CTAs an SM, whose weight ring is
+// filled before the CTA is set up; a CTA pair of gemm_pair_kernel has to meet first, and ends with an exchange of 4-byte
+// loads.  Four linears, bf16, us, pair / this: Llama-3.1-8B 1 token 87.7 / 76.7, 16 89.2 / 82.3, 24 90.5 / 86.2; at TP 4 1
+// token 37.1 / 30.9, 24 39.1 / 37.9, 32 38.6 / 39.6; Qwen2.5-32B at TP 2 1 token 94.1 / 84.8.
+constexpr int kDenseSmallMax = 24;
+template <int KIND, typename OutT>
+static int launch_dense_small(const void* x, int64_t ldx, const void* w, int64_t ldw, const GemmEpilogueParams& ep,
+                              cudaStream_t st) {
+  SmallMParams p = {};
+  p.out = ep.out;
+  p.ldc = ep.ldc;
+  p.bias = ep.bias;
+  p.M = ep.M;
+  p.N = ep.N;
+  p.K = ep.K;
+  const bool big = static_cast<int64_t>(ep.N) * ep.K * 2 >= (48ll << 20);
+  if (ep.M > 16) return launch_smallm_ks<32, false, OutT, false, 1, true, KIND>(x, ldx, w, ldw, p, st, "dense_gemm");
+  if (ep.M > 4)
+    return big ? launch_smallm_ks<16, false, OutT, false, 2, true, KIND>(x, ldx, w, ldw, p, st, "dense_gemm")
+               : launch_smallm_ks<16, false, OutT, false, 1, true, KIND>(x, ldx, w, ldw, p, st, "dense_gemm");
+  return big ? launch_smallm_ks<16, false, OutT, false, 2, false, KIND>(x, ldx, w, ldw, p, st, "dense_gemm")
+             : launch_smallm_ks<16, false, OutT, false, 1, false, KIND>(x, ldx, w, ldw, p, st, "dense_gemm");
+}
 
 static int gemm_16bit(const void* x, int64_t ldx, const void* w, int64_t ldw, const void* bias, void* out,
                       int64_t ldc, int M, int N, int K, bool act, float act_pos, float act_neg, int dtype,
@@ -37,6 +62,9 @@ static int gemm_16bit(const void* x, int64_t ldx, const void* w, int64_t ldw, co
   if (act)
     return dtype == B200_BF16 ? launch_gemm_pair<kKindBf16, __nv_bfloat16, true>(x, ldx, w, ldw, ep, st, "dense_gemm")
                               : launch_gemm_pair<kKindF16, __half, true>(x, ldx, w, ldw, ep, st, "dense_gemm");
+  if (M <= kDenseSmallMax)
+    return dtype == B200_BF16 ? launch_dense_small<kKindBf16, __nv_bfloat16>(x, ldx, w, ldw, ep, st)
+                              : launch_dense_small<kKindF16, __half>(x, ldx, w, ldw, ep, st);
   return dtype == B200_BF16 ? launch_gemm_pair<kKindBf16, __nv_bfloat16>(x, ldx, w, ldw, ep, st, "dense_gemm")
                             : launch_gemm_pair<kKindF16, __half>(x, ldx, w, ldw, ep, st, "dense_gemm");
 }

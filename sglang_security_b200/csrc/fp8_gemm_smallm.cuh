@@ -41,6 +41,7 @@ struct SmallMParams {
   const void* bias;
   int M, N, K;
   int kb_per_split;
+  int* wait_error;  // 16-bit kinds: tc::report_gave_up
   int vec4;      // rows of `out` take 8-byte stores
   int pdl_late;  // trigger dependents after the main loop instead of right after the dependency wait
   // Row-parallel fusion (RowParallelLinear.forward, linear.py:1277-1299): when use_comm != 0 the
@@ -95,12 +96,15 @@ struct SmallMCfg {
 // AR: the epilogue reduces across the tensor-parallel group (p.comm); a separate instantiation so
 // the plain kernel's unrolled epilogue carries none of that code (it cost 12-26 % at M = 16-32).
 // PULL: how a split's partials meet, see the epilogue.
-template <int MT, bool BLK, typename OutT, bool AR, int KSUB, bool PULL>
+// KIND: e4m3 operands, or 16-bit ones of the output's type without scales (a 128-byte K block is 64 of them; dense_gemm.cu).
+// The waits of the 16-bit instances are bounded, as in gemm_pair.cuh.
+template <int MT, bool BLK, typename OutT, bool AR, int KSUB, bool PULL, int KIND = kKindFp8>
 __global__ void __launch_bounds__(192, (BLK && MT == 128) ? 1 : 2)
 fp8_gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w,
                        const __grid_constant__ CUtensorMap tmap_x, const SmallMParams p) {
   using C = SmallMCfg<MT, BLK, KSUB>;
   constexpr int NW = C::NW, NX = C::NX, NBUF = C::NBUF;
+  constexpr int EK = 128 / GemmKindTraits<KIND>::ELT;   // elements of a 128-byte K block
   extern __shared__ __align__(1024) uint8_t smem_raw[];  // SWIZZLE_128B tiles need 1024-byte alignment
   const uint32_t smem_base = smem_u32(smem_raw);
   const uint32_t ring_x = smem_base + NW * C::W_BYTES;
@@ -125,7 +129,7 @@ fp8_gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w,
   const uint32_t rank = cluster_ctarank();
   const uint32_t S = cluster_nctarank();
   const int n_tile = blockIdx.x / S;
-  const int num_kb = ceil_div(p.K, 128 * C::KS);
+  const int num_kb = ceil_div(p.K, EK * C::KS);
   const int kb0 = min(num_kb, static_cast<int>(rank) * p.kb_per_split);
   const int kb1 = min(num_kb, kb0 + p.kb_per_split);
   const int nkb = kb1 - kb0;
@@ -139,16 +143,23 @@ fp8_gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w,
     const uint32_t sw = smem_base + s * C::W_BYTES;
 #pragma unroll
     for (int u = 0; u < C::KS; ++u)
-      tc::tma_load_2d_hint(sw + u * C::W_SUB, &tmap_w, full_bar(s), ((kb0 + i) * C::KS + u) * 128,
+      tc::tma_load_2d_hint(sw + u * C::W_SUB, &tmap_w, full_bar(s), ((kb0 + i) * C::KS + u) * EK,
                            n_tile * 128, tc::kEvictFirst);
   };
   auto issue_x = [&](int i) {
 #pragma unroll
     for (int u = 0; u < C::KS; ++u)
       tc::tma_load_2d_hint(ring_x + (i % NX) * C::X_BYTES + u * C::X_SUB, &tmap_x, full_bar(i % NW),
-                           ((kb0 + i) * C::KS + u) * 128, 0, tc::kEvictLast);
+                           ((kb0 + i) * C::KS + u) * EK, 0, tc::kEvictLast);
   };
-  auto wait_mma_done = [&](int i) { tc::mbar_wait(empty_bar(i % NW), (i / NW) & 1u); };
+  __shared__ uint32_t gave_up_s;
+  const uint32_t gave_up = smem_u32(&gave_up_s);
+  bool dead = false;
+  auto wait_bar = [&](uint32_t bar, uint32_t parity) {
+    if constexpr (KIND == kKindFp8) tc::mbar_wait(bar, parity);
+    else tc::mbar_wait_bounded(bar, parity, dead, gave_up);
+  };
+  auto wait_mma_done = [&](int i) { wait_bar(empty_bar(i % NW), (i / NW) & 1u); };
 
   if (warp == 0 && tc::elect_one()) {
     if ((smem_base & 1023u) != 0) __trap();
@@ -162,6 +173,7 @@ fp8_gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w,
       tc::mbar_init(tfull_bar(a), 1);
       tc::mbar_init(tempty_bar(a), 4);
     }
+    gave_up_s = 0;
     tc::fence_barrier_init();
     // Fill the weight ring BEFORE the CTA-wide setup barrier AND before the programmatic-launch
     // dependency wait: weights are never written during a step, so their first NW x 16 KiB are in
@@ -200,11 +212,11 @@ fp8_gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w,
     if (p.pdl_late) griddep_launch_dependents();  // every load of this CTA has been issued
   } else if (warp == 1) {
     // ===================== MMA issuer ==========================================================
-    constexpr uint32_t idesc = tc::make_idesc(0, 0, 128, MT, 0, 0);
+    constexpr uint32_t idesc = tc::make_idesc(GemmKindTraits<KIND>::FMT, GemmKindTraits<KIND>::FMT, 128, MT, 0, 0);
     for (int i = 0; i < nkb; ++i) {
       const int buf = BLK ? i % NBUF : 0;
-      if (BLK) tc::mbar_wait(tempty_bar(buf), ((i / NBUF) & 1u) ^ 1u);
-      tc::mbar_wait(full_bar(i % NW), (i / NW) & 1u);
+      if (BLK) wait_bar(tempty_bar(buf), ((i / NBUF) & 1u) ^ 1u);
+      wait_bar(full_bar(i % NW), (i / NW) & 1u);
       tc::tc_fence_after();
       const uint64_t adesc = tc::make_smem_desc_sw128(smem_base + (i % NW) * C::W_BYTES, 1024, 16);
       const uint64_t bdesc = tc::make_smem_desc_sw128(ring_x + (i % NX) * C::X_BYTES, 1024, 16);
@@ -215,8 +227,9 @@ fp8_gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w,
 #pragma unroll
           for (int k = 0; k < 4; ++k) {   // 32 bytes of K further on: 2 in the address field
             const uint32_t accum = BLK ? (k != 0) : ((i != 0) | (u != 0) | (k != 0));
-            tc::mma_f8f6f4(tmem_d, adesc + (u * C::W_SUB >> 4) + 2 * k, bdesc + (u * C::X_SUB >> 4) + 2 * k, idesc,
-                           accum ? 1u : 0u);
+            const uint64_t da = adesc + (u * C::W_SUB >> 4) + 2 * k, db = bdesc + (u * C::X_SUB >> 4) + 2 * k;
+            if constexpr (KIND == kKindFp8) tc::mma_f8f6f4(tmem_d, da, db, idesc, accum ? 1u : 0u);
+            else tc::mma_f16(tmem_d, da, db, idesc, accum ? 1u : 0u);
           }
         }
         tc::mma_commit(empty_bar(i % NW));
@@ -371,7 +384,7 @@ fp8_gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w,
         if (m < p.M) emit(m, acc[m]);
     } else {
       if (has_work) {
-        tc::mbar_wait(tfull_bar(0), 0);
+        wait_bar(tfull_bar(0), 0);
         tc::tc_fence_after();
       }
       if (!PULL && S > 1) {
@@ -474,7 +487,10 @@ fp8_gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w,
   }
   tc::tc_fence_before();
   __syncthreads();
-  if (warp == 1) tc::tmem_dealloc(tmem_base, C::TCOLS);
+  if (warp == 1) {
+    if constexpr (KIND != kKindFp8) tc::report_gave_up(gave_up, p.wait_error);
+    tc::tmem_dealloc(tmem_base, C::TCOLS);
+  }
 }
 
 // Host side --------------------------------------------------------------------------------------
@@ -486,16 +502,18 @@ bool smallm_forced();                      // threshold set explicitly through t
 bool comm_can_fuse(const void* comm, int M, int N);
 int comm_all_reduce_rows(void* comm, void* out, int64_t ldc, int M, int N, int dtype, void* stream);
 
-template <int MT, bool BLK, typename OutT, bool AR, int KSUB, bool PULL>
+template <int MT, bool BLK, typename OutT, bool AR, int KSUB, bool PULL, int KIND = kKindFp8>
 int launch_smallm_ks(const void* x, int64_t ldx, const void* w, int64_t ldw, SmallMParams p,
                      cudaStream_t st, const char* timer_name) {
   using C = SmallMCfg<MT, BLK, KSUB>;
   CUtensorMap tw, tx;
-  int rc = make_tmap_2d(&tw, w, p.N, p.K, ldw, 128, 128, 1, true);
+  constexpr int ELT = GemmKindTraits<KIND>::ELT, EK = 128 / ELT;
+  int rc = make_tmap_2d(&tw, w, p.N, p.K, ldw * ELT, 128, EK, ELT, true);
   if (rc) return rc;
-  rc = make_tmap_2d(&tx, x, p.M, p.K, ldx, MT, 128, 1, false);
+  rc = make_tmap_2d(&tx, x, p.M, p.K, ldx * ELT, MT, EK, ELT, false);
   if (rc) return rc;
-  auto kern = fp8_gemm_smallm_kernel<MT, BLK, OutT, AR, KSUB, PULL>;
+  if (KIND != kKindFp8 && (rc = wait_error_arm(timer_name, &p.wait_error))) return rc;
+  auto kern = fp8_gemm_smallm_kernel<MT, BLK, OutT, AR, KSUB, PULL, KIND>;
   static bool attr_done = false;
   if (!attr_done) {
     B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -504,8 +522,8 @@ int launch_smallm_ks(const void* x, int64_t ldx, const void* w, int64_t ldw, Sma
   }
   const int n_tiles = ceil_div(p.N, 128);
   // the split factor is chosen on 128-wide K blocks as before; slices are whole ring blocks
-  int S = smallm_pick_splits(n_tiles, ceil_div(p.K, 128));
-  const int num_kb = ceil_div(p.K, 128 * C::KS);
+  int S = smallm_pick_splits(n_tiles, ceil_div(p.K, EK));
+  const int num_kb = ceil_div(p.K, EK * C::KS);
   if (S > num_kb) S = num_kb;
   p.kb_per_split = ceil_div(num_kb, S);
   p.pdl_late = pdl_late();
@@ -516,7 +534,10 @@ int launch_smallm_ks(const void* x, int64_t ldx, const void* w, int64_t ldw, Sma
     (void)cudaGetLastError();
     ctas_per_sm = 0;
   }
-  note_variant("fp8_smallm mt=%d blk=%d ar=%d ksub=%d splits=%d tiles=%d ctas_per_sm=%d", MT,
+  if (KIND != kKindFp8)
+    note_variant("gemm_tn kind=%d smallm mt=%d ksub=%d splits=%d tiles=%d ctas_per_sm=%d", KIND, MT, KSUB, S, n_tiles, ctas_per_sm);
+  else
+    note_variant("fp8_smallm mt=%d blk=%d ar=%d ksub=%d splits=%d tiles=%d ctas_per_sm=%d", MT,
                BLK ? 1 : 0, AR ? 1 : 0, KSUB, S, n_tiles, ctas_per_sm);
   {
     ScopedKernelTimer timer(timer_name, st);
