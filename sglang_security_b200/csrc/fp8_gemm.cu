@@ -219,14 +219,14 @@ static int fp8_gemm_rowcol_impl(const void* a, int64_t lda, const void* b, int64
   ep.N = N;
   ep.K = K;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // Decode regime: weight streaming, swap-AB + cluster split-K, two CTAs per SM.  Against the CTA-pair kernel (us, qkv /
-  // o / gate_up / down of Llama-3.1-8B): this one at 32 tokens 8.3 / 7.3 / 19.8 / 12.7, the pair kernel at 64 tokens 8.9 /
-  // 8.2 / - / 15.1, where this one's accumulators halve the CTAs per SM.
+  // Decode regime: weight streaming, swap-AB + cluster split-K, two CTAs per SM.  Against the CTA-pair kernel (four linears
+  // with quantisers, us, pair / this): Llama-3.1-8B 40 tokens 65.8 / 63.7, 48 67.3 / 65.3, 64 67.3 / 67.8; at TP 4 40 tokens
+  // 37.0 / 35.3, 48 37.0 / 37.0, 64 36.8 / 41.1; Qwen2.5-32B at TP 2 40 tokens 68.3 / 68.0, 48 68.8 / 67.8.
   const bool fuse_ar = comm_can_fuse(comm, M, N);
   // A weight with more 128-row tiles than SMs (gate_up 28672x4096) streams best here up to 64 tokens: 21.8 us at 64,
   // the pair kernel 23.5 at 128.
   const bool wide = ceil_div(N, 128) > device_sm_count();
-  if (fuse_ar || (M <= smallm_max_m() && (M <= 32 || (wide && M <= 64) || smallm_forced()))) {
+  if (fuse_ar || (M <= smallm_max_m() && (M <= 48 || (wide && M <= 64) || smallm_forced()))) {
     SmallMParams sp = {};
     if (fuse_ar) {
       sp.use_comm = 1;

@@ -47,3 +47,19 @@ def test_rows_that_wide_stores_do_not_fit(m, n, k, pad, shift, block):
     _lib.check(rc, "fp8 gemm")
     _check(out[:, :n], ref + bias.double(), mags + bias.double().abs(), k)
     assert bool((out[:, n:] == 7.0).all()) and bool((whole[:shift] == 7.0).all()) and bool((whole[shift + m * ld:] == 7.0).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("m", [33, 47, 48, 49])
+@pytest.mark.parametrize("n,k", [(136, 4096), (6000, 1040), (520, 14336)])
+def test_rowcol_up_to_48_tokens(m, n, k, dtype):
+    from sglang_security_b200 import _lib
+    from sglang_security_b200.layers.quantization.fp8_kernel import fp8_scaled_mm
+
+    a, b, sa, sb, bias, _, _ = _problem(m, n, k, dtype)
+    ts, cs = sa[:, :1].contiguous(), sb[:, 0].repeat_interleave(128)[:n].contiguous()
+    x, w = a.double() * ts.double(), b.double() * cs.double()[:, None]
+    out = fp8_scaled_mm(a, b.t(), ts, cs, dtype, bias)
+    assert ("smallm" in _lib.last_variant()) == (m <= 48)
+    _check(out, x @ w.t() + bias.double(), x.abs() @ w.abs().t() + bias.double().abs(), k)
+    assert torch.equal(out, fp8_scaled_mm(a, b.t(), ts, cs, dtype, bias))
