@@ -402,23 +402,9 @@ int b200_fp8_quant_group128(const void* x, int64_t ldx, void* q, int64_t ldq, fl
     const unsigned total = static_cast<unsigned>(rows) * gpr;
     const int64_t xo = static_cast<int64_t>(m0) * ldx, qo = static_cast<int64_t>(m0) * ldq;
     float* sc = scales + static_cast<int64_t>(m0) * scale_row_stride;
-    // four groups per lane once that still leaves every SM its eight blocks, one where blocks are scarce
-    const bool many = total >= static_cast<unsigned>(device_sm_count()) * 8u * 64u;
-    const unsigned blocks = (total + (many ? 63u : 15u)) / (many ? 64u : 16u);
-    const char* ev = getenv("GQ");
-    if (ev && *ev != '0' && rows <= 65535 * 32) {
-      const int gpt = *ev - '0';
-#define LAUNCH_ROWS(T, GPT)                                                                                                 \
-  B200_CUDA_OK(launch_kernel(fp8_quant_group128_rows_kernel<T, GPT>, dim3(ceil_div(gpr, GPT), ceil_div(rows, 32)), dim3(256), 0, \
-                             st, 1, getenv("GP") ? kPdlQuant : pdl_family(M, kPdlQuant), static_cast<const T*>(x) + xo, ldx, static_cast<uint8_t*>(q) + qo, \
-                             ldq, sc, scale_row_stride, scale_col_stride, rows, gpr, eps))
-      if (dtype == B200_BF16) { if (gpt == 1) LAUNCH_ROWS(__nv_bfloat16, 1); else if (gpt == 2) LAUNCH_ROWS(__nv_bfloat16, 2); else LAUNCH_ROWS(__nv_bfloat16, 4); }
-      else { if (gpt == 1) LAUNCH_ROWS(__half, 1); else if (gpt == 2) LAUNCH_ROWS(__half, 2); else LAUNCH_ROWS(__half, 4); }
-      continue;
-    }
 #define LAUNCH_GROUP(KERNEL, BLOCKS)                                                                                  \
-  B200_CUDA_OK(launch_kernel(KERNEL, dim3(BLOCKS), dim3(256), 0, st, 1, pdl_family(M, kPdlQuant), static_cast<const T*>(x) + xo, ldx,       \
-                             static_cast<uint8_t*>(q) + qo, ldq, sc, scale_row_stride, scale_col_stride, rows, gpr, eps))
+  B200_CUDA_OK(launch_kernel(KERNEL, dim3(BLOCKS), dim3(256), 0, st, 1, pdl_family(M, kPdlQuant),                     \
+                             static_cast<const T*>(x) + xo, ldx, static_cast<uint8_t*>(q) + qo, ldq, sc, scale_row_stride, scale_col_stride, rows, gpr, eps))
     auto launch = [&](auto type) -> int {
       using T = decltype(type);
       if (total >= 65536) LAUNCH_GROUP((fp8_quant_group128_rows_kernel<T, 2>), ceil_div(gpr, 2) * ceil_div(rows, 32));
