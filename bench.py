@@ -317,7 +317,7 @@ def run_b200(args):
     d_ids, d_pos, d_lens, d_loc = h_ids.to(dev), h_pos.to(dev), h_lens.to(dev), h_loc.to(dev)
     d_req = torch.arange(bs, dtype=torch.int64, device=dev)
     d_out = torch.zeros((bs,), dtype=torch.int64, device=dev)
-    fb = model.make_forward_batch(bs, d_req, d_lens, d_loc, bs * ctx)
+    fb = model.make_forward_batch(bs, d_req, d_lens, d_loc, bs * ctx, own_slots=True)
 
     def step():
         model.forward(d_ids, d_pos, fb, d_out)

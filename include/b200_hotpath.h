@@ -43,6 +43,10 @@ enum b200_dtype {
  * byte (sign | 0x7c), NaN -> sign | 0x7f.  The e5m2 decode kernel has no in-kernel tail: a ticket
  * buffer passed to the _fused entry point is ignored (one merge / merge+quantise launch).        */
 #define B200_KV_FP8_E5M2 0x100
+/* Flag on the dtype argument of b200_attn_decode_layer / _fp8kv_layer: a decode batch as schedulers build them, every entry
+ * another request that was given a slot of its own: entry b's page table names loc[b] at position seq_lens[b] - 1 or not at
+ * all, and no other entry's new slot within its length. */
+#define B200_OWN_SLOTS 0x200
 
 /* ---- library ---------------------------------------------------------- */
 int b200_version(void);
@@ -142,9 +146,9 @@ int b200_attn_decode(const void* q, int64_t q_stride, const void* k_cache, const
                      void* workspace, size_t workspace_bytes, int num_splits, void* stream);
 
 /* A layer's decode in one call: entry b's new K/V row (k, v [bs, Hkv, D] in the dtype of q, token strides in elements) goes
- * to slot loc[b] of the pool, then attention as b200_attn_decode / _fused (tickets, q_out and q_scales may be NULL).  The
- * split kernel stores the rows itself, so a request's page table may name its own new slot but none that another request
- * of the batch is given in this call.  _fp8kv_: rows quantised as b200_kv_write_fp8 does (divided by the scales where
+ * to slot loc[b] of the pool, then attention as b200_attn_decode / _fused (tickets, q_out and q_scales may be NULL).  All
+ * rows are in the pool before any is read, as with b200_kv_write before it; with B200_OWN_SLOTS in dtype the split kernel
+ * stores them itself, entry by entry.  _fp8kv_: rows quantised as b200_kv_write_fp8 does (divided by the scales where
  * has_scale), then b200_attn_decode_fp8kv / _fused.  k NULL: the rows are in the pool.
  * pieces > 0 (at least bs, at most 128 requests, no tail): the batch is cut into that many pieces at most, of about equal
  * length, instead of num_splits a request (b200_attn_decode_pieces: how many, 0 where splits serve the batch); workspace from b200_attn_decode_pieces_workspace_bytes, 16-byte aligned. */

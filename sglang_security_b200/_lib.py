@@ -17,6 +17,7 @@ _lib = None
 # dtype codes (enum b200_dtype)
 BF16, F16, F32, FP8_E4M3 = 0, 1, 2, 3
 KV_FP8_E5M2 = 0x100  # B200_KV_FP8_E5M2: flag on the dtype argument of the FP8-KV-pool entry points
+OWN_SLOTS = 0x200    # B200_OWN_SLOTS: flag on the dtype argument of b200_attn_decode_layer / _fp8kv_layer
 
 # b200_extend_layer_args: 8-byte fields in the order of the header
 EXTEND_LAYER_ARGS = struct.Struct("=Pq2PqPqPq2P3P2P2qPqP2qP7q3q4dqP".replace("P", "Q"))

@@ -60,13 +60,13 @@ struct DecodeParams {
   const void* gate;
   int64_t gate_stride;
   // b200_attn_decode_layer: entry b's new K/V row [Hkv, D] in T, stored to slot loc[b] of the pool before it is read
-  // (null: the pool holds it already)
+  // (null: the pool holds it already); new_all: every CTA stores the rows of all entries (see store_new_rows)
   const void* new_k;
   const void* new_v;
   int64_t new_k_stride, new_v_stride;
   const int64_t* loc;
   float k_scale_w, v_scale_w;   // FP8 pool: divisors of the stored rows, where scale_new
-  int scale_new;
+  int scale_new, new_all;
   // PIECES instances: the batch is cut into this many pieces at most (decode_piece); grid.x is the piece
   int pieces;
   int2* plan;                   // [bs] first partial row and count of a request, for the merge
@@ -229,12 +229,19 @@ __device__ __forceinline__ DecodePiece decode_piece(const int64_t* seq_lens, int
   return out;
 }
 
-// One warp stores entry b's new K and V rows of one kv head to the pool, 16 bytes of the source a lane and pass.  The caller
-// synchronises the warp before it requests the tile that holds the new token; other CTAs read other slots (a request's page
-// table names no slot that another request of the batch is being given).
-// A KV write launch of its own cost a dependent launch of ~2 us in front of every layer's attention, with 1 to 64 requests
-// (us, 32 / 8 heads of 128, bf16: 1 x 1000 10.4 -> 8.4, 8 x 1000 14.4 -> 12.4, 64 x 300 14.5 -> 12.4, 64 x 3000 101.3 ->
-// 100.5; 1.086 x over 110 batches, none slower).  The store's latency hides beside the page table's.
+// One warp stores entry b's new K and V rows of one kv head to the pool, 16 bytes of the source a lane and pass.  A KV write
+// launch of its own costs 0.5 to 1.5 us in front of every layer's attention; the store's latency hides beside the page
+// table's.  Two forms, and who may read a new slot in the same launch differs:
+//  own slots   (the caller says so): entry b's page table names loc[b] at position seq_lens[b] - 1 or nowhere, and no other
+//              entry's new slot.  The warp whose last tile holds the new token stores the row, nothing else reads it.
+//  new_all     any page table (two positions of one request as two entries, a fork of a request beside it): the warps of
+//              every CTA store the rows of all entries, and the CTA synchronises before it reads the pool.  CTAs store the
+//              same bytes, so what a CTA reads behind its own store does not depend on the others.  Up to kNewRowsAll
+//              entries; beyond, the stores cost what the write launch does.
+// us, ten calls in a graph, own slots / new_all / write launch, 32 / 8 heads of 128, bf16: 1 x 1500 6.62 / 6.59 / 7.39,
+// 2 x 1500 7.82 / 8.20 / 8.63, 4 x 1000 8.22 / 8.46 / 9.25, 8 x 1000 10.29 / 11.09 / 11.31, 16 x 1024 13.03 / 15.14 / 14.16,
+// 64 x 300 11.59 / 19.49 / 12.64, 64 x 4096 160.3 / 169.8 / 161.9; e4m3 27 x up to 6000 42.1 / 46.9 / 43.6.
+constexpr int kNewRowsAll = 4;
 template <typename T, int D, bool FP8, bool E5M2>
 __device__ __forceinline__ void store_new_rows(const DecodeParams& p, int b, int kvh, int lane) {
   constexpr int CPR = D / 8;
@@ -518,9 +525,14 @@ attn_decode_mma_kernel(const DecodeParams p) {
   };
 
   load_slots(0, std::false_type{});
-  if (NEW && p.new_k && end == len && warp == (ntiles - 1) % NW) {   // this warp's last tile holds the new token
-    store_new_rows<T, D, false, false>(p, b, kvh, lane);
-    __syncwarp();
+  if (NEW && p.new_k) {
+    if (p.new_all) {
+      for (int i = warp; i < p.bs; i += NW) store_new_rows<T, D, false, false>(p, i, kvh, lane);
+      __syncthreads();
+    } else if (end == len && warp == (ntiles - 1) % NW) {   // this warp's last tile holds the new token
+      store_new_rows<T, D, false, false>(p, b, kvh, lane);
+      __syncwarp();
+    }
   }
 #pragma unroll
   for (int s = 0; s < STAGES - 1; ++s) {
@@ -1163,15 +1175,19 @@ struct DecodeNewRows {
   int64_t k_stride, v_stride;
   const int64_t* loc;
   int has_scale;
+  int own_slots;
 };
 
-// The split kernel stores the rows itself where 16-byte pieces of a head fit them and it is not the instance with the
-// in-kernel tail; else they are written by a launch of their own before it.
+// The split kernel stores the rows itself where 16-byte pieces of a head fit them, it is not the instance with the
+// in-kernel tail, and either no entry reads another's new slot or the entries are few (store_new_rows); else they are
+// written by a launch of their own before it, which takes pools without gaps between the rows only.
 static int apply_new_rows(DecodeParams& p, const DecodeNewRows* rows, int D, int dtype, bool fp8, int e5m2, float k_scale,
                           float v_scale, void* stream, const char* who) {
   if (!rows) return 0;
   B200_REQUIRE(rows->k && rows->v && rows->loc, "%s: null pointer", who);
-  if (!p.tickets && aligned16(rows->k) && aligned16(rows->v) && rows->k_stride % 8 == 0 && rows->v_stride % 8 == 0) {
+  const bool dense = p.kv_row_stride == static_cast<int64_t>(p.Hkv) * D;
+  if (!p.tickets && aligned16(rows->k) && aligned16(rows->v) && rows->k_stride % 8 == 0 && rows->v_stride % 8 == 0 &&
+      (rows->own_slots || p.bs <= kNewRowsAll || !dense)) {
     p.new_k = rows->k;
     p.new_v = rows->v;
     p.new_k_stride = rows->k_stride;
@@ -1180,9 +1196,10 @@ static int apply_new_rows(DecodeParams& p, const DecodeNewRows* rows, int D, int
     p.k_scale_w = k_scale;
     p.v_scale_w = v_scale;
     p.scale_new = rows->has_scale;
+    p.new_all = !rows->own_slots;
     return 0;
   }
-  B200_REQUIRE(p.kv_row_stride == static_cast<int64_t>(p.Hkv) * D, "%s: pool rows of %lld elements for %d heads", who,
+  B200_REQUIRE(dense, "%s: pool rows of %lld elements for %d heads", who,
                static_cast<long long>(p.kv_row_stride), p.Hkv);
   void *kc = const_cast<void*>(p.k_cache), *vc = const_cast<void*>(p.v_cache);
   const int row = p.Hkv * D;
@@ -1635,7 +1652,8 @@ int b200_attn_decode_layer(const void* k, int64_t k_stride, const void* v, int64
                            int pieces, void* tickets, size_t ticket_bytes, void* q_out, int64_t q_out_stride, float* q_scales,
                            void* stream) {
   const b200::DecodeTail tail = {tickets, ticket_bytes, q_out, q_out_stride, q_scales};
-  const b200::DecodeNewRows rows = {k, v, k_stride, v_stride, loc, 0};
+  const b200::DecodeNewRows rows = {k, v, k_stride, v_stride, loc, 0, dtype & B200_OWN_SLOTS};
+  dtype &= ~B200_OWN_SLOTS;
   return attn_decode_impl(q, q_stride, k_cache, v_cache, kv_row_stride, o, o_stride, req_to_token, req_to_token_stride,
                           req_pool_indices, seq_lens, bs, Hq, Hkv, D, Dv, scale, logit_cap, dtype, workspace, workspace_bytes,
                           num_splits, stream, tickets || q_out ? &tail : nullptr, nullptr, nullptr, 0, k ? &rows : nullptr, pieces);
@@ -1650,7 +1668,8 @@ int b200_attn_decode_fp8kv_layer(const void* k, int64_t k_stride, const void* v,
                                  void* tickets, size_t ticket_bytes, void* q_out, int64_t q_out_stride, float* q_scales,
                                  void* stream) {
   const b200::DecodeTail tail = {tickets, ticket_bytes, q_out, q_out_stride, q_scales};
-  const b200::DecodeNewRows rows = {k, v, k_stride, v_stride, loc, has_scale};
+  const b200::DecodeNewRows rows = {k, v, k_stride, v_stride, loc, has_scale, dtype & B200_OWN_SLOTS};
+  dtype &= ~B200_OWN_SLOTS;
   return attn_decode_fp8kv_impl(q, q_stride, k_cache, v_cache, kv_row_stride, o, o_stride, req_to_token, req_to_token_stride,
                                 req_pool_indices, seq_lens, bs, Hq, Hkv, D, Dv, scale, logit_cap, k_scale, v_scale, dtype,
                                 workspace, workspace_bytes, num_splits, stream, tickets || q_out ? &tail : nullptr, k ? &rows : nullptr, pieces);

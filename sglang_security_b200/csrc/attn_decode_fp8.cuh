@@ -188,9 +188,14 @@ attn_decode_fp8kv_kernel(const DecodeParams p) {
   };
 
   load_slots(0, std::false_type{});
-  if (NEW && p.new_k && end == len && warp == (ntiles - 1) % NW) {   // this warp's last tile holds the new token
-    store_new_rows<T, D, true, E5M2>(p, b, kvh, lane);
-    __syncwarp();
+  if (NEW && p.new_k) {
+    if (p.new_all) {
+      for (int i = warp; i < p.bs; i += NW) store_new_rows<T, D, true, E5M2>(p, i, kvh, lane);
+      __syncthreads();
+    } else if (end == len && warp == (ntiles - 1) % NW) {   // this warp's last tile holds the new token
+      store_new_rows<T, D, true, E5M2>(p, b, kvh, lane);
+      __syncwarp();
+    }
   }
 #pragma unroll
   for (int s = 0; s < STAGES - 1; ++s) {

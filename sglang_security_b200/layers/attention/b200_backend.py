@@ -6,9 +6,10 @@ implementation of the same interface, triton_backend.py:151-835).  It indexes
 `req_to_token_pool.req_to_token` and the `MHATokenToKVPool` buffers in place (layouts unchanged)
 and calls the sm_100a kernels through the C-ABI (include/b200_hotpath.h):
 
-  forward_decode : b200_kv_write -> b200_attn_decode_fused (split-KV gather kernel whose last CTA per
-                   request merges the splits and, on request, quantises the row for o_proj);
-                   B200_ATTN_FUSED_TAIL=0 restores split kernel + merge kernel
+  forward_decode : b200_attn_decode_layer / _fp8kv_layer: pool write of the new rows, split-KV gather kernel, merge of the
+                   splits (which on request quantises the row for o_proj).  A ForwardBatch with own_slots set says that
+                   no entry reads another's new slot; its rows are stored by the split kernel itself.
+                   B200_ATTN_FUSED_TAIL=0: without the quantiser in the merge
   forward_extend : b200_extend_layer_planned: pool write, 16-bit copy of an FP8 pool's rows, attention (tcgen05
                    prefix rectangle + causal triangle) in one native call.  Short extends are bound by the host: 64 fresh
                    tokens took 62 us a call in three native calls with torch's Stream objects, 37 in one; behind an
@@ -286,7 +287,7 @@ class B200AttnBackend(AttentionBackend):
         v_cache = pool.get_value_buffer(layer.layer_id)
         rows = None
         if save_kv_cache:
-            # one new row a request: the attention kernel stores it itself
+            # one new row an entry: stored by the attention call
             if bs and forward_batch.out_cache_loc.numel() == bs:
                 rows = self._new_rows(q.dtype, k, v, k_cache, v_cache, pool, forward_batch.out_cache_loc, hkv, d)
             if rows is None:
@@ -320,7 +321,10 @@ class B200AttnBackend(AttentionBackend):
                 if (ks is None) != (vs is None):
                     raise _lib.B200Error("forward_decode: k_scale and v_scale must be given together")
                 new = new + (0 if ks is None else 1,)
-        common = common + (_lib.kv_dtype_code(q.dtype, k_cache.dtype), _lib.ptr(ws),
+        dtype = _lib.kv_dtype_code(q.dtype, k_cache.dtype)
+        if new is not None and getattr(forward_batch, "own_slots", False):
+            dtype |= _lib.OWN_SLOTS
+        common = common + (dtype, _lib.ptr(ws),
                            0 if ws is None else ws.numel(), md.num_splits)
         layer_fn = self.lib.b200_attn_decode_fp8kv_layer if fp8kv else self.lib.b200_attn_decode_layer
         # the tail only pays when it replaces a launch: the merge (splits > 1) or the quantiser

@@ -94,6 +94,8 @@ def prepare(items: List[StepItem], req_to_token_pool, allocator, token_to_kv_poo
                       extend_start_loc=ext_start, extend_seq_lens_cpu=ext, extend_prefix_lens_cpu=pre,
                       extend_num_tokens=total, req_to_token_pool=req_to_token_pool,
                       token_to_kv_pool=token_to_kv_pool)
+    # the new slots are fresh from the allocator: only the rows of req_to_token that were just written name them
+    fb.own_slots = len({it.req.req_pool_idx for it in items}) == bs
     fb.tok_pos = positions.to(torch.int32)
     fb.tok_b = tok_b
     fb.ext_start = ext_start

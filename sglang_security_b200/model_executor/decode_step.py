@@ -188,12 +188,14 @@ class B200DecodeStep:
                 + bs * ctx * self.kv_bytes_per_token() + bs * ctx * 4 * self.layers_n)
 
     # ------------------------------------------------------------------ forward
-    def make_forward_batch(self, bs, req_pool_indices, seq_lens, out_cache_loc, seq_lens_sum):
+    def make_forward_batch(self, bs, req_pool_indices, seq_lens, out_cache_loc, seq_lens_sum, own_slots=False):
+        """own_slots: every entry is another request with a new slot of its own (ForwardBatch.own_slots)."""
         return ForwardBatch(forward_mode=ForwardMode.DECODE, batch_size=bs,
                             req_pool_indices=req_pool_indices, seq_lens=seq_lens,
                             out_cache_loc=out_cache_loc, seq_lens_sum=seq_lens_sum,
                             req_to_token_pool=self.req_to_token_pool,
-                            token_to_kv_pool=self.token_to_kv_pool, attn_backend=self.attn_backend)
+                            token_to_kv_pool=self.token_to_kv_pool, attn_backend=self.attn_backend,
+                            own_slots=own_slots)
 
     def forward(self, input_ids, positions, forward_batch, out_token_ids) -> None:
         """One decode step; the greedy next-token ids land in `out_token_ids` (int64 [bs])."""

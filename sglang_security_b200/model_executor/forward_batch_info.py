@@ -78,4 +78,7 @@ class ForwardBatch:
     max_seq_len: int = 0
     state_pool: Any = None
     encoder_lens: Optional[torch.Tensor] = None
+    # DECODE: whoever builds the batch says that every entry is another request with a new slot of its own, which its page
+    # table names last and no other entry's names.  The attention kernel then stores the new rows itself.
+    own_slots: bool = False
     extra: dict = field(default_factory=dict)

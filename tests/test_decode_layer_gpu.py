@@ -49,7 +49,7 @@ def _run(monkeypatch, own, heads, act, pool_dtype, lens, splits, scales, pad, pi
     fb = ForwardBatch(forward_mode=ForwardMode.DECODE, batch_size=bs,
                       req_pool_indices=torch.arange(bs, dtype=torch.int64, device=DEV), seq_lens=t.to(DEV),
                       out_cache_loc=torch.stack(loc), seq_lens_sum=sum(lens), seq_lens_cpu=t, req_to_token_pool=rtp,
-                      token_to_kv_pool=kvp, attn_backend=backend)
+                      token_to_kv_pool=kvp, attn_backend=backend, own_slots=True)
     backend.init_forward_metadata(fb)
     if pieces:
         backend.forward_metadata.pieces = pieces
