@@ -21,6 +21,12 @@ def _check_2d_cuda(x: torch.Tensor, what: str):
         raise _lib.B200Error(f"{what}: expected a 2-D tensor with contiguous rows")
 
 
+def _check_on_device(what: str, *operands: Optional[torch.Tensor]):
+    for t in operands:
+        if t is not None and not t.is_cuda:
+            raise _lib.B200Error(f"{what}: tensor must live on a CUDA device (no CPU path)")
+
+
 def sglang_per_token_quant_fp8(x: torch.Tensor, dtype: torch.dtype = fp8_dtype
                                ) -> Tuple[torch.Tensor, torch.Tensor]:
     """Dynamic per-token quantisation -> (x_q [M,K] e4m3, x_s [M,1] fp32)   (fp8_kernel.py:317-333)."""
@@ -92,6 +98,7 @@ def fp8_scaled_mm(mat_a: torch.Tensor, mat_b: torch.Tensor, scales_a: torch.Tens
     B [K,N] COLUMN-major e4m3 (the `.t()` view of the [N,K] weight), as sgl_kernel.fp8_scaled_mm
     (sgl-kernel/csrc/gemm/fp8_gemm_kernel.cu:1071-1146)."""
     _check_2d_cuda(mat_a, "fp8_scaled_mm")
+    _check_on_device("fp8_scaled_mm", mat_b, scales_a, scales_b, bias)
     if mat_b.dim() != 2 or mat_b.stride(0) != 1:
         raise _lib.B200Error("fp8_scaled_mm: mat_b must be a column-major [K, N] tensor")
     m, k = mat_a.shape
@@ -125,6 +132,7 @@ def fp8_blockwise_scaled_mm(mat_a: torch.Tensor, weight: torch.Tensor, scales_a:
     (w8a8_block_fp8_matmul, fp8_kernel.py:774-891 / sgl_kernel.fp8_blockwise_scaled_mm)."""
     _check_2d_cuda(mat_a, "fp8_blockwise_scaled_mm")
     _check_2d_cuda(weight, "fp8_blockwise_scaled_mm")
+    _check_on_device("fp8_blockwise_scaled_mm", scales_a, scales_b, bias)
     m, k = mat_a.shape
     n, kw = weight.shape
     if kw != k:

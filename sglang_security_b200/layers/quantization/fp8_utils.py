@@ -40,8 +40,8 @@ def _native_linear(x: torch.Tensor, weight: torch.Tensor, ldw: int, n: int, w_sc
     if dtype is not torch.bfloat16 and dtype is not torch.float16:
         return None
     m, k = x.shape
-    if m == 0 or not x.is_cuda or w_scale.dtype is not torch.float32 or weight.dtype is not torch.float8_e4m3fn or (
-            bias is not None and bias.dtype is not dtype):
+    if m == 0 or not (x.is_cuda and weight.is_cuda and w_scale.is_cuda) or w_scale.dtype is not torch.float32 or (
+            weight.dtype is not torch.float8_e4m3fn) or (bias is not None and not (bias.is_cuda and bias.dtype is dtype)):
         return None
     out = torch.empty((m, n), device=x.device, dtype=dtype)
     q_bytes = (m * k + 255) // 256 * 256

@@ -19,6 +19,45 @@ def test_cpu_tensors_and_other_types_are_not_taken():
         U.apply_w8a8_block_fp8_linear(x, w, [128, 128], torch.ones(1, 2))
 
 
+class _OnDevice:
+    """A CPU tensor that says it is on the GPU."""
+
+    is_cuda = True
+
+    def __init__(self, t):
+        self._t = t
+
+    def __getattr__(self, name):
+        return getattr(self._t, name)
+
+
+@pytest.mark.parametrize("host", ["weight", "scale", "bias"])
+@pytest.mark.parametrize("block", [False, True])
+def test_an_operand_in_host_memory_reaches_no_kernel(block, host, monkeypatch):
+    def no_kernel():
+        raise AssertionError("a kernel was called")
+
+    monkeypatch.setattr(U._lib, "load", no_kernel)
+    monkeypatch.setattr(U._lib, "current_stream", lambda: 0)
+    x = torch.zeros(4, 256, dtype=torch.bfloat16)
+    t = {"weight": torch.zeros(8, 256).to(FP8), "scale": torch.ones(1, 2) if block else torch.ones(8),
+         "bias": torch.zeros(8, dtype=torch.bfloat16)}
+    t["weight"] = t["weight"] if block else t["weight"].t()
+    ops = {name: v if name == host else _OnDevice(v) for name, v in t.items()}
+    assert U._native_linear(_OnDevice(x), ops["weight"], 256, 8, ops["scale"], 1, ops["bias"], block) is None
+    mm = U.fp8_blockwise_scaled_mm if block else U.fp8_scaled_mm
+    a_scale = torch.ones(4, 2 if block else 1)
+    with pytest.raises(U._lib.B200Error, match="CUDA"):
+        mm(_OnDevice(x.to(FP8)), ops["weight"], _OnDevice(a_scale), ops["scale"], torch.bfloat16, ops["bias"])
+
+
+def test_scales_of_another_length_are_refused():
+    x, w = torch.zeros(4, 256, dtype=torch.bfloat16), torch.zeros(8, 256).to(FP8)
+    for n in (2, 3, 7, 9):
+        with pytest.raises(ValueError, match="per-channel"):
+            U.apply_fp8_linear(_OnDevice(x), w.t(), torch.ones(n))
+
+
 def _both(monkeypatch, call):
     taken = []
     native = U._native_linear
