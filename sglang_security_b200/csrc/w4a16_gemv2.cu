@@ -510,7 +510,7 @@ static bool gemv2_plan(int M, int N, int K, int group, Gemv2Plan* pl) {
   if (forced > 0) {
     S = forced > 8 ? 8 : forced;
   } else {
-    // at least two CTAs per SM, at least two slice units per rank
+    // at least two CTAs per SM, at least two slice units per rank (the last may have fewer)
     const int sms = device_sm_count();
     while (n_groups * S < 2 * sms && S < 8 &&
            (units >= 4 * S || (MT == 1 && ceil_div(units, 2 * S) == 2 && (2 * S - 1) * 2 < units)))
@@ -529,11 +529,11 @@ static bool gemv2_plan(int M, int N, int K, int group, Gemv2Plan* pl) {
   }
   if (S > units) S = units;
   if (S < 1) S = 1;
-  for (;; S = MT == 1 ? S + 1 : 2 * S) {
-    const int kb_per_rank = ceil_div(units, S) * upg;
+  for (;; S = MT == 1 ? S + 1 : (S < 4 ? 2 * S : 8)) {   // 8: the largest cluster that every device takes
+    const int per = ceil_div(units, S), kb_per_rank = per * upg;
     const int xs_stride = kb_per_rank * 128 + 64;  // +64: conflict-free LDS.128 across token rows
     const int ng = ceil_div(kb_per_rank * 64, group) + 1;
-    pl->S = S;
+    pl->S = ceil_div(units, per);   // no rank without a slice
     pl->kb_per_rank = kb_per_rank;
     pl->xs_stride = xs_stride;
     pl->sz_off = (M + (M < MT * 8)) * xs_stride;  // M token rows + the shared zero row

@@ -30,6 +30,26 @@ def test_cluster_sizes(splits, m, dtype, gemv2_cfg):  # noqa: F811
     _run(m, 288, 2560, 64, dtype)
 
 
+@pytest.mark.parametrize("m,splits,used", [(16, 5, 8), (16, 6, 8), (16, 7, 8), (16, 3, 8), (9, 5, 8), (8, 5, 8), (1, 5, 6), (16, 1, 8)])
+def test_a_slice_that_does_not_fit_grows_to_eight_ranks_at_most(m, splits, used, gemv2_cfg):  # noqa: F811
+    """28672 input channels in 5 to 7 slices exceed what three CTAs share."""
+    from sglang_security_b200 import _lib
+
+    gemv2_cfg(splits)
+    _run(m, 144, 28672, 128, torch.float16)
+    assert f"splits={used} " in _lib.last_variant()
+
+
+@pytest.mark.parametrize("units,splits,used", [(19, 6, 5), (20, 6, 5), (25, 6, 5), (40, 7, 7), (9, 8, 5), (3, 8, 3), (2, 7, 2)])
+def test_no_rank_is_without_a_slice(units, splits, used, gemv2_cfg):  # noqa: F811
+    from sglang_security_b200 import _lib
+
+    gemv2_cfg(splits)
+    for m in (1, 13):
+        _run(m, 144, units * 128, 128, torch.bfloat16)
+        assert f"splits={used} " in _lib.last_variant()
+
+
 @pytest.mark.parametrize("m,n,k,splits", [(1, 7168, 4096, 6), (8, 7168, 4096, 6), (1, 896, 896, 4), (1, 28672, 1024, 2)])
 def test_default_sizes(m, n, k, splits):
     """7168 channels: eight slices are more clusters than are resident at once."""
