@@ -490,7 +490,7 @@ static int launch_block_pair(const void* a, int64_t lda, const void* b, int64_t 
   p.vec_ok = p.ldc % 8 == 0 && aligned16(p.out);
   p.splits = 1;
   p.kb_per_split = ceil_div(p.K, 128);
-  note_variant("fp8_block_gemm bn=256 pair tiles=%d", tiles);
+  note_variant("fp8_block_gemm pair tiles=%d", tiles);
   {
     ScopedKernelTimer timer("fp8_block_gemm", st);
     B200_CUDA_OK(launch_kernel(fp8_block_pair_kernel<OutT>, dim3(2 * (tiles < pairs ? tiles : pairs)), dim3(kBlkThreads),
@@ -503,17 +503,15 @@ static int launch_block_pair(const void* a, int64_t lda, const void* b, int64_t 
 template <typename OutT>
 static int launch_block_gemm(const void* a, int64_t lda, const void* b, int64_t ldb,
                              const BlockGemmParams& p, cudaStream_t st) {
-  // Estimated us of the three forms, waves x (K blocks x rate + tile) + launch, fitted to 91 problems of 300 to 3001 tokens
-  // timed on all of them (K 1024 to 14336, N 1000 to 28672): the pick is 0.2 % slower than the best on average, and 17 %
-  // faster than the rule and kernels before (128 x 256 tiles from 1.5 an SM on, scales read by the epilogue).  Narrow
-  // tiles that are split over K (fewer than half the SMs) are one wave, which is always theirs.
+  // Estimated us of the three forms, waves x (K blocks x rate + tile) + launch.  Over 137 problems of 300 to 3001 tokens
+  // timed on all of them (K 512 to 14336, N 1000 to 28672, profiles/fp8_block_forms.json) the pick is 0.9 % slower than the
+  // best on average, and in five more than a tenth (600 x 1000 x 2064 19.9, 14.6 in pairs).  Narrow tiles that are split
+  // over K (fewer than half the SMs) are one wave, which is always theirs.
   const int num_kb = ceil_div(p.K, 128), sms = device_sm_count(), pairs = block_pairs<OutT>();
   const int mb = ceil_div(p.M, 128), nb = ceil_div(p.N, 256);
   const double narrow = ceil_div(mb * ceil_div(p.N, 128), sms) * (0.28 * num_kb + 2.7) + 3.7;
   const double wide = ceil_div(mb * nb, sms) * (0.41 * num_kb + 6.0) + 2.9;
   const double pair = pairs > 0 ? ceil_div(ceil_div(p.M, 256) * nb, pairs) * (0.37 * num_kb + 5.5) + 2.8 : wide;
-  // a short K leaves little for wide tiles to save: only where there are 1.5 of them an SM
-  if (num_kb < 12 && 2 * mb * nb < 3 * sms) return launch_block_gemm_bn<OutT, 128>(a, lda, b, ldb, p, st);
   if (pair < wide && pair < narrow) return launch_block_pair<OutT>(a, lda, b, ldb, p, pairs, st);
   if (wide < narrow) return launch_block_gemm_bn<OutT, 256>(a, lda, b, ldb, p, st);
   return launch_block_gemm_bn<OutT, 128>(a, lda, b, ldb, p, st);

@@ -14,7 +14,9 @@ pytestmark = pytest.mark.gpu
     (2049, 3000, 4112, "pair"),      # a second wave, one token in the last tile, 33 blocks
     (1024, 4096, 4096, "pair"),
     (640, 6100, 2176, "pair"),       # the last tile's second half lies past N
-    (520, 7176, 2064, "bn=256 tiles"), (769, 6000, 16, "bn=128"), (2048, 2112, 1152, "bn=128"),
+    (520, 7176, 2064, "bn=256 tiles"), (769, 6000, 16, "bn=128"), (2048, 2112, 1152, "pair"), (900, 2112, 1152, "bn=128"),
+    (3001, 4100, 48, "pair"),        # one block
+    (2048, 1536, 512, "pair"),       # four blocks, which the ring of six takes whole
 ])
 def test_forms(m, n, k, form, dtype):
     from sglang_security_b200 import _lib

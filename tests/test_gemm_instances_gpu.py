@@ -103,9 +103,9 @@ def _block_oracle_gpu(a, b, a_s, b_s, out_dtype):
     return c.to(out_dtype)
 
 
-@pytest.mark.parametrize("m,n,k", [(4096, 6144, 4096), (8192, 4096, 14336), (3000, 28672, 4096),
-                                   (2048, 2112, 1152)])
-def test_fp8_block_bn256_instance(m, n, k):
+@pytest.mark.parametrize("m,n,k,form", [(4096, 6144, 4096, "pair"), (8192, 4096, 14336, "pair"), (3000, 28672, 4096, "pair"),
+                                        (2048, 2112, 1152, "pair"), (1100, 4096, 3584, "bn=256"), (900, 2112, 1152, "bn=128")])
+def test_fp8_block_forms(m, n, k, form):
     from sglang_security_b200.layers.quantization.fp8_kernel import fp8_blockwise_scaled_mm
 
     g = torch.Generator(device="cuda").manual_seed(m + n + k)
@@ -114,11 +114,7 @@ def test_fp8_block_bn256_instance(m, n, k):
     b_s = torch.rand(((n + 127) // 128, (k + 127) // 128), generator=g, device="cuda") * 1e-2
     out = fp8_blockwise_scaled_mm(a, b, a_s, b_s, torch.bfloat16)
     v = _variant()
-    tiles256 = ((m + 127) // 128) * ((n + 255) // 256)
-    sms = torch.cuda.get_device_properties(0).multi_processor_count
-    assert v.startswith("fp8_block_gemm bn=256" if 2 * tiles256 >= 3 * sms else "fp8_block_gemm bn=128"), v
-    if (m, n, k) != (2048, 2112, 1152):
-        assert "bn=256" in v, v
+    assert v.startswith(f"fp8_block_gemm {form} "), v
     ref = _block_oracle_gpu(a, b, a_s, b_s, torch.bfloat16)
     rel = (out.float() - ref.float()).abs().mean() / ref.float().abs().mean()
     assert rel.item() < 1e-3, rel.item()
