@@ -172,6 +172,7 @@ __device__ __forceinline__ uint32_t pack2<__half>(float lo, float hi) {
 constexpr int kPieceMaxBatch = 128;
 struct DecodePiece {
   int b, start, end, len, count;   // b < 0: no such piece
+  unsigned empty[kPieceMaxBatch / 32];   // entries without tokens
 };
 __device__ __forceinline__ DecodePiece decode_piece(const int64_t* seq_lens, int bs, int pieces, int x, int align, int lane) {
   constexpr int R = kPieceMaxBatch / 32;
@@ -200,11 +201,12 @@ __device__ __forceinline__ DecodePiece decode_piece(const int64_t* seq_lens, int
     else lo = mid + 1;
   }
   const float inv = 1.0f / static_cast<float>(lo);
-  DecodePiece out = {-1, 0, 0, 0, 0};
+  DecodePiece out = {-1, 0, 0, 0, 0, {}};
   int before = 0;
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     if (r * 32 >= bs) break;
+    out.empty[r] = __ballot_sync(0xffffffffu, r * 32 + lane < bs && u[r] == 0);
     const int n = count_of(u[r], inv);
     int incl = n;
 #pragma unroll
@@ -431,11 +433,13 @@ attn_decode_mma_kernel(const DecodeParams p) {
   if constexpr (PIECES) {
     const DecodePiece piece = decode_piece(p.seq_lens, p.bs, p.pieces, split, C::ALIGN, lane);
     if (split == 0 && warp == 0) {       // entries without tokens
-      for (int i = 0; i < p.bs; ++i) {
-        if (p.seq_lens[i] > 0) continue;
-        if (p.new_k) store_new_rows<T, D, false, false>(p, i, kvh, lane);
-        if (blockIdx.y == 0 && lane == 0) p.plan[i] = make_int2(0, 0);
-      }
+#pragma unroll
+      for (int r = 0; r < kPieceMaxBatch / 32; ++r)
+        for (unsigned z = piece.empty[r]; z; z &= z - 1) {
+          const int i = r * 32 + __ffs(z) - 1;
+          if (p.new_k) store_new_rows<T, D, false, false>(p, i, kvh, lane);
+          if (blockIdx.y == 0 && lane == 0) p.plan[i] = make_int2(0, 0);
+        }
     }
     if (piece.b < 0) return;
     b = piece.b;

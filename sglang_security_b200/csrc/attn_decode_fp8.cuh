@@ -97,11 +97,13 @@ attn_decode_fp8kv_kernel(const DecodeParams p) {
   if constexpr (PIECES) {
     const DecodePiece piece = decode_piece(p.seq_lens, p.bs, p.pieces, split, C::ALIGN, lane);
     if (split == 0 && warp == 0) {       // entries without tokens
-      for (int i = 0; i < p.bs; ++i) {
-        if (p.seq_lens[i] > 0) continue;
-        if (p.new_k) store_new_rows<T, D, true, E5M2>(p, i, kvh, lane);
-        if (blockIdx.y == 0 && lane == 0) p.plan[i] = make_int2(0, 0);
-      }
+#pragma unroll
+      for (int r = 0; r < kPieceMaxBatch / 32; ++r)
+        for (unsigned z = piece.empty[r]; z; z &= z - 1) {
+          const int i = r * 32 + __ffs(z) - 1;
+          if (p.new_k) store_new_rows<T, D, true, E5M2>(p, i, kvh, lane);
+          if (blockIdx.y == 0 && lane == 0) p.plan[i] = make_int2(0, 0);
+        }
     }
     if (piece.b < 0) return;
     b = piece.b;
