@@ -151,7 +151,7 @@ int b200_attn_decode(const void* q, int64_t q_stride, const void* k_cache, const
  * stores them itself, entry by entry.  _fp8kv_: rows quantised as b200_kv_write_fp8 does (divided by the scales where
  * has_scale), then b200_attn_decode_fp8kv / _fused.  k NULL: the rows are in the pool.
  * pieces > 0 (at least bs, at most 128 requests, no tail): the batch is cut into that many pieces at most, of about equal
- * length, instead of num_splits a request (b200_attn_decode_pieces: how many, 0 where splits serve the batch); workspace from b200_attn_decode_pieces_workspace_bytes, 16-byte aligned. */
+ * length, instead of num_splits a request (b200_attn_decode_pieces_for: how many, 0 where splits serve the batch); workspace from b200_attn_decode_pieces_workspace_bytes, 16-byte aligned. */
 int b200_attn_decode_layer(const void* k, int64_t k_stride, const void* v, int64_t v_stride, const int64_t* loc,
                            const void* q, int64_t q_stride, void* k_cache, void* v_cache, int64_t kv_row_stride, void* o,
                            int64_t o_stride, const int32_t* req_to_token, int64_t req_to_token_stride,
@@ -167,7 +167,8 @@ int b200_attn_decode_fp8kv_layer(const void* k, int64_t k_stride, const void* v,
                                  int dtype, void* workspace, size_t workspace_bytes, int num_splits, int pieces,
                                  void* tickets, size_t ticket_bytes, void* q_out, int64_t q_out_stride, float* q_scales,
                                  void* stream);
-int b200_attn_decode_pieces(int bs, int Hkv, int group, int64_t total_len, int64_t max_len, int num_sms);
+int b200_attn_decode_pieces(int bs, int Hkv, int group, int64_t total_len, int64_t max_len, int num_sms);   /* D = 128 */
+int b200_attn_decode_pieces_for(int bs, int Hkv, int group, int D, int64_t total_len, int64_t max_len, int num_sms);
 size_t b200_attn_decode_pieces_workspace_bytes(int bs, int Hq, int Dv, int pieces);
 
 /* b200_attn_decode for callers that cannot allocate device memory (CUDA graph capture, tight serving

@@ -105,6 +105,7 @@ _SIGNATURES = {
                                        c_size_t, c_int, c_int, c_void_p, c_size_t, c_void_p, c_int64,
                                        c_void_p, c_void_p]),
     "b200_attn_decode_pieces": (c_int, [c_int, c_int, c_int, c_int64, c_int64, c_int]),
+    "b200_attn_decode_pieces_for": (c_int, [c_int, c_int, c_int, c_int, c_int64, c_int64, c_int]),
     "b200_attn_decode_pieces_workspace_bytes": (c_size_t, [c_int, c_int, c_int, c_int]),
     # split-KV scratch built into the library (8 MiB, B200_ATTN_DECODE_NOALLOC_SCRATCH_BYTES): allocates nothing
     "b200_attn_decode_noalloc": (c_int, [c_void_p, c_int64, c_void_p, c_void_p, c_int64, c_void_p,

@@ -168,7 +168,7 @@ __device__ __forceinline__ uint32_t pack2<__half>(float lo, float hi) {
 // the lengths on the device, so a captured launch follows them.  us, splits / pieces (random lengths, 32 / 8 heads of 128):
 // bf16 16 x up to 6000 51.2 -> 43.0, 32 x up to 1000 20.2 -> 16.0; e4m3 27 x up to 6000 46.8 -> 42.8, 32 x up to 3000 35.2
 // -> 28.7.  Tried: exact equal pieces, ranges that begin and end inside requests; a CTA then starts on up to two requests,
-// which costs what the even end gives below ~1000 tokens a CTA (e4m3 48 x up to 1500: splits 27.2, pieces 21.3, pieces 25.0).
+// which costs what the even end gives below ~1000 tokens a CTA (e4m3 48 x up to 1500: splits 27.2, pieces 21.3, shares 25.0).
 constexpr int kPieceMaxBatch = 128;
 struct DecodePiece {
   int b, start, end, len, count;   // b < 0: no such piece
@@ -1355,19 +1355,30 @@ static int merge_pieces(const b200::DecodeParams& p, int D, int dtype, void* str
 }
 
 /* How many pieces a decode batch of unequal requests is cut into, or 0 where a split count for all serves it. */
-int b200_attn_decode_pieces(int bs, int Hkv, int group, int64_t total_len, int64_t max_len, int num_sms) {
+int b200_attn_decode_pieces_for(int bs, int Hkv, int group, int D, int64_t total_len, int64_t max_len, int num_sms) {
   using namespace b200;
-  if (bs < 2 || bs > kPieceMaxBatch || Hkv <= 0 || group <= 0) return 0;
+  if (bs < 2 || bs > kPieceMaxBatch || Hkv <= 0 || group <= 0 || D <= 0) return 0;
   if (num_sms <= 0) num_sms = 148;
   // One wave at four CTAs an SM (two and three waves were slower in every batch timed).  Not where the longest request is
   // within an eighth of the average; from 1.5 pieces a request on (64 x up to 1500 tokens, 1.2 pieces a request: 50.1 us in
   // splits, 53.0 in pieces); up to 16 (4 x up to 4000, 18 a request: 10.3 / 11.4, where splits of every request fill the
   // wave as well); and from 250 tokens a piece on (8 x up to 2000, 135 a piece: 11.6 / 12.1; 16 x up to 2000, 270: 17.5 /
   // 15.2), below which the plan and the merge cost what the even end gives.
-  const int64_t pieces = static_cast<int64_t>(num_sms) * 4 / (Hkv * ceil_div(group, tile_heads(group)));
+  const int64_t tiles = static_cast<int64_t>(Hkv) * ceil_div(group, tile_heads(group));
+  const int64_t slots = static_cast<int64_t>(num_sms) * 4, pieces = slots / tiles;
   const bool unequal = max_len * 8 * bs > total_len * 9;
   if (!unequal || 2 * pieces < 3 * bs || pieces > 16 * bs || total_len < 250 * pieces || pieces > 65535) return 0;
+  // And, where the splits are all resident at once, only if the longest of them is 220 tokens of head size 128 longer than a
+  // piece: short splits end early and leave their SM to the long ones, so less unevenness than that is evened out anyway.
+  // Of 450 random batches that pass the lines above (profiles/decode_pieces_batches.json) this one keeps 396, 1.150 x (0.969
+  // at worst, 5 below 0.98); the 54 others were 0.98 x (D 64, 34 x up to 3663 FP8 11.9 us in splits, 13.3 in pieces).
+  const int64_t splits = decode_num_splits(bs, Hkv, group, D, total_len / bs > 1 ? total_len / bs : 1, max_len, num_sms);
+  if (bs * tiles * splits <= slots && (max_len / splits - total_len / pieces) * D < 220 * 128) return 0;
   return static_cast<int>(pieces);
+}
+
+int b200_attn_decode_pieces(int bs, int Hkv, int group, int64_t total_len, int64_t max_len, int num_sms) {
+  return b200_attn_decode_pieces_for(bs, Hkv, group, 128, total_len, max_len, num_sms);
 }
 
 static int attn_merge_impl(const float* part_o, const float* part_lse, void* o, int64_t o_stride,

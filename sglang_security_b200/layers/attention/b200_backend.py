@@ -148,8 +148,8 @@ class B200AttnBackend(AttentionBackend):
             s = self._num_splits(bs, head_dim, max(1, total // bs), longest)
             pieces = 0
             if longest and self.fixed_num_kv_splits <= 0:
-                pieces = self.lib.b200_attn_decode_pieces(bs, self.num_kv_head, self.num_head // self.num_kv_head, int(total),
-                                                          longest, self.num_sms)
+                pieces = self.lib.b200_attn_decode_pieces_for(bs, self.num_kv_head, self.num_head // self.num_kv_head, head_dim,
+                                                              int(total), longest, self.num_sms)
             self.forward_metadata = ForwardMetadata(num_splits=s, pieces=pieces,
                                                     workspace=self._ensure_workspace(bs, s, pieces))
         else:

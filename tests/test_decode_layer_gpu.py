@@ -117,4 +117,6 @@ def test_rule_of_the_pieces():
     assert f(27, 27 * 3750, 6000) == 74 and f(16, 20000, 2000) == 74
     assert f(27, 27 * 4096, 4096) == 0                           # equal requests
     assert f(64, 64 * 1000, 1500) == 0 and f(4, 10000, 4000) == 0 and f(8, 10000, 2000) == 0 and f(129, 10 ** 6, 10 ** 5) == 0
+    d64 = lambda bs, total, longest: lib.b200_attn_decode_pieces_for(bs, 2, 7, 64, total, longest, 148)  # noqa: E731
+    assert d64(34, 80826, 3663) == 0 and d64(23, 176120, 15900) == 296         # splits even out the first by themselves
     assert f(40, 40 * 1915, 3064, 4, 5) == 148 and f(27, 27 * 3750, 6000, 2, 24) == 148
