@@ -15,13 +15,15 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda"
 
 
-def _run(monkeypatch, own, heads, act, pool_dtype, lens, splits, scales, pad, pieces=0):
+def _run(monkeypatch, own, heads, act, pool_dtype, lens, splits, scales, pad, pieces=0, width=9, cap=0.0, replay=None,
+         replay_eager=False):
+    """replay: lengths (none longer) that a graph, captured with `lens`, is replayed with, or a direct call made."""
     from sglang_security_b200 import _lib
 
     hq, hkv, d = heads
     g = torch.Generator(device=DEV).manual_seed(7)
     bs, total = len(lens), sum(lens) + len(lens)
-    rtp = ReqToTokenPool(bs + 1, max(lens) + 9, DEV)
+    rtp = ReqToTokenPool(bs + 1, max(lens) + width, DEV)
     kvp = MHATokenToKVPool(total + 16, 1, pool_dtype, hkv, d, 1, DEV)
     for buf in (kvp.k_buffer[0], kvp.v_buffer[0]):
         rows = torch.randn(buf.shape, device=DEV, generator=g)
@@ -42,7 +44,7 @@ def _run(monkeypatch, own, heads, act, pool_dtype, lens, splits, scales, pad, pi
     monkeypatch.setattr(backend, "_num_splits", lambda *a: splits)
     if not own:
         monkeypatch.setattr(backend, "_new_rows", lambda *a: None)
-    layer = RadixAttention(hq, d, d ** -0.5, hkv, 0)
+    layer = RadixAttention(hq, d, d ** -0.5, hkv, 0, logit_cap=cap)
     if scales:
         layer.k_scale_float, layer.v_scale_float = scales
     t = torch.tensor(lens, dtype=torch.int64)
@@ -55,8 +57,27 @@ def _run(monkeypatch, own, heads, act, pool_dtype, lens, splits, scales, pad, pi
         backend.forward_metadata.pieces = pieces
         backend.forward_metadata.workspace = backend._ensure_workspace(bs, splits, pieces)
         backend.forward_metadata.workspace.fill_(0xff)       # NaN in every partial row
+    if replay:
+        pools = [buf.clone() for buf in (kvp.k_buffer[0], kvp.v_buffer[0])]
+        layer(q, k, v, fb)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            o = layer(q, k, v, fb)
+        lens = replay
+        fb.seq_lens.copy_(torch.tensor(lens))
+        fb.out_cache_loc.copy_(rtp.req_to_token[torch.arange(bs), (fb.seq_lens.cpu() - 1).clamp(min=0)])
+        for buf, old in zip((kvp.k_buffer[0], kvp.v_buffer[0]), pools):
+            buf.copy_(old)
+        if pieces:
+            backend.forward_metadata.workspace.fill_(0xff)
+        if replay_eager:
+            o = layer(q, k, v, fb)
+        else:
+            graph.replay()
+        torch.cuda.synchronize()
     n0 = _lib.load().b200_launch_count()
-    o = layer(q, k, v, fb)
+    if not replay:
+        o = layer(q, k, v, fb)
     launches = _lib.load().b200_launch_count() - n0
     live = torch.tensor([n > 0 for n in lens], device=DEV)
     return o[live].clone(), kvp.k_buffer[0].clone(), kvp.v_buffer[0].clone(), launches
@@ -107,6 +128,56 @@ def test_pieces_of_equal_length(heads, act, pool, scales, lens, pieces, monkeypa
     assert bool(a.isfinite().all())
     assert (a - b).norm() <= 2.0 ** -8 * b.norm()
     assert (a - b).abs().max() <= 2.0 ** -8 * 6 * (scales[1] if scales else 1.0)
+
+
+FORMS = [((32, 8, 128), torch.bfloat16, torch.bfloat16, None), ((14, 2, 64), torch.float16, torch.float16, None),
+         ((48, 2, 128), torch.bfloat16, torch.bfloat16, None), ((20, 4, 128), torch.float16, torch.float8_e4m3fn, (0.5, 1.5)),
+         ((8, 2, 64), torch.bfloat16, torch.float8_e5m2, None)]
+UNEQUAL = [3000, 0, 17, 1448, 649, 2300, 96, 1197, 1]
+
+
+def _same(a, b):
+    for x, y in zip(a[:3], b[:3]):
+        assert torch.equal(x.view(torch.uint8), y.view(torch.uint8))
+
+
+@pytest.mark.parametrize("heads,act,pool,scales", FORMS)
+@pytest.mark.parametrize("splits,pieces", [(3, 0), (1, 24), (1, 60)])
+def test_page_tables_that_take_wide_loads(heads, act, pool, scales, splits, pieces, monkeypatch):
+    """Rows of a multiple of four entries: 16-byte loads, and from five tiles a warp on the step without checks.  The same
+    bytes as from rows whose entries are loaded and checked one by one; new rows stored by the kernel, or before it."""
+    for own in (True, False):
+        wide = _run(monkeypatch, own, heads, act, pool, UNEQUAL, splits, scales, 0, pieces, width=12)
+        _same(wide, _run(monkeypatch, own, heads, act, pool, UNEQUAL, splits, scales, 0, pieces, width=9))
+
+
+@pytest.mark.parametrize("heads,act,pool,scales", FORMS[:3])         # FP8 pools refuse such rows
+@pytest.mark.parametrize("pieces", [14, 40])
+def test_pieces_with_rows_that_do_not_start_on_16_bytes(heads, act, pool, scales, pieces, monkeypatch):
+    got = _run(monkeypatch, True, heads, act, pool, UNEQUAL, 1, scales, 3, pieces, width=12)
+    _same(got, _run(monkeypatch, False, heads, act, pool, UNEQUAL, 1, scales, 3, pieces, width=12))
+
+
+@pytest.mark.parametrize("heads,act,pool,scales", FORMS)
+def test_pieces_with_a_logit_cap(heads, act, pool, scales, monkeypatch):
+    """Bounds as above; the cap's own arithmetic is the same in both."""
+    got = _run(monkeypatch, True, heads, act, pool, UNEQUAL, 1, scales, 0, 40, width=12, cap=5.0)
+    ref = _run(monkeypatch, True, heads, act, pool, UNEQUAL, 1, scales, 0, width=12, cap=5.0)
+    plain = _run(monkeypatch, True, heads, act, pool, UNEQUAL, 1, scales, 0, 40, width=12)
+    a, b = got[0].double(), ref[0].double()
+    assert (a - b).norm() <= 2.0 ** -8 * b.norm() and (a - b).abs().max() <= 2.0 ** -8 * 6 * (scales[1] if scales else 1.0)
+    assert (a - plain[0].double()).norm() > 2.0 ** -6 * b.norm()          # the cap does something
+
+
+@pytest.mark.parametrize("heads,act,pool,scales", FORMS)
+@pytest.mark.parametrize("width", [9, 12])
+@pytest.mark.parametrize("lens", [[1, 2999, 0, 700, 5, 2300, 0, 33, 1100], [1] * 9, [0, 0, 3000, 0, 0, 0, 0, 0, 0],
+                                  [2999] * 9])
+def test_a_captured_launch_follows_the_lengths(lens, width, heads, act, pool, scales, monkeypatch):
+    """The plan is made from the lengths on the device: a graph captured with other lengths gives the bytes of a direct call."""
+    run = lambda eager: _run(monkeypatch, True, heads, act, pool, [3000] * 9, 1, scales, 0, 40, width=width,  # noqa: E731
+                             replay=lens, replay_eager=eager)
+    _same(run(False), run(True))
 
 
 def test_rule_of_the_pieces():
