@@ -59,17 +59,22 @@ struct DecodeParams {
   // optional output gate [rows, gate_stride] in T: o is multiplied by sigmoid(gate[row, head * D + d])
   const void* gate;
   int64_t gate_stride;
-  // b200_attn_decode_layer: entry b's new K/V row [Hkv, D] in T, stored to slot loc[b] of the pool before it is read
-  // (null: the pool holds it already); new_all: every CTA stores the rows of all entries (see store_new_rows)
+  // PIECES instances: the batch is cut into this many pieces at most (decode_piece); grid.x is the piece
+  int pieces;
+  int2* plan;                   // [bs] first partial row and count of a request, for the merge
+};
+
+// b200_attn_decode_layer: entry b's new K/V row [Hkv, D] in T, stored to slot loc[b] of the pool before it is read (null: the
+// pool holds it already); new_all: every CTA stores the rows of all entries (see store_new_rows).  Kernels that take these
+// parameters are instances of their own: with the stores in them, the others were slower by up to 7 % on short requests (us,
+// behind a write launch, 41 x 105 tokens of head size 64 5.06 -> 4.71, 6 x up to 92 4.75 -> 4.65, 64 x 600 30.4 -> 30.2).
+struct DecodeParamsNew : DecodeParams {
   const void* new_k;
   const void* new_v;
   int64_t new_k_stride, new_v_stride;
   const int64_t* loc;
   float k_scale_w, v_scale_w;   // FP8 pool: divisors of the stored rows, where scale_new
   int scale_new, new_all;
-  // PIECES instances: the batch is cut into this many pieces at most (decode_piece); grid.x is the piece
-  int pieces;
-  int2* plan;                   // [bs] first partial row and count of a request, for the merge
 };
 
 constexpr float kLog2e = 1.4426950408889634f;
@@ -239,13 +244,14 @@ __device__ __forceinline__ DecodePiece decode_piece(const int64_t* seq_lens, int
 //  new_all     any page table (two positions of one request as two entries, a fork of a request beside it): the warps of
 //              every CTA store the rows of all entries, and the CTA synchronises before it reads the pool.  CTAs store the
 //              same bytes, so what a CTA reads behind its own store does not depend on the others.  Up to kNewRowsAll
-//              entries; beyond, the stores cost what the write launch does.
-// us, ten calls in a graph, own slots / new_all / write launch, 32 / 8 heads of 128, bf16: 1 x 1500 6.62 / 6.59 / 7.39,
-// 2 x 1500 7.82 / 8.20 / 8.63, 4 x 1000 8.22 / 8.46 / 9.25, 8 x 1000 10.29 / 11.09 / 11.31, 16 x 1024 13.03 / 15.14 / 14.16,
-// 64 x 300 11.59 / 19.49 / 12.64, 64 x 4096 160.3 / 169.8 / 161.9; e4m3 27 x up to 6000 42.1 / 46.9 / 43.6.
-constexpr int kNewRowsAll = 4;
+//              entries; beyond, the stores cost what the write launch does or more.
+// us, calls in a graph, own slots / new_all / write launch, bf16, 32 / 8 heads of 128: 1 x 1500 6.48 / 6.34 / 7.18, 2 x 1500
+// 7.57 / 7.93 / 8.47, 2 x 8000 14.1 / 14.6 / 15.5, 3 x 8000 17.7 / 18.4 / 17.4, 4 x 8000 28.0 / 29.1 / 29.4, 16 x 1024 13.0 /
+// 15.1 / 14.2, 64 x 4096 160.3 / 169.8 / 161.9; e4m3 2 x 8000 11.5 / 11.9 / 12.3, 27 x up to 6000 42.1 / 46.9 / 43.6, 8 / 2
+// heads 4 x 8000 10.5 / 11.1 / 10.5.
+constexpr int kNewRowsAll = 2;
 template <typename T, int D, bool FP8, bool E5M2>
-__device__ __forceinline__ void store_new_rows(const DecodeParams& p, int b, int kvh, int lane) {
+__device__ __forceinline__ void store_new_rows(const DecodeParamsNew& p, int b, int kvh, int lane) {
   constexpr int CPR = D / 8;
   const int64_t slot = p.loc[b];
 #pragma unroll
@@ -407,9 +413,9 @@ namespace b200 {
 
 // HI: the tile holds more than 8 heads (rows 8..15 of the MMA are live).  ROWS: the row list and the output gate
 // of b200_attn_decode_rows (an instance of its own: the others stay at their register limit without spills).
-template <typename T, int D, int NT, int STAGES, int NW, bool HI, bool TAIL, bool ROWS = false, bool PIECES = false>
+template <typename P, typename T, int D, int NT, int STAGES, int NW, bool HI, bool TAIL, bool ROWS = false, bool PIECES = false>
 __global__ void __launch_bounds__(NW * 32, TAIL ? 4 : 0)
-attn_decode_mma_kernel(const DecodeParams p) {
+attn_decode_mma_kernel(const P p) {
   using C = MmaCfg<D, NT, STAGES, NW>;
   constexpr int CPR = C::CPR, RPG = C::RPG, ROW_BYTES = C::ROW_BYTES;
   constexpr int STAGE_BYTES = C::STAGE_BYTES;
@@ -427,7 +433,8 @@ attn_decode_mma_kernel(const DecodeParams p) {
   const int ht = blockIdx.y - kvh * p.head_tiles;
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
-  constexpr bool NEW = !TAIL && !ROWS;
+  constexpr bool NEW = std::is_same<P, DecodeParamsNew>::value;
+  static_assert(!NEW || !(TAIL || ROWS), "new rows are written before these");
   int b = blockIdx.z, len, chunk = 0, start, end;
   bool whole = false;                    // PIECES: writes the output row, not a partial one
   if constexpr (PIECES) {
@@ -437,7 +444,7 @@ attn_decode_mma_kernel(const DecodeParams p) {
       for (int r = 0; r < kPieceMaxBatch / 32; ++r)
         for (unsigned z = piece.empty[r]; z; z &= z - 1) {
           const int i = r * 32 + __ffs(z) - 1;
-          if (p.new_k) store_new_rows<T, D, false, false>(p, i, kvh, lane);
+          if constexpr (NEW) store_new_rows<T, D, false, false>(p, i, kvh, lane);
           if (blockIdx.y == 0 && lane == 0) p.plan[i] = make_int2(0, 0);
         }
     }
@@ -453,7 +460,9 @@ attn_decode_mma_kernel(const DecodeParams p) {
     chunk = split_chunk(len, p.num_splits, C::ALIGN);
     start = split * chunk;
     if (start >= len) {
-      if (NEW && p.new_k && len <= 0 && split == 0 && warp == 0) store_new_rows<T, D, false, false>(p, b, kvh, lane);
+      if constexpr (NEW) {
+        if (len <= 0 && split == 0 && warp == 0) store_new_rows<T, D, false, false>(p, b, kvh, lane);
+      }
       return;
     }
     end = min(len, start + chunk);
@@ -529,7 +538,7 @@ attn_decode_mma_kernel(const DecodeParams p) {
   };
 
   load_slots(0, std::false_type{});
-  if (NEW && p.new_k) {
+  if constexpr (NEW) {
     if (p.new_all) {
       for (int i = warp; i < p.bs; i += NW) store_new_rows<T, D, false, false>(p, i, kvh, lane);
       __syncthreads();
@@ -1018,64 +1027,40 @@ static int decode_ctas_per_sm(int D) {
   return n < 1 ? 1 : n;
 }
 
-// launcher of the fused-tail instantiations (own attribute flag per kernel through the template)
-template <typename C>
-static int launch_decode_any(void (*kern)(const DecodeParams), const DecodeParams& p, cudaStream_t st,
-                             const char* timer_name, const char* kernel_name) {
-  static void (*configured[64])(const DecodeParams) = {};
-  static int n_configured = 0;
-  bool done = false;
-  for (int i = 0; i < n_configured; ++i) done |= configured[i] == kern;
-  if (!done) {
-    B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      C::SMEM_BYTES));
-    if (n_configured < 64) configured[n_configured++] = kern;
+template <typename C, auto KERN>
+static int launch_decode_kernel(const DecodeParamsNew& p, cudaStream_t st, const char* timer_name, const char* kernel_name) {
+  static std::atomic<bool> attr_done{false};
+  if (!attr_done.load(std::memory_order_relaxed)) {
+    B200_CUDA_OK(cudaFuncSetAttribute(KERN, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
+    attr_done.store(true, std::memory_order_relaxed);
   }
   const dim3 grid = p.pieces ? dim3(p.pieces, p.Hkv * p.head_tiles) : dim3(p.num_splits, p.Hkv * p.head_tiles, p.bs);
   {
     ScopedKernelTimer timer(timer_name, st);
-    B200_CUDA_OK(launch_kernel(kern, grid, dim3(C::THREADS), C::SMEM_BYTES, st, 1,
-                               pdl_family(p.bs, kPdlAttn), p));
+    B200_CUDA_OK(launch_kernel(KERN, grid, dim3(C::THREADS), C::SMEM_BYTES, st, 1, pdl_family(p.bs, kPdlAttn), p));
   }
-  g_launch_count.fetch_add(1, std::memory_order_relaxed);
-  cudaError_t e = cudaPeekAtLastError();
-  if (e != cudaSuccess) {
-    set_error("%s: launch failed: %s", kernel_name, cudaGetErrorString(e));
-    (void)cudaGetLastError();
-    return 2;
-  }
+  B200_CHECK_LAUNCH(kernel_name);
   return 0;
 }
 
 template <typename T, int D, bool HI>
-static int launch_decode(const DecodeParams& p, cudaStream_t st) {
+static int launch_decode(const DecodeParamsNew& p, cudaStream_t st) {
   using C = MmaCfg<D, kNT, kStages, kNW>;
-  if (p.tickets) return launch_decode_any<C>(attn_decode_mma_kernel<T, D, kNT, kStages, kNW, HI, true>, p, st,
-                                             "attn_decode_split", "attn_decode_mma_kernel");
-  if (p.row_list || p.gate)
-    return launch_decode_any<C>(attn_decode_mma_kernel<T, D, kNT, kStages, kNW, HI, false, true>, p, st,
-                                "attn_decode_split", "attn_decode_mma_kernel");
+  using P = DecodeParams;
+  using N = DecodeParamsNew;
+#define DECODE_LAUNCH(...) \
+  launch_decode_kernel<C, attn_decode_mma_kernel<__VA_ARGS__>>(p, st, "attn_decode_split", "attn_decode_mma_kernel")
+  if (p.tickets) return DECODE_LAUNCH(P, T, D, kNT, kStages, kNW, HI, true);
+  if (p.row_list || p.gate) return DECODE_LAUNCH(P, T, D, kNT, kStages, kNW, HI, false, true);
   if (p.pieces)
-    return launch_decode_any<C>(attn_decode_mma_kernel<T, D, kNT, kStages, kNW, HI, false, false, true>, p, st,
-                                "attn_decode_split", "attn_decode_mma_kernel");
-  auto kern = attn_decode_mma_kernel<T, D, kNT, kStages, kNW, HI, false>;
-  static bool attr_done = false;
-  if (!attr_done) {
-    B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      C::SMEM_BYTES));
-    attr_done = true;
-  }
-  dim3 grid(p.num_splits, p.Hkv * p.head_tiles, p.bs);
-  {
-    ScopedKernelTimer timer("attn_decode_split", st);
-    B200_CUDA_OK(launch_kernel(kern, grid, dim3(C::THREADS), C::SMEM_BYTES, st, 1, pdl_family(p.bs, kPdlAttn), p));
-  }
-  B200_CHECK_LAUNCH("attn_decode_mma_kernel");
-  return 0;
+    return p.new_k ? DECODE_LAUNCH(N, T, D, kNT, kStages, kNW, HI, false, false, true)
+                   : DECODE_LAUNCH(P, T, D, kNT, kStages, kNW, HI, false, false, true);
+  return p.new_k ? DECODE_LAUNCH(N, T, D, kNT, kStages, kNW, HI, false) : DECODE_LAUNCH(P, T, D, kNT, kStages, kNW, HI, false);
+#undef DECODE_LAUNCH
 }
 
 template <typename T>
-static int dispatch_decode(const DecodeParams& p, int D, int G, cudaStream_t st) {
+static int dispatch_decode(const DecodeParamsNew& p, int D, int G, cudaStream_t st) {
   if (D == 128) return G > 8 ? launch_decode<T, 128, true>(p, st) : launch_decode<T, 128, false>(p, st);
   if (D == 64) return G > 8 ? launch_decode<T, 64, true>(p, st) : launch_decode<T, 64, false>(p, st);
   set_error("b200_attn_decode: unsupported head_dim %d (supported: 64, 128)", D);
@@ -1096,31 +1081,22 @@ static int fp8kv_stages() {
 }
 
 template <typename T, int D, bool HI, int ST>
-static int launch_decode_fp8kv_st(const DecodeParams& p, cudaStream_t st) {
+static int launch_decode_fp8kv_st(const DecodeParamsNew& p, cudaStream_t st) {
   using C = Fp8KvCfg<D, kNT8, ST, kNW>;
-  if (p.tickets) return launch_decode_any<C>(attn_decode_fp8kv_kernel<T, D, kNT8, ST, kNW, HI, true>, p, st,
-                                             "attn_decode_fp8kv", "attn_decode_fp8kv_kernel");
-  if (p.pieces) return launch_decode_any<C>(attn_decode_fp8kv_kernel<T, D, kNT8, ST, kNW, HI, false, false, true>, p, st,
-                                            "attn_decode_fp8kv", "attn_decode_fp8kv_kernel");
-  auto kern = attn_decode_fp8kv_kernel<T, D, kNT8, ST, kNW, HI, false>;
-  static bool attr_done = false;
-  if (!attr_done) {
-    B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      C::SMEM_BYTES));
-    attr_done = true;
-  }
-  dim3 grid(p.num_splits, p.Hkv * p.head_tiles, p.bs);
-  {
-    ScopedKernelTimer timer("attn_decode_fp8kv", st);
-    B200_CUDA_OK(launch_kernel(kern, grid, dim3(C::THREADS), C::SMEM_BYTES, st, 1,
-                               pdl_family(p.bs, kPdlAttn), p));
-  }
-  B200_CHECK_LAUNCH("attn_decode_fp8kv_kernel");
-  return 0;
+  using P = DecodeParams;
+  using N = DecodeParamsNew;
+#define DECODE_LAUNCH(...) \
+  launch_decode_kernel<C, attn_decode_fp8kv_kernel<__VA_ARGS__>>(p, st, "attn_decode_fp8kv", "attn_decode_fp8kv_kernel")
+  if (p.tickets) return DECODE_LAUNCH(P, T, D, kNT8, ST, kNW, HI, true);
+  if (p.pieces)
+    return p.new_k ? DECODE_LAUNCH(N, T, D, kNT8, ST, kNW, HI, false, false, true)
+                   : DECODE_LAUNCH(P, T, D, kNT8, ST, kNW, HI, false, false, true);
+  return p.new_k ? DECODE_LAUNCH(N, T, D, kNT8, ST, kNW, HI, false) : DECODE_LAUNCH(P, T, D, kNT8, ST, kNW, HI, false);
+#undef DECODE_LAUNCH
 }
 
 template <typename T, int D, bool HI>
-static int launch_decode_fp8kv(const DecodeParams& p, cudaStream_t st) {
+static int launch_decode_fp8kv(const DecodeParamsNew& p, cudaStream_t st) {
   return fp8kv_stages() == 3 ? launch_decode_fp8kv_st<T, D, HI, 3>(p, st)
                              : launch_decode_fp8kv_st<T, D, HI, 2>(p, st);
 }
@@ -1128,29 +1104,21 @@ static int launch_decode_fp8kv(const DecodeParams& p, cudaStream_t st) {
 // e5m2 pool (`--kv-cache-dtype fp8_e5m2`): the same kernel with the byte -> f16 conversion swapped
 // (one PRMT instead of a cvt); 2-stage ring, no in-kernel tail.
 template <typename T, int D, bool HI>
-static int launch_decode_e5m2kv(const DecodeParams& p, cudaStream_t st) {
+static int launch_decode_e5m2kv(const DecodeParamsNew& p, cudaStream_t st) {
   using C = Fp8KvCfg<D, kNT8, 2, kNW>;
-  if (p.pieces) return launch_decode_any<C>(attn_decode_fp8kv_kernel<T, D, kNT8, 2, kNW, HI, false, true, true>, p, st,
-                                            "attn_decode_fp8kv", "attn_decode_fp8kv_kernel<e5m2>");
-  auto kern = attn_decode_fp8kv_kernel<T, D, kNT8, 2, kNW, HI, false, true>;
-  static bool attr_done = false;
-  if (!attr_done) {
-    B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      C::SMEM_BYTES));
-    attr_done = true;
-  }
-  dim3 grid(p.num_splits, p.Hkv * p.head_tiles, p.bs);
-  {
-    ScopedKernelTimer timer("attn_decode_fp8kv", st);
-    B200_CUDA_OK(launch_kernel(kern, grid, dim3(C::THREADS), C::SMEM_BYTES, st, 1,
-                               pdl_family(p.bs, kPdlAttn), p));
-  }
-  B200_CHECK_LAUNCH("attn_decode_fp8kv_kernel<e5m2>");
-  return 0;
+  using P = DecodeParams;
+  using N = DecodeParamsNew;
+#define DECODE_LAUNCH(...) \
+  launch_decode_kernel<C, attn_decode_fp8kv_kernel<__VA_ARGS__>>(p, st, "attn_decode_fp8kv", "attn_decode_fp8kv_kernel<e5m2>")
+  if (p.pieces)
+    return p.new_k ? DECODE_LAUNCH(N, T, D, kNT8, 2, kNW, HI, false, true, true)
+                   : DECODE_LAUNCH(P, T, D, kNT8, 2, kNW, HI, false, true, true);
+  return p.new_k ? DECODE_LAUNCH(N, T, D, kNT8, 2, kNW, HI, false, true) : DECODE_LAUNCH(P, T, D, kNT8, 2, kNW, HI, false, true);
+#undef DECODE_LAUNCH
 }
 
 template <typename T>
-static int dispatch_decode_fp8kv(const DecodeParams& p, int D, int G, bool e5m2, cudaStream_t st) {
+static int dispatch_decode_fp8kv(const DecodeParamsNew& p, int D, int G, bool e5m2, cudaStream_t st) {
   if (e5m2 && D == 128)
     return G > 8 ? launch_decode_e5m2kv<T, 128, true>(p, st) : launch_decode_e5m2kv<T, 128, false>(p, st);
   if (e5m2 && D == 64)
@@ -1185,7 +1153,7 @@ struct DecodeNewRows {
 // The split kernel stores the rows itself where 16-byte pieces of a head fit them, it is not the instance with the
 // in-kernel tail, and either no entry reads another's new slot or the entries are few (store_new_rows); else they are
 // written by a launch of their own before it, which takes pools without gaps between the rows only.
-static int apply_new_rows(DecodeParams& p, const DecodeNewRows* rows, int D, int dtype, bool fp8, int e5m2, float k_scale,
+static int apply_new_rows(DecodeParamsNew& p, const DecodeNewRows* rows, int D, int dtype, bool fp8, int e5m2, float k_scale,
                           float v_scale, void* stream, const char* who) {
   if (!rows) return 0;
   B200_REQUIRE(rows->k && rows->v && rows->loc, "%s: null pointer", who);
@@ -1449,7 +1417,7 @@ static int attn_decode_impl(const void* q, int64_t q_stride, const void* k_cache
   B200_REQUIRE(num_splits == 1 || pieces > 0 || (workspace && workspace_bytes >= need),
                "b200_attn_decode: workspace too small (%zu < %zu)", workspace_bytes, need);
 
-  DecodeParams p = {};
+  DecodeParamsNew p = {};
   p.q = q;
   p.q_stride = q_stride;
   p.k_cache = k_cache;
@@ -1583,7 +1551,7 @@ static int attn_decode_fp8kv_impl(const void* q, int64_t q_stride, const void* k
   const size_t need = b200_attn_decode_workspace_bytes(bs, Hq, Dv, num_splits);
   B200_REQUIRE(num_splits == 1 || pieces > 0 || (workspace && workspace_bytes >= need),
                "b200_attn_decode_fp8kv: workspace too small (%zu < %zu)", workspace_bytes, need);
-  DecodeParams p = {};
+  DecodeParamsNew p = {};
   p.q = q;
   p.q_stride = q_stride;
   p.k_cache = k_cache;

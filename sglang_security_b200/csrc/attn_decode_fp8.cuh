@@ -71,9 +71,9 @@ __device__ __forceinline__ void q4_to_f16<__nv_bfloat16>(const __nv_bfloat16* q,
   hi = *reinterpret_cast<const uint32_t*>(&hb);
 }
 
-template <typename T, int D, int NT, int STAGES, int NW, bool HI, bool TAIL, bool E5M2 = false, bool PIECES = false>
+template <typename P, typename T, int D, int NT, int STAGES, int NW, bool HI, bool TAIL, bool E5M2 = false, bool PIECES = false>
 __global__ void __launch_bounds__(NW * 32, TAIL ? 4 : 0)
-attn_decode_fp8kv_kernel(const DecodeParams p) {
+attn_decode_fp8kv_kernel(const P p) {
   using C = Fp8KvCfg<D, NT, STAGES, NW>;
   constexpr int CPR = C::CPR, RPG = C::RPG, RB = C::RB;
   constexpr int STAGE_BYTES = C::STAGE_BYTES;
@@ -91,7 +91,8 @@ attn_decode_fp8kv_kernel(const DecodeParams p) {
   const int ht = blockIdx.y - kvh * p.head_tiles;
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
-  constexpr bool NEW = !TAIL;
+  constexpr bool NEW = std::is_same<P, DecodeParamsNew>::value;
+  static_assert(!NEW || !TAIL, "new rows are written before this");
   int b = blockIdx.z, len, chunk = 0, start, end;
   bool whole = false;                    // PIECES: writes the output row, not a partial one
   if constexpr (PIECES) {
@@ -101,7 +102,7 @@ attn_decode_fp8kv_kernel(const DecodeParams p) {
       for (int r = 0; r < kPieceMaxBatch / 32; ++r)
         for (unsigned z = piece.empty[r]; z; z &= z - 1) {
           const int i = r * 32 + __ffs(z) - 1;
-          if (p.new_k) store_new_rows<T, D, true, E5M2>(p, i, kvh, lane);
+          if constexpr (NEW) store_new_rows<T, D, true, E5M2>(p, i, kvh, lane);
           if (blockIdx.y == 0 && lane == 0) p.plan[i] = make_int2(0, 0);
         }
     }
@@ -117,7 +118,9 @@ attn_decode_fp8kv_kernel(const DecodeParams p) {
     chunk = split_chunk(len, p.num_splits, C::ALIGN);
     start = split * chunk;
     if (start >= len) {
-      if (NEW && p.new_k && len <= 0 && split == 0 && warp == 0) store_new_rows<T, D, true, E5M2>(p, b, kvh, lane);
+      if constexpr (NEW) {
+        if (len <= 0 && split == 0 && warp == 0) store_new_rows<T, D, true, E5M2>(p, b, kvh, lane);
+      }
       return;
     }
     end = min(len, start + chunk);
@@ -190,7 +193,7 @@ attn_decode_fp8kv_kernel(const DecodeParams p) {
   };
 
   load_slots(0, std::false_type{});
-  if (NEW && p.new_k) {
+  if constexpr (NEW) {
     if (p.new_all) {
       for (int i = warp; i < p.bs; i += NW) store_new_rows<T, D, true, E5M2>(p, i, kvh, lane);
       __syncthreads();

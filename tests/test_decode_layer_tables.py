@@ -113,7 +113,7 @@ def _twice(bs, n):
     ((14, 2, 64), torch.bfloat16, torch.float8_e5m2, None),
 ])
 @pytest.mark.parametrize("splits,pieces", [(1, 0), (6, 0), (1, 40)])
-@pytest.mark.parametrize("bs", [1, 2, 4, 5, 19])
+@pytest.mark.parametrize("bs", [1, 2, 3, 4, 19])
 @pytest.mark.parametrize("tables", [_positions, _forks, _twice])
 def test_same_bytes_as_a_write_before(tables, bs, splits, pieces, heads, act, pool, scales, monkeypatch):
     for n in (49, 900):
@@ -123,4 +123,4 @@ def test_same_bytes_as_a_write_before(tables, bs, splits, pieces, heads, act, po
             got = _decode(monkeypatch, False, *case, heads, act, pool, scales, splits, pieces)
             for a, b in zip(got[:3], ref[:3]):
                 assert torch.equal(a.view(torch.uint8), b.view(torch.uint8))
-        assert got[3] == ref[3] - (bs <= 4)
+        assert got[3] == ref[3] - (bs <= 2)
