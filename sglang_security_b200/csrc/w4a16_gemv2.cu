@@ -510,7 +510,9 @@ static bool gemv2_plan(int M, int N, int K, int group, Gemv2Plan* pl) {
   if (forced > 0) {
     S = forced > 8 ? 8 : forced;
   } else {
-    // at least two CTAs per SM, at least two slice units per rank (the last may have fewer)
+    // At least two CTAs per SM, at least two slice units per rank but the last, which may be left with none (20 units in 8
+    // ranks of 3): a cluster without that rank has an odd size, which is slower (5120 x 2560, 12 tokens of four linears of
+    // Qwen2.5-32B at TP 2, us: 8 ranks 69.8, 7 74.1).
     const int sms = device_sm_count();
     while (n_groups * S < 2 * sms && S < 8 &&
            (units >= 4 * S || (MT == 1 && ceil_div(units, 2 * S) == 2 && (2 * S - 1) * 2 < units)))
@@ -530,10 +532,10 @@ static bool gemv2_plan(int M, int N, int K, int group, Gemv2Plan* pl) {
   if (S > units) S = units;
   if (S < 1) S = 1;
   for (;; S = MT == 1 ? S + 1 : (S < 4 ? 2 * S : 8)) {   // 8: the largest cluster that every device takes
-    const int per = ceil_div(units, S), kb_per_rank = per * upg;
+    const int kb_per_rank = ceil_div(units, S) * upg;
     const int xs_stride = kb_per_rank * 128 + 64;  // +64: conflict-free LDS.128 across token rows
     const int ng = ceil_div(kb_per_rank * 64, group) + 1;
-    pl->S = ceil_div(units, per);   // no rank without a slice
+    pl->S = S;
     pl->kb_per_rank = kb_per_rank;
     pl->xs_stride = xs_stride;
     pl->sz_off = (M + (M < MT * 8)) * xs_stride;  // M token rows + the shared zero row
