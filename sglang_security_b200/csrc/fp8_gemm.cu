@@ -219,14 +219,17 @@ static int fp8_gemm_rowcol_impl(const void* a, int64_t lda, const void* b, int64
   ep.N = N;
   ep.K = K;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // Decode regime: weight streaming, swap-AB + cluster split-K, two CTAs per SM.  Against the CTA-pair kernel (four linears
-  // with quantisers, us, pair / this): Llama-3.1-8B 40 tokens 65.8 / 63.7, 48 67.3 / 65.3, 64 67.3 / 67.8; at TP 4 40 tokens
-  // 37.0 / 35.3, 48 37.0 / 37.0, 64 36.8 / 41.1; Qwen2.5-32B at TP 2 40 tokens 68.3 / 68.0, 48 68.8 / 67.8.
+  // Decode regime: weight streaming, swap-AB + cluster split-K, two CTAs per SM.  From 33 to 48 tokens only where K is cut
+  // into eight slices (few channels, long K; profiles/fp8_small_m_forms.json).  One linear with its quantiser, us, pair /
+  // this: in 8 slices 1536 x 4096 40 tokens 8.5 / 7.2, 48 8.5 / 7.4, 56 8.7 / 8.4; 4096 x 4096 10.6 / 9.9, 10.5 / 10.2, 10.6 /
+  // 11.0; fewer slices 4096 x 1024 6.3 / 7.3, 6.4 / 7.6, 6.4 / 8.7; 6144 x 4096 10.3 / 11.1, 10.3 / 11.3; 896 x 896 6.1 / 7.1,
+  // 6.1 / 7.6; 5120 x 13824 alone gains, 18.8 / 18.2, 18.7 / 18.5.
   const bool fuse_ar = comm_can_fuse(comm, M, N);
   // A weight with more 128-row tiles than SMs (gate_up 28672x4096) streams best here up to 64 tokens: 21.8 us at 64,
   // the pair kernel 23.5 at 128.
   const bool wide = ceil_div(N, 128) > device_sm_count();
-  if (fuse_ar || (M <= smallm_max_m() && (M <= 48 || (wide && M <= 64) || smallm_forced()))) {
+  const bool sliced = M <= 48 && smallm_pick_splits(ceil_div(N, 128), ceil_div(K, 128)) == 8;
+  if (fuse_ar || (M <= smallm_max_m() && (M <= 32 || sliced || (wide && M <= 64) || smallm_forced()))) {
     SmallMParams sp = {};
     if (fuse_ar) {
       sp.use_comm = 1;
