@@ -13,9 +13,17 @@ static WaitCounter wait_counter_registered(tc::wait_counter());
 
 // Decode sizes: the swap-AB kernel with K split over a cluster (fp8_gemm_smallm.cuh), two CTAs an SM, whose weight ring is
 // filled before the CTA is set up; a CTA pair of gemm_pair_kernel has to meet first, and ends with an exchange of 4-byte
-// loads.  Four linears, bf16, us, pair / this: Llama-3.1-8B 1 token 87.7 / 76.7, 16 89.2 / 82.3, 24 90.5 / 86.2; at TP 4 1
-// token 37.1 / 30.9, 24 39.1 / 37.9, 32 38.6 / 39.6; Qwen2.5-32B at TP 2 1 token 94.1 / 84.8.
-constexpr int kDenseSmallMax = 24;
+// loads.  Its sums meet token by token, so it pays with a long K: of 24 shapes timed on both (profiles/dense_small_m_forms.json)
+// from K 2048 up to 24 tokens (us, pair / this: 4096 x 4096 1 token 10.2 / 7.1, 24 10.2 / 9.4; 5120 x 2560 8.8 / 6.9), up to 12
+// where K is not split (128256 x 4096 1 token 154.8 / 153.1, 24 159.6 / 166.1); with a short K up to 4 tokens and 8192 channels
+// (4096 x 1024 1 token equal, 24 4.8 / 5.6; 9728 x 896 1 token 5.5 / 5.7, 24 5.8 / 7.7).
+// Four linears, bf16: Llama-3.1-8B 1 token 87.7 / 76.7, 16 89.2 / 82.3, 24 90.5 / 86.2; at TP 4 1 token 37.1 / 30.9;
+// Qwen2.5-32B at TP 2 1 token 94.1 / 84.8.
+static bool dense_small(int M, int N, int K) {
+  const int tiles = ceil_div(N, 128), num_kb = ceil_div(K, 64);
+  if (num_kb < 32) return M <= 4 && tiles <= 64;
+  return M <= (smallm_pick_splits(tiles, num_kb) == 1 ? 12 : 24);
+}
 template <int KIND, typename OutT>
 static int launch_dense_small(const void* x, int64_t ldx, const void* w, int64_t ldw, const GemmEpilogueParams& ep,
                               cudaStream_t st) {
@@ -62,7 +70,7 @@ static int gemm_16bit(const void* x, int64_t ldx, const void* w, int64_t ldw, co
   if (act)
     return dtype == B200_BF16 ? launch_gemm_pair<kKindBf16, __nv_bfloat16, true>(x, ldx, w, ldw, ep, st, "dense_gemm")
                               : launch_gemm_pair<kKindF16, __half, true>(x, ldx, w, ldw, ep, st, "dense_gemm");
-  if (M <= kDenseSmallMax)
+  if (dense_small(M, N, K))
     return dtype == B200_BF16 ? launch_dense_small<kKindBf16, __nv_bfloat16>(x, ldx, w, ldw, ep, st)
                               : launch_dense_small<kKindF16, __half>(x, ldx, w, ldw, ep, st);
   return dtype == B200_BF16 ? launch_gemm_pair<kKindBf16, __nv_bfloat16>(x, ldx, w, ldw, ep, st, "dense_gemm")

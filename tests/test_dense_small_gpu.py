@@ -25,7 +25,8 @@ def _check(out, ref, mags, k):
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("m", [1, 4, 5, 16, 17, 24, 25])
-@pytest.mark.parametrize("n,k", [(136, 64), (136, 72), (128, 1096), (264, 4096), (24000, 1032), (20000, 2048), (24, 8192)])
+@pytest.mark.parametrize("n,k", [(136, 64), (136, 72), (128, 1096), (264, 4096), (264, 4104), (24000, 1032), (20000, 2048),
+                                 (20000, 2056), (24, 8192)])
 def test_small(m, n, k, dtype):
     from sglang_security_b200 import _lib
     from sglang_security_b200.layers.dense_kernel import gemm_16bit
@@ -33,7 +34,9 @@ def test_small(m, n, k, dtype):
     x, w, bias, ref, mags = _problem(m, n, k, dtype)
     out = gemm_16bit(x, w, bias)
     v = _lib.last_variant()
-    assert v.startswith("gemm_tn kind=") and ("smallm" in v) == (m <= 24)
+    short = k < 2000
+    whole = n >= 148 * 128                  # a tile for every SM: K is not split
+    assert v.startswith("gemm_tn kind=") and ("smallm" in v) == (m <= (4 if short else 12 if whole else 24) and not (short and whole))
     _check(out, ref, mags, k)
     assert torch.equal(out, gemm_16bit(x, w, bias))
 
