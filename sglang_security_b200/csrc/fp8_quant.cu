@@ -162,6 +162,37 @@ fp8_quant_row_kernel(const T* __restrict__ x, int64_t ldx, uint8_t* __restrict__
 // a multiple of 2^-57 scale, which fp32 holds from a scale of 2^-92 on.  Smaller scales (a caller's eps; below 3e-39
 // their reciprocal is infinite) and infinite ones are divided by.  The compiler's division and one load in flight per lane bound the kernel.
 constexpr float kReciprocalMin = 0x1p-90f;
+// The general rules (NaN, infinities and tiny scales among them): a group's maximum from `amax` up, over LANES lanes that
+// hold N pairs each, and its elements divided by the scale and clamped.
+template <int LANES, int N>
+__device__ __forceinline__ float group_max(const float2 (&f)[N], float amax) {
+#pragma unroll
+  for (int e = 0; e < N; ++e) amax = fmaxf(amax, fmaxf(fabsf(f[e].x), fabsf(f[e].y)));
+#pragma unroll
+  for (int off = LANES / 2; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
+  return amax;
+}
+template <int N>
+__device__ __forceinline__ void group_scale(float2 (&f)[N], float s) {
+  if (s >= kReciprocalMin && s < INFINITY) {
+    const float r = 1.0f / s;
+#pragma unroll
+    for (int e = 0; e < N; ++e) {
+      const float qx = f[e].x * r, qy = f[e].y * r;
+      f[e].x = copysignf(fmaf(fmaf(-qx, s, f[e].x), r, qx), qx);   // -0 stays -0
+      f[e].y = copysignf(fmaf(fmaf(-qy, s, f[e].y), r, qy), qy);
+    }
+  } else {
+#pragma unroll
+    for (int e = 0; e < N; ++e) f[e] = make_float2(f[e].x / s, f[e].y / s);
+  }
+#pragma unroll
+  for (int e = 0; e < N; ++e) {
+    f[e].x = fminf(fmaxf(f[e].x, -kFp8Max), kFp8Max);
+    f[e].y = fminf(fmaxf(f[e].y, -kFp8Max), kFp8Max);
+  }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256)
 fp8_quant_group128_kernel(const T* __restrict__ x, int64_t ldx, uint8_t* __restrict__ q,
@@ -178,34 +209,12 @@ fp8_quant_group128_kernel(const T* __restrict__ x, int64_t ldx, uint8_t* __restr
   const uint4 raw = gid < total ? *reinterpret_cast<const uint4*>(x + m * ldx + g * 128 + lane * 8) : make_uint4(0, 0, 0, 0);
   const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
   float2 f[4];
-  float amax = eps;
 #pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    f[e] = unpack2<T>(w[e]);
-    amax = fmaxf(amax, fmaxf(fabsf(f[e].x), fabsf(f[e].y)));
-  }
-#pragma unroll
-  for (int off = 8; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
+  for (int e = 0; e < 4; ++e) f[e] = unpack2<T>(w[e]);
+  const float s = group_max<16>(f, eps) / kFp8Max;
   if (gid >= total) return;
-  const float s = amax / kFp8Max;
   if (lane == 0) scales[m * s_row + g * s_col] = s;
-  if (s >= kReciprocalMin && s < INFINITY) {
-    const float r = 1.0f / s;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float qx = f[e].x * r, qy = f[e].y * r;
-      f[e].x = copysignf(fmaf(fmaf(-qx, s, f[e].x), r, qx), qx);   // -0 stays -0
-      f[e].y = copysignf(fmaf(fmaf(-qy, s, f[e].y), r, qy), qy);
-    }
-  } else {
-#pragma unroll
-    for (int e = 0; e < 4; ++e) f[e] = make_float2(f[e].x / s, f[e].y / s);
-  }
-#pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    f[e].x = fminf(fmaxf(f[e].x, -kFp8Max), kFp8Max);
-    f[e].y = fminf(fmaxf(f[e].y, -kFp8Max), kFp8Max);
-  }
+  group_scale(f, s);
   *reinterpret_cast<uint2*>(q + m * ldq + g * 128 + lane * 8) = make_uint2(e4m3x4(f[0], f[1]), e4m3x4(f[2], f[3]));
 }
 
@@ -220,43 +229,21 @@ __device__ __forceinline__ float max_nan(float a, float b) {
   asm("max.NaN.f32 %0, %1, %2;\n" : "=f"(r) : "f"(a), "f"(b));
   return r;
 }
-// One group by the general rules (NaN, infinities, tiny scales: a true division, clamped), 8 lanes of a full warp.
+// One group by the general rules, 8 lanes of a full warp.
 template <typename T>
 __device__ __noinline__ void quant_group_general(const T* src, uint8_t* out, float* scale, bool store, bool lane0, float eps) {
   float2 f[8];
-  float amax = eps;
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     const uint4 raw = *reinterpret_cast<const uint4*>(src + h * 64);
     const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      f[h * 4 + e] = unpack2<T>(w[e]);
-      amax = fmaxf(amax, fmaxf(fabsf(f[h * 4 + e].x), fabsf(f[h * 4 + e].y)));
-    }
+    for (int e = 0; e < 4; ++e) f[h * 4 + e] = unpack2<T>(w[e]);
   }
-#pragma unroll
-  for (int off = 4; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
-  const float s = amax / kFp8Max;
-  if (s >= kReciprocalMin && s < INFINITY) {
-    const float r = 1.0f / s;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const float qx = f[e].x * r, qy = f[e].y * r;
-      f[e].x = copysignf(fmaf(fmaf(-qx, s, f[e].x), r, qx), qx);   // -0 stays -0
-      f[e].y = copysignf(fmaf(fmaf(-qy, s, f[e].y), r, qy), qy);
-    }
-  } else {
-#pragma unroll
-    for (int e = 0; e < 8; ++e) f[e] = make_float2(f[e].x / s, f[e].y / s);
-  }
+  const float s = group_max<8>(f, eps) / kFp8Max;
   if (!store) return;
   if (lane0) *scale = s;
-#pragma unroll
-  for (int e = 0; e < 8; ++e) {
-    f[e].x = fminf(fmaxf(f[e].x, -kFp8Max), kFp8Max);
-    f[e].y = fminf(fmaxf(f[e].y, -kFp8Max), kFp8Max);
-  }
+  group_scale(f, s);
   *reinterpret_cast<uint2*>(out) = make_uint2(e4m3x4(f[0], f[1]), e4m3x4(f[2], f[3]));
   *reinterpret_cast<uint2*>(out + 64) = make_uint2(e4m3x4(f[4], f[5]), e4m3x4(f[6], f[7]));
 }
