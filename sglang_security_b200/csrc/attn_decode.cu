@@ -92,7 +92,7 @@ __host__ __device__ inline int split_chunk(int len, int num_splits, int align) {
 // The dot products of a GQA group run on mma.sync m16n8k16 (rows = query heads of the group,
 // padded to 16), so the per-token instruction count does not scale with the group size and the
 // SM front end stays far below the HBM-bound gather stream (a CUDA-core FFMA version of this
-// kernel was issue-bound at 78 % of the HBM peak; profiles/r01_decode_tuning.md).
+// kernel was issue-bound at 78 % of the HBM peak).
 //
 //   S[16 heads, NT tokens] = Q[16, D] . K^T   (K rows from swizzled smem via ldmatrix)
 //   P = exp2(S*scale - m)  (fp32 registers; the accumulator layout of S is the A layout of P)
@@ -1012,7 +1012,7 @@ static int launch_merge_quant(const DecodeParams& p, int Dv, int align, cudaStre
 }
 
 // ---- host-side dispatch -----------------------------------------------------------------------
-// One instance family, tuned on the B200 for the HBM-bound regime (profiles/r01_decode_tuning.md):
+// One instance family, tuned on the B200 for the HBM-bound regime:
 // 16-token tiles, 2 stages, 3 warps -> 48 KiB per CTA at D=128, 4 CTAs (12 warps) per SM.  More
 // resident warps beat deeper per-warp rings; 12 warps x 8 KiB keeps ~100 KiB of gathers in flight.
 constexpr int kNT = 16, kStages = 2, kNW = 3;

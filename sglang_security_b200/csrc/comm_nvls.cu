@@ -126,7 +126,7 @@ static int64_t nvls_min_bytes() {
   static int64_t v = [] {
     const char* e = std::getenv("B200_COMM_NVLS_MIN");
     // 128 KiB: below that the LL protocol's single NVLink trip wins (TP 8: 9.4 vs 10.7 us at 64 KiB,
-    // 14.9 vs 12.9 us at 256 KiB; profiles/r02_bench_allreduce_tp8.json)
+    // 14.9 vs 12.9 us at 256 KiB)
     return (e && *e) ? std::atoll(e) : static_cast<int64_t>(128 << 10);
   }();
   return v;

@@ -77,7 +77,7 @@ extern std::atomic<int> g_pdl_on;  // bit mask over PdlFamily (all bits = every 
 enum PdlFamily { kPdlGemmSmall = 1, kPdlGemmBig = 2, kPdlAttn = 4, kPdlMerge = 8, kPdlRow = 16,
                  kPdlRope = 32, kPdlQuant = 64, kPdlOther = 128 };
 
-// Measured on the Llama-3.1-8B FP8 decode step (profiles/r01_pdl_sweep.md): overlapping launches
+// Measured on the Llama-3.1-8B FP8 decode step: overlapping launches
 // pays while the step is latency-bound (-7..-10 % at batch <= 32) and costs 3-6 % at batch 64+, where
 // early-resident dependents only take SM resources from a bandwidth-bound predecessor.  Call sites
 // therefore pass pdl_family(tokens, family): the family bit for small token counts, 0 otherwise.

@@ -528,7 +528,7 @@ int b200_rmsnorm(const void* x, int64_t ldx, void* residual, int64_t ldr, const 
     // Optional cluster split of a row (B200_RMSNORM_TARGET_CTAS = CTA count to aim for).  Off by default:
     // unlike SiLU*mul (56 exp + divide per thread on a 14336-wide row) a 4096-wide norm row is a short
     // chain of dependent latencies that the extra cluster barriers only lengthen — measured 10.65 vs
-    // 9.74 us per launch, whole step 8.238 vs 8.232 ms at 64 tokens (profiles/r02_bench_rmsnorm_split.json).
+    // 9.74 us per launch, whole step 8.238 vs 8.232 ms at 64 tokens.
     static const int target = [] {
       const char* e = std::getenv("B200_RMSNORM_TARGET_CTAS");
       return (e && *e) ? std::atoi(e) : 0;
@@ -578,7 +578,7 @@ int b200_silu_and_mul(const void* x, int64_t ldx, void* out, int64_t ldo, void* 
     // cluster size: spread few rows over more SMs while every CTA keeps >= 256 vectors
     const int nvec = d / 8;
     // (one CTA per row leaves a 14336-wide row — 56 exp + divide per thread — to 8 warps of one SM:
-    // 11.7 us at M = 64 in the whole-model launch list, profiles/r02_ncu_launches.json), so rows are
+    // 11.7 us at M = 64 in the whole-model launch list), so rows are
     // split until about two CTAs per SM exist; B200_SILU_TARGET_CTAS overrides the target
     static const int target = [] {
       const char* e = std::getenv("B200_SILU_TARGET_CTAS");

@@ -140,9 +140,9 @@ int smallm_pick_splits(int n_tiles, int num_kb) {
 
 // Row-parallel fusion: the small-M kernel can reduce across the TP group in its epilogue when the
 // dense [M, N] partial fits one receive slot and the grid fits the flag table.
-// Policy measured on B200: at TP = 2 (profiles/r01_bench_allreduce_tp2.json) fusing wins while the
+// Policy measured on B200: at TP = 2 fusing wins while the
 // swap-AB kernel itself is the right GEMM (M <= 32: 7.7 vs 8.2 us at M = 1, 13.1 vs 15.4 us at
-// M = 32, against GEMM + stand-alone LL all-reduce).  At TP = 8 (profiles/r01_bench_allreduce_tp8.json)
+// M = 32, against GEMM + stand-alone LL all-reduce).  At TP = 8
 // every tile pushes to 7 peers and the fused epilogue only wins at the smallest batches (o_proj:
 // 8.4 vs 10.8 us at M = 1 but 16.1 vs 12.7 at M = 8 and 51.6 vs 20.2 at M = 32), so the limit
 // shrinks with the group: 32 / 8 / 4 tokens at world 2 / 4 / 8 (world 4 interpolated).

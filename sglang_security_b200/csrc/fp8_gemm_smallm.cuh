@@ -59,14 +59,14 @@ __device__ __forceinline__ void named_bar_sync(int id, int threads) {
 template <int MT, bool BLK, int KSUB = 1>
 struct SmallMCfg {
   // A ring slot ("block") spans KS sub-blocks of 128 K: every barrier hand-off of the pipeline costs
-  // a fixed ~0.3 us round trip per role (profiles/r01_w4a16_notes.md), so the decode instances
+  // a fixed ~0.3 us round trip per role, so the decode instances
   // can move 32 KiB of weights per hand-off (KSUB = 2): measured +5-8 % on the wide weights
   // (gate_up M = 1: 20.7 -> 19.6 us = 6.0 TB/s, 92 % of the HBM peak; down 11.1 us) but -7 % on
   // qkv / o, whose short K slices then hold too few blocks, so the launcher picks it by weight size.
   // The block-scaled variant needs one TMEM buffer per 128 K and keeps KS = 1.
   // MT = 16 only: the MT = 32 instance with 32 KiB ring blocks sits at the two-CTAs-per-SM shared
   // memory limit and fell to one CTA per SM once the epilogue's scale staging was added (gate_up
-  // M = 32: 21.5 -> 26.8 us, down 13.3 -> 25.7 us, profiles/r02_bench_gemm_midm.json)
+  // M = 32: 21.5 -> 26.8 us, down 13.3 -> 25.7 us)
   static constexpr int KS = (!BLK && MT <= 16) ? KSUB : 1;
   static constexpr int W_SUB = 128 * 128, X_SUB = MT * 128;
   static constexpr int W_BYTES = KS * W_SUB;
@@ -80,7 +80,7 @@ struct SmallMCfg {
   static constexpr int BUDGET = (BLK && MT == 128) ? 208 * 1024 : (MT == 64 ? 108 * 1024 : 112 * 1024);
   // MT = 64: three activation slots like the smaller instances.  With two, the x tile of block i is only requested when the
   // MMA of block i - 2 retires, so every other K block exposed an L2 round trip (measured: the same
-  // 25 MB weight took 9.4 us at MT = 32 and 14-16 us at MT = 64, profiles/r02_bench_gemm_midm_mt64.json)
+  // 25 MB weight took 9.4 us at MT = 32 and 14-16 us at MT = 64)
   static constexpr int NX = (MT <= 32 && KS == 1) ? 3 : (MT == 64 ? 3 : 2);
   static constexpr int NW = (BUDGET - NX * X_BYTES) / W_BYTES;
   static constexpr int NBUF = BLK ? (MT <= 64 ? 4 : 2) : 1;

@@ -28,7 +28,7 @@ static const char* pdl_limit() {
 int pdl_max_tokens() {
   static int v = [] {
     const char* e = pdl_limit();
-    // 512: measured on the whole-model decode step (profiles/r02_bench_pdl.json): batch
+    // 512: measured on the whole-model decode step: batch
     // 64 x 4k 8.11 ms with PDL against 8.25 ms without; batch 128 / 256 @ 1k 5.99 / 9.62 ms against
     // 6.20 / 9.84 ms with a limit of 64 tokens
     return e ? std::atoi(e) : 512;

@@ -1,7 +1,7 @@
 // Greedy sampling step of the decode loop: row-wise argmax of the logits (first index of the maximum,
 // torch.argmax semantics).  The reference does this with torch.argmax in Sampler.forward
 // (python/sglang/srt/layers/sampler.py:60-66); torch's reduce kernel puts ONE CTA on a 128k-entry row
-// (46 us per decode step in the whole-model launch list, profiles/r01_ncu_decode_model_bs1_launches.json).
+// (46 us per decode step in the whole-model launch list).
 // Here a row is spread over a cluster of 8 CTAs (16-byte loads), the per-CTA candidates are combined
 // through distributed shared memory by rank 0.
 #include "common.cuh"

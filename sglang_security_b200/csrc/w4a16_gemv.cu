@@ -330,8 +330,8 @@ static std::atomic<int> g_gemv_max_m{-1};
 static std::atomic<int> g_gemv_splits{-1};
 
 // Largest M the dispatch in b200_w4a16_gemm hands to the GEMV for an N-column weight.  Explicit
-// settings (b200_w4a16_gemv_config / B200_W4A16_GEMV_MAX_M) win.  Default, from the cfg-4 sweep
-// (profiles/r01_bench_w4a16_crossover.json): the swap-AB split-K tcgen05 kernel is as fast or faster
+// settings (b200_w4a16_gemv_config / B200_W4A16_GEMV_MAX_M) win.  Default, from a sweep of int4 shapes:
+// the swap-AB split-K tcgen05 kernel is as fast or faster
 // from M = 1 on every shape whose tiles can be split over a cluster (N / 128 <= 64); the GEMV keeps
 // M <= 2 on the wide gate_up weights, which fill the machine without split-K.
 int w4a16_gemv_max_m(int N) {

@@ -6,8 +6,8 @@
 // awq_kernel.cu:126-219) and vllm's gptq_gemm (quantization/gptq.py:17-31).
 //
 // Why a second kernel: w4a16_gemv.cu stages [K, N/8] rows through a shared-memory ring with a CTA
-// barrier per 64 k rows and regroups nibbles with PRMT; it measured 9-23 % of the HBM peak
-// (profiles/r01_bench_w4a16_crossover.json) — latency-bound on 12 warps per SM.  Here:
+// barrier per 64 k rows and regroups nibbles with PRMT; it measured 9-23 % of the HBM peak,
+// latency-bound on 12 warps per SM.  Here:
 //   * one-time repack (process_weights_after_loading) into a STREAM layout: tiles of 16 output
 //     columns x 64 k, 512 contiguous bytes, ordered [n / 16][k / 64]; lane l = 4 g + t owns one
 //     uint4 = { W(g,0), W(g+8,0), W(g,1), W(g+8,1) } where W(c, s) packs the 8 weights of column

@@ -62,7 +62,7 @@ class B200AllReduce:
                                         ctypes.byref(h)), "b200_comm_create")
         self.handle = h
         self.max_size = int(lib.b200_comm_max_bytes(h))
-        # measured crossover with NCCL (NVLS) on 8 x B200 (profiles/r01_bench_allreduce_tp8.json): the
+        # measured crossover with NCCL (NVLS) on 8 x B200: the
         # one-shot kernel is 24 vs 36 us at 1 MiB, equal at 2 MiB, 70 vs 61 us at 4 MiB; at TP = 2 it
         # stays ahead up to the 4 MiB buffer limit
         self.crossover = self.max_size if self.world_size <= 4 else min(self.max_size, 2 << 20)
@@ -72,7 +72,7 @@ class B200AllReduce:
         # the driver or the container does not offer multicast objects
         self.nvls = False
         self._nvls_buf = None
-        # Default: on for groups of 8 (measured on 8 x B200, profiles/r02_bench_allreduce_tp8.json:
+        # Default: on for groups of 8 (measured on 8 x B200:
         # 15.9 vs 24.3 us at 512 KiB, whole-model TP 8 decode 3.86 vs 4.67 ms per step), off below
         # (TP 2: the LL kernel is 2x faster).  B200_COMM_NVLS=1 / 0 forces it on / off.
         want = os.environ.get("B200_COMM_NVLS", "")

@@ -99,7 +99,7 @@ class B200AttnBackend(AttentionBackend):
         # structure).  True = ONE merge+quantise launch after the split kernel (a cluster of CTAs per
         # request).  The in-kernel variant (ticket counters inside the split kernel, batch <=
         # tail_in_kernel_max_bs) measured slower than both at every batch on B200
-        # (profiles/r02_decode_tail_modes.json) and is therefore off by default.
+        # and is therefore off by default.
         self.fused_tail = os.environ.get("B200_ATTN_FUSED_TAIL", "1") != "0"
         self.tail_in_kernel_max_bs = int(os.environ.get("B200_ATTN_TAIL_IN_KERNEL_MAX_BS", "0"))
         self._tickets = torch.zeros(256 * (1 + self.num_head), dtype=torch.int32, device=self.device)

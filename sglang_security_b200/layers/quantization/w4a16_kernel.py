@@ -240,7 +240,7 @@ def w4a16_gemv_v2_config(splits: int = 0) -> None:
 
 
 # largest token count handed to the stream GEMV (its two-tile instance for 9..16 tokens is at par or
-# ahead of the tcgen05 swap-AB kernel on every cfg-4 shape, profiles/r02_bench_w4a16_gemv2.json)
+# ahead of the tcgen05 swap-AB kernel on every shape of Qwen2.5-32B at TP 2)
 GEMV_V2_MAX_M = int(os.environ.get("B200_W4A16_GEMV2_MAX_M", "16"))
 
 
