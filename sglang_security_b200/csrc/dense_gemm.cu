@@ -13,16 +13,16 @@ static WaitCounter wait_counter_registered(tc::wait_counter());
 
 // Decode sizes: the swap-AB kernel with K split over a cluster (fp8_gemm_smallm.cuh), two CTAs an SM, whose weight ring is
 // filled before the CTA is set up; a CTA pair of gemm_pair_kernel has to meet first, and ends with an exchange of 4-byte
-// loads.  Its sums meet token by token, so it pays with a long K: of 24 shapes timed on both (profiles/dense_small_m_forms.json)
-// from K 2048 up to 24 tokens (us, pair / this: 4096 x 4096 1 token 10.2 / 7.1, 24 10.2 / 9.4; 5120 x 2560 8.8 / 6.9), up to 12
-// where K is not split (128256 x 4096 1 token 154.8 / 153.1, 24 159.6 / 166.1); with a short K up to 4 tokens and 8192 channels
-// (4096 x 1024 1 token equal, 24 4.8 / 5.6; 9728 x 896 1 token 5.5 / 5.7, 24 5.8 / 7.7).
-// Four linears, bf16: Llama-3.1-8B 1 token 87.7 / 76.7, 16 89.2 / 82.3, 24 90.5 / 86.2; at TP 4 1 token 37.1 / 30.9;
-// Qwen2.5-32B at TP 2 1 token 94.1 / 84.8.
+// loads.  Its sums meet token by token, so it pays with a long K: of 24 shapes timed on both, one call after the other
+// (profiles/dense_small_m_forms.json), from K 2048 up to 24 tokens (us, pair / this: 4096 x 4096 1 token 10.2 / 7.1, 24 10.2 /
+// 9.4; 5120 x 2560 8.8 / 6.9 and equal); with a short K up to 4 tokens and 8192 channels (4096 x 1024 1 token equal, 24 4.8 /
+// 5.6; 9728 x 896 1 token 5.5 / 5.7, 24 5.8 / 7.7; 151936 x 896 24 tokens 43.1 / 54.9).  Where K is not split the two are even
+// call after call, or pairs up to 4 % ahead from 16 tokens on, but not between other linears, whose kernel it shares (four
+// linears of Llama-3.1-8B, 16 tokens, all here 79.1, gate_up in pairs 85.9; a whole step with the head here / in pairs, 20
+// tokens, 399 / 402).  Four linears, bf16: Llama-3.1-8B 1 token 83.9 / 73.7, 16 86.1 / 79.2, 24 86.6 / 81.9; at TP 4 34.5 /
+// 28.9, 36.1 / 30.4, 36.6 / 33.2; Qwen2.5-32B at TP 2 90.0 / 81.8, 91.5 / 85.2, 92.0 / 88.5.
 static bool dense_small(int M, int N, int K) {
-  const int tiles = ceil_div(N, 128), num_kb = ceil_div(K, 64);
-  if (num_kb < 32) return M <= 4 && tiles <= 64;
-  return M <= (smallm_pick_splits(tiles, num_kb) == 1 ? 12 : 24);
+  return ceil_div(K, 64) >= 32 ? M <= 24 : M <= 4 && ceil_div(N, 128) <= 64;
 }
 template <int KIND, typename OutT>
 static int launch_dense_small(const void* x, int64_t ldx, const void* w, int64_t ldw, const GemmEpilogueParams& ep,

@@ -34,9 +34,7 @@ def test_small(m, n, k, dtype):
     x, w, bias, ref, mags = _problem(m, n, k, dtype)
     out = gemm_16bit(x, w, bias)
     v = _lib.last_variant()
-    short = k < 2000
-    whole = n >= 148 * 128                  # a tile for every SM: K is not split
-    assert v.startswith("gemm_tn kind=") and ("smallm" in v) == (m <= (4 if short else 12 if whole else 24) and not (short and whole))
+    assert v.startswith("gemm_tn kind=") and ("smallm" in v) == (m <= 24 if k > 1984 else m <= 4 and n <= 8192)
     _check(out, ref, mags, k)
     assert torch.equal(out, gemm_16bit(x, w, bias))
 
