@@ -124,3 +124,43 @@ def test_same_bytes_as_a_write_before(tables, bs, splits, pieces, heads, act, po
             for a, b in zip(got[:3], ref[:3]):
                 assert torch.equal(a.view(torch.uint8), b.view(torch.uint8))
         assert got[3] == ref[3] - (bs <= 2)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("own", [False, True])
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("bs", [1, 2, 5, 40])
+def test_pools_with_gaps_between_the_rows(bs, fp8, own):
+    """A pool whose rows are wider than the heads, which the KV write launch does not take: the same output and rows as from a
+    pool without gaps, and the gaps keep their bytes."""
+    lib, hq, hkv, d, pad = _lib.load(), 8, 2, 64, 32
+    g = torch.Generator(device=DEV).manual_seed(bs)
+    lens = [1 + 37 * b % 200 for b in range(bs)]
+    width = max(lens) + 3
+    table = (torch.randperm(bs * width, device=DEV, generator=g) + 1).view(bs, width).to(torch.int32)
+    seq = torch.tensor(lens, device=DEV)
+    loc = table[torch.arange(bs, device=DEV), seq - 1].long()
+    req = torch.arange(bs, device=DEV)
+    act = torch.bfloat16
+    q, k, v = (torch.randn(bs, n * d, device=DEV, generator=g).to(act) for n in (hq, hkv, hkv))
+    pools = torch.randn(2, bs * width + 1, hkv * d, device=DEV, generator=g)
+    pools = pools.to(torch.float8_e4m3fn).view(torch.uint8) if fp8 else pools.to(act)
+    splits, out = 3, []
+    ws = torch.empty(lib.b200_attn_decode_workspace_bytes(bs, hq, d, splits), dtype=torch.uint8, device=DEV)
+    for gap in (0, pad):
+        kv = torch.full((2, bs * width + 1, hkv * d + gap), 9, device=DEV, dtype=pools.dtype)
+        kv[..., :hkv * d] = pools
+        o = torch.empty(bs, hq * d, device=DEV, dtype=act)
+        head = (k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0), loc.data_ptr()) + ((0,) if fp8 else ())
+        mid = (q.data_ptr(), q.stride(0), kv[0].data_ptr(), kv[1].data_ptr(), kv.stride(1), o.data_ptr(), o.stride(0),
+               table.data_ptr(), table.stride(0), req.data_ptr(), seq.data_ptr(), bs, hq, hkv, d, d, d ** -0.5, 0.0)
+        mid += ((1.0, 1.0) if fp8 else ()) + (_lib.dtype_code(act) | (_lib.OWN_SLOTS if own else 0),)
+        fn = lib.b200_attn_decode_fp8kv_layer if fp8 else lib.b200_attn_decode_layer
+        rc = fn(*head, *mid, ws.data_ptr(), ws.numel(), splits, 0, None, 0, None, 0, None, _lib.current_stream())
+        _lib.check(rc, "decode")
+        assert bool((kv[..., hkv * d:] == 9).all())
+        out.append((o, kv[..., :hkv * d].clone()))
+    for a, b in zip(*out):
+        assert torch.equal(a.contiguous().view(torch.uint8), b.contiguous().view(torch.uint8))
+    want = v.to(torch.float8_e4m3fn).view(torch.uint8) if fp8 else v
+    assert torch.equal(out[0][1][1][loc], want)
