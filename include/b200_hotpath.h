@@ -179,7 +179,7 @@ size_t b200_attn_decode_pieces_workspace_bytes(int bs, int Hq, int Dv, int piece
  * Limit: b200_attn_decode_workspace_bytes(bs, Hq, Dv, num_splits) must not exceed
  * B200_ATTN_DECODE_NOALLOC_SCRATCH_BYTES (8 MiB: e.g. 64 requests x 32 heads x 7 splits at Dv 128);
  * larger requests are rejected with an error (status 1, b200_last_error()), nothing is launched.
- * The device that owns `stream` must be current.  Every call on a device pieces the scratch and
+ * The device that owns `stream` must be current.  Every call on a device shares the scratch and
  * finds the previous call's contents in it (none of it has to be zero); calls that overlap on the
  * GPU (different streams, concurrent graph launches) race on it - serialise them on one stream.  */
 #define B200_ATTN_DECODE_NOALLOC_SCRATCH_BYTES (8u << 20)

@@ -83,9 +83,10 @@ enum PdlFamily { kPdlGemmSmall = 1, kPdlGemmBig = 2, kPdlAttn = 4, kPdlMerge = 8
 // therefore pass pdl_family(tokens, family): the family bit for small token counts, 0 otherwise.
 int pdl_max_tokens();
 inline int pdl_family(int tokens, int family) { return tokens <= pdl_max_tokens() ? family : 0; }
-// The CTA-pair GEMM's launch: dependent at every token count unless B200_PDL_MAX_M sets a limit.  Its barriers, tensor
-// memory and descriptors are ready when its predecessor ends (the four linears of a Llama-3.1-8B layer, bf16, 777
-// tokens: 321 us without, 303 with).  What it reads before its dependency wait keeps to pdl_max_tokens().
+// Kernels that are dependent launches at every token count unless B200_PDL_MAX_M sets a limit: the CTA-pair GEMM, the
+// block-scaled GEMMs, the KV writes and all extend kernels.  Their barriers, tensor memory and descriptors are ready when
+// their predecessor ends (the four linears of a Llama-3.1-8B layer, bf16, 777 tokens: 321 us without, 303 with; 46 extends
+// 1.025 x, profiles/extend_dependent_launches.json).  What they read before their dependency wait keeps to pdl_max_tokens().
 int pdl_gemm_family(int tokens, int family);
 
 template <typename... KArgs, typename... Args>
