@@ -223,7 +223,8 @@ fp8_quant_group128_kernel(const T* __restrict__ x, int64_t ldx, uint8_t* __restr
 // (nearly all) need no clamp, since the conversion saturates; the general rules are a function of their own, so that six
 // or eight blocks fit an SM.  Issue slots and, with fewer blocks, bytes in flight bounded the kernel above: 3001 x 14336
 // bf16 32.7 -> 22.0 us (19.7 of HBM time), 2048 x 4096 9.5 -> 7.0, 512 x 4096 3.2 -> 2.4.  Two groups a lane from 65536 on
-// (3001 x 14336 one / two / four 23.9 / 22.0 / 29.6; 1024 x 4096 4.4 / 5.0).
+// (3001 x 14336 one / two / four 23.9 / 22.0 / 29.6; 1024 x 4096 4.4 / 5.0).  Of 154 sizes of 100 to 3001 rows 1.2 x on
+// average; slower at 19000 to 22400 groups alone, where its 600 to 700 blocks are an uneven few an SM (300 x 8192 2.85 / 3.13).
 __device__ __forceinline__ float max_nan(float a, float b) {
   float r;
   asm("max.NaN.f32 %0, %1, %2;\n" : "=f"(r) : "f"(a), "f"(b));

@@ -145,6 +145,8 @@ __device__ __forceinline__ uint32_t g2_hmul2(uint32_t a, uint32_t b) {
 // (checks on every tile, all the way: 47 -> 61 us), and a round of four leaves, with groups of 128, nothing or two tiles
 // that need none.  Four linears, us, six and a tail of up to two rounds with checks / this: Qwen2.5-32B at TP 2, f16, 1
 // token 47.2 / 41.2, 8 49.9 / 45.2, 16 73.4 / 71.5; Llama-3.1-8B 45.4 / 41.1, 49.0 / 44.4, 69.8 / 66.8.  Two: 49.9.
+// Over 16 shapes call after call 1.05 x (groups of 128, 9 to 16 tokens) to 1.13 x (1 to 8); groups of 32, 64, 256 1.01 to 1.09 x,
+// with some shapes slower (64, 9 tokens, 28672 x 4096 31.7 / 33.8; 256, 4 tokens, 3584 x 5120 7.6 / 8.3).
 //  SPG = 32-k steps per quantisation group
 // known at compile time (1, 2, 4 = groups of 32, 64, 128: the fold sits at fixed places of the
 // unrolled round, no counters) or 0 = any other group size (run-time step counter).
